@@ -148,10 +148,13 @@ def _close(moes):
 class _Layer:
     """The ranks' dispatchers of one expert-parallel layer."""
 
-    def __init__(self, case):
-        self.ranks = [MoeDispatcher(c, case["tokens"], case["hidden"], case["topk"], case["experts"], _capacity(case))
-                      for c in _world()]
+    def __init__(self, tokens, hidden, topk, experts, capacity):
+        self.ranks = [MoeDispatcher(c, tokens, hidden, topk, experts, capacity) for c in _world()]
         weakref.finalize(self, _close, self.ranks)
+
+
+# A program creates a layer once and keeps it; a pass uses it from dispatch to combine.
+_layer = functools.lru_cache(maxsize=2)(_Layer)
 
 
 def prepare(case, seed):
@@ -169,7 +172,7 @@ def prepare(case, seed):
         _world()
         s["out"] = [torch.empty_like(t) for t in s["x"]]
     elif kind == "moe":
-        s["layer"] = _Layer(case)
+        s["layer"] = _layer(case["tokens"], case["hidden"], case["topk"], case["experts"], _capacity(case))
         s["out"] = [torch.empty_like(t) for t in s["x"]]
     elif kind == "block":
         s["fn"] = build_units(LlamaConfig.llama3_8b())[1].fn
