@@ -1,0 +1,213 @@
+// split_gemm.cu -- the plain tcgen05 GEMM D[M,N] = A[M,K] * B[N,K]^T for outputs that have
+// too few 256-wide tiles to occupy the chip (few rows: decoding, short prompts).
+//
+// The persistent kernel of tp_gemm.cu gives a whole K to one CTA (pair) per tile: 128 x 3584
+// x 8192 is 14 tiles, so 14 of 148 SMs stream the 59 MB of weights.  Here a cluster of S
+// CTAs owns a tile and each takes 1/S of K, so tiles x S SMs stream at once; tiles are 128 x
+// BN with BN = 256, 128 or 64.  Each CTA accumulates its part in TMEM, leaves it as fp32 in
+// its own shared memory (the operand ring is free by then), and after one cluster barrier
+// every CTA adds up 1/S of the tile's rows out of the S shared memories (distributed shared
+// memory, fixed order 0..S-1: the result does not depend on timing) and stores it as bf16.
+// The partial sums never leave the chip, no workspace is needed, and no CTA waits for
+// another except at that barrier, which the hardware's cluster scheduling makes safe.
+#include <cuda_bf16.h>
+
+#include <atomic>
+
+#include "split_gemm.h"
+#include "tcgen05.cuh"
+
+namespace fcx {
+namespace {
+
+using bf16 = __nv_bfloat16;
+using namespace tc;
+
+constexpr int BM = 128, BK = 64, kThreads = 256;
+constexpr unsigned long long kWaitLimitNs = 4000000000ull; // 4 s
+
+template <int BN>
+struct __align__(1024) Smem {
+  static constexpr int STAGES = 192 * 1024 / ((BM + BN) * BK * 2); // 4, 6, 8
+  bf16 a[STAGES][BM * BK];
+  bf16 b[STAGES][BN * BK];
+  uint64_t full[STAGES], empty[STAGES], done;
+  uint32_t tmemBase;
+  int abortFlag, bad;
+};
+
+__device__ __forceinline__ float4 ldCluster16(uint32_t addr) {
+  float4 v;
+  asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];"
+               : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w)
+               : "r"(addr)
+               : "memory");
+  return v;
+}
+__device__ __forceinline__ int ldClusterInt(uint32_t addr) {
+  int v;
+  asm volatile("ld.shared::cluster.s32 %0, [%1];" : "=r"(v) : "r"(addr) : "memory");
+  return v;
+}
+
+template <int BN>
+__global__ void __launch_bounds__(kThreads, 1)
+    splitGemmKernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
+                    bf16 *__restrict__ D, int N, int kBlocks, int tilesM, int S) {
+  extern __shared__ uint8_t rawSmem[];
+  using SmemT = Smem<BN>;
+  constexpr int STAGES = SmemT::STAGES;
+  constexpr uint32_t kStageBytes = (BM + BN) * BK * 2;
+  constexpr int kChunks = BN / 4; // 16-byte chunks of an fp32 tile row
+  static_assert(BM * BN * 4 <= (int)(STAGES * kStageBytes), "the fp32 tile reuses the operand ring");
+  SmemT &s = *reinterpret_cast<SmemT *>((reinterpret_cast<uintptr_t>(rawSmem) + 1023) & ~(uintptr_t)1023);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int part = (int)clusterCtaRank(), tile = blockIdx.x / S;
+  const int tm = tile % tilesM, tn = tile / tilesM; // neighbours share the rows of B
+  const int kb0 = (int)((long)kBlocks * part / S), kb1 = (int)((long)kBlocks * (part + 1) / S);
+
+  if (threadIdx.x == 0) {
+    prefetchTensorMap(&tmA);
+    prefetchTensorMap(&tmB);
+    for (int i = 0; i < STAGES; ++i) { mbarInit(&s.full[i], 1); mbarInit(&s.empty[i], 1); }
+    mbarInit(&s.done, 1);
+    s.abortFlag = 0;
+    s.bad = 0;
+    mbarInitFence();
+  }
+  if (warp == 1) { tmemAlloc(&s.tmemBase, BN); tmemRelinquish(); }
+  fenceBeforeSync();
+  __syncthreads();
+  fenceAfterSync();
+  const uint32_t tmemBase = s.tmemBase;
+  volatile int *abortFlag = &s.abortFlag;
+
+  if (warp == 0) {
+    if (lane == 0) { // TMA producer
+      int stage = 0, issued = 0;
+      uint32_t phase = 0;
+      for (int kb = kb0; kb < kb1; ++kb) {
+        if (!mbarWait(&s.empty[stage], phase ^ 1, abortFlag, kWaitLimitNs)) break;
+        mbarExpectTx(&s.full[stage], kStageBytes);
+        tmaLoad2d(s.a[stage], &tmA, kb * BK, tm * BM, &s.full[stage]);
+        tmaLoad2d(s.b[stage], &tmB, kb * BK, tn * BN, &s.full[stage]);
+        ++issued;
+        if (++stage == STAGES) { stage = 0; phase ^= 1; }
+      }
+      if (*abortFlag) { // given up: copies that are still under way land before the CTA goes on
+        int never = 0;
+        for (int j = issued > STAGES ? issued - STAGES : 0; j < issued; ++j)
+          mbarWait(&s.full[j % STAGES], (uint32_t)(j / STAGES) & 1u, &never, kWaitLimitNs);
+      }
+    }
+    __syncwarp();
+  } else if (warp == 1) {
+    if (lane == 0) { // MMA issuer
+      constexpr uint32_t idesc = instrDescBf16(BM, BN);
+      int stage = 0;
+      uint32_t phase = 0;
+      bool ok = true;
+      for (int kb = kb0; kb < kb1; ++kb) {
+        if (!mbarWait(&s.full[stage], phase, abortFlag, kWaitLimitNs)) { ok = false; break; }
+        fenceAfterSync();
+        const uint64_t da = smemDescSw128(s.a[stage]), db = smemDescSw128(s.b[stage]);
+#pragma unroll
+        for (int k4 = 0; k4 < BK / 16; ++k4) mmaBf16(tmemBase, da + 2 * k4, db + 2 * k4, idesc, (kb > kb0) || k4 != 0);
+        mmaCommit(&s.empty[stage]);
+        if (++stage == STAGES) { stage = 0; phase ^= 1; }
+      }
+      if (ok) mmaCommit(&s.done);
+    }
+    __syncwarp();
+  }
+  // every MMA has finished (and with them every load and every read of the ring)
+  const bool ok = mbarWait(&s.done, 0, abortFlag, kWaitLimitNs);
+  fenceAfterSync();
+  float4 *tileBuf = reinterpret_cast<float4 *>(s.a);
+  if (__syncthreads_and(ok ? 1 : 0)) {
+    // warp w reads TMEM lanes 32 (w % 4) .. and half of the columns; a row's chunks are
+    // swizzled by its number, so that the eight lanes of a phase hit different banks
+    const int row = (warp & 3) * 32 + lane;
+#pragma unroll 1
+    for (int c = (warp >> 2) * (BN / 2); c < ((warp >> 2) + 1) * (BN / 2); c += 32) {
+      uint32_t r[32];
+      tmemLoad32(tmemBase + ((uint32_t)((warp & 3) * 32) << 16) + c, r);
+      tmemLoadWait();
+#pragma unroll
+      for (int i = 0; i < 8; ++i)
+        tileBuf[row * kChunks + ((c / 4 + i) ^ (row & 7))] =
+            make_float4(__uint_as_float(r[4 * i]), __uint_as_float(r[4 * i + 1]), __uint_as_float(r[4 * i + 2]),
+                        __uint_as_float(r[4 * i + 3]));
+    }
+  } else if (threadIdx.x == 0) {
+    s.bad = 1; // the whole tile becomes NaN, in every CTA of the cluster
+  }
+  fenceBeforeSync();
+  __syncwarp();
+  clusterSync();
+  const uint32_t base = smemAddr(tileBuf), badAddr = smemAddr(&s.bad);
+  bool bad = false;
+  for (int p = 0; p < S; ++p) bad |= ldClusterInt(mapToCta(badAddr, p)) != 0;
+  const int r0 = BM * part / S, r1 = BM * (part + 1) / S;
+  for (int i = threadIdx.x; i < (r1 - r0) * kChunks; i += kThreads) {
+    const int row = r0 + i / kChunks, ch = i % kChunks;
+    const uint32_t off = base + (uint32_t)(row * kChunks + (ch ^ (row & 7))) * 16u;
+    float4 v[kSplitGemmMaxParts];
+#pragma unroll
+    for (int p = 0; p < kSplitGemmMaxParts; ++p)
+      if (p < S) v[p] = ldCluster16(mapToCta(off, p));
+    float4 t = v[0];
+#pragma unroll
+    for (int p = 1; p < kSplitGemmMaxParts; ++p)
+      if (p < S) { t.x += v[p].x; t.y += v[p].y; t.z += v[p].z; t.w += v[p].w; }
+    if (bad) t = make_float4(NAN, NAN, NAN, NAN);
+    __align__(8) __nv_bfloat162 o[2] = {__floats2bfloat162_rn(t.x, t.y), __floats2bfloat162_rn(t.z, t.w)};
+    *reinterpret_cast<uint2 *>(D + (size_t)(tm * BM + row) * N + tn * BN + ch * 4) = *reinterpret_cast<uint2 *>(o);
+  }
+  __syncwarp();
+  clusterSync(); // no CTA leaves while another may still read its part
+  if (warp == 1) tmemDealloc(tmemBase, BN);
+}
+
+template <int BN>
+cudaError_t launch(cudaStream_t stream, const CUtensorMap &tmA, const CUtensorMap &tmB, void *D, int M, int N, int K, int S) {
+  static std::atomic<unsigned long long> ready{0}; // bit per device: the attribute belongs to the device's context
+  const size_t smem = sizeof(Smem<BN>) + 1024;
+  int dev = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e != cudaSuccess) return e;
+  const unsigned long long bit = 1ull << (dev & 63);
+  if (dev > 63 || !(ready.load(std::memory_order_acquire) & bit)) {
+    e = cudaFuncSetAttribute(splitGemmKernel<BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return e;
+    if (dev <= 63) ready.fetch_or(bit, std::memory_order_release);
+  }
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = (unsigned)S;
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = 1;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)((M / BM) * (N / BN) * S));
+  cfg.blockDim = dim3(kThreads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, splitGemmKernel<BN>, tmA, tmB, (bf16 *)D, N, K / BK, M / BM, S);
+}
+
+} // namespace
+
+cudaError_t launchSplitGemm(cudaStream_t stream, const CUtensorMap &tmA, const CUtensorMap &tmB, void *D, int M, int N, int K,
+                            const SplitGemmPlan &p) {
+  if (p.parts < 1 || p.parts > kSplitGemmMaxParts || p.parts > K / BK) return cudaErrorInvalidValue;
+  switch (p.tileN) {
+    case 256: return launch<256>(stream, tmA, tmB, D, M, N, K, p.parts);
+    case 128: return launch<128>(stream, tmA, tmB, D, M, N, K, p.parts);
+    case 64: return launch<64>(stream, tmA, tmB, D, M, N, K, p.parts);
+    default: return cudaErrorInvalidValue;
+  }
+}
+
+} // namespace fcx

@@ -25,6 +25,28 @@ def test_tcgen05_gemm_matches_fp32_reference(M, N, K, pair, monkeypatch):
     assert err < 2 ** -7, err
 
 
+# parts that do not divide K's steps or the 128 rows of a tile, one step per part, and what the
+# size rule picks at the ends of its range (0: automatic)
+@pytest.mark.parametrize("M,N,K,parts", [(128, 256, 512, 8), (128, 512, 2112, 3), (384, 256, 576, 5), (256, 768, 1024, 7),
+                                         (128, 256, 128, 2), (128, 256, 256, 0), (128, 3584, 8192, 0), (1024, 2048, 320, 0),
+                                         (512, 256, 4160, 0)])
+@pytest.mark.parametrize("tile_n", [256, 128, 64])
+def test_gemm_with_k_split_over_a_cluster(M, N, K, parts, tile_n, monkeypatch):
+    from flagcx_b200.parallel.tp import gemm_bf16
+    monkeypatch.setenv("FLAGCX_GEMM_SPLIT", str(parts))
+    monkeypatch.setenv("FLAGCX_GEMM_SPLIT_N", str(tile_n))
+    g = torch.Generator(device="cuda").manual_seed(M + N + K)
+    a = torch.randn(M, K, generator=g, device="cuda").to(torch.bfloat16)
+    b = torch.randn(N, K, generator=g, device="cuda").to(torch.bfloat16)
+    out = torch.full((M, N), float("nan"), dtype=torch.bfloat16, device="cuda")
+    gemm_bf16(a, b, out)
+    ref = a.double() @ b.double().T
+    # one rounding to bf16 (2^-9 of the value) and fp32 sums of K products: each of the K additions
+    # errs by at most 2^-24 of the running sum, bounded by the sum of the products' magnitudes
+    bound = ref.abs() * 2 ** -8 + (a.double().abs() @ b.double().abs().T) * K * 2 ** -24
+    assert bool(((out.double() - ref).abs() <= bound).all())
+
+
 @pytest.mark.skipif(torch.cuda.device_count() < 2, reason="needs at least 2 GPUs")
 def test_fused_tensor_parallel_kernels_on_real_peers():
     n = 8 if torch.cuda.device_count() >= 8 else 4 if torch.cuda.device_count() >= 4 else 2
