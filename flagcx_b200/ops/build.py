@@ -8,7 +8,7 @@ import shutil
 HERE = os.path.dirname(os.path.abspath(__file__))
 ROOT = os.path.dirname(os.path.dirname(HERE))
 NAME = "_flagcx_ops_C"
-SOURCES = ["fused_elementwise.cu"]
+SOURCES = ["fused_elementwise.cu", "torch_ops.cpp"]
 NVCC_FLAGS = ["-O3", "-std=c++17", "-lineinfo", "-gencode", "arch=compute_100a,code=sm_100a", "--use_fast_math"]
 
 

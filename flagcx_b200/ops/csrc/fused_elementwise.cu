@@ -4,15 +4,14 @@
 // cross-entropy with the gradient written in place of the logits, and a flat
 // AdamW step.  All are sm_100a kernels with 16-byte accesses and fp32 math; each
 // reads its operands once and writes its results once.
-#include <ATen/cuda/CUDAContext.h>
-#include <c10/cuda/CUDAException.h>
-#include <c10/cuda/CUDAGuard.h>
 #include <cooperative_groups.h>
 #include <cuda_bf16.h>
-#include <torch/extension.h>
 
 #include <algorithm>
+#include <cstdint>
 #include <cstdlib>
+
+#include "fused_elementwise.h"
 
 namespace cg = cooperative_groups;
 
@@ -622,175 +621,98 @@ __global__ void adamwFlat(bf16 *__restrict__ p, const bf16 *__restrict__ g, bf16
   }
 }
 
-// ---------------------------------------------------------------------------
-// host wrappers
-// ---------------------------------------------------------------------------
-void checkBf16(const at::Tensor &t, const char *name) {
-  TORCH_CHECK(t.is_cuda() && t.scalar_type() == at::kBFloat16 && t.is_contiguous(), name,
-              " must be a contiguous CUDA bfloat16 tensor");
-  TORCH_CHECK(((uintptr_t)t.data_ptr() & 15) == 0, name, " must be 16-byte aligned");
-}
-
-int gridFor(size_t items, int threads, int perSm = 8) {
-  int sms = at::cuda::getCurrentDeviceProperties()->multiProcessorCount;
+int gridFor(size_t items, int threads, int sms, int perSm = 8) {
   size_t want = (items + threads - 1) / threads;
   return (int)std::max<size_t>(1, std::min<size_t>(want, (size_t)sms * perSm));
 }
 
-std::vector<at::Tensor> rmsnorm_fwd(const at::Tensor &x, const at::Tensor &w, double eps) {
-  checkBf16(x, "x");
-  checkBf16(w, "weight");
-  const int H = (int)x.size(-1);
-  TORCH_CHECK(H % 8 == 0 && H <= 8 * 512 * 4 && w.numel() == H, "rmsnorm: hidden size must be a multiple of 8, at most 16384");
-  const c10::cuda::CUDAGuard guard(x.device());
-  const int64_t rows = x.numel() / H;
-  auto y = at::empty_like(x);
-  auto rstd = at::empty({rows}, x.options().dtype(at::kFloat));
-  auto stream = at::cuda::getCurrentCUDAStream();
+#define RETURN_IF(e)                        \
+  do {                                      \
+    const cudaError_t err_ = (e);           \
+    if (err_ != cudaSuccess) return err_;   \
+  } while (0)
+
+} // namespace
+
+// ---------------------------------------------------------------------------
+// launchers (see fused_elementwise.h)
+// ---------------------------------------------------------------------------
+namespace fcxops {
+
+cudaError_t rmsnormForward(const void *x, const void *w, void *y, float *rstd, long rows, int H, float eps, int sms,
+                           cudaStream_t stream) {
   const int threads = 512, packs = H / 8;
   const int maxp = (packs + threads - 1) / threads;
   auto launch = [&](auto tag) {
-    rmsnormFwd<decltype(tag)::value><<<(unsigned)rows, threads, 0, stream>>>(
-        (const bf16 *)x.data_ptr(), (const bf16 *)w.data_ptr(), (bf16 *)y.data_ptr(), rstd.data_ptr<float>(), H, (float)eps);
+    rmsnormFwd<decltype(tag)::value><<<(unsigned)rows, threads, 0, stream>>>((const bf16 *)x, (const bf16 *)w, (bf16 *)y,
+                                                                             rstd, H, eps);
   };
   auto launchWarp = [&](auto tag) { // one warp per row, eight rows per CTA
-    rmsnormFwdWarp<decltype(tag)::value><<<(unsigned)((rows + 7) / 8), 256, 0, stream>>>(
-        (const bf16 *)x.data_ptr(), (const bf16 *)w.data_ptr(), (bf16 *)y.data_ptr(), rstd.data_ptr<float>(), (long)rows, H,
-        (float)eps);
+    rmsnormFwdWarp<decltype(tag)::value><<<(unsigned)((rows + 7) / 8), 256, 0, stream>>>((const bf16 *)x, (const bf16 *)w,
+                                                                                       (bf16 *)y, rstd, rows, H, eps);
   };
-  if (rows > 0) {
-    if (packs <= 32 * 4) launchWarp(std::integral_constant<int, 4>());
-    else if (packs <= 32 * 8) launchWarp(std::integral_constant<int, 8>());
-    else if (packs <= 32 * 16) launchWarp(std::integral_constant<int, 16>());
-    else if (maxp <= 1) launch(std::integral_constant<int, 1>());
-    else if (maxp <= 2) launch(std::integral_constant<int, 2>());
-    else launch(std::integral_constant<int, 4>());
-    C10_CUDA_KERNEL_LAUNCH_CHECK();
-  }
-  return {y, rstd};
+  if (packs <= 32 * 4) launchWarp(std::integral_constant<int, 4>());
+  else if (packs <= 32 * 8) launchWarp(std::integral_constant<int, 8>());
+  else if (packs <= 32 * 16) launchWarp(std::integral_constant<int, 16>());
+  else if (maxp <= 1) launch(std::integral_constant<int, 1>());
+  else if (maxp <= 2) launch(std::integral_constant<int, 2>());
+  else launch(std::integral_constant<int, 4>());
+  return cudaGetLastError();
 }
 
-// `add`, when given, has x's shape and is added to dx inside the kernel (the gradient that
-// reaches x through a residual connection around the norm).
-std::vector<at::Tensor> rmsnorm_bwd(const at::Tensor &g, const at::Tensor &x, const at::Tensor &w,
-                                    const at::Tensor &rstd, const c10::optional<at::Tensor> &add) {
-  checkBf16(g, "grad");
-  if (add.has_value()) {
-    checkBf16(*add, "add");
-    TORCH_CHECK(add->numel() == x.numel(), "rmsnorm_bwd: `add` must have x's shape");
-  }
-  checkBf16(x, "x");
-  checkBf16(w, "weight");
-  const int H = (int)x.size(-1);
-  const c10::cuda::CUDAGuard guard(x.device());
-  const int64_t rows = x.numel() / H;
-  auto dx = at::empty_like(x);
-  TORCH_CHECK(H % 8 == 0 && H <= 8 * 512 * 4 && w.numel() == H, "rmsnorm: hidden size must be a multiple of 8, at most 16384");
-  const int sms = at::cuda::getCurrentDeviceProperties()->multiProcessorCount;
-  const int ctas = (int)std::max<int64_t>(1, std::min<int64_t>(rows, sms * 2));
-  auto partial = at::empty({ctas, H}, x.options().dtype(at::kFloat));
-  auto dw = at::empty({H}, x.options());
-  auto stream = at::cuda::getCurrentCUDAStream();
+int rmsnormPartials(long rows, int H, int sms) { return (int)std::max<long>(1, std::min<long>(rows, sms * 2)); }
+
+cudaError_t rmsnormBackward(const void *g, const void *x, const void *w, const float *rstd, const void *add, void *dx, void *dw,
+                            float *partial, long rows, int H, int sms, cudaStream_t stream) {
+  const int ctas = rmsnormPartials(rows, H, sms);
   const int packs = H / 8;
   const int maxp = (packs + kNormBwdThreads - 1) / kNormBwdThreads;
   // ring of (g row, x row) slots: about 96 KiB per CTA so that two CTAs share an SM
-  const size_t slot = (size_t)H * (add.has_value() ? 6 : 4);
+  const size_t slot = (size_t)H * (add ? 6 : 4);
   const int stages = (int)std::max<size_t>(2, std::min<size_t>(kNormBwdMaxStages, ((size_t)96 << 10) / slot));
   const size_t smem = slot * stages;
   auto launch = [&](auto tag) {
     auto kern = rmsnormBwdPipelined<decltype(tag)::value>;
-    C10_CUDA_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    kern<<<ctas, kNormBwdThreads, smem, stream>>>((const bf16 *)g.data_ptr(), (const bf16 *)x.data_ptr(),
-                                                  (const bf16 *)w.data_ptr(), rstd.data_ptr<float>(),
-                                                  add.has_value() ? (const bf16 *)add->data_ptr() : nullptr,
-                                                  (bf16 *)dx.data_ptr(), partial.data_ptr<float>(), (int)rows, H, stages);
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return e;
+    kern<<<ctas, kNormBwdThreads, smem, stream>>>((const bf16 *)g, (const bf16 *)x, (const bf16 *)w, rstd, (const bf16 *)add,
+                                                  (bf16 *)dx, partial, (int)rows, H, stages);
+    return cudaGetLastError();
   };
-  if (rows == 0) {
-    dw.zero_();
-    return {dx, dw};
-  }
-  TORCH_CHECK(smem <= ((size_t)200 << 10), "rmsnorm_bwd: hidden size too large for the shared-memory ring");
-  if (maxp <= 1) launch(std::integral_constant<int, 1>());
-  else if (maxp <= 2) launch(std::integral_constant<int, 2>());
-  else launch(std::integral_constant<int, 4>());
-  C10_CUDA_KERNEL_LAUNCH_CHECK();
-  columnSumToBf16<<<(H + 31) / 32, dim3(32, 32), 0, stream>>>(partial.data_ptr<float>(), (bf16 *)dw.data_ptr(), ctas, H);
-  C10_CUDA_KERNEL_LAUNCH_CHECK();
-  return {dx, dw};
+  if (maxp <= 1) RETURN_IF(launch(std::integral_constant<int, 1>()));
+  else if (maxp <= 2) RETURN_IF(launch(std::integral_constant<int, 2>()));
+  else RETURN_IF(launch(std::integral_constant<int, 4>()));
+  columnSumToBf16<<<(H + 31) / 32, dim3(32, 32), 0, stream>>>(partial, (bf16 *)dw, ctas, H);
+  return cudaGetLastError();
 }
 
-void rope_inplace(at::Tensor &x, const c10::optional<at::Tensor> &positions, double theta, bool backward) {
-  checkBf16(x, "x");
-  TORCH_CHECK(x.dim() >= 3, "rope: expected [..., heads, head_dim]");
-  const int D = (int)x.size(-1), heads = (int)x.size(-2);
-  TORCH_CHECK(D % 16 == 0, "rope: head_dim must be a multiple of 16");
-  const int64_t tokens = x.numel() / ((int64_t)D * heads);
-  const int *pos = nullptr;
-  if (positions.has_value()) {
-    TORCH_CHECK(positions->scalar_type() == at::kInt && positions->numel() == tokens && positions->is_cuda(), "rope: bad positions");
-    pos = positions->data_ptr<int>();
-  }
-  const c10::cuda::CUDAGuard guard(x.device());
-  size_t items = (size_t)tokens * heads * (D / 16);
-  ropeKernel<<<gridFor(items, 256), 256, 0, at::cuda::getCurrentCUDAStream()>>>(
-      (bf16 *)x.data_ptr(), pos, (int)tokens, heads, D, logf((float)theta), backward ? -1.f : 1.f);
+cudaError_t rope(void *x, const int *positions, int tokens, int heads, int D, float logTheta, float sign, int sms,
+                 cudaStream_t stream) {
+  const size_t items = (size_t)tokens * heads * (D / 16);
+  ropeKernel<<<gridFor(items, 256, sms), 256, 0, stream>>>((bf16 *)x, positions, tokens, heads, D, logTheta, sign);
+  return cudaGetLastError();
 }
 
-// qkv: [tokens, (ropeHeads + otherHeads) * D]; returns a new tensor of the same shape.
-at::Tensor rope_fused_qkv(const at::Tensor &qkv, int64_t ropeHeads, int64_t totalHeads, int64_t D, double theta,
-                          bool backward) {
-  checkBf16(qkv, "qkv");
-  TORCH_CHECK(D % 16 == 0 && qkv.size(-1) == totalHeads * D && ropeHeads <= totalHeads, "rope_fused_qkv: bad shape");
-  const int64_t tokens = qkv.numel() / (totalHeads * D);
-  const c10::cuda::CUDAGuard guard(qkv.device());
-  auto out = at::empty_like(qkv);
-  if (qkv.numel() == 0) return out;
-  size_t items = (size_t)tokens * totalHeads * (D / 16);
-  ropeFusedQkv<<<gridFor(items, 256), 256, 0, at::cuda::getCurrentCUDAStream()>>>(
-      (const bf16 *)qkv.data_ptr(), (bf16 *)out.data_ptr(), (int)tokens, (int)ropeHeads, (int)totalHeads, (int)D,
-      logf((float)theta), backward ? -1.f : 1.f);
-  C10_CUDA_KERNEL_LAUNCH_CHECK();
-  return out;
+cudaError_t ropeQkv(const void *qkv, void *out, int tokens, int ropeHeads, int totalHeads, int D, float logTheta, float sign,
+                    int sms, cudaStream_t stream) {
+  const size_t items = (size_t)tokens * totalHeads * (D / 16);
+  ropeFusedQkv<<<gridFor(items, 256, sms), 256, 0, stream>>>((const bf16 *)qkv, (bf16 *)out, tokens, ropeHeads, totalHeads,
+                                                             D, logTheta, sign);
+  return cudaGetLastError();
 }
 
-at::Tensor swiglu_fwd(const at::Tensor &ab) {
-  checkBf16(ab, "ab");
-  const int F = (int)ab.size(-1) / 2;
-  TORCH_CHECK(F % 8 == 0, "swiglu: width must be a multiple of 8");
-  const c10::cuda::CUDAGuard guard(ab.device());
-  auto sizes = ab.sizes().vec();
-  sizes.back() = F;
-  auto out = at::empty(sizes, ab.options());
-  size_t T = ab.numel() / (2 * (size_t)F);
-  swigluFwd<<<gridFor(T * (F / 8), 256), 256, 0, at::cuda::getCurrentCUDAStream()>>>((const bf16 *)ab.data_ptr(),
-                                                                                    (bf16 *)out.data_ptr(), T, F);
-  return out;
+cudaError_t swigluForward(const void *ab, void *out, size_t T, int F, int sms, cudaStream_t stream) {
+  swigluFwd<<<gridFor(T * (F / 8), 256, sms), 256, 0, stream>>>((const bf16 *)ab, (bf16 *)out, T, F);
+  return cudaGetLastError();
 }
 
-at::Tensor swiglu_bwd(const at::Tensor &g, const at::Tensor &ab) {
-  checkBf16(g, "grad");
-  checkBf16(ab, "ab");
-  const int F = (int)ab.size(-1) / 2;
-  const c10::cuda::CUDAGuard guard(ab.device());
-  auto dab = at::empty_like(ab);
-  size_t T = ab.numel() / (2 * (size_t)F);
-  swigluBwd<<<gridFor(T * (F / 8), 256), 256, 0, at::cuda::getCurrentCUDAStream()>>>(
-      (const bf16 *)g.data_ptr(), (const bf16 *)ab.data_ptr(), (bf16 *)dab.data_ptr(), T, F);
-  return dab;
+cudaError_t swigluBackward(const void *g, const void *ab, void *dab, size_t T, int F, int sms, cudaStream_t stream) {
+  swigluBwd<<<gridFor(T * (F / 8), 256, sms), 256, 0, stream>>>((const bf16 *)g, (const bf16 *)ab, (bf16 *)dab, T, F);
+  return cudaGetLastError();
 }
 
-// Returns per-row losses; `logits` now holds gradScale * dLoss/dlogits.
-at::Tensor cross_entropy_fwd_bwd_(at::Tensor &logits, const at::Tensor &targets, double gradScale) {
-  checkBf16(logits, "logits");
-  TORCH_CHECK(targets.is_cuda() && targets.scalar_type() == at::kLong && targets.is_contiguous(), "targets must be int64 CUDA");
-  const int V = (int)logits.size(-1);
-  TORCH_CHECK(V % 8 == 0, "cross-entropy: vocabulary must be a multiple of 8");
-  const int64_t rows = logits.numel() / V;
-  TORCH_CHECK(targets.numel() == rows, "cross-entropy: one target per row");
-  const c10::cuda::CUDAGuard guard(logits.device());
-  auto loss = at::empty({rows}, logits.options().dtype(at::kFloat));
-  if (rows == 0) return loss;
-  auto stream = at::cuda::getCurrentCUDAStream();
+cudaError_t crossEntropy(void *logits, const long *targets, float *loss, long rows, int V, float gradScale, int sms,
+                         cudaStream_t stream) {
   // Smallest cluster whose per-CTA part of a row fits beside two other CTAs on the SM
   // (72 KiB each); failing that, one CTA per SM with up to 200 KiB; failing that, the
   // kernel that streams the row three times.
@@ -806,13 +728,11 @@ at::Tensor cross_entropy_fwd_bwd_(at::Tensor &logits, const at::Tensor &targets,
   }
   static const bool forceStreaming = std::getenv("FLAGCX_OPS_CE_STREAMING") && atoi(std::getenv("FLAGCX_OPS_CE_STREAMING")) != 0;
   if (!cluster || forceStreaming || rows * cluster > 0x7fffffffLL) {
-    crossEntropyFwdBwd<<<(unsigned)rows, 1024, 0, stream>>>((bf16 *)logits.data_ptr(), targets.data_ptr<long>(),
-                                                            loss.data_ptr<float>(), V, (float)gradScale);
-    C10_CUDA_KERNEL_LAUNCH_CHECK();
-    return loss;
+    crossEntropyFwdBwd<<<(unsigned)rows, 1024, 0, stream>>>((bf16 *)logits, targets, loss, V, gradScale);
+    return cudaGetLastError();
   }
   const size_t smem = (size_t)per * 16;
-  C10_CUDA_CHECK(cudaFuncSetAttribute(crossEntropyCluster, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  RETURN_IF(cudaFuncSetAttribute(crossEntropyCluster, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((unsigned)(rows * cluster));
   static const int ceThreads = std::getenv("FLAGCX_OPS_CE_THREADS") ? std::min(kCeMaxThreads, std::max(32, atoi(std::getenv("FLAGCX_OPS_CE_THREADS")) / 32 * 32)) : 256;
@@ -826,36 +746,14 @@ at::Tensor cross_entropy_fwd_bwd_(at::Tensor &logits, const at::Tensor &targets,
   attr[0].val.clusterDim.z = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  C10_CUDA_CHECK(cudaLaunchKernelEx(&cfg, crossEntropyCluster, (bf16 *)logits.data_ptr(), (const long *)targets.data_ptr<long>(),
-                                    loss.data_ptr<float>(), V, (float)gradScale, per));
-  return loss;
+  return cudaLaunchKernelEx(&cfg, crossEntropyCluster, (bf16 *)logits, targets, loss, V, gradScale, per);
 }
 
-void adamw_flat_(at::Tensor &p, const at::Tensor &g, at::Tensor &m, at::Tensor &v, double lr, double beta1, double beta2,
-                 double eps, double wd, int64_t step) {
-  checkBf16(p, "param");
-  checkBf16(g, "grad");
-  checkBf16(m, "exp_avg");
-  checkBf16(v, "exp_avg_sq");
-  TORCH_CHECK(p.numel() == g.numel() && p.numel() == m.numel() && p.numel() == v.numel(), "adamw: size mismatch");
-  const c10::cuda::CUDAGuard guard(p.device());
-  const size_t n = p.numel();
-  if (n == 0) return;
-  float bc1 = 1.f - (float)std::pow(beta1, (double)step), bc2 = 1.f - (float)std::pow(beta2, (double)step);
-  adamwFlat<<<gridFor(n / 8 + 8, 256), 256, 0, at::cuda::getCurrentCUDAStream()>>>(
-      (bf16 *)p.data_ptr(), (const bf16 *)g.data_ptr(), (bf16 *)m.data_ptr(), (bf16 *)v.data_ptr(), n, (float)lr,
-      (float)beta1, (float)beta2, (float)eps, (float)wd, bc1, bc2);
+cudaError_t adamw(void *p, const void *g, void *m, void *v, size_t n, float lr, float beta1, float beta2, float eps, float wd,
+                  float bc1, float bc2, int sms, cudaStream_t stream) {
+  adamwFlat<<<gridFor(n / 8 + 8, 256, sms), 256, 0, stream>>>((bf16 *)p, (const bf16 *)g, (bf16 *)m, (bf16 *)v, n, lr, beta1,
+                                                              beta2, eps, wd, bc1, bc2);
+  return cudaGetLastError();
 }
 
-} // namespace
-
-PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
-  m.def("rmsnorm_fwd", &rmsnorm_fwd);
-  m.def("rmsnorm_bwd", &rmsnorm_bwd, py::arg("g"), py::arg("x"), py::arg("w"), py::arg("rstd"), py::arg("add") = py::none());
-  m.def("rope_inplace", &rope_inplace);
-  m.def("rope_fused_qkv", &rope_fused_qkv);
-  m.def("swiglu_fwd", &swiglu_fwd);
-  m.def("swiglu_bwd", &swiglu_bwd);
-  m.def("cross_entropy_fwd_bwd_", &cross_entropy_fwd_bwd_);
-  m.def("adamw_flat_", &adamw_flat_);
-}
+} // namespace fcxops
