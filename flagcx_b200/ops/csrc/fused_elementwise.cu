@@ -8,6 +8,7 @@
 #include <cuda_bf16.h>
 
 #include <algorithm>
+#include <atomic>
 #include <cstdint>
 #include <cstdlib>
 
@@ -465,7 +466,146 @@ __global__ void crossEntropyFwdBwd(bf16 *__restrict__ logits, const long *__rest
 }
 
 // ---------------------------------------------------------------------------
-// The same operation with the row held on chip.  A thread-block cluster of C CTAs
+// The same operation, persistent, for vocabularies up to 8 x 16 x 2048 = 262144.  A cluster
+// of C CTAs walks over rows; each CTA's 1/C of a row comes into a shared-memory slot by bulk
+// copy, moves on into registers (PPT packs of 8 per thread), and the copy of the next row
+// into the slot starts at once: while a row is being reduced, scaled and stored, the next one
+// is already on its way.  The exponentials are taken relative to the WARP's maximum and stay
+// in registers (as bf16), so that a row needs one exchange only: every warp publishes its
+// (maximum, sum), one cluster barrier, and every warp combines all pairs of the cluster.  A
+// warp whose logits are all -inf (a masked stretch) contributes nothing.
+//
+// Bound: HBM (one read and one write of the logits).  The kernel below it in this file, which
+// loads, reduces and stores one row per CTA with nothing overlapped, took 458 us for
+// 4096 x 128256; this one takes 355 (5.9 TB/s, 0.92 of a copy).
+// ---------------------------------------------------------------------------
+constexpr int kCeRowThreads = 256, kCeRowWarps = kCeRowThreads / 32;
+constexpr int kCeRowMaxPacks = 16 * kCeRowThreads; // packs of a row that one CTA can hold
+constexpr uint32_t kCeBulkPiece = 32768;
+
+__device__ __forceinline__ void clusterSyncAll() {
+  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+
+__device__ __forceinline__ float lowBf16(uint32_t u) { return __uint_as_float(u << 16); }
+__device__ __forceinline__ float highBf16(uint32_t u) { return __uint_as_float(u & 0xffff0000u); }
+__device__ __forceinline__ uint32_t packBf16x2(float lo, float hi) {
+  uint32_t r;
+  asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(r) : "f"(hi), "f"(lo));
+  return r;
+}
+__device__ __forceinline__ uint32_t maxBf16x2(uint32_t a, uint32_t b) {
+  uint32_t r;
+  asm("max.bf16x2 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(b));
+  return r;
+}
+
+template <int PPT>
+__global__ void __launch_bounds__(kCeRowThreads, PPT > 10 ? 2 : PPT > 8 ? 3 : PPT == 8 ? 4 : PPT == 4 ? 5 : 8)
+crossEntropyRows(bf16 *__restrict__ logits, const long *__restrict__ targets, float *__restrict__ loss, long rows, int V,
+                 float gradScale, int packsPerCta) {
+  extern __shared__ __align__(128) unsigned char ceSlot[];
+  __shared__ float2 stat[2][kCeRowWarps]; // (maximum, sum) of every warp, two rows deep
+  __shared__ __align__(8) uint64_t bar;
+  cg::cluster_group cluster = cg::this_cluster();
+  const int C = (int)cluster.num_blocks(), cr = (int)cluster.block_rank();
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const long step = gridDim.x / C;
+  const int p0 = cr * packsPerCta, n = max(0, min(packsPerCta, V / 8 - p0));
+  const uint32_t bytes = (uint32_t)n * 16u;
+  const uint4 *slot = (const uint4 *)ceSlot;
+  auto part = [&](long row) { return (unsigned char *)(logits + (size_t)row * V + (size_t)p0 * 8); };
+  auto issue = [&](long row) { // thread 0
+    mbarExpect(&bar, bytes);
+    for (uint32_t off = 0; off < bytes; off += kCeBulkPiece)
+      bulkLoad(ceSlot + off, part(row) + off, min(kCeBulkPiece, bytes - off), &bar);
+  };
+  long row = blockIdx.x / C;
+  if (tid == 0) {
+    mbarInit(&bar);
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    if (row < rows && n > 0) issue(row);
+  }
+  __syncthreads();
+  constexpr float kLog2e = 1.4426950408889634f;
+  bool ok = true; // a copy that never arrived poisons the loss and the gradient of its row
+  for (int it = 0; row < rows; row += step, ++it) {
+    if (n > 0 && ok) ok = mbarWaitBounded(&bar, (uint32_t)it & 1u);
+    const long tLocal = targets[row] - (long)p0 * 8; // index of the target inside this CTA's part, if it is here
+    const bool own = tLocal >= 0 && tLocal < (long)n * 8;
+    const float tgtLogit = own ? __bfloat162float(((const bf16 *)ceSlot)[tLocal]) : 0.f;
+    uint32_t v[PPT][4];
+#pragma unroll
+    for (int k = 0; k < PPT; ++k) {
+      const int p = tid + k * kCeRowThreads;
+      const uint4 q = p < n ? slot[p] : make_uint4(0xff80ff80u, 0xff80ff80u, 0xff80ff80u, 0xff80ff80u); // -inf
+      v[k][0] = q.x; v[k][1] = q.y; v[k][2] = q.z; v[k][3] = q.w;
+    }
+    __syncthreads(); // the slot has been read
+    if (tid == 0 && row + step < rows && n > 0 && ok) issue(row + step);
+    uint32_t m2 = 0xff80ff80u;
+#pragma unroll
+    for (int k = 0; k < PPT; ++k)
+#pragma unroll
+      for (int i = 0; i < 4; ++i) m2 = maxBf16x2(m2, v[k][i]);
+    const float wmax = warpMax(fmaxf(lowBf16(m2), highBf16(m2)));
+    // exponentials: 2^(v*log2e - max*log2e), one FMA and one MUFU each
+    const float ref = wmax == -INFINITY ? 0.f : wmax * kLog2e;
+    float sum = 0.f;
+#pragma unroll
+    for (int k = 0; k < PPT; ++k)
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const float e0 = exp2f(fmaf(lowBf16(v[k][i]), kLog2e, -ref)), e1 = exp2f(fmaf(highBf16(v[k][i]), kLog2e, -ref));
+        sum += e0 + e1;
+        v[k][i] = packBf16x2(e0, e1);
+      }
+    sum = warpSum(ok ? sum : NAN);
+    if (lane == 0) stat[it & 1][warp] = make_float2(wmax, sum);
+    __syncwarp();
+    // One barrier per row: the pairs of the row before last are overwritten only now, when
+    // every CTA has passed the last row's barrier and so has read them.
+    if (C > 1) clusterSyncAll(); else __syncthreads();
+    float M = -INFINITY, S = 0.f;
+    float2 st[2];
+#pragma unroll
+    for (int j = 0; j < 2; ++j) {
+      const int i = lane + 32 * j;
+      st[j] = i < C * kCeRowWarps ? cluster.map_shared_rank(&stat[it & 1][0], i / kCeRowWarps)[i % kCeRowWarps]
+                                  : make_float2(-INFINITY, 0.f);
+      M = fmaxf(M, st[j].x);
+    }
+    M = warpMax(M);
+#pragma unroll
+    for (int j = 0; j < 2; ++j)
+      if (st[j].y != 0.f) S += st[j].y * __expf(st[j].x - M);
+    S = warpSum(S);
+    if (own && tid == 0) loss[row] = M + __logf(S) - tgtLogit;
+    const float f = __expf(wmax - M) / S * gradScale;
+    uint4 *out = (uint4 *)part(row);
+#pragma unroll
+    for (int k = 0; k < PPT; ++k) {
+      const int p = tid + k * kCeRowThreads;
+      if (p < n) {
+        uint4 o;
+        o.x = packBf16x2(lowBf16(v[k][0]) * f, highBf16(v[k][0]) * f);
+        o.y = packBf16x2(lowBf16(v[k][1]) * f, highBf16(v[k][1]) * f);
+        o.z = packBf16x2(lowBf16(v[k][2]) * f, highBf16(v[k][2]) * f);
+        o.w = packBf16x2(lowBf16(v[k][3]) * f, highBf16(v[k][3]) * f);
+        out[p] = o;
+      }
+    }
+    // the one element that is softmax - 1, redone in fp32 by the thread that stored its pack
+    if (own && tid == (int)((tLocal >> 3) % kCeRowThreads))
+      ((bf16 *)out)[tLocal] = __float2bfloat16_rn(exp2f(fmaf(tgtLogit, kLog2e, -ref)) * f - gradScale);
+  }
+  __syncwarp();
+  if (C > 1) clusterSyncAll(); // no CTA leaves while another may still read its pairs
+}
+
+// ---------------------------------------------------------------------------
+// The same operation for vocabularies beyond that (part of a row stays in shared memory, up to
+// 200 KiB per CTA).  A thread-block cluster of C CTAs
 // owns one row; each CTA brings its 1/C of the row into shared memory with one
 // bulk asynchronous copy, finds its own maximum and sum of exponentials (the
 // exponentials replace the logits in shared memory, as bf16), trades (max, sum)
@@ -475,7 +615,6 @@ __global__ void crossEntropyFwdBwd(bf16 *__restrict__ logits, const long *__rest
 // exponential instead of two.
 // ---------------------------------------------------------------------------
 constexpr int kCeMaxThreads = 1024;
-constexpr uint32_t kCeBulkPiece = 32768;
 
 __global__ void __launch_bounds__(kCeMaxThreads)
 crossEntropyCluster(bf16 *__restrict__ logits, const long *__restrict__ targets, float *__restrict__ loss, int V,
@@ -521,7 +660,7 @@ crossEntropyCluster(bf16 *__restrict__ logits, const long *__restrict__ targets,
   mx = blockMax(mx, red); // its barriers also order the read of the target logit before the overwrite below
   // exponentials: 2^(v*log2e - mx*log2e), one FMA and one MUFU each
   constexpr float kLog2e = 1.4426950408889634f;
-  const float mxs = mx * kLog2e;
+  const float mxs = mx == -INFINITY ? 0.f : mx * kLog2e; // a part that is all -inf contributes nothing
   float sum = 0.f;
   for (int p = threadIdx.x; p < n; p += (int)blockDim.x) {
     const uint4 v = buf[p];
@@ -632,6 +771,42 @@ int gridFor(size_t items, int threads, int sms, int perSm = 8) {
     if (err_ != cudaSuccess) return err_;   \
   } while (0)
 
+template <int PPT>
+cudaError_t launchCeRows(bf16 *logits, const long *targets, float *loss, long rows, int V, float gradScale, int C, int per,
+                         int sms, cudaStream_t stream) {
+  auto kern = crossEntropyRows<PPT>;
+  const int smem = per * 16;
+  cudaLaunchConfig_t cfg = {};
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = (unsigned)C;
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = 1;
+  cfg.blockDim = dim3(kCeRowThreads);
+  cfg.dynamicSmemBytes = (size_t)smem;
+  cfg.stream = stream;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  RETURN_IF(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+  // As many clusters as run at once: rows are dealt out evenly, so a second wave would be waste.
+  long clusters = rows;
+  if (rows * C > sms) {
+    static std::atomic<uint64_t> known{0}; // last answer: shared memory << 32 | cluster size << 16 | clusters
+    uint64_t k = known.load(std::memory_order_relaxed);
+    const uint64_t key = (uint64_t)smem << 16 | (uint64_t)C;
+    if (k >> 16 != key) {
+      int active = 0;
+      cfg.gridDim = dim3((unsigned)C);
+      RETURN_IF(cudaOccupancyMaxActiveClusters(&active, kern, &cfg));
+      k = key << 16 | (uint64_t)std::min(std::max(active, 1), 0xffff);
+      known.store(k, std::memory_order_relaxed);
+    }
+    clusters = std::min<long>(rows, (long)(k & 0xffff));
+  }
+  cfg.gridDim = dim3((unsigned)(clusters * C));
+  return cudaLaunchKernelEx(&cfg, kern, logits, targets, loss, rows, V, gradScale, per);
+}
+
 } // namespace
 
 // ---------------------------------------------------------------------------
@@ -713,21 +888,37 @@ cudaError_t swigluBackward(const void *g, const void *ab, void *dab, size_t T, i
 
 cudaError_t crossEntropy(void *logits, const long *targets, float *loss, long rows, int V, float gradScale, int sms,
                          cudaStream_t stream) {
-  // Smallest cluster whose per-CTA part of a row fits beside two other CTAs on the SM
-  // (72 KiB each); failing that, one CTA per SM with up to 200 KiB; failing that, the
-  // kernel that streams the row three times.
+  // Smallest cluster whose per-CTA part of a row fits the registers of crossEntropyRows; more
+  // CTAs per row while that leaves SMs idle and a CTA still has two packs per thread.  Longer
+  // rows: up to 200 KiB of shared memory per CTA; failing that, the kernel that streams the
+  // row three times.
   const int packs = V / 8;
   int cluster = 0, per = 0;
-  static const size_t partKb = std::getenv("FLAGCX_OPS_CE_PART_KB") ? (size_t)atoi(std::getenv("FLAGCX_OPS_CE_PART_KB")) : 72;
-  for (size_t limit : {partKb << 10, (size_t)200 << 10}) {
+  static const size_t partKb = std::getenv("FLAGCX_OPS_CE_PART_KB") ? (size_t)atoi(std::getenv("FLAGCX_OPS_CE_PART_KB")) : 64;
+  static const bool forceStreaming = std::getenv("FLAGCX_OPS_CE_STREAMING") && atoi(std::getenv("FLAGCX_OPS_CE_STREAMING")) != 0;
+  if (!forceStreaming) {
     for (int c : {1, 2, 4, 8}) {
       per = (packs + c - 1) / c;
-      if ((size_t)per * 16 <= limit) { cluster = c; break; }
+      if (per <= kCeRowMaxPacks && ((size_t)per * 16 <= partKb << 10 || c == 8)) { cluster = c; break; }
     }
-    if (cluster) break;
+    if (cluster) {
+      while (cluster < 8 && rows * cluster < 2 * sms && packs >= 4 * kCeRowThreads * cluster) cluster *= 2;
+      per = (packs + cluster - 1) / cluster;
+      auto go = [&](auto tag) {
+        return launchCeRows<decltype(tag)::value>((bf16 *)logits, targets, loss, rows, V, gradScale, cluster, per, sms, stream);
+      };
+      if (per <= kCeRowThreads) return go(std::integral_constant<int, 1>());
+      if (per <= 2 * kCeRowThreads) return go(std::integral_constant<int, 2>());
+      if (per <= 4 * kCeRowThreads) return go(std::integral_constant<int, 4>());
+      if (per <= 8 * kCeRowThreads) return go(std::integral_constant<int, 8>());
+      if (per <= 10 * kCeRowThreads) return go(std::integral_constant<int, 10>());
+      if (per <= 13 * kCeRowThreads) return go(std::integral_constant<int, 13>());
+      return go(std::integral_constant<int, 16>());
+    }
+    per = (packs + 7) / 8;
+    if ((size_t)per * 16 <= (size_t)200 << 10) cluster = 8;
   }
-  static const bool forceStreaming = std::getenv("FLAGCX_OPS_CE_STREAMING") && atoi(std::getenv("FLAGCX_OPS_CE_STREAMING")) != 0;
-  if (!cluster || forceStreaming || rows * cluster > 0x7fffffffLL) {
+  if (!cluster || rows * cluster > 0x7fffffffLL) {
     crossEntropyFwdBwd<<<(unsigned)rows, 1024, 0, stream>>>((bf16 *)logits, targets, loss, V, gradScale);
     return cudaGetLastError();
   }

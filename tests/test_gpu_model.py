@@ -146,6 +146,31 @@ def test_cross_entropy_loss_and_gradient(T, V):
         assert rel < 1.2e-2
 
 
+# edges of what one CTA of a row holds (256 threads x 1, 2, 4, 8, 10, 13, 16 packs of 8, one to
+# eight CTAs per row), the last row size of the persistent kernel and the first of the next one,
+# and more rows than clusters run at once; a stretch of -inf (masked vocabulary) in every second row
+@pytest.mark.parametrize("T,V", [(1, 8), (3, 2048), (5, 2056), (2, 4104), (3, 8200), (2, 16392), (2, 20488), (3, 32768),
+                                 (2, 32776), (7, 65544), (2, 151936), (700, 128256), (2, 262144), (2, 262152)])
+def test_cross_entropy_at_the_edges_of_its_row_split(T, V):
+    ops = _ops()
+    g = torch.Generator(device="cuda").manual_seed(V)
+    logits = (torch.randn(T, V, generator=g, device="cuda") * 3).to(torch.bfloat16)
+    tgt = torch.randint(0, V // 2, (T,), generator=g, device="cuda")
+    tgt[0] = V - 1
+    logits[1::2, V // 2:] = float("-inf")
+    lp = logits.double().log_softmax(-1)
+    at = torch.arange(T, device="cuda")
+    want = -lp[at, tgt].mean()
+    d = lp.exp_()
+    d[at, tgt] -= 1
+    d /= T
+    loss = ops.cross_entropy_(logits, tgt)
+    assert abs(loss.double() - want) <= 1e-5 * want + 1e-5
+    # the exponential and the gradient are each rounded to bf16 (2^-9 of the value each), the
+    # fp32 exponential and the sum add less than 2^-15; at the target softmax and 1 cancel
+    assert bool(((logits.double() - d).abs() <= d.abs() * 2 ** -7 + 2 ** -15 / T * (d < 0)).all())
+
+
 def test_adamw_matches_torch():
     ops = _ops()
     torch.manual_seed(5)
