@@ -8,6 +8,8 @@
 // its own shared memory (the operand ring is free by then), and after one cluster barrier
 // every CTA adds up 1/S of the tile's rows out of the S shared memories (distributed shared
 // memory, fixed order 0..S-1: the result does not depend on timing) and stores it as bf16.
+// The same kernel takes the last, nearly empty wave of a large product (SplitGemmTail): the
+// persistent kernel stops after its full waves.
 // The partial sums never leave the chip, no workspace is needed, and no CTA waits for
 // another except at that barrier, which the hardware's cluster scheduling makes safe.
 #include <cuda_bf16.h>
@@ -53,7 +55,7 @@ __device__ __forceinline__ int ldClusterInt(uint32_t addr) {
 template <int BN>
 __global__ void __launch_bounds__(kThreads, 1)
     splitGemmKernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
-                    bf16 *__restrict__ D, int N, int kBlocks, int tilesM, int S) {
+                    bf16 *__restrict__ D, int N, int kBlocks, int tilesM, int S, const SplitGemmTail tail) {
   extern __shared__ uint8_t rawSmem[];
   using SmemT = Smem<BN>;
   constexpr int STAGES = SmemT::STAGES;
@@ -63,7 +65,15 @@ __global__ void __launch_bounds__(kThreads, 1)
   SmemT &s = *reinterpret_cast<SmemT *>((reinterpret_cast<uintptr_t>(rawSmem) + 1023) & ~(uintptr_t)1023);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int part = (int)clusterCtaRank(), tile = blockIdx.x / S;
-  const int tm = tile % tilesM, tn = tile / tilesM; // neighbours share the rows of B
+  int tm = tile % tilesM, tn = tile / tilesM; // neighbours share the rows of B
+  if (tail.count) {
+    // part q of one of the persistent kernel's tiles (its order: tileCoords in tp_gemm.cu)
+    const int down = tail.tileRows / BM, per = down * (256 / BN), t = tail.first + tile / per, q = tile % per;
+    const int wide = N / 256, g = t / (tail.groupRows * wide), wg = t - g * tail.groupRows * wide;
+    const int gsize = min(tail.groupRows, tilesM / down - g * tail.groupRows);
+    tm = (g * tail.groupRows + wg % gsize) * down + q % down;
+    tn = wg / gsize * (256 / BN) + q / down;
+  }
   const int kb0 = (int)((long)kBlocks * part / S), kb1 = (int)((long)kBlocks * (part + 1) / S);
 
   if (threadIdx.x == 0) {
@@ -170,7 +180,8 @@ __global__ void __launch_bounds__(kThreads, 1)
 }
 
 template <int BN>
-cudaError_t launch(cudaStream_t stream, const CUtensorMap &tmA, const CUtensorMap &tmB, void *D, int M, int N, int K, int S) {
+cudaError_t launch(cudaStream_t stream, const CUtensorMap &tmA, const CUtensorMap &tmB, void *D, int M, int N, int K, int S,
+                   const SplitGemmTail &tail) {
   static std::atomic<unsigned long long> ready{0}; // bit per device: the attribute belongs to the device's context
   const size_t smem = sizeof(Smem<BN>) + 1024;
   int dev = 0;
@@ -188,24 +199,25 @@ cudaError_t launch(cudaStream_t stream, const CUtensorMap &tmA, const CUtensorMa
   attr[0].val.clusterDim.y = 1;
   attr[0].val.clusterDim.z = 1;
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3((unsigned)((M / BM) * (N / BN) * S));
+  const int tiles = tail.count ? tail.count * (tail.tileRows / BM) * (256 / BN) : (M / BM) * (N / BN);
+  cfg.gridDim = dim3((unsigned)(tiles * S));
   cfg.blockDim = dim3(kThreads);
   cfg.dynamicSmemBytes = smem;
   cfg.stream = stream;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  return cudaLaunchKernelEx(&cfg, splitGemmKernel<BN>, tmA, tmB, (bf16 *)D, N, K / BK, M / BM, S);
+  return cudaLaunchKernelEx(&cfg, splitGemmKernel<BN>, tmA, tmB, (bf16 *)D, N, K / BK, M / BM, S, tail);
 }
 
 } // namespace
 
 cudaError_t launchSplitGemm(cudaStream_t stream, const CUtensorMap &tmA, const CUtensorMap &tmB, void *D, int M, int N, int K,
-                            const SplitGemmPlan &p) {
+                            const SplitGemmPlan &p, const SplitGemmTail &tail) {
   if (p.parts < 1 || p.parts > kSplitGemmMaxParts || p.parts > K / BK) return cudaErrorInvalidValue;
   switch (p.tileN) {
-    case 256: return launch<256>(stream, tmA, tmB, D, M, N, K, p.parts);
-    case 128: return launch<128>(stream, tmA, tmB, D, M, N, K, p.parts);
-    case 64: return launch<64>(stream, tmA, tmB, D, M, N, K, p.parts);
+    case 256: return launch<256>(stream, tmA, tmB, D, M, N, K, p.parts, tail);
+    case 128: return launch<128>(stream, tmA, tmB, D, M, N, K, p.parts, tail);
+    case 64: return launch<64>(stream, tmA, tmB, D, M, N, K, p.parts, tail);
     default: return cudaErrorInvalidValue;
   }
 }

@@ -204,7 +204,7 @@ __global__ void __launch_bounds__(kThreads, 1)
   const int unit = PAIR ? blockIdx.x / 2 : blockIdx.x, units = PAIR ? G / 2 : G;
   const int TM = PAIR ? 2 * BM : BM;
   const int tilesN = a.N / BN;
-  const int nTiles = (a.M / TM) * tilesN;
+  const int nTiles = a.tiles ? a.tiles : (a.M / TM) * tilesN;
   const int kBlocks = a.K / BK;
 
   if (!alive) {

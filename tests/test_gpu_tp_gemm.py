@@ -47,6 +47,22 @@ def test_gemm_with_k_split_over_a_cluster(M, N, K, parts, tile_n, monkeypatch):
     assert bool(((out.double() - ref).abs() <= bound).all())
 
 
+# full waves by the persistent kernel, the rest of the tiles by the split one: CTA pairs, single
+# CTAs, and row blocks that do not fill the tile order's last group
+@pytest.mark.parametrize("M,N,K", [(2048, 2816, 8192), (1408, 3584, 4096), (2816, 1792, 4096)])
+def test_gemm_whose_last_wave_is_nearly_empty(M, N, K):
+    from flagcx_b200.parallel.tp import gemm_bf16
+    g = torch.Generator(device="cuda").manual_seed(M + N + K)
+    a = torch.randn(M, K, generator=g, device="cuda").to(torch.bfloat16)
+    b = torch.randn(N, K, generator=g, device="cuda").to(torch.bfloat16)
+    out = torch.full((M, N), float("nan"), dtype=torch.bfloat16, device="cuda")
+    gemm_bf16(a, b, out)
+    ref = a.double() @ b.double().T
+    # the bound of the test above
+    bound = ref.abs() * 2 ** -8 + (a.double().abs() @ b.double().abs().T) * K * 2 ** -24
+    assert bool(((out.double() - ref).abs() <= bound).all())
+
+
 @pytest.mark.skipif(torch.cuda.device_count() < 2, reason="needs at least 2 GPUs")
 def test_fused_tensor_parallel_kernels_on_real_peers():
     n = 8 if torch.cuda.device_count() >= 8 else 4 if torch.cuda.device_count() >= 4 else 2
