@@ -283,6 +283,149 @@ rmsnormBwdPipelined(const bf16 *__restrict__ g, const bf16 *__restrict__ x, cons
   }
 }
 
+// The same where one row does not keep 512 threads busy (see rmsnormBackward for where the line
+// lies).  A CTA is cut into groups of GT threads, the fewest (a power of two from 32) that hold a row with four packs
+// per thread; every group owns a ring of row slots in shared memory, which its first thread
+// keeps full with bulk copies that complete on one mbarrier per slot, and reduces its rows by
+// itself: shuffles, and for GT > 32 one named barrier of the group.  So a CTA has 512 / GT rows
+// in work and as many or more on their way, and nothing waits for the whole block.  Bound: the
+// chain wait -> dot product -> sum -> store of each row.  With one row per CTA 8192 x 1024
+// took 39.2 us, 8192 x 256 37.0, 4096 x 2560 30.8, 2048 x 5120 32.9, 512 x 8192 20.5; in groups
+// they take 22.9, 12.4, 24.7, 23.0 and 16.5.
+constexpr int kNormThreads = 512, kNormMaxStages = 6, kNormPacks = 4;
+
+// Sum over a group of GT threads; every thread gets it.  red holds one float per warp of the
+// CTA, alternately the first and the second 16 (parity), so that one barrier per sum is enough:
+// a half is written again only after the next sum's barrier, which follows its last read.
+template <int GT>
+__device__ __forceinline__ float groupSum(float v, float (*red)[kNormThreads / 32], int parity, int group) {
+  v = warpSum(v);
+  if constexpr (GT > 32) {
+    constexpr int W = GT / 32;
+    const int warp = threadIdx.x >> 5;
+    if ((threadIdx.x & 31) == 0) red[parity][warp] = v;
+    asm volatile("bar.sync %0, %1;" ::"r"(group + 1), "n"(GT) : "memory");
+    v = 0.f;
+#pragma unroll
+    for (int i = 0; i < W; ++i) v += red[parity][group * W + i];
+  } else {
+    __syncwarp();
+  }
+  return v;
+}
+
+// The weight gradient is summed in fp32 per group (a thread owns the same columns for all of
+// its rows), then over the CTA's groups in their order, then over CTAs by columnSumToBf16.
+template <int GT, int PPT>
+__global__ void __launch_bounds__(kNormThreads)
+rmsnormBwdRing(const bf16 *__restrict__ g, const bf16 *__restrict__ x, const bf16 *__restrict__ w,
+               const float *__restrict__ rstdIn, const bf16 *__restrict__ addIn, bf16 *__restrict__ dx,
+               float *__restrict__ dwPartial, long rows, int H, int stages) {
+  extern __shared__ __align__(128) unsigned char ring[];
+  constexpr int G = kNormThreads / GT;
+  __shared__ float red[2][kNormThreads / 32];
+  __shared__ __align__(8) uint64_t full[G * kNormMaxStages];
+  const int group = threadIdx.x / GT, t = threadIdx.x % GT;
+  const int nPacks = H / 8;
+  const uint32_t rowBytes = (uint32_t)H * 2u;
+  // a slot holds the g row, the x row and, when a gradient of the same shape is to be added
+  // to dx (the residual branch around the norm), that gradient's row
+  const uint32_t slotBytes = (addIn ? 3u : 2u) * rowBytes;
+  unsigned char *slots = ring + (size_t)group * stages * slotBytes;
+  uint64_t *bars = full + group * kNormMaxStages;
+  const long first = (long)blockIdx.x * G + group, step = (long)gridDim.x * G;
+  auto issue = [&](long k) { // the group's first thread: row k of the group into slot k % stages
+    const long row = first + k * step;
+    if (row >= rows) return;
+    const int s = (int)(k % stages);
+    unsigned char *dst = slots + (size_t)s * slotBytes;
+    mbarExpect(&bars[s], slotBytes);
+    bulkLoad(dst, g + (size_t)row * H, rowBytes, &bars[s]);
+    bulkLoad(dst + rowBytes, x + (size_t)row * H, rowBytes, &bars[s]);
+    if (addIn) bulkLoad(dst + 2 * rowBytes, addIn + (size_t)row * H, rowBytes, &bars[s]);
+  };
+  if (t == 0) {
+    for (int s = 0; s < stages; ++s) mbarInit(&bars[s]);
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    for (int k = 0; k < stages; ++k) issue(k);
+  }
+  __syncthreads();
+  float dwAcc[PPT][8];
+  Pack8 pw[PPT];
+#pragma unroll
+  for (int k = 0; k < PPT; ++k) {
+    const int p = t + k * GT;
+    if (p < nPacks) pw[k].raw = ((const uint4 *)w)[p];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) dwAcc[k][i] = 0.f;
+  }
+  // A wait that ran out marks the group's part of the weight gradient as NaN.
+  bool ok = true;
+  int it = 0;
+  for (long row = first; row < rows; row += step, ++it) {
+    const int s = it % stages;
+    const float rstd = rstdIn[row];
+    if (ok) ok = mbarWaitBounded(&bars[s], (uint32_t)(it / stages) & 1u);
+    const uint4 *gs = (const uint4 *)(slots + (size_t)s * slotBytes), *xs = gs + nPacks, *as = xs + nPacks;
+    Pack8 pg[PPT], px[PPT], pa[PPT];
+    float dot = 0.f;
+#pragma unroll
+    for (int k = 0; k < PPT; ++k) {
+      const int p = t + k * GT;
+      if (p < nPacks) {
+        pg[k].raw = gs[p];
+        px[k].raw = xs[p];
+        if (addIn) pa[k].raw = as[p];
+#pragma unroll
+        for (int i = 0; i < 8; ++i) dot += pg[k].get(i) * pw[k].get(i) * px[k].get(i);
+      }
+    }
+    dot = groupSum<GT>(dot, red, it & 1, group); // the whole group has read the slot
+    if (t == 0 && ok) issue(it + stages);
+    const float c = dot * rstd * rstd / H;
+    uint4 *dxr = (uint4 *)(dx + (size_t)row * H);
+#pragma unroll
+    for (int k = 0; k < PPT; ++k) {
+      const int p = t + k * GT;
+      if (p < nPacks) {
+        Pack8 po;
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+          const float gv = pg[k].get(i), xv = px[k].get(i);
+          float d = rstd * (gv * pw[k].get(i) - xv * c);
+          if (addIn) d += pa[k].get(i);
+          po.set(i, d);
+          dwAcc[k][i] += gv * xv * rstd;
+        }
+        dxr[p] = po.raw;
+      }
+    }
+  }
+  // The groups' sums meet in the ring (all copies have landed and been read), a group's sums in
+  // its own slots: G x H floats fit since a slot holds at least two rows of 16 bits.
+  const float bad = ok ? 0.f : NAN;
+  float *mine = (float *)ring + (size_t)group * H;
+  __syncthreads();
+#pragma unroll
+  for (int k = 0; k < PPT; ++k) {
+    const int p = t + k * GT;
+    if (p < nPacks) {
+      *(float4 *)(mine + p * 8) = make_float4(dwAcc[k][0] + bad, dwAcc[k][1] + bad, dwAcc[k][2] + bad, dwAcc[k][3] + bad);
+      *(float4 *)(mine + p * 8 + 4) = make_float4(dwAcc[k][4] + bad, dwAcc[k][5] + bad, dwAcc[k][6] + bad, dwAcc[k][7] + bad);
+    }
+  }
+  __syncthreads();
+  float *out = dwPartial + (size_t)blockIdx.x * H;
+  for (int c = threadIdx.x; c < H / 4; c += kNormThreads) {
+    float4 sum = ((const float4 *)ring)[c];
+    for (int q = 1; q < G; ++q) {
+      const float4 v = ((const float4 *)((const float *)ring + (size_t)q * H))[c];
+      sum.x += v.x; sum.y += v.y; sum.z += v.z; sum.w += v.w;
+    }
+    ((float4 *)out)[c] = sum;
+  }
+}
+
 // dw[c] = sum over the CTAs' partials, in a fixed order, rounded to bf16 once.
 // Block (32, 32): 32 neighbouring columns, 32 lanes over the rows.
 __global__ void columnSumToBf16(const float *__restrict__ partial, bf16 *__restrict__ dw, int R, int H) {
@@ -771,6 +914,25 @@ int gridFor(size_t items, int threads, int sms, int perSm = 8) {
     if (err_ != cudaSuccess) return err_;   \
   } while (0)
 
+// Calls f(GT, PPT) for rows of `packs` packs of 8: the smallest group whose threads hold a row
+// with at most four packs each (512 threads and four packs: 16384 elements).
+template <typename F>
+cudaError_t withNormShape(int packs, F &&f) {
+  auto ppt = [&](auto gt) -> cudaError_t {
+    constexpr int GT = decltype(gt)::value;
+    const int n = (packs + GT - 1) / GT;
+    if (n <= 1) return f(gt, std::integral_constant<int, 1>());
+    if (n <= 2) return f(gt, std::integral_constant<int, 2>());
+    if (n <= 3) return f(gt, std::integral_constant<int, 3>());
+    return f(gt, std::integral_constant<int, 4>());
+  };
+  if (packs <= 32 * kNormPacks) return ppt(std::integral_constant<int, 32>());
+  if (packs <= 64 * kNormPacks) return ppt(std::integral_constant<int, 64>());
+  if (packs <= 128 * kNormPacks) return ppt(std::integral_constant<int, 128>());
+  if (packs <= 256 * kNormPacks) return ppt(std::integral_constant<int, 256>());
+  return ppt(std::integral_constant<int, 512>());
+}
+
 template <int PPT>
 cudaError_t launchCeRows(bf16 *logits, const long *targets, float *loss, long rows, int V, float gradScale, int C, int per,
                          int sms, cudaStream_t stream) {
@@ -835,28 +997,57 @@ cudaError_t rmsnormForward(const void *x, const void *w, void *y, float *rstd, l
   return cudaGetLastError();
 }
 
-int rmsnormPartials(long rows, int H, int sms) { return (int)std::max<long>(1, std::min<long>(rows, sms * 2)); }
+// One CTA of 512 threads per row where a row fills them (one or two packs per thread, 0.9 of the
+// threads with work) and a third tensor is added: its two CTAs per SM need fewer registers (4096
+// x 4096 33.6 us against 35.4 in groups, 16384 x 4096 100.1 against 104.4).  Groups elsewhere
+// (without the third tensor 16384 x 4096 takes 90.4 us in groups against 96.3).
+static bool rowPerCta(int H, bool add) {
+  const int packs = H / 8, perThread = (packs + kNormBwdThreads - 1) / kNormBwdThreads;
+  return add && perThread <= 2 && packs * 10 > 9 * perThread * kNormBwdThreads;
+}
+
+int rmsnormPartials(long rows, int H, bool add, int sms) {
+  if (rowPerCta(H, add)) return (int)std::max<long>(1, std::min<long>(rows, sms * 2));
+  int ctas = 0;
+  withNormShape(H / 8, [&](auto gt, auto) {
+    constexpr int G = kNormThreads / decltype(gt)::value;
+    ctas = (int)std::max<long>(1, std::min<long>((rows + G - 1) / G, sms));
+    return cudaSuccess;
+  });
+  return ctas;
+}
 
 cudaError_t rmsnormBackward(const void *g, const void *x, const void *w, const float *rstd, const void *add, void *dx, void *dw,
                             float *partial, long rows, int H, int sms, cudaStream_t stream) {
-  const int ctas = rmsnormPartials(rows, H, sms);
-  const int packs = H / 8;
-  const int maxp = (packs + kNormBwdThreads - 1) / kNormBwdThreads;
-  // ring of (g row, x row) slots: about 96 KiB per CTA so that two CTAs share an SM
-  const size_t slot = (size_t)H * (add ? 6 : 4);
-  const int stages = (int)std::max<size_t>(2, std::min<size_t>(kNormBwdMaxStages, ((size_t)96 << 10) / slot));
-  const size_t smem = slot * stages;
-  auto launch = [&](auto tag) {
-    auto kern = rmsnormBwdPipelined<decltype(tag)::value>;
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return e;
-    kern<<<ctas, kNormBwdThreads, smem, stream>>>((const bf16 *)g, (const bf16 *)x, (const bf16 *)w, rstd, (const bf16 *)add,
-                                                  (bf16 *)dx, partial, (int)rows, H, stages);
-    return cudaGetLastError();
-  };
-  if (maxp <= 1) RETURN_IF(launch(std::integral_constant<int, 1>()));
-  else if (maxp <= 2) RETURN_IF(launch(std::integral_constant<int, 2>()));
-  else RETURN_IF(launch(std::integral_constant<int, 4>()));
+  const int ctas = rmsnormPartials(rows, H, add != nullptr, sms);
+  if (rowPerCta(H, add != nullptr)) {
+    // ring of (g, x, add) slots: about 96 KiB per CTA so that two CTAs share an SM
+    const size_t slot = (size_t)H * 6;
+    const int stages = (int)std::max<size_t>(2, std::min<size_t>(kNormBwdMaxStages, ((size_t)96 << 10) / slot));
+    const size_t smem = slot * stages;
+    auto launch = [&](auto tag) {
+      auto kern = rmsnormBwdPipelined<decltype(tag)::value>;
+      RETURN_IF(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+      kern<<<ctas, kNormBwdThreads, smem, stream>>>((const bf16 *)g, (const bf16 *)x, (const bf16 *)w, rstd, (const bf16 *)add,
+                                                    (bf16 *)dx, partial, (int)rows, H, stages);
+      return cudaGetLastError();
+    };
+    if (H / 8 <= kNormBwdThreads) RETURN_IF(launch(std::integral_constant<int, 1>()));
+    else RETURN_IF(launch(std::integral_constant<int, 2>()));
+  } else {
+    RETURN_IF(withNormShape(H / 8, [&](auto gt, auto ppt) {
+      constexpr int GT = decltype(gt)::value, PPT = decltype(ppt)::value, G = kNormThreads / GT;
+      // slots of all groups, about 200 KiB: one CTA per SM
+      const size_t slots = (size_t)H * (add ? 6 : 4) * G;
+      const int stages = (int)std::max<size_t>(1, std::min<size_t>(kNormMaxStages, ((size_t)200 << 10) / slots));
+      const size_t smem = slots * stages;
+      auto kern = rmsnormBwdRing<GT, PPT>;
+      RETURN_IF(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+      kern<<<ctas, kNormThreads, smem, stream>>>((const bf16 *)g, (const bf16 *)x, (const bf16 *)w, rstd, (const bf16 *)add,
+                                                 (bf16 *)dx, partial, rows, H, stages);
+      return cudaGetLastError();
+    }));
+  }
   columnSumToBf16<<<(H + 31) / 32, dim3(32, 32), 0, stream>>>(partial, (bf16 *)dw, ctas, H);
   return cudaGetLastError();
 }

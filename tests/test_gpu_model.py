@@ -34,6 +34,34 @@ def test_rmsnorm_forward_backward():
         assert ((w.grad.float() - wf.grad).abs() / wf.grad.abs().clamp(min=1)).max() < 0.05, (rows, H)
 
 
+# every group size of the backward (32 to 512 threads, one to four packs each), the line where one
+# row per CTA takes over (0.9 of 512 threads), a single row, and rows that the groups share unevenly
+@pytest.mark.parametrize("rows,H", [(1, 8), (17, 256), (5, 1024), (33, 1032), (300, 2048), (7, 2056), (149, 3688), (149, 3680),
+                                    (9, 4104), (200, 7176), (3, 8200), (5, 12296), (2, 16384), (2500, 264)])
+@pytest.mark.parametrize("skip", [True, False])
+def test_rmsnorm_backward_at_the_edges_of_its_row_groups(rows, H, skip):
+    ops = _ops()
+    gen = torch.Generator(device="cuda").manual_seed(rows + H)
+    x, g, gs = [torch.randn(rows, H, generator=gen, device="cuda").to(torch.bfloat16) for _ in range(3)]
+    w = (1 + 0.1 * torch.randn(H, generator=gen, device="cuda")).to(torch.bfloat16)
+    x.requires_grad_()
+    w.requires_grad_()
+    if skip:
+        dx, dw = torch.autograd.grad(ops.rmsnorm_branch(x, w, 1e-5), (x, w), (g, gs))
+    else:
+        dx, dw = torch.autograd.grad(ops.rmsnorm(x, w, 1e-5), (x, w), g)
+    xd, wd, gd = x.detach().double().requires_grad_(), w.detach().double().requires_grad_(), g.double()
+    xhat = xd * torch.rsqrt(xd.square().mean(-1, keepdim=True) + 1e-5)
+    rdx, rdw = torch.autograd.grad(xhat * wd, (xd, wd), gd)
+    if skip:
+        rdx = rdx + gs.double()
+    # one rounding to bf16; the fp32 terms before it are a few and at most |g w| + |x| + |skip| large
+    scale = (gd * wd).abs() + xd.abs() + gs.double().abs()
+    assert bool(((dx.double() - rdx).abs() <= rdx.abs() * 2 ** -8 + scale.detach() * 2 ** -18).all())
+    terms = (gd * xhat).abs().sum(0).detach()
+    assert bool(((dw.double() - rdw).abs() <= rdw.abs() * 2 ** -8 + terms * 2 ** -16).all())
+
+
 def test_rope_matches_reference_and_backward_is_inverse():
     ops = _ops()
     T, Hn, D = 64, 4, 128
