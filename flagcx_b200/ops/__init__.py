@@ -10,11 +10,12 @@ import importlib.util
 import os
 
 import torch
+import torch.autograd.forward_ad as _forward_ad
 
 from . import build as _build
 
 _ext = None
-launch_count = 0  # kernels launched through this module (bench.py reports it)
+_launches = 0  # see __getattr__ at the end of this file
 # When the loss is only ever differentiated with gradient 1 (loss.backward()), the
 # cross-entropy backward can hand out the stored gradient without another pass.
 assume_unit_loss_grad = False
@@ -36,8 +37,16 @@ def ext():
 
 
 def _count(n=1):
-    global launch_count
-    launch_count += n
+    global _launches
+    _launches += n
+
+
+def _in_python():
+    """Whether an operator has to go through its torch.autograd.Function below: a tracer records
+    that as a call, and function transforms and forward-mode differentiation refuse it with their
+    own errors.  Otherwise the same function in C++ (torch_ops.cpp) is used."""
+    return (torch._C._get_tracing_state() is not None or torch._C._are_functorch_transforms_active()
+            or _forward_ad._current_level >= 0)
 
 
 class _RMSNorm(torch.autograd.Function):
@@ -57,7 +66,9 @@ class _RMSNorm(torch.autograd.Function):
 
 
 def rmsnorm(x: torch.Tensor, weight: torch.Tensor, eps: float = 1e-5) -> torch.Tensor:
-    return _RMSNorm.apply(x.contiguous(), weight, eps)
+    if _in_python():
+        return _RMSNorm.apply(x.contiguous(), weight, eps)
+    return ext().rmsnorm(x, weight, eps)
 
 
 class _RMSNormBranch(torch.autograd.Function):
@@ -86,7 +97,9 @@ class _RMSNormBranch(torch.autograd.Function):
 
 def rmsnorm_branch(x: torch.Tensor, weight: torch.Tensor, eps: float = 1e-5):
     """(rmsnorm(x), x): see _RMSNormBranch.  Use the second value for the residual add."""
-    return _RMSNormBranch.apply(x.contiguous(), weight, eps)
+    if _in_python():
+        return _RMSNormBranch.apply(x.contiguous(), weight, eps)
+    return ext().rmsnorm_branch(x, weight, eps)
 
 
 class _Rope(torch.autograd.Function):
@@ -130,7 +143,9 @@ def rope_fused_qkv(qkv: torch.Tensor, n_heads: int, n_kv_heads: int, head_dim: i
     (queries, keys, values side by side).  Rotates the query and key heads (token t at
     position t) and copies the value heads, in one pass; q, k and v are then views of the
     result and no per-tensor copy is needed before attention."""
-    return _RopeFusedQkv.apply(qkv.contiguous(), n_heads + n_kv_heads, n_heads + 2 * n_kv_heads, head_dim, theta)
+    if _in_python():
+        return _RopeFusedQkv.apply(qkv.contiguous(), n_heads + n_kv_heads, n_heads + 2 * n_kv_heads, head_dim, theta)
+    return ext().rope_qkv(qkv, n_heads + n_kv_heads, n_heads + 2 * n_kv_heads, head_dim, theta)
 
 
 class _SwiGLU(torch.autograd.Function):
@@ -150,7 +165,9 @@ class _SwiGLU(torch.autograd.Function):
 
 def swiglu(ab: torch.Tensor) -> torch.Tensor:
     """ab = [a | b] along the last dimension; returns silu(a) * b."""
-    return _SwiGLU.apply(ab)
+    if _in_python():
+        return _SwiGLU.apply(ab)
+    return ext().swiglu(ab)
 
 
 def _mm_residual(x, w, residual):
@@ -247,3 +264,11 @@ def cross_entropy_(logits: torch.Tensor, targets: torch.Tensor) -> torch.Tensor:
 def adamw_flat_(p, g, m, v, lr, beta1, beta2, eps, weight_decay, step) -> None:
     ext().adamw_flat_(p, g, m, v, lr, beta1, beta2, eps, weight_decay, step)
     _count()
+
+
+def __getattr__(name):
+    """`launch_count` (read only): kernels launched through this module, from Python and from C++
+    (bench.py reports it)."""
+    if name == "launch_count":
+        return _launches + (_ext.launch_count() if _ext is not None else 0)
+    raise AttributeError(f"module {__name__!r} has no attribute {name!r}")

@@ -62,6 +62,28 @@ def test_rmsnorm_backward_at_the_edges_of_its_row_groups(rows, H, skip):
     assert bool(((dw.double() - rdw).abs() <= rdw.abs() * 2 ** -8 + terms * 2 ** -16).all())
 
 
+def test_operators_keep_hooks_tracing_and_transforms():
+    """The operators run as C++ autograd functions, except under a tracer, a function transform or
+    forward-mode differentiation."""
+    ops = _ops()
+    x = torch.randn(5, 256, device="cuda").to(torch.bfloat16).requires_grad_()
+    w, g = torch.ones_like(x[0]).requires_grad_(), torch.randn_like(x)
+    before = ops.launch_count
+    plain = torch.autograd.grad(ops.rmsnorm(x, w), (x, w), g)
+    assert ops.launch_count - before == 2
+    saved = []
+    with torch.autograd.graph.saved_tensors_hooks(lambda t: (saved.append(1), t.cpu())[1], lambda t: t.cuda()):
+        y = ops.rmsnorm(x, w)
+    assert len(saved) == 3 and all(torch.equal(a, b) for a, b in zip(plain, torch.autograd.grad(y, (x, w), g)))
+    other = torch.randn_like(g)
+    traced = torch.jit.trace(lambda t: ops.swiglu(t), (g,), check_trace=False)
+    assert torch.equal(traced(other), ops.swiglu(other))
+    with pytest.raises(RuntimeError, match="functorch transforms"):
+        torch.vmap(ops.swiglu)(g[None])
+    with torch.autograd.forward_ad.dual_level(), pytest.raises(NotImplementedError):
+        ops.swiglu(torch.autograd.forward_ad.make_dual(g, other))
+
+
 def test_rope_matches_reference_and_backward_is_inverse():
     ops = _ops()
     T, Hn, D = 64, 4, 128
