@@ -30,18 +30,33 @@ namespace {
 // registers for them; the host launches twice as many CTAs as it would of the 512-thread kind.
 constexpr int kMoeThreads = 256;
 
-// One warp copies one row (H bf16) with 16-byte accesses, four loads in flight per lane.
-__device__ __forceinline__ void warpCopyRow(char *dst, const char *src, int vecs, int lane, bool srcIsPeerWritten) {
+// One warp copies one row (H bf16) to every non-null destination.  The row is read once, eight
+// 16-byte loads in flight per lane, and each piece goes to all destinations: a token's row was
+// read again for every rank it went to (and every local copy re-read the leader row), with four
+// loads in flight, which with 8 warps per SM is 16 KiB of the 35 that latency asks for.  Eight
+// emulated ranks, 512 tokens x 7168, top 8 of 256: dispatch 225 -> 209 us; with two vectors of
+// every row in flight in the pulling combine 189 -> 163.
+__device__ __forceinline__ void warpCopyRow(char *const (&dst)[FLAGCX_MOE_MAX_TOPK], const char *src, int vecs, int lane,
+                                            bool srcIsPeerWritten) {
+  constexpr int U = 8;
   const uint4 *s = (const uint4 *)src;
-  uint4 *d = (uint4 *)dst;
-  int v = lane;
-  for (; v + 96 < vecs; v += 128) {
-    uint4 r0, r1, r2, r3;
-    if (srcIsPeerWritten) { r0 = ldSys16(s + v); r1 = ldSys16(s + v + 32); r2 = ldSys16(s + v + 64); r3 = ldSys16(s + v + 96); }
-    else { r0 = s[v]; r1 = s[v + 32]; r2 = s[v + 64]; r3 = s[v + 96]; }
-    st16(d + v, r0); st16(d + v + 32, r1); st16(d + v + 64, r2); st16(d + v + 96, r3);
+  for (int v0 = lane; v0 < vecs; v0 += 32 * U) {
+    uint4 r[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const int v = v0 + 32 * u;
+      if (v < vecs) r[u] = srcIsPeerWritten ? ldSys16(s + v) : s[v];
+    }
+#pragma unroll
+    for (int k = 0; k < FLAGCX_MOE_MAX_TOPK; ++k)
+      if (dst[k]) {
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+          const int v = v0 + 32 * u;
+          if (v < vecs) st16((uint4 *)dst[k] + v, r[u]);
+        }
+      }
   }
-  for (; v < vecs; v += 32) st16(d + v, srcIsPeerWritten ? ldSys16(s + v) : s[v]);
 }
 
 // A group record (FLAGCX_MOE_MAX_TOPK ints written by a peer) as two 16-byte loads.
@@ -227,12 +242,14 @@ __device__ void dispatchBody(const flagcxDevComm &c, const MoeArgs &a) {
       if (isFirst)
         for (int j = groupSize; j < FLAGCX_MOE_MAX_TOPK; ++j) rec[j] = -1;
     }
-    const char *src = (const char *)(a.x + (size_t)tok * a.H);
-    for (int k = 0; k < a.K; ++k) {
+    char *dst[FLAGCX_MOE_MAX_TOPK];
+#pragma unroll
+    for (int k = 0; k < FLAGCX_MOE_MAX_TOPK; ++k) { // lanes from K on hold no pair
       const int dk = __shfl_sync(0xffffffffu, d, k), rowk = __shfl_sync(0xffffffffu, row, k);
       const bool fk = __shfl_sync(0xffffffffu, isFirst ? 1 : 0, k) != 0;
-      if (fk) warpCopyRow(a.recv[dk] + (size_t)rowk * rowBytes, src, vecs, lane, false);
+      dst[k] = fk ? a.recv[dk] + (size_t)rowk * rowBytes : nullptr;
     }
+    warpCopyRow(dst, (const char *)(a.x + (size_t)tok * a.H), vecs, lane, false);
   }
   __syncthreads();
   if (t < n) a.grpCount[t][(size_t)rank * FLAGCX_COLL_BARRIER_SLOTS + b] = grpN[t] < capPer ? grpN[t] : capPer;
@@ -245,10 +262,12 @@ __device__ void dispatchBody(const flagcxDevComm &c, const MoeArgs &a) {
       int rows[FLAGCX_MOE_MAX_TOPK];
       loadGroup(recs + (size_t)r * FLAGCX_MOE_MAX_TOPK, rows);
       if ((size_t)rows[0] >= a.capacity) continue;
+      char *dst[FLAGCX_MOE_MAX_TOPK];
+      dst[0] = nullptr;
 #pragma unroll
       for (int j = 1; j < FLAGCX_MOE_MAX_TOPK; ++j)
-        if (rows[j] >= 0 && (size_t)rows[j] < a.capacity)
-          warpCopyRow(a.recv[rank] + (size_t)rows[j] * rowBytes, a.recv[rank] + (size_t)rows[0] * rowBytes, vecs, lane, true);
+        dst[j] = rows[j] >= 0 && (size_t)rows[j] < a.capacity ? a.recv[rank] + (size_t)rows[j] * rowBytes : nullptr;
+      if (rows[1] >= 0) warpCopyRow(dst, a.recv[rank] + (size_t)rows[0] * rowBytes, vecs, lane, true); // packed: none after -1
     }
   }
 }
@@ -281,24 +300,37 @@ __device__ void combinePullBody(const flagcxDevComm &c, const MoeArgs &a) {
       }
     }
     uint4 *dst = (uint4 *)(a.out + (size_t)tok * a.H);
-    for (int v = lane; v < vecs; v += 32) {
-      uint4 r[FLAGCX_MOE_MAX_TOPK];
+    constexpr int U = 2; // vectors of every row in flight per lane
+    for (int v0 = lane; v0 < vecs; v0 += 32 * U) {
+      uint4 r[U][FLAGCX_MOE_MAX_TOPK];
 #pragma unroll
-      for (int k = 0; k < FLAGCX_MOE_MAX_TOPK; ++k)
-        if (rows[k]) r[k] = ldSys16(rows[k] + (size_t)v * 16);
-      float acc[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+      for (int u = 0; u < U; ++u) {
+        const int v = v0 + 32 * u;
+        if (v < vecs) {
 #pragma unroll
-      for (int k = 0; k < FLAGCX_MOE_MAX_TOPK; ++k)
-        if (rows[k]) {
-          const __nv_bfloat16 *e = (const __nv_bfloat16 *)&r[k];
-#pragma unroll
-          for (int j = 0; j < 8; ++j) acc[j] += w[k] * __bfloat162float(e[j]);
+          for (int k = 0; k < FLAGCX_MOE_MAX_TOPK; ++k)
+            if (rows[k]) r[u][k] = ldSys16(rows[k] + (size_t)v * 16);
         }
-      uint4 o;
-      __nv_bfloat16 *oe = (__nv_bfloat16 *)&o;
+      }
 #pragma unroll
-      for (int j = 0; j < 8; ++j) oe[j] = __float2bfloat16_rn(acc[j]);
-      dst[v] = o;
+      for (int u = 0; u < U; ++u) {
+        const int v = v0 + 32 * u;
+        if (v < vecs) {
+          float acc[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+#pragma unroll
+          for (int k = 0; k < FLAGCX_MOE_MAX_TOPK; ++k)
+            if (rows[k]) {
+              const __nv_bfloat16 *e = (const __nv_bfloat16 *)&r[u][k];
+#pragma unroll
+              for (int j = 0; j < 8; ++j) acc[j] += w[k] * __bfloat162float(e[j]);
+            }
+          uint4 o;
+          __nv_bfloat16 *oe = (__nv_bfloat16 *)&o;
+#pragma unroll
+          for (int j = 0; j < 8; ++j) oe[j] = __float2bfloat16_rn(acc[j]);
+          dst[v] = o;
+        }
+      }
     }
   }
   ctaBarrier(c, b); // peers may overwrite their expert outputs only after everyone has read them
