@@ -949,7 +949,8 @@ cudaError_t launchCeRows(bf16 *logits, const long *targets, float *loss, long ro
   cfg.stream = stream;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  RETURN_IF(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+  if (smem > (47 << 10)) // beyond what a kernel gets without asking
+    RETURN_IF(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
   // As many clusters as run at once: rows are dealt out evenly, so a second wave would be waste.
   long clusters = rows;
   if (rows * C > sms) {
