@@ -5,9 +5,9 @@
 #include <map>
 
 #include "../kernels/launch.h"
-#include "../kernels/split_gemm.h"
 #include "../kernels/tp_gemm_args.h"
 #include "comm.h"
+#include "gemm_plan.h"
 #include "flagcx_ext.h"
 
 namespace fcx {
@@ -44,79 +44,6 @@ int smCount() {
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   return sms > 0 ? sms : 1;
-}
-
-// Estimates for split_gemm.cu: fixed cost and cost of a K step (us) by tile width, and how many
-// CTAs run at once by cluster size.
-struct { int tileN; double fixedUs, stepUs; } const kSplitKinds[] = {{256, 11.5, 0.384}, {128, 10.3, 0.27}, {64, 8.7, 0.2875}};
-struct { int parts, ctas; } const kSplits[] = {{8, 112}, {4, 132}, {2, 148}, {1, 148}};
-
-// Which kernel takes a plain product: the persistent one (tileN = 0), or K split over clusters
-// of S CTAs that own 128 x tileN tiles.  The split pays while the persistent kernel's 128 x 256
-// tiles leave most SMs idle (back-to-back calls, operands not in L2, us: 128 x 3584 x 8192
-// 54.6 -> 20.2, 256 x 3584 x 8192 45.2 -> 25.1, 128 x 256 x 8192 47.7 -> 12.4, 512 x 3584 x
-// 8192 45.5 -> 36.8); from about 64 tiles on the persistent kernel's CTA pairs and overlapped
-// epilogues win (1024 x 3584 x 8192: 53 against 68 us).  Below that the smallest of the
-// estimates decides: a fixed cost plus the largest of one CTA's K steps, the operands out of
-// HBM (6.4 TB/s) and what all CTAs together pull out of L2 (13 TB/s); the figures are fitted to
-// 26 shapes from 128 x 256 x 4096 to 1024 x 1280 x 8192 and within 2 us of all of them.
-// Clusters stay within what is co-resident (33 of 4 CTAs, 14 of 8): a second wave costs more
-// than the split gains (28 clusters of 5: 37 us against 27).
-SplitGemmPlan splitPlan(int M, int N, int K, bool pair) {
-  SplitGemmPlan best;
-  const int kb = K / 64;
-  const int forced = (int)readParam("GEMM_SPLIT", 0);
-  if (forced == 1) return best;
-  if (forced > 1 && forced <= kSplitGemmMaxParts && forced <= kb) {
-    best.parts = forced;
-    best.tileN = (int)readParam("GEMM_SPLIT_N", 256);
-    return best;
-  }
-  const long tiles256 = (long)(M / 128) * (N / 256);
-  if (tiles256 > 64 || kb < 4) return best;
-  const double hbmUs = ((double)M + N) * K * 2 / 6.4e6;
-  double bestUs = pair ? 7.2 + kb * 0.33 : 8.5 + kb * 0.38;
-  for (auto &k : kSplitKinds) {
-    const long tiles = tiles256 * (256 / k.tileN);
-    for (auto &sp : kSplits) {
-      if (tiles * sp.parts > sp.ctas || sp.parts * 4 > kb) continue;
-      const double steps = (kb + sp.parts - 1) / sp.parts * k.stepUs;
-      const double bytes = (double)tiles * kb * (128 + k.tileN) * 128;
-      const double us = k.fixedUs + std::max({steps, hbmUs, bytes / 13e6});
-      if (us < bestUs) {
-        bestUs = us;
-        best.tileN = k.tileN;
-        best.parts = sp.parts;
-      }
-    }
-  }
-  return best;
-}
-
-// The tiles of the persistent kernel's last wave, where handing them to the split kernel (parts
-// CTAs per tile) is quicker than a wave of whole tiles in which most SMs are idle.  8192 x 3584
-// x 8192 is 6 waves of 74 CTA pairs and 4 tiles: 336 -> 325 us; 2048 x 5120 x 4096 119 -> 86,
-// 1408 x 3584 x 8192 99 -> 76.  3 us are asked for as margin (the second launch; 2304 x 2560 x
-// 3072 lost 2 %), and beyond 9 waves the last one no longer counts.
-SplitGemmTail tailPlan(int M, int N, int K, bool pair, int units, SplitGemmPlan *plan) {
-  SplitGemmTail t;
-  const int kb = K / 64, tiles = (M / (pair ? 256 : 128)) * (N / 256), rest = tiles % units;
-  if (tiles <= units || tiles > 9 * units || rest == 0 || readParam("GEMM_SPLIT", 0) == 1) return t;
-  const int parts128 = rest * (pair ? 2 : 1);
-  for (auto &sp : kSplits) {
-    if (sp.parts < 2 || parts128 * sp.parts > sp.ctas || sp.parts * 4 > kb) continue;
-    const double steps = (kb + sp.parts - 1) / sp.parts * kSplitKinds[0].stepUs;
-    const double bytes = (double)parts128 * kb * (128 + 256) * 128;
-    if (kSplitKinds[0].fixedUs + std::max(steps, bytes / 13e6) + 3.0 > kb * 0.38) break;
-    plan->tileN = 256;
-    plan->parts = sp.parts;
-    t.first = tiles - rest;
-    t.count = rest;
-    t.tileRows = pair ? 256 : 128;
-    t.groupRows = groupRows(pair);
-    break;
-  }
-  return t;
 }
 
 flagcxResult_t checkShape(int M, int N, int K) {
@@ -172,7 +99,8 @@ flagcxResult_t flagcxGemmBf16(const void *A, const void *B, void *D, int M, int 
   CUtensorMap ta, tb;
   FCXCHECK(cu::tensorMap2dBf16(&ta, A, M, K, 128, 64));
   const bool pair = usePair(M);
-  SplitGemmPlan plan = splitPlan(M, N, K, pair);
+  const int forced = (int)readParam("GEMM_SPLIT", 0);
+  SplitGemmPlan plan = splitPlan(M, N, K, pair, forced, (int)readParam("GEMM_SPLIT_N", 256));
   if (plan.tileN) {
     FCXCHECK(cu::tensorMap2dBf16(&tb, B, N, K, plan.tileN, 64));
     cudaError_t e = launchSplitGemm(stream ? stream->base : nullptr, ta, tb, D, M, N, K, plan);
@@ -194,7 +122,8 @@ flagcxResult_t flagcxGemmBf16(const void *A, const void *B, void *D, int M, int 
   int tiles = (M / 128) * (N / 256);
   if (pair) tiles = 2 * ((M / 256) * (N / 256));
   const int sms = smCount();
-  const SplitGemmTail tail = tailPlan(M, N, K, pair, pair ? sms / 2 : sms, &plan);
+  SplitGemmTail tail;
+  if (forced != 1) tail = tailPlan(M, N, K, pair, pair ? sms / 2 : sms, groupRows(pair), &plan);
   a.tiles = tail.first;
   cudaError_t e = launchTpGemm(stream ? stream->base : nullptr, ta, tb, nullptr, c, a, std::min(tiles, sms), pair);
   if (e == cudaSuccess && tail.count) {

@@ -14,6 +14,7 @@
 #include "../host/bootstrap.h"
 #include "../host/comm.h"
 #include "../host/cpu_coll.h"
+#include "../host/gemm_plan.h"
 #include "../host/reg_cache.h"
 #include "../host/shm.h"
 #include "../host/tuner.h"
@@ -441,7 +442,28 @@ static void testP2pEngine() {
   EXPECT(flagcxP2pEngineDestroy(owner) == flagcxSuccess);
 }
 
+static void testGemmPlan() {
+  // measured device times (us): the persistent kernel is quicker at small K ...
+  EXPECT(splitPlan(1664, 768, 1024, false).tileN == 0);  // 11.1 against 12.6
+  EXPECT(splitPlan(2432, 512, 1152, false).tileN == 0);   // 12.0 against 13.4
+  EXPECT(splitPlan(128, 9728, 1280, false).tileN == 0);  // 14.1 against 15.6
+  EXPECT(splitPlan(3456, 512, 1472, false).tileN == 0);  // 15.1 against 17.0
+  EXPECT(splitPlan(128, 8704, 320, false).tileN == 0);   // 7.4 against 7.7
+  // ... and the split where few tiles share a long K
+  EXPECT(splitPlan(128, 3584, 8192, false).parts == 4 && splitPlan(128, 3584, 8192, false).tileN == 128); // 55 against 20
+  EXPECT(splitPlan(128, 256, 8192, false).parts == 8);   // 48 against 12
+  EXPECT(splitPlan(896, 2048, 2240, false).tileN == 256);  // 18.2 against 16.4
+  EXPECT(splitPlan(128, 256, 8192, false, 1).tileN == 0 && splitPlan(128, 256, 8192, false, 3, 64).parts == 3);
+  for (int M = 128; M <= 8192; M += 128) // a plan never asks for more parts than K has steps or than run at once
+    for (int N = 256; N <= 8192; N += 768)
+      for (int K = 64; K <= 8192; K += 192) {
+        const SplitGemmPlan p = splitPlan(M, N, K, M % 256 == 0);
+        EXPECT(p.tileN == 0 || (p.parts * 64 <= K && (long)(M / 128) * (N / p.tileN) * p.parts <= 148));
+      }
+}
+
 int main() {
+  testGemmPlan();
   testRegCache();
   testShmRing();
   testParams();
