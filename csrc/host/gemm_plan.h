@@ -60,9 +60,14 @@ inline SplitGemmPlan splitPlan(int M, int N, int K, bool pair, int forced = 0, i
 
 // The tiles of the persistent kernel's last wave, where handing them to the split kernel (parts
 // CTAs per tile) is quicker than a wave of whole tiles in which most SMs are idle.  8192 x 3584
-// x 8192 is 6 waves of 74 CTA pairs and 4 tiles: 336 -> 325 us; 2048 x 5120 x 4096 119 -> 86,
-// 1408 x 3584 x 8192 99 -> 76.  3 us are asked for as margin (the second launch; 2304 x 2560 x
-// 3072 lost 2 %), and beyond 9 waves the last one no longer counts.
+// x 8192 is 6 waves of 74 CTA pairs and 4 tiles: 339 -> 328 us; 1408 x 5120 x 12352 213 -> 177,
+// 6400 x 768 x 8896 142 -> 92.  A wave costs 0.363 us per K step, of pairs 0.33 (several waves:
+// the clock is lower than in splitPlan's single one); the split kernel its estimate and 5.25 us
+// for the second launch.  Measured on 283 shapes with both routes: at 0.38 us for pairs,
+// too, 21 of the 162 that took a second launch lost 1 to 5 % (6400 x 4096 x 7040 269 -> 282, 768 x 8448 x 6336 80 -> 83), and
+// with less for the launch 5504 x 3584 x 2880 did (123 -> 130).  The gain falls
+// with the number of full waves (on average 17 % after one, 11 after two, 3 after six, 1 after
+// eight); beyond nine it is within the noise (twelve shapes to 13 waves: 0.95 to 1.05).
 inline SplitGemmTail tailPlan(int M, int N, int K, bool pair, int units, int groupRows, SplitGemmPlan *plan) {
   SplitGemmTail t;
   const int kb = K / 64, tiles = (M / (pair ? 256 : 128)) * (N / 256), rest = tiles % units;
@@ -70,9 +75,9 @@ inline SplitGemmTail tailPlan(int M, int N, int K, bool pair, int units, int gro
   const int parts128 = rest * (pair ? 2 : 1);
   for (auto &sp : kSplitSizes) {
     if (sp.parts < 2 || parts128 * sp.parts > sp.ctas || sp.parts * 4 > kb) continue;
-    const double steps = (kb + sp.parts - 1) / sp.parts * 0.384;
+    const double steps = (kb + sp.parts - 1) / sp.parts * kSplitKinds[0].stepUs;
     const double bytes = (double)parts128 * kb * (128 + 256) * 128;
-    if (11.5 + std::max(steps, bytes / 13e6) + 3.0 > kb * 0.38) break;
+    if (kSplitKinds[0].fixedUs + std::max(steps, bytes / 13e6) + 5.25 > kb * (pair ? 0.33 : 0.363)) break;
     plan->tileN = 256;
     plan->parts = sp.parts;
     t.first = tiles - rest;

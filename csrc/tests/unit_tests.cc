@@ -454,6 +454,21 @@ static void testGemmPlan() {
   EXPECT(splitPlan(128, 256, 8192, false).parts == 8);   // 48 against 12
   EXPECT(splitPlan(896, 2048, 2240, false).tileN == 256);  // 18.2 against 16.4
   EXPECT(splitPlan(128, 256, 8192, false, 1).tileN == 0 && splitPlan(128, 256, 8192, false, 3, 64).parts == 3);
+  // the last wave: measured with and without a second launch (us)
+  auto tail = [](int M, int N, int K) {
+    SplitGemmPlan p;
+    const bool pair = M % 256 == 0;
+    const SplitGemmTail t = tailPlan(M, N, K, pair, pair ? 74 : 148, pair ? 8 : 16, &p);
+    EXPECT(t.count == 0 || (p.tileN == 256 && t.first + t.count == M / t.tileRows * (N / 256)));
+    return t.count;
+  };
+  EXPECT(tail(6400, 4096, 7040) == 0);  // 269 against 282
+  EXPECT(tail(768, 8448, 6336) == 0);   // 80 against 83
+  EXPECT(tail(5504, 3584, 2880) == 0);  // 123 against 130
+  EXPECT(tail(1024, 4864, 3072) == 0);  // 39.7 either way
+  EXPECT(tail(8192, 3584, 8192) == 4);  // 339 against 328
+  EXPECT(tail(6400, 768, 8896) == 1);   // 142 against 92
+  EXPECT(tail(1408, 5120, 12352) == 72); // 213 against 177
   for (int M = 128; M <= 8192; M += 128) // a plan never asks for more parts than K has steps or than run at once
     for (int N = 256; N <= 8192; N += 768)
       for (int K = 64; K <= 8192; K += 192) {
