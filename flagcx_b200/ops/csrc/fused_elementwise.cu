@@ -13,12 +13,14 @@
 #include <cstdlib>
 
 #include "fused_elementwise.h"
+#include "norm_route.h"
 
 namespace cg = cooperative_groups;
 
 namespace {
 
 using bf16 = __nv_bfloat16;
+using fcxops::kNormBwdThreads;
 
 __device__ __forceinline__ float warpSum(float v) {
 #pragma unroll
@@ -186,7 +188,7 @@ rmsnormFwdWarp(const bf16 *__restrict__ x, const bf16 *__restrict__ w, bf16 *__r
 // ring of `stages` slots in shared memory; one thread keeps the ring full with bulk
 // asynchronous copies of (g row, x row) that complete on one mbarrier per slot, so several
 // rows per CTA are in flight while the 512 threads reduce and write the current one.
-constexpr int kNormBwdThreads = 512, kNormBwdMaxStages = 8;
+constexpr int kNormBwdMaxStages = 8;
 
 template <int MAXP>
 __global__ void __launch_bounds__(kNormBwdThreads)
@@ -283,7 +285,7 @@ rmsnormBwdPipelined(const bf16 *__restrict__ g, const bf16 *__restrict__ x, cons
   }
 }
 
-// The same where one row does not keep 512 threads busy (see rmsnormBackward for where the line
+// The same where one row does not keep 512 threads busy (norm_route.h says where the line
 // lies).  A CTA is cut into groups of GT threads, the fewest (a power of two from 32) that hold a row with four packs
 // per thread; every group owns a ring of row slots in shared memory, which its first thread
 // keeps full with bulk copies that complete on one mbarrier per slot, and reduces its rows by
@@ -998,17 +1000,8 @@ cudaError_t rmsnormForward(const void *x, const void *w, void *y, float *rstd, l
   return cudaGetLastError();
 }
 
-// One CTA of 512 threads per row where a row fills them (one or two packs per thread, 0.9 of the
-// threads with work) and a third tensor is added: its two CTAs per SM need fewer registers (4096
-// x 4096 33.6 us against 35.4 in groups, 16384 x 4096 100.1 against 104.4).  Groups elsewhere
-// (without the third tensor 16384 x 4096 takes 90.4 us in groups against 96.3).
-static bool rowPerCta(int H, bool add) {
-  const int packs = H / 8, perThread = (packs + kNormBwdThreads - 1) / kNormBwdThreads;
-  return add && perThread <= 2 && packs * 10 > 9 * perThread * kNormBwdThreads;
-}
-
 int rmsnormPartials(long rows, int H, bool add, int sms) {
-  if (rowPerCta(H, add)) return (int)std::max<long>(1, std::min<long>(rows, sms * 2));
+  if (rmsnormRowPerCta(rows, H, add, sms)) return (int)std::max<long>(1, std::min<long>(rows, sms * 2));
   int ctas = 0;
   withNormShape(H / 8, [&](auto gt, auto) {
     constexpr int G = kNormThreads / decltype(gt)::value;
@@ -1021,9 +1014,9 @@ int rmsnormPartials(long rows, int H, bool add, int sms) {
 cudaError_t rmsnormBackward(const void *g, const void *x, const void *w, const float *rstd, const void *add, void *dx, void *dw,
                             float *partial, long rows, int H, int sms, cudaStream_t stream) {
   const int ctas = rmsnormPartials(rows, H, add != nullptr, sms);
-  if (rowPerCta(H, add != nullptr)) {
+  if (rmsnormRowPerCta(rows, H, add != nullptr, sms)) {
     // ring of (g, x, add) slots: about 96 KiB per CTA so that two CTAs share an SM
-    const size_t slot = (size_t)H * 6;
+    const size_t slot = (size_t)H * (add ? 6 : 4);
     const int stages = (int)std::max<size_t>(2, std::min<size_t>(kNormBwdMaxStages, ((size_t)96 << 10) / slot));
     const size_t smem = slot * stages;
     auto launch = [&](auto tag) {

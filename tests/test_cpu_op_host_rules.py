@@ -1,0 +1,27 @@
+"""Host-side rules of the model kernels (flagcx_b200/ops/csrc), compiled without CUDA."""
+import os
+import subprocess
+
+ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+
+
+def _run(tmp_path, text, flags=()):
+    src, exe = tmp_path / "t.cc", tmp_path / "t"
+    src.write_text(text)
+    subprocess.check_call(["g++", "-std=c++17", "-O1", "-Wall", *flags, "-I" + os.path.join(ROOT, "flagcx_b200", "ops", "csrc"),
+                           str(src), "-lpthread", "-o", str(exe)])
+    res = subprocess.run([str(exe)], capture_output=True, text=True, timeout=60)
+    assert res.returncode == 0, res.stdout + res.stderr
+    return res.stdout
+
+
+def test_norm_backward_of_few_rows_runs_one_row_per_cta(tmp_path):
+    # rows, hidden size, skip gradient -> one row per CTA, where both kernels were measured and
+    # differ by more than 3 % on 148 SMs
+    cases = [(1, 1024, 0, 1), (64, 4096, 0, 1), (148, 8192, 1, 1), (257, 2048, 1, 1), (257, 3584, 0, 1), (592, 1024, 1, 1),
+             (800, 3584, 1, 1), (8192, 7168, 1, 1), (4096, 4096, 1, 1), (257, 256, 1, 1), (360, 2560, 0, 1), (8192, 8192, 1, 1),
+             (592, 256, 0, 0), (4096, 256, 1, 0), (1021, 2048, 1, 0), (592, 3072, 0, 0), (200, 5120, 1, 0), (257, 7168, 1, 0),
+             (4096, 5120, 0, 0), (4096, 4096, 0, 0), (148, 12288, 0, 0), (1, 16384, 1, 0), (2048, 1024, 0, 0)]
+    rows = "".join(f"  bad += fcxops::rmsnormRowPerCta({r}, {h}, {s}, 148) != {w} && printf(\"{r} x {h} skip {s}\\n\");\n"
+                   for r, h, s, w in cases)
+    _run(tmp_path, '#include <cstdio>\n#include "norm_route.h"\nint main() {\n  int bad = 0;\n' + rows + "  return bad != 0;\n}\n")
