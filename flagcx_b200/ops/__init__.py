@@ -8,6 +8,8 @@ from __future__ import annotations
 
 import importlib.util
 import os
+import sys
+import types
 
 import torch
 import torch.autograd.forward_ad as _forward_ad
@@ -15,7 +17,7 @@ import torch.autograd.forward_ad as _forward_ad
 from . import build as _build
 
 _ext = None
-_launches = 0  # see __getattr__ at the end of this file
+_launches = 0  # see _Module at the end of this file
 # When the loss is only ever differentiated with gradient 1 (loss.backward()), the
 # cross-entropy backward can hand out the stored gradient without another pass.
 assume_unit_loss_grad = False
@@ -266,9 +268,18 @@ def adamw_flat_(p, g, m, v, lr, beta1, beta2, eps, weight_decay, step) -> None:
     _count()
 
 
-def __getattr__(name):
-    """`launch_count` (read only): kernels launched through this module, from Python and from C++
-    (bench.py reports it)."""
-    if name == "launch_count":
+class _Module(types.ModuleType):
+    """`launch_count`: kernels launched through this module, from Python and from C++ (bench.py
+    reports it); assigning sets what it reads from then on."""
+
+    @property
+    def launch_count(self):
         return _launches + (_ext.launch_count() if _ext is not None else 0)
-    raise AttributeError(f"module {__name__!r} has no attribute {name!r}")
+
+    @launch_count.setter
+    def launch_count(self, value):
+        global _launches
+        _launches = value - (_ext.launch_count() if _ext is not None else 0)
+
+
+sys.modules[__name__].__class__ = _Module

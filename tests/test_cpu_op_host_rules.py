@@ -25,3 +25,14 @@ def test_norm_backward_of_few_rows_runs_one_row_per_cta(tmp_path):
     rows = "".join(f"  bad += fcxops::rmsnormRowPerCta({r}, {h}, {s}, 148) != {w} && printf(\"{r} x {h} skip {s}\\n\");\n"
                    for r, h, s, w in cases)
     _run(tmp_path, '#include <cstdio>\n#include "norm_route.h"\nint main() {\n  int bad = 0;\n' + rows + "  return bad != 0;\n}\n")
+
+
+def test_launch_count_can_be_set():
+    from flagcx_b200 import ops
+    before = ops.launch_count
+    try:
+        ops.launch_count = 5
+        ops._count(2)
+        assert ops.launch_count == 7
+    finally:
+        ops.launch_count = before
