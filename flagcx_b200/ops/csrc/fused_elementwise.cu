@@ -13,6 +13,7 @@
 #include <cstdlib>
 
 #include "fused_elementwise.h"
+#include "launch_state.h"
 #include "norm_route.h"
 
 namespace cg = cooperative_groups;
@@ -188,7 +189,7 @@ rmsnormFwdWarp(const bf16 *__restrict__ x, const bf16 *__restrict__ w, bf16 *__r
 // ring of `stages` slots in shared memory; one thread keeps the ring full with bulk
 // asynchronous copies of (g row, x row) that complete on one mbarrier per slot, so several
 // rows per CTA are in flight while the 512 threads reduce and write the current one.
-constexpr int kNormBwdMaxStages = 8;
+constexpr int kNormBwdMaxStages = 8, kNormBwdRingBytes = 96 << 10; // two CTAs share an SM
 
 template <int MAXP>
 __global__ void __launch_bounds__(kNormBwdThreads)
@@ -294,7 +295,7 @@ rmsnormBwdPipelined(const bf16 *__restrict__ g, const bf16 *__restrict__ x, cons
 // chain wait -> dot product -> sum -> store of each row.  With one row per CTA 8192 x 1024
 // took 39.2 us, 8192 x 256 37.0, 4096 x 2560 30.8, 2048 x 5120 32.9, 512 x 8192 20.5; in groups
 // they take 22.9, 12.4, 24.7, 23.0 and 16.5.
-constexpr int kNormThreads = 512, kNormMaxStages = 6, kNormPacks = 4;
+constexpr int kNormThreads = 512, kNormMaxStages = 6, kNormPacks = 4, kNormRingBytes = 200 << 10;
 
 // Sum over a group of GT threads; every thread gets it.  red holds one float per warp of the
 // CTA, alternately the first and the second 16 (parity), so that one barrier per sum is enough:
@@ -759,7 +760,7 @@ crossEntropyRows(bf16 *__restrict__ logits, const long *__restrict__ targets, fl
 // [T, V] tensor crosses L2/HBM once in each direction and every element costs one
 // exponential instead of two.
 // ---------------------------------------------------------------------------
-constexpr int kCeMaxThreads = 1024;
+constexpr int kCeMaxThreads = 1024, kCePartBytes = 200 << 10;
 
 __global__ void __launch_bounds__(kCeMaxThreads)
 crossEntropyCluster(bf16 *__restrict__ logits, const long *__restrict__ targets, float *__restrict__ loss, int V,
@@ -916,6 +917,17 @@ int gridFor(size_t items, int threads, int sms, int perSm = 8) {
     if (err_ != cudaSuccess) return err_;   \
   } while (0)
 
+// Lets every launch of Kern on this device have `bytes` of dynamic shared memory, the most that any
+// of its sizes asks for.  The limit belongs to the kernel, not to a launch: set to each call's own
+// size, two threads could lower it between the other's call and launch.
+template <auto Kern>
+cudaError_t allowShared(int bytes) {
+  static fcxops::OncePerDevice once;
+  int dev = 0;
+  RETURN_IF(cudaGetDevice(&dev));
+  return once(dev, [&] { return cudaFuncSetAttribute(Kern, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes); });
+}
+
 // Calls f(GT, PPT) for rows of `packs` packs of 8: the smallest group whose threads hold a row
 // with at most four packs each (512 threads and four packs: 16384 elements).
 template <typename F>
@@ -951,8 +963,8 @@ cudaError_t launchCeRows(bf16 *logits, const long *targets, float *loss, long ro
   cfg.stream = stream;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  if (smem > (47 << 10)) // beyond what a kernel gets without asking
-    RETURN_IF(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+  constexpr int kMost = PPT * kCeRowThreads * 16;
+  if constexpr (kMost > (47 << 10)) RETURN_IF(allowShared<crossEntropyRows<PPT>>(kMost)); // beyond what a kernel gets without asking
   // As many clusters as run at once: rows are dealt out evenly, so a second wave would be waste.
   long clusters = rows;
   if (rows * C > sms) {
@@ -1015,13 +1027,13 @@ cudaError_t rmsnormBackward(const void *g, const void *x, const void *w, const f
                             float *partial, long rows, int H, int sms, cudaStream_t stream) {
   const int ctas = rmsnormPartials(rows, H, add != nullptr, sms);
   if (rmsnormRowPerCta(rows, H, add != nullptr, sms)) {
-    // ring of (g, x, add) slots: about 96 KiB per CTA so that two CTAs share an SM
+    // ring of (g, x, add) slots, two at least (8192 x 6 bytes each)
     const size_t slot = (size_t)H * (add ? 6 : 4);
-    const int stages = (int)std::max<size_t>(2, std::min<size_t>(kNormBwdMaxStages, ((size_t)96 << 10) / slot));
+    const int stages = (int)std::min<size_t>(kNormBwdMaxStages, kNormBwdRingBytes / slot);
     const size_t smem = slot * stages;
     auto launch = [&](auto tag) {
-      auto kern = rmsnormBwdPipelined<decltype(tag)::value>;
-      RETURN_IF(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+      constexpr auto kern = rmsnormBwdPipelined<decltype(tag)::value>;
+      RETURN_IF(allowShared<kern>(kNormBwdRingBytes));
       kern<<<ctas, kNormBwdThreads, smem, stream>>>((const bf16 *)g, (const bf16 *)x, (const bf16 *)w, rstd, (const bf16 *)add,
                                                     (bf16 *)dx, partial, (int)rows, H, stages);
       return cudaGetLastError();
@@ -1031,12 +1043,12 @@ cudaError_t rmsnormBackward(const void *g, const void *x, const void *w, const f
   } else {
     RETURN_IF(withNormShape(H / 8, [&](auto gt, auto ppt) {
       constexpr int GT = decltype(gt)::value, PPT = decltype(ppt)::value, G = kNormThreads / GT;
-      // slots of all groups, about 200 KiB: one CTA per SM
+      // slots of all groups, two for each at least: one CTA per SM
       const size_t slots = (size_t)H * (add ? 6 : 4) * G;
-      const int stages = (int)std::max<size_t>(1, std::min<size_t>(kNormMaxStages, ((size_t)200 << 10) / slots));
+      const int stages = (int)std::min<size_t>(kNormMaxStages, kNormRingBytes / slots);
       const size_t smem = slots * stages;
-      auto kern = rmsnormBwdRing<GT, PPT>;
-      RETURN_IF(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+      constexpr auto kern = rmsnormBwdRing<GT, PPT>;
+      RETURN_IF(allowShared<kern>(kNormRingBytes));
       kern<<<ctas, kNormThreads, smem, stream>>>((const bf16 *)g, (const bf16 *)x, (const bf16 *)w, rstd, (const bf16 *)add,
                                                  (bf16 *)dx, partial, rows, H, stages);
       return cudaGetLastError();
@@ -1101,14 +1113,14 @@ cudaError_t crossEntropy(void *logits, const long *targets, float *loss, long ro
       return go(std::integral_constant<int, 16>());
     }
     per = (packs + 7) / 8;
-    if ((size_t)per * 16 <= (size_t)200 << 10) cluster = 8;
+    if (per * 16 <= kCePartBytes) cluster = 8;
   }
   if (!cluster || rows * cluster > 0x7fffffffLL) {
     crossEntropyFwdBwd<<<(unsigned)rows, 1024, 0, stream>>>((bf16 *)logits, targets, loss, V, gradScale);
     return cudaGetLastError();
   }
   const size_t smem = (size_t)per * 16;
-  RETURN_IF(cudaFuncSetAttribute(crossEntropyCluster, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  RETURN_IF(allowShared<crossEntropyCluster>(kCePartBytes));
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((unsigned)(rows * cluster));
   static const int ceThreads = std::getenv("FLAGCX_OPS_CE_THREADS") ? std::min(kCeMaxThreads, std::max(32, atoi(std::getenv("FLAGCX_OPS_CE_THREADS")) / 32 * 32)) : 256;

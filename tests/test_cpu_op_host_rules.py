@@ -27,6 +27,36 @@ def test_norm_backward_of_few_rows_runs_one_row_per_cta(tmp_path):
     _run(tmp_path, '#include <cstdio>\n#include "norm_route.h"\nint main() {\n  int bad = 0;\n' + rows + "  return bad != 0;\n}\n")
 
 
+def test_a_limit_is_set_once_per_device_and_never_skipped(tmp_path):
+    """Eight threads on three devices; the first call of a device fails and is tried again."""
+    _run(tmp_path, """
+#include <cstdio>
+#include <thread>
+#include <vector>
+#include "launch_state.h"
+int main() {
+  fcxops::OncePerDevice once;
+  std::atomic<int> calls[3] = {}, bad{0};
+  if (once(1, [&] { return ++calls[1], 7; }) != 7) return 1; // passed on
+  std::vector<std::thread> ts;
+  for (int k = 0; k < 8; ++k)
+    ts.emplace_back([&, k] {
+      for (int i = 0; i < 3000; ++i) {
+        const int d = (k + i) % 3;
+        if (once(d, [&] { return ++calls[d], 0; }) != 0) ++bad;
+        if (calls[d] == 0) ++bad; // whoever goes on finds it set
+      }
+    });
+  for (auto &t : ts) t.join();
+  for (int d = 0; d < 3; ++d)
+    if (calls[d] < 1 || calls[d] > 9) return 2; // at most once per thread that came first together
+  int far = 0;
+  for (int i = 0; i < 2; ++i) once(64, [&] { return ++far, 0; });
+  return bad || far != 2;
+}
+""")
+
+
 def test_launch_count_can_be_set():
     from flagcx_b200 import ops
     before = ops.launch_count

@@ -62,6 +62,44 @@ def test_rmsnorm_backward_at_the_edges_of_its_row_groups(rows, H, skip):
     assert bool(((dw.double() - rdw).abs() <= rdw.abs() * 2 ** -8 + terms * 2 ** -16).all())
 
 
+def test_norm_backward_from_two_threads_with_different_sizes():
+    """The backward of an autograd graph runs without the GIL, so its launches interleave with
+    another thread's; 8 and 256 columns share a kernel and ask for 3 and 144 KiB of shared memory."""
+    import threading
+    import time
+    ops = _ops()
+    made = {}
+    for H in (8, 256):
+        x, g, skip = [torch.randn(300, H, device="cuda").to(torch.bfloat16) for _ in range(3)]
+        w = torch.ones(H, device="cuda", dtype=torch.bfloat16)
+        made[H] = x, w, g, skip, ops.ext().rmsnorm_fwd(x, w, 1e-5)[1]
+    errors, stop = [], threading.Event()
+
+    def small():
+        x, w, g, _, rstd = made[8]
+        try:
+            while not stop.is_set():
+                for _ in range(20):
+                    ops.ext().rmsnorm_bwd(g, x, w, rstd)
+                torch.cuda.synchronize()  # a full launch queue would keep the other thread out
+        except RuntimeError as e:
+            errors.append(e)
+
+    other = threading.Thread(target=small)
+    other.start()
+    try:
+        x, w, g, skip, _ = made[256]
+        x.requires_grad_()
+        end = time.monotonic() + 3
+        while time.monotonic() < end:
+            torch.autograd.grad(ops.rmsnorm_branch(x, w, 1e-5), x, (g, skip))
+    finally:
+        stop.set()
+        other.join()
+    torch.cuda.synchronize()
+    assert not errors, errors
+
+
 def test_operators_keep_hooks_tracing_and_transforms():
     """The operators run as C++ autograd functions, except under a tracer, a function transform or
     forward-mode differentiation."""
