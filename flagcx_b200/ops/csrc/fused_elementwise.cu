@@ -8,7 +8,6 @@
 #include <cuda_bf16.h>
 
 #include <algorithm>
-#include <atomic>
 #include <cstdint>
 #include <cstdlib>
 
@@ -968,17 +967,12 @@ cudaError_t launchCeRows(bf16 *logits, const long *targets, float *loss, long ro
   // As many clusters as run at once: rows are dealt out evenly, so a second wave would be waste.
   long clusters = rows;
   if (rows * C > sms) {
-    static std::atomic<uint64_t> known{0}; // last answer: shared memory << 32 | cluster size << 16 | clusters
-    uint64_t k = known.load(std::memory_order_relaxed);
-    const uint64_t key = (uint64_t)smem << 16 | (uint64_t)C;
-    if (k >> 16 != key) {
-      int active = 0;
-      cfg.gridDim = dim3((unsigned)C);
-      RETURN_IF(cudaOccupancyMaxActiveClusters(&active, kern, &cfg));
-      k = key << 16 | (uint64_t)std::min(std::max(active, 1), 0xffff);
-      known.store(k, std::memory_order_relaxed);
-    }
-    clusters = std::min<long>(rows, (long)(k & 0xffff));
+    static fcxops::ClusterCount count;
+    int dev = 0, active = 0;
+    RETURN_IF(cudaGetDevice(&dev));
+    cfg.gridDim = dim3((unsigned)C);
+    RETURN_IF(count(dev, smem, C, [&](int *n) { return cudaOccupancyMaxActiveClusters(n, kern, &cfg); }, &active));
+    clusters = std::min<long>(rows, active);
   }
   cfg.gridDim = dim3((unsigned)(clusters * C));
   return cudaLaunchKernelEx(&cfg, kern, logits, targets, loss, rows, V, gradScale, per);

@@ -57,6 +57,27 @@ int main() {
 """)
 
 
+def test_cluster_count_is_kept_per_device_and_shape(tmp_path):
+    _run(tmp_path, """
+#include "launch_state.h"
+int main() {
+  fcxops::ClusterCount count;
+  int asked = 0, n = 0, bad = 0;
+  auto get = [&](int dev, int smem, int ctas, int answer) {
+    if (count(dev, smem, ctas, [&](int *c) { ++asked; *c = answer; return 0; }, &n) != 0) ++bad;
+    return n;
+  };
+  bad += get(0, 65536, 4, 71) != 71 || get(0, 65536, 4, 99) != 71 || asked != 1;
+  bad += get(1, 65536, 4, 30) != 30 || asked != 2; // another device
+  bad += get(1, 65520, 4, 31) != 31 || get(1, 65520, 8, 12) != 12 || asked != 4;
+  bad += get(1, 0, 1, 0) != 1 || get(2, 0, 1, 1 << 20) != 0xffff;
+  if (count(3, 16, 1, [&](int *) { return 5; }, &n) != 5) ++bad; // passed on, nothing kept
+  bad += get(3, 16, 1, 9) != 9;
+  return bad;
+}
+""")
+
+
 def test_launch_count_can_be_set():
     from flagcx_b200 import ops
     before = ops.launch_count
