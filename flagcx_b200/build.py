@@ -19,22 +19,34 @@ def build_core(jobs: int | None = None, verbose: bool = False) -> str:
     return os.path.join(ROOT, "flagcx_b200", "lib", "libflagcx.so")
 
 
-def build_devtest(verbose: bool = False) -> str:
-    """The device-API conformance kernels (csrc/tests/device_api_kernels.cu) as a shared
-    library next to their source; tests/test_gpu_device_api.py loads it."""
-    src = os.path.join(ROOT, "csrc", "tests", "device_api_kernels.cu")
-    lib = os.path.join(ROOT, "csrc", "tests", "libflagcx_devtest.so")
-    inc = os.path.join(ROOT, "csrc", "include")
-    deps = [src] + [os.path.join(inc, f) for f in os.listdir(inc)]
-    if os.path.exists(lib) and os.path.getmtime(lib) >= max(os.path.getmtime(d) for d in deps):
+def _build_test_kernels(name: str, lib: str, deps: list[str], flags: list[str], verbose: bool) -> str:
+    src = os.path.join(ROOT, "csrc", "tests", name)
+    lib = os.path.join(ROOT, "csrc", "tests", lib)
+    if os.path.exists(lib) and os.path.getmtime(lib) >= max(os.path.getmtime(d) for d in deps + [src]):
         return lib
-    cmd = ["/usr/local/cuda/bin/nvcc", "-std=c++17", "-O2", "-lineinfo", "-gencode", "arch=compute_100a,code=sm_100a",
-           "-shared", "-Xcompiler", "-fPIC", "-cudart", "shared", "-I" + os.path.join(ROOT, "csrc", "include"), src, "-o", lib]
+    cmd = ["/usr/local/cuda/bin/nvcc", "-std=c++17", "-lineinfo", "-gencode", "arch=compute_100a,code=sm_100a",
+           "-shared", "-Xcompiler", "-fPIC", "-cudart", "shared", *flags, src, "-o", lib]
     res = subprocess.run(cmd, capture_output=not verbose, text=True)
     if res.returncode != 0:
         sys.stderr.write((res.stdout or "") + (res.stderr or ""))
-        raise RuntimeError("building the device-API test kernels failed")
+        raise RuntimeError(f"building the test kernels of {name} failed")
     return lib
+
+
+def build_devtest(verbose: bool = False) -> str:
+    """The device-API conformance kernels (csrc/tests/device_api_kernels.cu) as a shared
+    library next to their source; tests/test_gpu_device_api.py loads it."""
+    inc = os.path.join(ROOT, "csrc", "include")
+    return _build_test_kernels("device_api_kernels.cu", "libflagcx_devtest.so", [os.path.join(inc, f) for f in os.listdir(inc)],
+                               ["-O2", "-I" + inc], verbose)
+
+
+def build_opwait(verbose: bool = False) -> str:
+    """The model kernels with a short wait limit (csrc/tests/op_wait_limits.cu), loaded by
+    tests/test_gpu_op_wait_limits.py."""
+    ops = os.path.join(ROOT, "flagcx_b200", "ops", "csrc")
+    return _build_test_kernels("op_wait_limits.cu", "libflagcx_opwait.so", [os.path.join(ops, f) for f in os.listdir(ops)],
+                               ["-O3", "--use_fast_math"], verbose)
 
 
 def build_bounds(jobs: int | None = None, verbose: bool = False) -> str:
@@ -53,6 +65,7 @@ def build(verbose: bool = False) -> None:
     build_core(verbose=verbose)
     build_bounds(verbose=verbose)
     build_devtest(verbose=verbose)
+    build_opwait(verbose=verbose)
     try:
         from flagcx_b200.torch_backend import build as tb
     except ImportError:

@@ -58,6 +58,13 @@ __device__ __forceinline__ float blockMax(float v, float *red) {
 
 __device__ __forceinline__ uint32_t sharedAddr(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }
 
+// How long a copy may take before a kernel gives up on it, and the row that is never fetched
+// (a test of the waits that run out sets both; there is none otherwise).
+#ifndef FLAGCX_OPS_WAIT_NS
+#define FLAGCX_OPS_WAIT_NS 1000000000ull
+#define FLAGCX_OPS_HELD_BACK(row) false
+#endif
+
 // Waits for a phase of an mbarrier for at most about one second.
 __device__ __forceinline__ bool mbarWaitBounded(uint64_t *bar, uint32_t parity) {
   unsigned long long t0 = 0;
@@ -75,7 +82,7 @@ __device__ __forceinline__ bool mbarWaitBounded(uint64_t *bar, uint32_t parity) 
       unsigned long long now;
       asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(now));
       if (t0 == 0) t0 = now;
-      else if (now - t0 > 1000000000ull) return false;
+      else if (now - t0 > FLAGCX_OPS_WAIT_NS) return false;
     }
   }
 }
@@ -336,10 +343,8 @@ rmsnormBwdRing(const bf16 *__restrict__ g, const bf16 *__restrict__ x, const bf1
   unsigned char *slots = ring + (size_t)group * stages * slotBytes;
   uint64_t *bars = full + group * kNormMaxStages;
   const long first = (long)blockIdx.x * G + group, step = (long)gridDim.x * G;
-  auto issue = [&](long k) { // the group's first thread: row k of the group into slot k % stages
-    const long row = first + k * step;
-    if (row >= rows) return;
-    const int s = (int)(k % stages);
+  auto issue = [&](long row, int s) { // the group's first thread: a row into slot s
+    if (row >= rows || FLAGCX_OPS_HELD_BACK(row)) return;
     unsigned char *dst = slots + (size_t)s * slotBytes;
     mbarExpect(&bars[s], slotBytes);
     bulkLoad(dst, g + (size_t)row * H, rowBytes, &bars[s]);
@@ -349,7 +354,7 @@ rmsnormBwdRing(const bf16 *__restrict__ g, const bf16 *__restrict__ x, const bf1
   if (t == 0) {
     for (int s = 0; s < stages; ++s) mbarInit(&bars[s]);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-    for (int k = 0; k < stages; ++k) issue(k);
+    for (int s = 0; s < stages; ++s) issue(first + s * step, s);
   }
   __syncthreads();
   float dwAcc[PPT][8];
@@ -361,13 +366,14 @@ rmsnormBwdRing(const bf16 *__restrict__ g, const bf16 *__restrict__ x, const bf1
 #pragma unroll
     for (int i = 0; i < 8; ++i) dwAcc[k][i] = 0.f;
   }
-  // A wait that ran out marks the group's part of the weight gradient as NaN.
-  bool ok = true;
-  int it = 0;
-  for (long row = first; row < rows; row += step, ++it) {
-    const int s = it % stages;
+  bool ok = true; // of the whole warp
+  int s = 0, half = 0;
+  uint32_t phase = 0;
+  long row = first;
+  for (; row < rows; row += step) {
     const float rstd = rstdIn[row];
-    if (ok) ok = mbarWaitBounded(&bars[s], (uint32_t)(it / stages) & 1u);
+    ok = __all_sync(0xffffffffu, mbarWaitBounded(&bars[s], phase));
+    if (!ok) break;
     const uint4 *gs = (const uint4 *)(slots + (size_t)s * slotBytes), *xs = gs + nPacks, *as = xs + nPacks;
     Pack8 pg[PPT], px[PPT], pa[PPT];
     float dot = 0.f;
@@ -382,8 +388,10 @@ rmsnormBwdRing(const bf16 *__restrict__ g, const bf16 *__restrict__ x, const bf1
         for (int i = 0; i < 8; ++i) dot += pg[k].get(i) * pw[k].get(i) * px[k].get(i);
       }
     }
-    dot = groupSum<GT>(dot, red, it & 1, group); // the whole group has read the slot
-    if (t == 0 && ok) issue(it + stages);
+    dot = groupSum<GT>(dot, red, half, group); // the whole group has read the slot
+    half ^= 1;
+    if (t == 0) issue(row + stages * step, s);
+    if (++s == stages) { s = 0; phase ^= 1u; }
     const float c = dot * rstd * rstd / H;
     uint4 *dxr = (uint4 *)(dx + (size_t)row * H);
 #pragma unroll
@@ -403,8 +411,24 @@ rmsnormBwdRing(const bf16 *__restrict__ g, const bf16 *__restrict__ x, const bf1
       }
     }
   }
-  // The groups' sums meet in the ring (all copies have landed and been read), a group's sums in
-  // its own slots: G x H floats fit since a slot holds at least two rows of 16 bits.
+  // A wait ran out: nothing more is fetched, copies still under way land (or are given as long
+  // again), and the rows from there on and the warp's part of the weight gradient are NaN.
+  if (!ok) {
+    if (t == 0)
+      for (long r = row; r < rows && r < row + stages * step; r += step) {
+        mbarWaitBounded(&bars[s], phase);
+        if (++s == stages) { s = 0; phase ^= 1u; }
+      }
+    __syncwarp();
+    for (; row < rows; row += step, half ^= 1) {
+      groupSum<GT>(NAN, red, half, group);
+      for (int p = t; p < nPacks; p += GT)
+        ((uint4 *)(dx + (size_t)row * H))[p] = make_uint4(0x7fff7fffu, 0x7fff7fffu, 0x7fff7fffu, 0x7fff7fffu);
+    }
+  }
+  // The groups' sums meet at the start of the ring: G x H floats fit since a slot holds at least
+  // two rows of 16 bits.  They lie across slots of other groups, so every group is through with
+  // its rows first, and no copy is under way then.
   const float bad = ok ? 0.f : NAN;
   float *mine = (float *)ring + (size_t)group * H;
   __syncthreads();

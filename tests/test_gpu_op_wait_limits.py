@@ -1,0 +1,50 @@
+"""What the model kernels make of a copy that never comes: the wait for it runs out (20 ms in this
+build of them), the kernel ends, what depends on it is NaN and everything else is right."""
+import ctypes
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def lib():
+    from flagcx_b200.build import build_opwait
+    torch.cuda.init()
+    so = ctypes.CDLL(build_opwait())
+    so.hold_back.argtypes = [ctypes.c_long]
+    so.norm_partials.argtypes = [ctypes.c_long, ctypes.c_int, ctypes.c_int, ctypes.c_int]
+    so.norm_backward.argtypes = [ctypes.c_void_p] * 8 + [ctypes.c_long, ctypes.c_int, ctypes.c_int]
+    yield so
+    so.hold_back(-1)
+
+
+def _norm_backward(lib, t, rows, H, skip, held):
+    assert lib.hold_back(held) == 0
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    dx, dw = torch.full_like(t["x"], 7.0), torch.full_like(t["w"], 7.0)
+    partial = torch.empty(lib.norm_partials(rows, H, skip, sms), H, device="cuda")
+    assert lib.norm_backward(*[p.data_ptr() for p in (t["g"], t["x"], t["w"], t["rstd"])], t["skip"].data_ptr() if skip else None,
+                             dx.data_ptr(), dw.data_ptr(), partial.data_ptr(), rows, H, sms) == 0
+    return dx, dw
+
+
+# groups of 32 to 512 threads, with rows for several rounds of their rings
+@pytest.mark.parametrize("rows,H,skip", [(9000, 256, 1), (4000, 1032, 0), (3000, 2560, 1), (2000, 5120, 0), (700, 12296, 1)])
+def test_norm_backward_without_one_row(lib, rows, H, skip):
+    g = torch.Generator(device="cuda").manual_seed(rows)
+    t = {k: torch.randn(rows, H, generator=g, device="cuda").to(torch.bfloat16) for k in ("x", "g", "skip")}
+    t["w"] = torch.ones(H, device="cuda", dtype=torch.bfloat16)
+    t["rstd"] = torch.rsqrt(t["x"].float().square().mean(-1) + 1e-5)
+    whole = _norm_backward(lib, t, rows, H, skip, -1)
+    assert not whole[0].isnan().any() and not whole[1].isnan().any()
+    held = rows // 2 + 1
+    dx, dw = _norm_backward(lib, t, rows, H, skip, held)
+    lost = dx.isnan().any(1)
+    assert torch.equal(lost, dx.isnan().all(1)) and bool(lost[held])  # a row is lost as a whole
+    assert 0 < int(lost.sum()) <= rows - held and not bool(lost[:held].any())  # from there on, in one group
+    assert torch.equal(dx[~lost], whole[0][~lost])
+    assert bool(dw.isnan().all())
+    again = _norm_backward(lib, t, rows, H, skip, -1)
+    assert all(torch.equal(a, b) for a, b in zip(again, whole))
