@@ -217,7 +217,7 @@ rmsnormBwdPipelined(const bf16 *__restrict__ g, const bf16 *__restrict__ x, cons
   __syncthreads();
   auto issue = [&](int k) { // thread 0: the row of iteration k into slot k % stages
     const size_t row = blockIdx.x + (size_t)k * gridDim.x;
-    if (row >= (size_t)rows) return;
+    if (row >= (size_t)rows || FLAGCX_OPS_HELD_BACK(row)) return;
     const int s = k % stages;
     unsigned char *dst = ring + (size_t)s * slotBytes;
     mbarExpect(&full[s], slotBytes);
@@ -242,9 +242,12 @@ rmsnormBwdPipelined(const bf16 *__restrict__ g, const bf16 *__restrict__ x, cons
   for (size_t row = blockIdx.x; row < (size_t)rows; row += gridDim.x, ++it) {
     const int s = it % stages;
     const float rstd = rstdIn[row];
-    // Every thread goes on through the same barriers whatever its wait returned; a wait
-    // that ran out marks this CTA's weight-gradient partial as NaN.
-    if (ok) ok = mbarWaitBounded(&full[s], (uint32_t)(it / stages) & 1u);
+    // Every thread goes on through the same barriers whatever its wait returned.  After one that
+    // ran out nothing more is fetched, and the rows from there on and this CTA's part of the weight
+    // gradient are NaN; the copies that are out land (or are given as long again) first.
+    if (ok && !(ok = mbarWaitBounded(&full[s], (uint32_t)(it / stages) & 1u)) && threadIdx.x == 0)
+      for (int k = it; k < it + stages && blockIdx.x + (size_t)k * gridDim.x < (size_t)rows; ++k)
+        mbarWaitBounded(&full[k % stages], (uint32_t)(k / stages) & 1u);
     const uint4 *gs = (const uint4 *)(ring + (size_t)s * slotBytes), *xs = gs + nPacks, *as = xs + nPacks;
     Pack8 pg[MAXP], px[MAXP], pa[MAXP];
     float dot = 0.f;
@@ -259,8 +262,8 @@ rmsnormBwdPipelined(const bf16 *__restrict__ g, const bf16 *__restrict__ x, cons
         for (int i = 0; i < 8; ++i) dot += pg[k].get(i) * pw[k].get(i) * px[k].get(i);
       }
     }
-    dot = blockSum(dot, red); // all threads have read the slot once its barriers are passed
-    if (threadIdx.x == 0) issue(it + stages);
+    dot = blockSum(ok ? dot : NAN, red); // all threads have read the slot once its barriers are passed
+    if (threadIdx.x == 0 && ok) issue(it + stages);
     const float c = dot * rstd * rstd / H;
     uint4 *dxr = (uint4 *)(dx + row * H);
 #pragma unroll

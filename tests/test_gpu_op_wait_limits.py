@@ -30,8 +30,10 @@ def _norm_backward(lib, t, rows, H, skip, held):
     return dx, dw
 
 
-# groups of 32 to 512 threads, with rows for several rounds of their rings
-@pytest.mark.parametrize("rows,H,skip", [(9000, 256, 1), (4000, 1032, 0), (3000, 2560, 1), (2000, 5120, 0), (700, 12296, 1)])
+# groups of 32 to 512 threads, and one row per CTA (with one and two packs per thread; a single
+# round of the ring without a skip gradient), with rows for several rounds of their rings
+@pytest.mark.parametrize("rows,H,skip", [(9000, 256, 1), (4000, 1032, 0), (3000, 2560, 1), (2000, 5120, 0), (700, 12296, 1),
+                                         (5000, 4096, 1), (3000, 8192, 1), (800, 3584, 0)])
 def test_norm_backward_without_one_row(lib, rows, H, skip):
     g = torch.Generator(device="cuda").manual_seed(rows)
     t = {k: torch.randn(rows, H, generator=g, device="cuda").to(torch.bfloat16) for k in ("x", "g", "skip")}
