@@ -10,7 +10,7 @@ extern "C" {
 
 int hold_back(long row) { return cudaMemcpyToSymbol(heldBackRow, &row, sizeof row); }
 
-int norm_partials(long rows, int H, int add, int sms) { return fcxops::rmsnormPartials(rows, H, add != 0, sms); }
+int norm_partials(long rows, int H, int sms) { return fcxops::rmsnormPartials(rows, H, sms); }
 
 int norm_backward(const void *g, const void *x, const void *w, const float *rstd, const void *add, void *dx, void *dw,
                   float *partial, long rows, int H, int sms) {

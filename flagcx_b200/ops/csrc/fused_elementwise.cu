@@ -21,6 +21,7 @@ namespace {
 
 using bf16 = __nv_bfloat16;
 using fcxops::kNormBwdThreads;
+using fcxops::kNormFewRows;
 
 __device__ __forceinline__ float warpSum(float v) {
 #pragma unroll
@@ -191,42 +192,37 @@ rmsnormFwdWarp(const bf16 *__restrict__ x, const bf16 *__restrict__ w, bf16 *__r
 // per CTA in fp32 (thread t owns the same columns for all of its CTA's rows) and the
 // partials are added up by columnSumToBf16.
 //
-// The backward with the rows brought in by the copy engine.  Each persistent CTA owns a
-// ring of `stages` slots in shared memory; one thread keeps the ring full with bulk
-// asynchronous copies of (g row, x row) that complete on one mbarrier per slot, so several
-// rows per CTA are in flight while the 512 threads reduce and write the current one.
-constexpr int kNormBwdMaxStages = 8, kNormBwdRingBytes = 96 << 10; // two CTAs share an SM
-
+// Few rows: one CTA of 512 threads per row, or two rows for each of the CTAs that run at once.
+// Both come in by bulk asynchronous copies of (g, x, the gradient to be added) that complete on one
+// mbarrier per row and are under way before the first is needed.  Bound: the latency of copy, dot
+// product, block-wide sum and store (64 x 4096 takes 5.7 us with the sum over CTAs that follows).
 template <int MAXP>
 __global__ void __launch_bounds__(kNormBwdThreads)
-rmsnormBwdPipelined(const bf16 *__restrict__ g, const bf16 *__restrict__ x, const bf16 *__restrict__ w,
-                    const float *__restrict__ rstdIn, const bf16 *__restrict__ addIn, bf16 *__restrict__ dx,
-                    float *__restrict__ dwPartial, int rows, int H, int stages) {
-  extern __shared__ __align__(128) unsigned char ring[];
+rmsnormBwdFewRows(const bf16 *__restrict__ g, const bf16 *__restrict__ x, const bf16 *__restrict__ w,
+                  const float *__restrict__ rstdIn, const bf16 *__restrict__ addIn, bf16 *__restrict__ dx,
+                  float *__restrict__ dwPartial, int rows, int H) {
+  extern __shared__ __align__(128) unsigned char slots[];
   __shared__ float red[32];
-  __shared__ __align__(8) uint64_t full[kNormBwdMaxStages];
+  __shared__ __align__(8) uint64_t full[kNormFewRows];
   const int nPacks = H / 8;
   const uint32_t rowBytes = (uint32_t)H * 2u;
   // a slot holds the g row, the x row and, when a gradient of the same shape is to be added
   // to dx (the residual branch around the norm), that gradient's row
   const uint32_t slotBytes = (addIn ? 3u : 2u) * rowBytes;
   if (threadIdx.x == 0) {
-    for (int s = 0; s < stages; ++s) mbarInit(&full[s]);
+    for (int s = 0; s < kNormFewRows; ++s) mbarInit(&full[s]);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    for (int s = 0; s < kNormFewRows; ++s) {
+      const size_t row = blockIdx.x + (size_t)s * gridDim.x;
+      if (row >= (size_t)rows || FLAGCX_OPS_HELD_BACK(row)) continue;
+      unsigned char *dst = slots + (size_t)s * slotBytes;
+      mbarExpect(&full[s], slotBytes);
+      bulkLoad(dst, g + row * H, rowBytes, &full[s]);
+      bulkLoad(dst + rowBytes, x + row * H, rowBytes, &full[s]);
+      if (addIn) bulkLoad(dst + 2 * rowBytes, addIn + row * H, rowBytes, &full[s]);
+    }
   }
   __syncthreads();
-  auto issue = [&](int k) { // thread 0: the row of iteration k into slot k % stages
-    const size_t row = blockIdx.x + (size_t)k * gridDim.x;
-    if (row >= (size_t)rows || FLAGCX_OPS_HELD_BACK(row)) return;
-    const int s = k % stages;
-    unsigned char *dst = ring + (size_t)s * slotBytes;
-    mbarExpect(&full[s], slotBytes);
-    bulkLoad(dst, g + row * H, rowBytes, &full[s]);
-    bulkLoad(dst + rowBytes, x + row * H, rowBytes, &full[s]);
-    if (addIn) bulkLoad(dst + 2 * rowBytes, addIn + row * H, rowBytes, &full[s]);
-  };
-  if (threadIdx.x == 0)
-    for (int k = 0; k < stages; ++k) issue(k);
 
   float dwAcc[MAXP][8];
   Pack8 pw[MAXP];
@@ -238,17 +234,16 @@ rmsnormBwdPipelined(const bf16 *__restrict__ g, const bf16 *__restrict__ x, cons
     for (int i = 0; i < 8; ++i) dwAcc[k][i] = 0.f;
   }
   bool ok = true;
-  int it = 0;
-  for (size_t row = blockIdx.x; row < (size_t)rows; row += gridDim.x, ++it) {
-    const int s = it % stages;
+  for (int s = 0; s < kNormFewRows; ++s) {
+    const size_t row = blockIdx.x + (size_t)s * gridDim.x;
+    if (row >= (size_t)rows) break;
     const float rstd = rstdIn[row];
     // Every thread goes on through the same barriers whatever its wait returned.  After one that
-    // ran out nothing more is fetched, and the rows from there on and this CTA's part of the weight
-    // gradient are NaN; the copies that are out land (or are given as long again) first.
-    if (ok && !(ok = mbarWaitBounded(&full[s], (uint32_t)(it / stages) & 1u)) && threadIdx.x == 0)
-      for (int k = it; k < it + stages && blockIdx.x + (size_t)k * gridDim.x < (size_t)rows; ++k)
-        mbarWaitBounded(&full[k % stages], (uint32_t)(k / stages) & 1u);
-    const uint4 *gs = (const uint4 *)(ring + (size_t)s * slotBytes), *xs = gs + nPacks, *as = xs + nPacks;
+    // ran out this CTA's row (or rows) from there on and its part of the weight gradient are NaN;
+    // the copies that are out land (or are given as long again) first.
+    if (ok && !(ok = mbarWaitBounded(&full[s], 0)) && threadIdx.x == 0)
+      for (int k = s; k < kNormFewRows && blockIdx.x + (size_t)k * gridDim.x < (size_t)rows; ++k) mbarWaitBounded(&full[k], 0);
+    const uint4 *gs = (const uint4 *)(slots + (size_t)s * slotBytes), *xs = gs + nPacks, *as = xs + nPacks;
     Pack8 pg[MAXP], px[MAXP], pa[MAXP];
     float dot = 0.f;
 #pragma unroll
@@ -262,8 +257,7 @@ rmsnormBwdPipelined(const bf16 *__restrict__ g, const bf16 *__restrict__ x, cons
         for (int i = 0; i < 8; ++i) dot += pg[k].get(i) * pw[k].get(i) * px[k].get(i);
       }
     }
-    dot = blockSum(ok ? dot : NAN, red); // all threads have read the slot once its barriers are passed
-    if (threadIdx.x == 0 && ok) issue(it + stages);
+    dot = blockSum(ok ? dot : NAN, red);
     const float c = dot * rstd * rstd / H;
     uint4 *dxr = (uint4 *)(dx + row * H);
 #pragma unroll
@@ -295,8 +289,7 @@ rmsnormBwdPipelined(const bf16 *__restrict__ g, const bf16 *__restrict__ x, cons
   }
 }
 
-// The same where one row does not keep 512 threads busy (norm_route.h says where the line
-// lies).  A CTA is cut into groups of GT threads, the fewest (a power of two from 32) that hold a row with four packs
+// The same for more rows (norm_route.h says where the line lies).  A CTA is cut into groups of GT threads, the fewest (a power of two from 32) that hold a row with four packs
 // per thread; every group owns a ring of row slots in shared memory, which its first thread
 // keeps full with bulk copies that complete on one mbarrier per slot, and reduces its rows by
 // itself: shuffles, and for GT > 32 one named barrier of the group.  So a CTA has 512 / GT rows
@@ -1033,8 +1026,8 @@ cudaError_t rmsnormForward(const void *x, const void *w, void *y, float *rstd, l
   return cudaGetLastError();
 }
 
-int rmsnormPartials(long rows, int H, bool add, int sms) {
-  if (rmsnormRowPerCta(rows, H, add, sms)) return (int)std::max<long>(1, std::min<long>(rows, sms * 2));
+int rmsnormPartials(long rows, int H, int sms) {
+  if (rmsnormRowPerCta(rows, H, sms)) return (int)std::max<long>(1, std::min<long>(rows, sms * 2));
   int ctas = 0;
   withNormShape(H / 8, [&](auto gt, auto) {
     constexpr int G = kNormThreads / decltype(gt)::value;
@@ -1046,17 +1039,15 @@ int rmsnormPartials(long rows, int H, bool add, int sms) {
 
 cudaError_t rmsnormBackward(const void *g, const void *x, const void *w, const float *rstd, const void *add, void *dx, void *dw,
                             float *partial, long rows, int H, int sms, cudaStream_t stream) {
-  const int ctas = rmsnormPartials(rows, H, add != nullptr, sms);
-  if (rmsnormRowPerCta(rows, H, add != nullptr, sms)) {
-    // ring of (g, x, add) slots, two at least (8192 x 6 bytes each)
-    const size_t slot = (size_t)H * (add ? 6 : 4);
-    const int stages = (int)std::min<size_t>(kNormBwdMaxStages, kNormBwdRingBytes / slot);
-    const size_t smem = slot * stages;
+  const int ctas = rmsnormPartials(rows, H, sms);
+  if (rmsnormRowPerCta(rows, H, sms)) {
+    const int shared = H * (add ? 6 : 4) * (rows > ctas ? kNormFewRows : 1);
     auto launch = [&](auto tag) {
-      constexpr auto kern = rmsnormBwdPipelined<decltype(tag)::value>;
-      RETURN_IF(allowShared<kern>(kNormBwdRingBytes));
-      kern<<<ctas, kNormBwdThreads, smem, stream>>>((const bf16 *)g, (const bf16 *)x, (const bf16 *)w, rstd, (const bf16 *)add,
-                                                    (bf16 *)dx, partial, (int)rows, H, stages);
+      constexpr int MAXP = decltype(tag)::value;
+      constexpr auto kern = rmsnormBwdFewRows<MAXP>;
+      RETURN_IF(allowShared<kern>(kNormFewRows * MAXP * kNormBwdThreads * 8 * 6));
+      kern<<<ctas, kNormBwdThreads, shared, stream>>>((const bf16 *)g, (const bf16 *)x, (const bf16 *)w, rstd, (const bf16 *)add,
+                                                      (bf16 *)dx, partial, (int)rows, H);
       return cudaGetLastError();
     };
     if (H / 8 <= kNormBwdThreads) RETURN_IF(launch(std::integral_constant<int, 1>()));

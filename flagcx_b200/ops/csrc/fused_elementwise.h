@@ -10,8 +10,8 @@ namespace fcxops {
 
 cudaError_t rmsnormForward(const void *x, const void *w, void *y, float *rstd, long rows, int H, float eps, int sms,
                            cudaStream_t stream);
-// partial: scratch of rmsnormPartials(rows, H, add != null, sms) x H floats; add may be null
-int rmsnormPartials(long rows, int H, bool add, int sms);
+// partial: scratch of rmsnormPartials(rows, H, sms) x H floats; add may be null
+int rmsnormPartials(long rows, int H, int sms);
 cudaError_t rmsnormBackward(const void *g, const void *x, const void *w, const float *rstd, const void *add, void *dx, void *dw,
                             float *partial, long rows, int H, int sms, cudaStream_t stream);
 cudaError_t rope(void *x, const int *positions, int tokens, int heads, int D, float logTheta, float sign, int sms,

@@ -59,7 +59,7 @@ std::vector<at::Tensor> rmsnorm_bwd(const at::Tensor &g, const at::Tensor &x, co
   auto dx = at::empty_like(x);
   TORCH_CHECK(H % 8 == 0 && H <= 8 * 512 * 4 && w.numel() == H, "rmsnorm: hidden size must be a multiple of 8, at most 16384");
   const int sms = smCount();
-  auto partial = at::empty({fcxops::rmsnormPartials(rows, H, add.has_value(), sms), H}, x.options().dtype(at::kFloat));
+  auto partial = at::empty({fcxops::rmsnormPartials(rows, H, sms), H}, x.options().dtype(at::kFloat));
   auto dw = at::empty({H}, x.options());
   if (rows == 0) {
     dw.zero_();

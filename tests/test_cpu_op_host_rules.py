@@ -16,15 +16,20 @@ def _run(tmp_path, text, flags=()):
 
 
 def test_norm_backward_of_few_rows_runs_one_row_per_cta(tmp_path):
-    # rows, hidden size, skip gradient -> one row per CTA, where both kernels were measured and
-    # differ by more than 3 % on 148 SMs
-    cases = [(1, 1024, 0, 1), (64, 4096, 0, 1), (148, 8192, 1, 1), (257, 2048, 1, 1), (257, 3584, 0, 1), (592, 1024, 1, 1),
-             (800, 3584, 1, 1), (8192, 7168, 1, 1), (4096, 4096, 1, 1), (257, 256, 1, 1), (360, 2560, 0, 1), (8192, 8192, 1, 1),
-             (592, 256, 0, 0), (4096, 256, 1, 0), (1021, 2048, 1, 0), (592, 3072, 0, 0), (200, 5120, 1, 0), (257, 7168, 1, 0),
-             (4096, 5120, 0, 0), (4096, 4096, 0, 0), (148, 12288, 0, 0), (1, 16384, 1, 0), (2048, 1024, 0, 0)]
-    rows = "".join(f"  bad += fcxops::rmsnormRowPerCta({r}, {h}, {s}, 148) != {w} && printf(\"{r} x {h} skip {s}\\n\");\n"
-                   for r, h, s, w in cases)
-    _run(tmp_path, '#include <cstdio>\n#include "norm_route.h"\nint main() {\n  int bad = 0;\n' + rows + "  return bad != 0;\n}\n")
+    # rows, hidden size -> one row per CTA, where both kernels were measured and differ by more
+    # than 3 % on 148 SMs
+    cases = [(1, 1024, 1), (64, 4096, 1), (148, 8192, 1), (257, 2048, 1), (257, 3584, 1), (592, 1024, 1), (257, 768, 1), (360, 3584, 1),
+             (16, 256, 1), (592, 2048, 1), (296, 1536, 1), (592, 256, 0), (4096, 256, 0), (1021, 2048, 0), (592, 3072, 0),
+             (200, 5120, 0), (257, 7168, 0), (4096, 5120, 0), (4096, 4096, 0), (8192, 7168, 0), (1024, 1024, 0), (200, 8192, 0)]
+    rows = "".join(f"  bad += fcxops::rmsnormRowPerCta({r}, {h}, 148) != {w} && printf(\"{r} x {h}\\n\");\n" for r, h, w in cases)
+    _run(tmp_path, '#include <cstdio>\n#include <initializer_list>\n#include "norm_route.h"\nint main() {\n  int bad = 0;\n' + rows + """
+  for (int sms : {1, 20, 148}) // no CTA ever gets more rows than the kernel has slots for
+    for (int H = 8; H <= 16384; H += 8)
+      for (long rows = 1; rows <= 5 * sms; ++rows)
+        if (fcxops::rmsnormRowPerCta(rows, H, sms)) bad += rows > fcxops::kNormFewRows * (rows < 2 * sms ? rows : 2L * sms) || H > 8192;
+  return bad != 0;
+}
+""")
 
 
 def test_a_limit_is_set_once_per_device_and_never_skipped(tmp_path):
