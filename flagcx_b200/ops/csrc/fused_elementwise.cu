@@ -948,14 +948,17 @@ cudaError_t allowShared(int bytes) {
 }
 
 // Calls f(GT, PPT) for rows of `packs` packs of 8: the smallest group whose threads hold a row
-// with at most four packs each (512 threads and four packs: 16384 elements).
+// with at most four packs each (512 threads and four packs: 16384 elements), so three or four in
+// every group but the smallest.
 template <typename F>
 cudaError_t withNormShape(int packs, F &&f) {
   auto ppt = [&](auto gt) -> cudaError_t {
     constexpr int GT = decltype(gt)::value;
     const int n = (packs + GT - 1) / GT;
-    if (n <= 1) return f(gt, std::integral_constant<int, 1>());
-    if (n <= 2) return f(gt, std::integral_constant<int, 2>());
+    if constexpr (GT == 32) {
+      if (n <= 1) return f(gt, std::integral_constant<int, 1>());
+      if (n <= 2) return f(gt, std::integral_constant<int, 2>());
+    }
     if (n <= 3) return f(gt, std::integral_constant<int, 3>());
     return f(gt, std::integral_constant<int, 4>());
   };
