@@ -18,4 +18,9 @@ int norm_backward(const void *g, const void *x, const void *w, const float *rstd
   return e != cudaSuccess ? e : cudaDeviceSynchronize();
 }
 
+int cross_entropy(void *logits, const long *targets, float *loss, long rows, int V, float gradScale, int sms) {
+  const cudaError_t e = fcxops::crossEntropy(logits, targets, loss, rows, V, gradScale, sms, nullptr);
+  return e != cudaSuccess ? e : cudaDeviceSynchronize();
+}
+
 } // extern "C"

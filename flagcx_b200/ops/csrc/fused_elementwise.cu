@@ -681,6 +681,7 @@ crossEntropyRows(bf16 *__restrict__ logits, const long *__restrict__ targets, fl
   const uint4 *slot = (const uint4 *)ceSlot;
   auto part = [&](long row) { return (unsigned char *)(logits + (size_t)row * V + (size_t)p0 * 8); };
   auto issue = [&](long row) { // thread 0
+    if (FLAGCX_OPS_HELD_BACK(row)) return;
     mbarExpect(&bar, bytes);
     for (uint32_t off = 0; off < bytes; off += kCeBulkPiece)
       bulkLoad(ceSlot + off, part(row) + off, min(kCeBulkPiece, bytes - off), &bar);
@@ -693,9 +694,11 @@ crossEntropyRows(bf16 *__restrict__ logits, const long *__restrict__ targets, fl
   }
   __syncthreads();
   constexpr float kLog2e = 1.4426950408889634f;
-  bool ok = true; // a copy that never arrived poisons the loss and the gradient of its row
+  // A copy that never arrived makes the loss and the gradient of its row NaN, and those of the rows
+  // after it, which are not fetched; it is given as long again to land before the CTA may leave.
+  bool ok = true;
   for (int it = 0; row < rows; row += step, ++it) {
-    if (n > 0 && ok) ok = mbarWaitBounded(&bar, (uint32_t)it & 1u);
+    if (n > 0 && ok && !(ok = mbarWaitBounded(&bar, (uint32_t)it & 1u)) && tid == 0) mbarWaitBounded(&bar, (uint32_t)it & 1u);
     const long tLocal = targets[row] - (long)p0 * 8; // index of the target inside this CTA's part, if it is here
     const bool own = tLocal >= 0 && tLocal < (long)n * 8;
     const float tgtLogit = own ? __bfloat162float(((const bf16 *)ceSlot)[tLocal]) : 0.f;

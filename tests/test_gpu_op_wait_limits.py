@@ -16,6 +16,7 @@ def lib():
     so.hold_back.argtypes = [ctypes.c_long]
     so.norm_partials.argtypes = [ctypes.c_long, ctypes.c_int, ctypes.c_int]
     so.norm_backward.argtypes = [ctypes.c_void_p] * 8 + [ctypes.c_long, ctypes.c_int, ctypes.c_int]
+    so.cross_entropy.argtypes = [ctypes.c_void_p] * 3 + [ctypes.c_long, ctypes.c_int, ctypes.c_float, ctypes.c_int]
     yield so
     so.hold_back(-1)
 
@@ -49,4 +50,31 @@ def test_norm_backward_without_one_row(lib, rows, H, skip):
     assert torch.equal(dx[~lost], whole[0][~lost])
     assert bool(dw.isnan().all())
     again = _norm_backward(lib, t, rows, H, skip, -1)
+    assert all(torch.equal(a, b) for a, b in zip(again, whole))
+
+
+def _cross_entropy(lib, logits, targets, held):
+    assert lib.hold_back(held) == 0
+    rows, V = logits.shape
+    d, loss = logits.clone(), torch.full((rows,), 7.0, device="cuda")
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    assert lib.cross_entropy(d.data_ptr(), targets.data_ptr(), loss.data_ptr(), rows, V, 1.0 / rows, sms) == 0
+    return d, loss
+
+
+# one, two, four and eight CTAs per row, with several rows for each
+@pytest.mark.parametrize("rows,V", [(5000, 1024), (900, 32768), (700, 65536), (600, 128256), (300, 262144)])
+def test_cross_entropy_without_one_row(lib, rows, V):
+    g = torch.Generator(device="cuda").manual_seed(V)
+    logits = torch.randn(rows, V, generator=g, device="cuda").to(torch.bfloat16)
+    targets = torch.randint(0, V, (rows,), generator=g, device="cuda")
+    whole = _cross_entropy(lib, logits, targets, -1)
+    assert not whole[0].isnan().any() and not whole[1].isnan().any()
+    held = rows // 2 + 1
+    d, loss = _cross_entropy(lib, logits, targets, held)
+    lost = loss.isnan()
+    assert bool(lost[held]) and not bool(lost[:held].any()) and not bool(lost[held:].all())
+    assert bool(d[lost].isnan().all())
+    assert torch.equal(loss[~lost], whole[1][~lost]) and torch.equal(d[~lost], whole[0][~lost])
+    again = _cross_entropy(lib, logits, targets, -1)
     assert all(torch.equal(a, b) for a, b in zip(again, whole))
