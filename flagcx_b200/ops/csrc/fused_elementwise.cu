@@ -807,11 +807,12 @@ crossEntropyCluster(bf16 *__restrict__ logits, const long *__restrict__ targets,
   __syncthreads();
   bool ok = true;
   if (n > 0) {
-    if (threadIdx.x == 0) {
+    if (threadIdx.x == 0 && !FLAGCX_OPS_HELD_BACK(row)) {
       mbarExpect(&bar, bytes);
       for (uint32_t off = 0; off < bytes; off += kCeBulkPiece) bulkLoad(ceRow + off, gRow + off, min(kCeBulkPiece, bytes - off), &bar);
     }
     ok = mbarWaitBounded(&bar, 0);
+    if (!ok && threadIdx.x == 0) mbarWaitBounded(&bar, 0); // nothing is written over a copy that is under way
   }
 
   const long tLocal = targets[row] - (long)p0 * 8; // index of the target inside this CTA's part, if it is here
@@ -844,10 +845,10 @@ crossEntropyCluster(bf16 *__restrict__ logits, const long *__restrict__ targets,
     }
     buf[p] = e;
   }
-  sum = blockSum(sum, red);
+  sum = blockSum(ok ? sum : NAN, red); // a copy that never arrived makes the whole row's loss and gradient NaN
   if (threadIdx.x == 0) {
     stat[0] = mx;
-    stat[1] = ok ? sum : NAN; // a copy that never arrived poisons the whole row's loss and gradient
+    stat[1] = sum;
   }
   cluster.sync();
   float M = -INFINITY, S = 0.f;
@@ -876,7 +877,7 @@ crossEntropyCluster(bf16 *__restrict__ logits, const long *__restrict__ targets,
     ((bf16 *)ceRow)[tLocal] = __float2bfloat16_rn(exp2f(fmaf(tgtLogit, kLog2e, -mxs)) * f - gradScale);
   asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); // the stores above, before the engine reads them
   __syncthreads();
-  if (threadIdx.x == 0 && n > 0 && ok) {
+  if (threadIdx.x == 0 && n > 0) {
     for (uint32_t off = 0; off < bytes; off += kCeBulkPiece) {
       const uint32_t sz = min(kCeBulkPiece, bytes - off);
       asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;" ::"l"(gRow + off),

@@ -62,8 +62,9 @@ def _cross_entropy(lib, logits, targets, held):
     return d, loss
 
 
-# one, two, four and eight CTAs per row, with several rows for each
-@pytest.mark.parametrize("rows,V", [(5000, 1024), (900, 32768), (700, 65536), (600, 128256), (300, 262144)])
+# one, two, four and eight CTAs per row, with several rows for each, and the kernel that takes one
+# row per cluster
+@pytest.mark.parametrize("rows,V", [(5000, 1024), (900, 32768), (700, 65536), (600, 128256), (300, 262144), (5, 262152)])
 def test_cross_entropy_without_one_row(lib, rows, V):
     g = torch.Generator(device="cuda").manual_seed(V)
     logits = torch.randn(rows, V, generator=g, device="cuda").to(torch.bfloat16)
