@@ -88,11 +88,8 @@ class _RMSNormBranch(torch.autograd.Function):
 
     @staticmethod
     def backward(ctx, g, g_skip):
-        x, weight, rstd = ctx.saved_tensors
-        if g is None:  # only the skip connection was used
-            return g_skip, None, None
-        add = g_skip.contiguous() if g_skip is not None else None
-        dx, dw = ext().rmsnorm_bwd(g.contiguous(), x, weight, rstd, add)
+        x, weight, rstd = ctx.saved_tensors  # an output that was not used has a gradient of zeros here
+        dx, dw = ext().rmsnorm_bwd(g.contiguous(), x, weight, rstd, g_skip.contiguous())
         _count()
         return dx, dw, None
 

@@ -188,11 +188,8 @@ struct RmsNormBranchFunction : public Function<RmsNormBranchFunction> {
     return {r[0], x.view_as(x)};
   }
   static variable_list backward(AutogradContext *ctx, variable_list g) {
-    auto s = ctx->get_saved_variables();
-    if (!g[0].defined()) return {g[1], at::Tensor(), at::Tensor()}; // only the skip connection was used
-    c10::optional<at::Tensor> add;
-    if (g[1].defined()) add = g[1].contiguous();
-    auto r = rmsnorm_bwd(g[0].contiguous(), s[0], s[1], s[2], add);
+    auto s = ctx->get_saved_variables(); // an output that was not used has a gradient of zeros here
+    auto r = rmsnorm_bwd(g[0].contiguous(), s[0], s[1], s[2], g[1].contiguous());
     ++launches;
     return {r[0], r[1], at::Tensor()};
   }

@@ -195,6 +195,12 @@ def test_norm_branch_and_residual_linear_match_the_unfused_graph():
     _, skip2 = ops.rmsnorm_branch(x2, wn.detach(), 1e-5)
     skip2.backward(g)
     assert torch.equal(x2.grad, g)
+    # one output used, in both implementations: the other one's gradient counts as zeros
+    for fn in (ops.rmsnorm_branch, ops._RMSNormBranch.apply):
+        dx, dw = torch.autograd.grad(fn(x, wn, 1e-5)[1], (x, wn), g)
+        assert torch.equal(dx, g) and not dw.any()
+        one = torch.autograd.grad(fn(x, wn, 1e-5)[0], (x, wn), g)
+        assert all(torch.equal(a, b) for a, b in zip(one, torch.autograd.grad(ops.rmsnorm(x, wn, 1e-5), (x, wn), g)))
 
 
 def test_swiglu_forward_backward():
