@@ -34,7 +34,7 @@ def build(verbose: bool = False) -> str:
         name=NAME,
         sources=[os.path.join(HERE, "csrc", s) for s in SOURCES],
         extra_cuda_cflags=NVCC_FLAGS,
-        extra_cflags=["-O2", "-std=c++17"],
+        extra_cflags=["-O3", "-std=c++17"],
         build_directory=build_dir,
         with_cuda=True,
         is_python_module=False,
