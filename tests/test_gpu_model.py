@@ -17,9 +17,9 @@ def _ops():
 def test_rmsnorm_forward_backward():
     ops = _ops()
     torch.manual_seed(0)
-    # widths: each forward variant (4 / 8 / 16 packs per lane, then one CTA per row) and each
-    # backward variant; 2500 rows make every persistent CTA of the backward wrap its ring of
-    # shared-memory slots, 37 rows leave most of the grid without work
+    # widths: each forward variant (4 / 8 / 16 packs per lane, then one CTA per row); the backward
+    # in groups with several rows each (2500, 700 rows) and with one row per CTA, most of the grid
+    # without work (37 rows)
     for rows, H in ((2500, 256), (37, 1000), (37, 2048), (2500, 4096), (37, 4096), (700, 8192), (37, 16384)):
         x = torch.randn(rows, H, device="cuda", dtype=torch.bfloat16, requires_grad=True)
         w = (1 + 0.1 * torch.randn(H, device="cuda")).to(torch.bfloat16).requires_grad_()
@@ -34,10 +34,14 @@ def test_rmsnorm_forward_backward():
         assert ((w.grad.float() - wf.grad).abs() / wf.grad.abs().clamp(min=1)).max() < 0.05, (rows, H)
 
 
-# every group size of the backward (32 to 512 threads, one to four packs each), the line where one
-# row per CTA takes over (0.9 of 512 threads), a single row, and rows that the groups share unevenly
+# one row per CTA (one and two packs of 8 per thread) and two, to the last count of rows; then every
+# group size (32 to 512 threads, one to four packs each), from the first count of rows that takes
+# groups to several more rows than a ring has slots, which the groups share unevenly
 @pytest.mark.parametrize("rows,H", [(1, 8), (17, 256), (5, 1024), (33, 1032), (300, 2048), (7, 2056), (149, 3688), (149, 3680),
-                                    (9, 4104), (200, 7176), (3, 8200), (5, 12296), (2, 16384), (2500, 264)])
+                                    (9, 4104), (200, 7176), (3, 8200), (5, 12296), (2, 16384), (2500, 264),
+                                    (148, 8192), (592, 1024), (593, 1024), (444, 3584), (445, 4096), (296, 2560), (297, 2560),
+                                    (17000, 256), (16600, 1024), (4800, 2048), (9000, 1288), (4200, 2560), (2500, 4096),
+                                    (1300, 7176), (2000, 5120), (1300, 8192), (1000, 12296), (700, 16384)])
 @pytest.mark.parametrize("skip", [True, False])
 def test_rmsnorm_backward_at_the_edges_of_its_row_groups(rows, H, skip):
     ops = _ops()
@@ -240,11 +244,17 @@ def test_cross_entropy_loss_and_gradient(T, V):
         assert rel < 1.2e-2
 
 
-# edges of what one CTA of a row holds (256 threads x 1, 2, 4, 8, 10, 13, 16 packs of 8, one to
-# eight CTAs per row), the last row size of the persistent kernel and the first of the next one,
-# and more rows than clusters run at once; a stretch of -inf (masked vocabulary) in every second row
+# few rows, which are spread over up to eight CTAs each; then the edges of what one CTA holds (256
+# threads x 1, 2, 4, 8, 10, 13, 16 packs of 8) with 300 rows and more, so that a row stays with as few
+# CTAs as can hold it, and with several rows for each of them: one (up to 32768 columns), two, four
+# and eight CTAs per row; the last row size of the persistent kernel and the first of the next one.
+# A stretch of -inf (masked vocabulary) in every second row
 @pytest.mark.parametrize("T,V", [(1, 8), (3, 2048), (5, 2056), (2, 4104), (3, 8200), (2, 16392), (2, 20488), (3, 32768),
-                                 (2, 32776), (7, 65544), (2, 151936), (700, 128256), (2, 262144), (2, 262152)])
+                                 (2, 32776), (7, 65544), (2, 151936), (700, 128256), (2, 262144), (2, 262152),
+                                 (5000, 1024), (3000, 2048), (3000, 2056), (3000, 4096), (3000, 4104), (1500, 8192), (1500, 8200),
+                                 (900, 16384), (700, 16392), (700, 20480), (500, 20488), (500, 26624), (500, 26632), (500, 32768),
+                                 (500, 32776), (400, 40960), (400, 65536), (300, 65544), (300, 100352), (300, 131080),
+                                 (300, 151936), (300, 262144)])
 def test_cross_entropy_at_the_edges_of_its_row_split(T, V):
     ops = _ops()
     g = torch.Generator(device="cuda").manual_seed(V)

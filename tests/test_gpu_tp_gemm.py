@@ -25,12 +25,15 @@ def test_tcgen05_gemm_matches_fp32_reference(M, N, K, pair, monkeypatch):
     assert err < 2 ** -7, err
 
 
-# parts that do not divide K's steps or the 128 rows of a tile, one step per part, and what the
-# size rule picks at the ends of its range (0: automatic)
-@pytest.mark.parametrize("M,N,K,parts", [(128, 256, 512, 8), (128, 512, 2112, 3), (384, 256, 576, 5), (256, 768, 1024, 7),
-                                         (128, 256, 128, 2), (128, 256, 256, 0), (128, 3584, 8192, 0), (1024, 2048, 320, 0),
-                                         (512, 256, 4160, 0)])
-@pytest.mark.parametrize("tile_n", [256, 128, 64])
+# parts that do not divide K's steps or the 128 rows of a tile and one step per part, with every
+# tile width; and what the size rule picks (parts 0), on both sides of its lines
+@pytest.mark.parametrize("M,N,K,parts,tile_n",
+                         [(M, N, K, parts, t) for M, N, K, parts in
+                          [(128, 256, 512, 8), (128, 512, 2112, 3), (384, 256, 576, 5), (256, 768, 1024, 7), (128, 256, 128, 2)]
+                          for t in (256, 128, 64)] +
+                         [(M, N, K, 0, 256) for M, N, K in
+                          [(128, 256, 256), (128, 3584, 8192), (1024, 2048, 320), (512, 256, 4160), (896, 2048, 2240),
+                           (1664, 768, 1024), (256, 256, 5120)]])
 def test_gemm_with_k_split_over_a_cluster(M, N, K, parts, tile_n, monkeypatch):
     from flagcx_b200.parallel.tp import gemm_bf16
     monkeypatch.setenv("FLAGCX_GEMM_SPLIT", str(parts))
