@@ -15,10 +15,14 @@
 
 namespace {
 
+// The address of a tensor's elements for a kernel.  Asking with the element type is refused where
+// there is no memory (fake and meta tensors); asked without, they give a null pointer.
+void *data(const at::Tensor &t) { return t.numel() ? t.data_ptr<at::BFloat16>() : nullptr; }
+
 void checkBf16(const at::Tensor &t, const char *name) {
   TORCH_CHECK(t.is_cuda() && t.scalar_type() == at::kBFloat16 && t.is_contiguous(), name,
               " must be a contiguous CUDA bfloat16 tensor");
-  TORCH_CHECK(((uintptr_t)t.data_ptr() & 15) == 0, name, " must be 16-byte aligned");
+  TORCH_CHECK(((uintptr_t)data(t) & 15) == 0, name, " must be 16-byte aligned");
 }
 
 void checkLaunch(cudaError_t e) {
@@ -37,7 +41,7 @@ std::vector<at::Tensor> rmsnorm_fwd(const at::Tensor &x, const at::Tensor &w, do
   auto y = at::empty_like(x);
   auto rstd = at::empty({rows}, x.options().dtype(at::kFloat));
   if (rows > 0)
-    checkLaunch(fcxops::rmsnormForward(x.data_ptr(), w.data_ptr(), y.data_ptr(), rstd.data_ptr<float>(), rows, H, (float)eps,
+    checkLaunch(fcxops::rmsnormForward(data(x), data(w), data(y), rstd.data_ptr<float>(), rows, H, (float)eps,
                                           smCount(), at::cuda::getCurrentCUDAStream()));
   return {y, rstd};
 }
@@ -65,8 +69,8 @@ std::vector<at::Tensor> rmsnorm_bwd(const at::Tensor &g, const at::Tensor &x, co
     dw.zero_();
     return {dx, dw};
   }
-  checkLaunch(fcxops::rmsnormBackward(g.data_ptr(), x.data_ptr(), w.data_ptr(), rstd.data_ptr<float>(),
-                                         add.has_value() ? add->data_ptr() : nullptr, dx.data_ptr(), dw.data_ptr(),
+  checkLaunch(fcxops::rmsnormBackward(data(g), data(x), data(w), rstd.data_ptr<float>(),
+                                         add.has_value() ? data(*add) : nullptr, data(dx), data(dw),
                                          partial.data_ptr<float>(), rows, H, sms, at::cuda::getCurrentCUDAStream()));
   return {dx, dw};
 }
@@ -83,7 +87,7 @@ void rope_inplace(at::Tensor &x, const c10::optional<at::Tensor> &positions, dou
     pos = positions->data_ptr<int>();
   }
   const c10::cuda::CUDAGuard guard(x.device());
-  checkLaunch(fcxops::rope(x.data_ptr(), pos, (int)tokens, heads, D, logf((float)theta), backward ? -1.f : 1.f, smCount(),
+  checkLaunch(fcxops::rope(data(x), pos, (int)tokens, heads, D, logf((float)theta), backward ? -1.f : 1.f, smCount(),
                               at::cuda::getCurrentCUDAStream()));
 }
 
@@ -96,7 +100,7 @@ at::Tensor rope_fused_qkv(const at::Tensor &qkv, int64_t ropeHeads, int64_t tota
   const c10::cuda::CUDAGuard guard(qkv.device());
   auto out = at::empty_like(qkv);
   if (qkv.numel() == 0) return out;
-  checkLaunch(fcxops::ropeQkv(qkv.data_ptr(), out.data_ptr(), (int)tokens, (int)ropeHeads, (int)totalHeads, (int)D,
+  checkLaunch(fcxops::ropeQkv(data(qkv), data(out), (int)tokens, (int)ropeHeads, (int)totalHeads, (int)D,
                                  logf((float)theta), backward ? -1.f : 1.f, smCount(), at::cuda::getCurrentCUDAStream()));
   return out;
 }
@@ -110,7 +114,7 @@ at::Tensor swiglu_fwd(const at::Tensor &ab) {
   sizes.back() = F;
   auto out = at::empty(sizes, ab.options());
   size_t T = ab.numel() / (2 * (size_t)F);
-  checkLaunch(fcxops::swigluForward(ab.data_ptr(), out.data_ptr(), T, F, smCount(), at::cuda::getCurrentCUDAStream()));
+  checkLaunch(fcxops::swigluForward(data(ab), data(out), T, F, smCount(), at::cuda::getCurrentCUDAStream()));
   return out;
 }
 
@@ -121,7 +125,7 @@ at::Tensor swiglu_bwd(const at::Tensor &g, const at::Tensor &ab) {
   const c10::cuda::CUDAGuard guard(ab.device());
   auto dab = at::empty_like(ab);
   size_t T = ab.numel() / (2 * (size_t)F);
-  checkLaunch(fcxops::swigluBackward(g.data_ptr(), ab.data_ptr(), dab.data_ptr(), T, F, smCount(),
+  checkLaunch(fcxops::swigluBackward(data(g), data(ab), data(dab), T, F, smCount(),
                                         at::cuda::getCurrentCUDAStream()));
   return dab;
 }
@@ -137,7 +141,7 @@ at::Tensor cross_entropy_fwd_bwd_(at::Tensor &logits, const at::Tensor &targets,
   const c10::cuda::CUDAGuard guard(logits.device());
   auto loss = at::empty({rows}, logits.options().dtype(at::kFloat));
   if (rows == 0) return loss;
-  checkLaunch(fcxops::crossEntropy(logits.data_ptr(), targets.data_ptr<int64_t>(), loss.data_ptr<float>(), rows, V,
+  checkLaunch(fcxops::crossEntropy(data(logits), targets.data_ptr<int64_t>(), loss.data_ptr<float>(), rows, V,
                                       (float)gradScale, smCount(), at::cuda::getCurrentCUDAStream()));
   return loss;
 }
@@ -153,7 +157,7 @@ void adamw_flat_(at::Tensor &p, const at::Tensor &g, at::Tensor &m, at::Tensor &
   const size_t n = p.numel();
   if (n == 0) return;
   float bc1 = 1.f - (float)std::pow(beta1, (double)step), bc2 = 1.f - (float)std::pow(beta2, (double)step);
-  checkLaunch(fcxops::adamw(p.data_ptr(), g.data_ptr(), m.data_ptr(), v.data_ptr(), n, (float)lr, (float)beta1, (float)beta2,
+  checkLaunch(fcxops::adamw(data(p), data(g), data(m), data(v), n, (float)lr, (float)beta1, (float)beta2,
                                (float)eps, (float)wd, bc1, bc2, smCount(), at::cuda::getCurrentCUDAStream()));
 }
 

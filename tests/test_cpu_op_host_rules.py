@@ -92,3 +92,21 @@ def test_launch_count_can_be_set():
         assert ops.launch_count == 7
     finally:
         ops.launch_count = before
+
+
+def test_tensors_without_memory_are_refused():
+    """Fake tensors (export, shape propagation) have no address: a kernel must not get it."""
+    import pytest
+    import torch
+    from torch._subclasses.fake_tensor import FakeTensorMode
+    from flagcx_b200 import ops
+    e = ops.ext()
+    with FakeTensorMode():
+        x = torch.empty(4, 512, device="cuda", dtype=torch.bfloat16)
+        w, r, t = x.new_empty(512), x.new_empty(4, dtype=torch.float32), x.new_empty(4, dtype=torch.long)
+        for call in (lambda: ops.swiglu(x), lambda: ops.rmsnorm_branch(x, w), lambda: ops.rope_fused_qkv(x, 4, 2, 64),
+                     lambda: e.swiglu_bwd(x[:, :256].contiguous(), x), lambda: e.rmsnorm_bwd(x, x, w, r),
+                     lambda: e.rope_inplace(x.view(4, 8, 64), None, 1e4, False), lambda: e.cross_entropy_fwd_bwd_(x, t, 1.0),
+                     lambda: ops.adamw_flat_(x, x, x, x, 1e-3, 0.9, 0.95, 1e-8, 0.1, 1)):
+            with pytest.raises(RuntimeError, match="not allocated"):
+                call()

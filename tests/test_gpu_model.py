@@ -126,6 +126,18 @@ def test_operators_keep_hooks_tracing_and_transforms():
         ops.swiglu(torch.autograd.forward_ad.make_dual(g, other))
 
 
+def test_results_without_memory_are_refused():
+    """Under a mode that makes every new tensor a fake one."""
+    from torch._subclasses.fake_tensor import FakeTensorMode
+    ops = _ops()
+    x = torch.randn(3, 512, device="cuda").to(torch.bfloat16)
+    for call in (lambda: ops.swiglu(x), lambda: ops.rmsnorm(x, x[0]), lambda: ops.rope_fused_qkv(x, 4, 2, 64),
+                 lambda: ops.ext().swiglu_bwd(x, torch.cat([x, x], 1))):
+        with FakeTensorMode(allow_non_fake_inputs=True), pytest.raises(RuntimeError, match="not allocated"):
+            call()
+    assert not ops.swiglu(x).isnan().any()
+
+
 def test_rope_matches_reference_and_backward_is_inverse():
     ops = _ops()
     T, Hn, D = 64, 4, 128
