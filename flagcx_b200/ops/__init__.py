@@ -43,12 +43,16 @@ def _count(n=1):
     _launches += n
 
 
-def _in_python():
+_PLAIN = (torch.Tensor, torch.nn.Parameter)
+
+
+def _in_python(x):
     """Whether an operator has to go through its torch.autograd.Function below: a tracer records
-    that as a call, and function transforms and forward-mode differentiation refuse it with their
-    own errors.  Otherwise the same function in C++ (torch_ops.cpp) is used."""
-    return (torch._C._get_tracing_state() is not None or torch._C._are_functorch_transforms_active()
-            or _forward_ad._current_level >= 0)
+    that as a call, function transforms and forward-mode differentiation refuse it with their own
+    errors, and a tensor subclass sees the operations on it.  Otherwise the same function in C++
+    (torch_ops.cpp) is used."""
+    return (type(x) not in _PLAIN or torch._C._get_tracing_state() is not None
+            or torch._C._are_functorch_transforms_active() or _forward_ad._current_level >= 0)
 
 
 class _RMSNorm(torch.autograd.Function):
@@ -68,7 +72,7 @@ class _RMSNorm(torch.autograd.Function):
 
 
 def rmsnorm(x: torch.Tensor, weight: torch.Tensor, eps: float = 1e-5) -> torch.Tensor:
-    if _in_python():
+    if _in_python(x):
         return _RMSNorm.apply(x.contiguous(), weight, eps)
     return ext().rmsnorm(x, weight, eps)
 
@@ -96,7 +100,7 @@ class _RMSNormBranch(torch.autograd.Function):
 
 def rmsnorm_branch(x: torch.Tensor, weight: torch.Tensor, eps: float = 1e-5):
     """(rmsnorm(x), x): see _RMSNormBranch.  Use the second value for the residual add."""
-    if _in_python():
+    if _in_python(x):
         return _RMSNormBranch.apply(x.contiguous(), weight, eps)
     return ext().rmsnorm_branch(x, weight, eps)
 
@@ -142,7 +146,7 @@ def rope_fused_qkv(qkv: torch.Tensor, n_heads: int, n_kv_heads: int, head_dim: i
     (queries, keys, values side by side).  Rotates the query and key heads (token t at
     position t) and copies the value heads, in one pass; q, k and v are then views of the
     result and no per-tensor copy is needed before attention."""
-    if _in_python():
+    if _in_python(qkv):
         return _RopeFusedQkv.apply(qkv.contiguous(), n_heads + n_kv_heads, n_heads + 2 * n_kv_heads, head_dim, theta)
     return ext().rope_qkv(qkv, n_heads + n_kv_heads, n_heads + 2 * n_kv_heads, head_dim, theta)
 
@@ -164,7 +168,7 @@ class _SwiGLU(torch.autograd.Function):
 
 def swiglu(ab: torch.Tensor) -> torch.Tensor:
     """ab = [a | b] along the last dimension; returns silu(a) * b."""
-    if _in_python():
+    if _in_python(ab):
         return _SwiGLU.apply(ab)
     return ext().swiglu(ab)
 

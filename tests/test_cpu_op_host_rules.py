@@ -110,3 +110,12 @@ def test_tensors_without_memory_are_refused():
                      lambda: ops.adamw_flat_(x, x, x, x, 1e-3, 0.9, 0.95, 1e-8, 0.1, 1)):
             with pytest.raises(RuntimeError, match="not allocated"):
                 call()
+
+
+def test_a_tensor_subclass_takes_the_python_functions():
+    """What they do to it goes through the subclass (the skip output of a norm keeps its class)."""
+    import torch
+    from flagcx_b200 import ops
+    x = torch.zeros(2)
+    assert not ops._in_python(x) and not ops._in_python(torch.nn.Parameter(x))
+    assert ops._in_python(x.as_subclass(type("Own", (torch.Tensor,), {})))

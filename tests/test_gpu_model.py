@@ -124,6 +124,9 @@ def test_operators_keep_hooks_tracing_and_transforms():
         torch.vmap(ops.swiglu)(g[None])
     with torch.autograd.forward_ad.dual_level(), pytest.raises(NotImplementedError):
         ops.swiglu(torch.autograd.forward_ad.make_dual(g, other))
+    own = type("Own", (torch.Tensor,), {})
+    y, skip = ops.rmsnorm_branch(g.as_subclass(own), w)
+    assert type(skip) is own and torch.equal(y, ops.rmsnorm(g, w))
 
 
 def test_results_without_memory_are_refused():
