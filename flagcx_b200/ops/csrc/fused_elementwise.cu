@@ -1158,9 +1158,9 @@ cudaError_t crossEntropy(void *logits, const long *targets, float *loss, long ro
 
 cudaError_t adamw(void *p, const void *g, void *m, void *v, size_t n, float lr, float beta1, float beta2, float eps, float wd,
                   float bc1, float bc2, int sms, cudaStream_t stream) {
-  adamwFlat<<<gridFor(n / 8 + 8, 256, sms), 256, 0, stream>>>((bf16 *)p, (const bf16 *)g, (bf16 *)m, (bf16 *)v, n, lr, beta1,
-                                                              beta2, eps, wd, bc1, bc2);
-  return cudaGetLastError();
+  // a small step is the host's: this launch reports its own error
+  void *args[] = {&p, &g, &m, &v, &n, &lr, &beta1, &beta2, &eps, &wd, &bc1, &bc2};
+  return cudaLaunchKernel((const void *)adamwFlat, dim3(gridFor(n / 8 + 8, 256, sms)), dim3(256), args, 0, stream);
 }
 
 } // namespace fcxops

@@ -19,10 +19,12 @@ namespace {
 // there is no memory (fake and meta tensors); asked without, they give a null pointer.
 void *data(const at::Tensor &t) { return t.numel() ? t.data_ptr<at::BFloat16>() : nullptr; }
 
-void checkBf16(const at::Tensor &t, const char *name) {
+void *checkBf16(const at::Tensor &t, const char *name) {
   TORCH_CHECK(t.is_cuda() && t.scalar_type() == at::kBFloat16 && t.is_contiguous(), name,
               " must be a contiguous CUDA bfloat16 tensor");
-  TORCH_CHECK(((uintptr_t)data(t) & 15) == 0, name, " must be 16-byte aligned");
+  void *p = data(t);
+  TORCH_CHECK(((uintptr_t)p & 15) == 0, name, " must be 16-byte aligned");
+  return p;
 }
 
 void checkLaunch(cudaError_t e) {
@@ -148,16 +150,13 @@ at::Tensor cross_entropy_fwd_bwd_(at::Tensor &logits, const at::Tensor &targets,
 
 void adamw_flat_(at::Tensor &p, const at::Tensor &g, at::Tensor &m, at::Tensor &v, double lr, double beta1, double beta2,
                  double eps, double wd, int64_t step) {
-  checkBf16(p, "param");
-  checkBf16(g, "grad");
-  checkBf16(m, "exp_avg");
-  checkBf16(v, "exp_avg_sq");
+  void *pp = checkBf16(p, "param"), *pg = checkBf16(g, "grad"), *pm = checkBf16(m, "exp_avg"), *pv = checkBf16(v, "exp_avg_sq");
   TORCH_CHECK(p.numel() == g.numel() && p.numel() == m.numel() && p.numel() == v.numel(), "adamw: size mismatch");
   const c10::cuda::CUDAGuard guard(p.device());
   const size_t n = p.numel();
   if (n == 0) return;
   float bc1 = 1.f - (float)std::pow(beta1, (double)step), bc2 = 1.f - (float)std::pow(beta2, (double)step);
-  checkLaunch(fcxops::adamw(data(p), data(g), data(m), data(v), n, (float)lr, (float)beta1, (float)beta2,
+  checkLaunch(fcxops::adamw(pp, pg, pm, pv, n, (float)lr, (float)beta1, (float)beta2,
                                (float)eps, (float)wd, bc1, bc2, smCount(), at::cuda::getCurrentCUDAStream()));
 }
 
