@@ -289,14 +289,16 @@ rmsnormBwdFewRows(const bf16 *__restrict__ g, const bf16 *__restrict__ x, const 
   }
 }
 
-// The same for more rows (norm_route.h says where the line lies).  A CTA is cut into groups of GT threads, the fewest (a power of two from 32) that hold a row with four packs
-// per thread; every group owns a ring of row slots in shared memory, which its first thread
-// keeps full with bulk copies that complete on one mbarrier per slot, and reduces its rows by
-// itself: shuffles, and for GT > 32 one named barrier of the group.  So a CTA has 512 / GT rows
-// in work and as many or more on their way, and nothing waits for the whole block.  Bound: the
-// chain wait -> dot product -> sum -> store of each row.  With one row per CTA 8192 x 1024
-// took 39.2 us, 8192 x 256 37.0, 4096 x 2560 30.8, 2048 x 5120 32.9, 512 x 8192 20.5; in groups
-// they take 22.9, 12.4, 24.7, 23.0 and 16.5.
+// The same for more rows (norm_route.h says where the line lies).  A CTA is cut into groups of GT
+// threads, the fewest (a power of two from 32) that hold a row with four packs per thread; every
+// group owns a ring of row slots in shared memory, which its first thread keeps full with bulk
+// copies that complete on one mbarrier per slot, and reduces its rows by itself: shuffles, and for
+// GT > 32 one named barrier of the group.  So a CTA has 512 / GT rows in work and as many or more
+// on their way, and nothing waits for the whole block.  Bound: the chain wait -> dot product ->
+// sum -> store of each row, and 128 registers (four packs per thread spill 16 bytes).  Device time
+// with the sum over CTAs and a skip gradient, against one row per CTA at every size: 8192 x 1024
+// 37.1 -> 18.8 us, 8192 x 256 34.2 -> 8.7, 4096 x 2560 27.9 -> 20.4, 2048 x 5120 28.7 -> 19.0,
+// 4096 x 4096 31.4 -> 29.1, 2048 x 16384 58.1 -> 51.0.
 constexpr int kNormThreads = 512, kNormMaxStages = 6, kNormPacks = 4, kNormRingBytes = 200 << 10;
 
 // Sum over a group of GT threads; every thread gets it.  red holds one float per warp of the
@@ -642,7 +644,7 @@ __global__ void crossEntropyFwdBwd(bf16 *__restrict__ logits, const long *__rest
 //
 // Bound: HBM (one read and one write of the logits).  The kernel below it in this file, which
 // loads, reduces and stores one row per CTA with nothing overlapped, took 458 us for
-// 4096 x 128256; this one takes 355 (5.9 TB/s, 0.92 of a copy).
+// 4096 x 128256; this one takes 355 (5.9 TB/s, 0.90 of a copy).
 // ---------------------------------------------------------------------------
 constexpr int kCeRowThreads = 256, kCeRowWarps = kCeRowThreads / 32;
 constexpr int kCeRowMaxPacks = 16 * kCeRowThreads; // packs of a row that one CTA can hold
@@ -1123,6 +1125,9 @@ cudaError_t crossEntropy(void *logits, const long *targets, float *loss, long ro
       auto go = [&](auto tag) {
         return launchCeRows<decltype(tag)::value>((bf16 *)logits, targets, loss, rows, V, gradScale, cluster, per, sms, stream);
       };
+      // Packs per thread decide the registers (4 each), and they how many CTAs share an SM: 10 let
+      // three, 16 two, 13 waste less of them than 16.  Without these two 1024 x 65544 took 79.9 us
+      // instead of 61.2, 1024 x 151936 170.9 instead of 134.7, 4096 x 100352 327.5 instead of 295.5.
       if (per <= kCeRowThreads) return go(std::integral_constant<int, 1>());
       if (per <= 2 * kCeRowThreads) return go(std::integral_constant<int, 2>());
       if (per <= 4 * kCeRowThreads) return go(std::integral_constant<int, 4>());
