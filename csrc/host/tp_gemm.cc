@@ -100,7 +100,7 @@ flagcxResult_t flagcxGemmBf16(const void *A, const void *B, void *D, int M, int 
   FCXCHECK(cu::tensorMap2dBf16(&ta, A, M, K, 128, 64));
   const bool pair = usePair(M);
   const int forced = (int)readParam("GEMM_SPLIT", 0);
-  SplitGemmPlan plan = splitPlan(M, N, K, pair, forced, (int)readParam("GEMM_SPLIT_N", 256));
+  SplitGemmPlan plan = splitPlan(M, N, K, pair, forced, forced > 1 ? (int)readParam("GEMM_SPLIT_N", 256) : 256);
   if (plan.tileN) {
     FCXCHECK(cu::tensorMap2dBf16(&tb, B, N, K, plan.tileN, 64));
     cudaError_t e = launchSplitGemm(stream ? stream->base : nullptr, ta, tb, D, M, N, K, plan);
