@@ -89,7 +89,7 @@ void rope_inplace(at::Tensor &x, const c10::optional<at::Tensor> &positions, dou
     pos = positions->data_ptr<int>();
   }
   const c10::cuda::CUDAGuard guard(x.device());
-  checkLaunch(fcxops::rope(data(x), pos, (int)tokens, heads, D, logf((float)theta), backward ? -1.f : 1.f, smCount(),
+  checkLaunch(fcxops::rope(data(x), pos, (int)tokens, heads, D, logf((float)theta), backward ? -1.f : 1.f,
                               at::cuda::getCurrentCUDAStream()));
 }
 
@@ -103,7 +103,7 @@ at::Tensor rope_fused_qkv(const at::Tensor &qkv, int64_t ropeHeads, int64_t tota
   auto out = at::empty_like(qkv);
   if (qkv.numel() == 0) return out;
   checkLaunch(fcxops::ropeQkv(data(qkv), data(out), (int)tokens, (int)ropeHeads, (int)totalHeads, (int)D,
-                                 logf((float)theta), backward ? -1.f : 1.f, smCount(), at::cuda::getCurrentCUDAStream()));
+                                 logf((float)theta), backward ? -1.f : 1.f, at::cuda::getCurrentCUDAStream()));
   return out;
 }
 
@@ -116,7 +116,7 @@ at::Tensor swiglu_fwd(const at::Tensor &ab) {
   sizes.back() = F;
   auto out = at::empty(sizes, ab.options());
   size_t T = ab.numel() / (2 * (size_t)F);
-  checkLaunch(fcxops::swigluForward(data(ab), data(out), T, F, smCount(), at::cuda::getCurrentCUDAStream()));
+  checkLaunch(fcxops::swigluForward(data(ab), data(out), T, F, at::cuda::getCurrentCUDAStream()));
   return out;
 }
 
@@ -127,7 +127,7 @@ at::Tensor swiglu_bwd(const at::Tensor &g, const at::Tensor &ab) {
   const c10::cuda::CUDAGuard guard(ab.device());
   auto dab = at::empty_like(ab);
   size_t T = ab.numel() / (2 * (size_t)F);
-  checkLaunch(fcxops::swigluBackward(data(g), data(ab), data(dab), T, F, smCount(),
+  checkLaunch(fcxops::swigluBackward(data(g), data(ab), data(dab), T, F,
                                         at::cuda::getCurrentCUDAStream()));
   return dab;
 }
@@ -157,7 +157,7 @@ void adamw_flat_(at::Tensor &p, const at::Tensor &g, at::Tensor &m, at::Tensor &
   if (n == 0) return;
   float bc1 = 1.f - (float)std::pow(beta1, (double)step), bc2 = 1.f - (float)std::pow(beta2, (double)step);
   checkLaunch(fcxops::adamw(pp, pg, pm, pv, n, (float)lr, (float)beta1, (float)beta2,
-                               (float)eps, (float)wd, bc1, bc2, smCount(), at::cuda::getCurrentCUDAStream()));
+                               (float)eps, (float)wd, bc1, bc2, at::cuda::getCurrentCUDAStream()));
 }
 
 // ---- autograd functions -------------------------------------------------------------------
