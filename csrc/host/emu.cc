@@ -10,12 +10,11 @@
 #include <algorithm>
 
 #include "../kernels/launch.h"
+#include "../kernels/moe_args.h"
 #include "comm.h"
 #include "tuner.h"
 
 namespace fcx {
-
-constexpr int kArgRing = 16;
 
 struct EmuWorld {
   int n = 0, dev = 0;
@@ -27,15 +26,9 @@ struct EmuWorld {
   std::vector<char> has;
   std::vector<CollArgs> coll;
   std::vector<P2pArgs> p2p;
-  // device copies
-  flagcxDevComm *dComms = nullptr;
-  CollArgs *dColl = nullptr; // kArgRing * n
-  P2pArgs *dP2p = nullptr;   // kArgRing * n
-  // generic kernels (MoE, fused GEMMs): opaque per-rank argument blocks
-  std::vector<std::vector<char>> blob;
-  char *dBlob = nullptr;     // kArgRing * n * kMaxBlobBytes
-  int blobKernel = -1;
-  int ring = 0;
+  std::vector<MoeArgs> moe;
+  EmuMoeOp moeOp = kEmuMoeDispatch;
+  std::vector<flagcxDevComm> devs; // what the launch in preparation hands to its kernel
   int maxGrid = 0;
 };
 
@@ -53,6 +46,8 @@ flagcxResult_t emuWorldCreate(int nranks, int dev, flagcxComm **out) {
   w->has.assign(nranks, 0);
   w->coll.resize(nranks);
   w->p2p.resize(nranks);
+  w->moe.resize(nranks);
+  w->devs.resize(nranks);
   SyncLayout layout{};
   for (int r = 0; r < nranks; ++r) {
     auto *c = new flagcxComm();
@@ -88,11 +83,6 @@ flagcxResult_t emuWorldCreate(int nranks, int dev, flagcxComm **out) {
     c->tuner.reset(new Tuner());
     FCXCHECK(c->tuner->init(c));
   }
-  FCX_CUDACHECK(cudaMalloc((void **)&w->dComms, sizeof(flagcxDevComm) * nranks));
-  FCX_CUDACHECK(cudaMalloc((void **)&w->dColl, sizeof(CollArgs) * nranks * kArgRing));
-  FCX_CUDACHECK(cudaMalloc((void **)&w->dP2p, sizeof(P2pArgs) * nranks * kArgRing));
-  FCX_CUDACHECK(cudaMalloc((void **)&w->dBlob, (size_t)kMaxEmuBlobBytes * nranks * kArgRing));
-  w->blob.resize(nranks);
   w->maxGrid = maxCoresidentCtas(FLAGCX_DEVICE_THREADS_PER_CTA);
   FCX_CUDACHECK(cudaDeviceSynchronize());
   for (int r = 0; r < nranks; ++r) out[r] = w->comms[r];
@@ -143,12 +133,19 @@ flagcxResult_t emuWorldDestroy(flagcxComm *any) {
     c->magic = 0;
     delete c;
   }
-  cudaFree(w->dComms);
-  cudaFree(w->dColl);
-  cudaFree(w->dP2p);
-  cudaFree(w->dBlob);
   delete w;
   return flagcxSuccess;
+}
+
+// The launch of the operation that every rank of `w` has posted by now.
+static LaunchCtx emuLaunchCtx(EmuWorld *w, cudaStream_t stream) {
+  LaunchCtx lc;
+  lc.stream = stream;
+  lc.emuRanks = w->n;
+  lc.nCtas = std::max(1, std::min(w->nCtas, std::max(1, w->maxGrid / w->n)));
+  for (int q = 0; q < w->n; ++q) w->devs[q] = w->comms[q]->dev;
+  lc.emuComms = w->devs.data();
+  return lc;
 }
 
 flagcxResult_t emuSubmit(flagcxComm *c, int family, const CollArgs *coll, const P2pArgs *p2p, int nCtas,
@@ -173,22 +170,12 @@ flagcxResult_t emuSubmit(flagcxComm *c, int family, const CollArgs *coll, const 
   // everybody is here: complete the peer tables and launch once
   w->posted = 0;
   std::fill(w->has.begin(), w->has.end(), 0);
-  const int slot = w->ring++ % kArgRing;
-  LaunchCtx lc;
-  lc.stream = stream;
-  lc.emuRanks = n;
-  lc.nCtas = std::max(1, std::min(w->nCtas, std::max(1, w->maxGrid / n)));
-  std::vector<flagcxDevComm> devs(n);
-  for (int q = 0; q < n; ++q) devs[q] = w->comms[q]->dev;
-  FCX_CUDACHECK(cudaMemcpyAsync(w->dComms, devs.data(), sizeof(flagcxDevComm) * n, cudaMemcpyHostToDevice, stream));
-  lc.emuComms = w->dComms;
+  LaunchCtx lc = emuLaunchCtx(w, stream);
   cudaError_t e;
   if (family == 3) {
     lc.nCtas = FLAGCX_P2P_CTAS;
     if (FLAGCX_P2P_CTAS * n > w->maxGrid) { FCX_WARN("p2p grid does not fit the device"); return flagcxInternalError; }
-    P2pArgs *d = w->dP2p + (size_t)slot * n;
-    FCX_CUDACHECK(cudaMemcpyAsync(d, w->p2p.data(), sizeof(P2pArgs) * n, cudaMemcpyHostToDevice, stream));
-    lc.emuP2p = d;
+    lc.emuP2p = w->p2p.data();
     e = launchP2pKernel(lc, w->p2p[0]);
   } else {
     for (int q = 0; q < n; ++q) {
@@ -200,9 +187,7 @@ flagcxResult_t emuSubmit(flagcxComm *c, int family, const CollArgs *coll, const 
       }
     }
     for (int q = 0; q < n; ++q) lc.emuBulk |= w->coll[q].bulkStage != 0;
-    CollArgs *d = w->dColl + (size_t)slot * n;
-    FCX_CUDACHECK(cudaMemcpyAsync(d, w->coll.data(), sizeof(CollArgs) * n, cudaMemcpyHostToDevice, stream));
-    lc.emuArgs = d;
+    lc.emuArgs = w->coll.data();
     e = family == 0   ? launchReduceKernel(lc, w->coll[0], n)
         : family == 1 ? launchCopyKernel(lc, w->coll[0])
         : family == 4 ? launchLlKernel(lc, w->coll[0])
@@ -215,44 +200,28 @@ flagcxResult_t emuSubmit(flagcxComm *c, int family, const CollArgs *coll, const 
   return flagcxSuccess;
 }
 
-// Generic variant for kernels with their own argument block (MoE, fused GEMMs): the
-// blocks are parked per rank; the last arrival copies them to the device and calls
-// `launch(ctx, deviceArray)`, which must do ONE cooperative launch with
-// gridDim.y = ctx.emuRanks.
-flagcxResult_t emuSubmitBlob(flagcxComm *c, int kernelId, const void *args, size_t argBytes, int nCtas,
-                             cudaStream_t stream, EmuBlobLaunch launch) {
+// The same for the expert-parallel kernels.
+flagcxResult_t emuSubmitMoe(flagcxComm *c, EmuMoeOp op, const MoeArgs &args, int nCtas, cudaStream_t stream) {
   EmuWorld *w = c->emu;
   const int n = w->n, r = c->rank;
-  if (argBytes > (size_t)kMaxEmuBlobBytes) return flagcxInternalError;
   if (w->has[r]) {
     FCX_WARN("emulated rank %d posted a second operation before the others posted their first", r);
     return flagcxInvalidUsage;
   }
-  if (w->posted == 0) { w->blobKernel = kernelId; w->nCtas = nCtas; }
-  if (kernelId != w->blobKernel) {
+  if (w->posted == 0) { w->moeOp = op; w->nCtas = nCtas; }
+  if (op != w->moeOp) {
     FCX_WARN("emulated ranks posted different kinds of operations");
     return flagcxInvalidUsage;
   }
   w->nCtas = std::min(w->nCtas, nCtas);
-  w->blob[r].assign((const char *)args, (const char *)args + argBytes);
+  w->moe[r] = args;
   w->has[r] = 1;
   if (++w->posted < n) return flagcxSuccess;
   w->posted = 0;
   std::fill(w->has.begin(), w->has.end(), 0);
-  const int slot = w->ring++ % kArgRing;
-  std::vector<flagcxDevComm> devs(n);
-  for (int q = 0; q < n; ++q) devs[q] = w->comms[q]->dev;
-  FCX_CUDACHECK(cudaMemcpyAsync(w->dComms, devs.data(), sizeof(flagcxDevComm) * n, cudaMemcpyHostToDevice, stream));
-  char *d = w->dBlob + (size_t)slot * n * kMaxEmuBlobBytes;
-  std::vector<char> packed((size_t)n * argBytes);
-  for (int q = 0; q < n; ++q) memcpy(packed.data() + (size_t)q * argBytes, w->blob[q].data(), argBytes);
-  FCX_CUDACHECK(cudaMemcpyAsync(d, packed.data(), packed.size(), cudaMemcpyHostToDevice, stream));
-  LaunchCtx lc;
-  lc.stream = stream;
-  lc.emuRanks = n;
-  lc.emuComms = w->dComms;
-  lc.nCtas = std::max(1, std::min(w->nCtas, std::max(1, w->maxGrid / n)));
-  cudaError_t e = launch(lc, d);
+  LaunchCtx lc = emuLaunchCtx(w, stream);
+  lc.emuMoe = w->moe.data();
+  const cudaError_t e = op == kEmuMoeDispatch ? launchMoeDispatch(lc, w->moe[0]) : launchMoeCombine(lc, w->moe[0]);
   if (e != cudaSuccess) {
     FCX_WARN("emulated-world launch failed: %s", cudaGetErrorString(e));
     return flagcxUnhandledDeviceError;

@@ -96,26 +96,6 @@ void fillArgs(flagcxMoe *m, MoeArgs &a, int nTokens) {
   a.capacity = m->capacity;
 }
 
-cudaError_t emuDispatch(const LaunchCtx &lc, const void *d) {
-  LaunchCtx l2 = lc;
-  l2.emuBlob = d;
-  MoeArgs dummy{};
-  dummy.E = 0;
-  return launchMoeDispatch(l2, dummy);
-}
-cudaError_t emuCombine(const LaunchCtx &lc, const void *d) {
-  LaunchCtx l2 = lc;
-  l2.emuBlob = d;
-  MoeArgs dummy{};
-  return launchMoeCombine(l2, dummy, false);
-}
-cudaError_t emuCombinePull(const LaunchCtx &lc, const void *d) {
-  LaunchCtx l2 = lc;
-  l2.emuBlob = d;
-  MoeArgs dummy{};
-  return launchMoeCombine(l2, dummy, true);
-}
-
 int moeCtas(flagcxComm *c) {
   int64_t v = readParam("MOE_CTAS", 128); // CTAs of 256 threads
   return (int)std::max<int64_t>(1, std::min<int64_t>(v, FLAGCX_COLL_BARRIER_SLOTS));
@@ -207,7 +187,7 @@ flagcxResult_t flagcxMoeDispatch(flagcxMoe_t m, const void *x, const int *topkId
   m->lastIdx = topkIdx;
   c->stats[flagcxCommOpAlltoAllv].calls++;
   c->stats[flagcxCommOpAlltoAllv].bytes += (size_t)nTokens * m->topk * m->hidden * 2;
-  if (c->emu) return emuSubmitBlob(c, 100, &a, sizeof a, moeCtas(c), s, emuDispatch);
+  if (c->emu) return emuSubmitMoe(c, kEmuMoeDispatch, a, moeCtas(c), s);
   LaunchCtx lc;
   lc.comm = &c->dev;
   lc.stream = s;
@@ -230,13 +210,12 @@ flagcxResult_t flagcxMoeCombine(flagcxMoe_t m, const float *topkWeights, void *o
   a.topkIdx = m->lastIdx;
   a.topkW = topkWeights;
   a.out = (__nv_bfloat16 *)out;
-  const bool pull = a.preReduce == 0;
-  if (c->emu) return emuSubmitBlob(c, pull ? 102 : 101, &a, sizeof a, moeCtas(c), s, pull ? emuCombinePull : emuCombine);
+  if (c->emu) return emuSubmitMoe(c, a.preReduce ? kEmuMoeCombineReduce : kEmuMoeCombinePull, a, moeCtas(c), s);
   LaunchCtx lc;
   lc.comm = &c->dev;
   lc.stream = s;
   lc.nCtas = moeCtas(c);
-  cudaError_t e = launchMoeCombine(lc, a, pull);
+  cudaError_t e = launchMoeCombine(lc, a);
   if (e != cudaSuccess) { FCX_WARN("moe combine launch failed: %s", cudaGetErrorString(e)); return flagcxUnhandledDeviceError; }
   return flagcxSuccess;
 }

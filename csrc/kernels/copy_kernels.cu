@@ -341,8 +341,8 @@ __global__ void __launch_bounds__(FLAGCX_DEVICE_THREADS_PER_CTA)
   copyBody(c, stageArgs(a));
 }
 __global__ void __launch_bounds__(FLAGCX_DEVICE_THREADS_PER_CTA)
-    copyKernelEmu(const flagcxDevComm *cs, const CollArgs *as) {
-  copyBody(cs[blockIdx.y], stageArgs(as[blockIdx.y]));
+    copyKernelEmu(const __grid_constant__ EmuLaunch<CollArgs> e) {
+  copyBody(e.comm[blockIdx.y], stageArgs(e.args[blockIdx.y]));
 }
 
 // ---------------------------------------------------------------------------
@@ -387,8 +387,8 @@ __global__ void __launch_bounds__(FLAGCX_DEVICE_THREADS_PER_CTA) p2pKernel(const
   p2pBody(c, a);
 }
 __global__ void __launch_bounds__(FLAGCX_DEVICE_THREADS_PER_CTA)
-    p2pKernelEmu(const flagcxDevComm *cs, const P2pArgs *as) {
-  p2pBody(cs[blockIdx.y], as[blockIdx.y]);
+    p2pKernelEmu(const __grid_constant__ EmuLaunch<P2pArgs> e) {
+  p2pBody(e.comm[blockIdx.y], e.args[blockIdx.y]);
 }
 
 } // namespace
@@ -396,7 +396,6 @@ __global__ void __launch_bounds__(FLAGCX_DEVICE_THREADS_PER_CTA)
 cudaError_t launchCopyKernel(const LaunchCtx &lc, const CollArgs &a) {
   dim3 grid(lc.nCtas, lc.emuRanks > 0 ? lc.emuRanks : 1), block(lc.nThreads);
   if (lc.emuRanks > 0) {
-    void *params[] = {(void *)&lc.emuComms, (void *)&lc.emuArgs};
     size_t emuSmem = 0;
     if (lc.emuBulk) {
       emuSmem = kBulkRingBytes;
@@ -407,7 +406,7 @@ cudaError_t launchCopyKernel(const LaunchCtx &lc, const CollArgs &a) {
         emuConfigured = true;
       }
     }
-    return cudaLaunchCooperativeKernel((const void *)copyKernelEmu, grid, block, params, emuSmem, lc.stream);
+    return launchEmu(copyKernelEmu, lc, lc.emuArgs, grid, block, emuSmem);
   }
   size_t smem = 0;
   if (a.bulkStage) {
@@ -425,10 +424,7 @@ cudaError_t launchCopyKernel(const LaunchCtx &lc, const CollArgs &a) {
 
 cudaError_t launchP2pKernel(const LaunchCtx &lc, const P2pArgs &a) {
   dim3 grid(FLAGCX_P2P_CTAS, lc.emuRanks > 0 ? lc.emuRanks : 1), block(lc.nThreads);
-  if (lc.emuRanks > 0) {
-    void *params[] = {(void *)&lc.emuComms, (void *)&lc.emuP2p};
-    return cudaLaunchCooperativeKernel((const void *)p2pKernelEmu, grid, block, params, 0, lc.stream);
-  }
+  if (lc.emuRanks > 0) return launchEmu(p2pKernelEmu, lc, lc.emuP2p, grid, block, 0);
   p2pKernel<<<grid, block, 0, lc.stream>>>(*lc.comm, a);
   return cudaGetLastError();
 }

@@ -129,8 +129,8 @@ __global__ void __launch_bounds__(FLAGCX_DEVICE_THREADS_PER_CTA)
 }
 template <typename T>
 __global__ void __launch_bounds__(FLAGCX_DEVICE_THREADS_PER_CTA)
-    llKernelEmu(const flagcxDevComm *cs, const CollArgs *as) {
-  llBody<T>(cs[blockIdx.y], as[blockIdx.y]);
+    llKernelEmu(const __grid_constant__ EmuLaunch<CollArgs> e) {
+  llBody<T>(e.comm[blockIdx.y], e.args[blockIdx.y]);
 }
 
 } // namespace
@@ -139,10 +139,7 @@ namespace {
 template <typename T>
 cudaError_t launchLlT(const LaunchCtx &lc, const CollArgs &a) {
   dim3 grid(lc.nCtas, lc.emuRanks > 0 ? lc.emuRanks : 1), block(lc.nThreads);
-  if (lc.emuRanks > 0) {
-    void *params[] = {(void *)&lc.emuComms, (void *)&lc.emuArgs};
-    return cudaLaunchCooperativeKernel((const void *)llKernelEmu<T>, grid, block, params, 0, lc.stream);
-  }
+  if (lc.emuRanks > 0) return launchEmu(llKernelEmu<T>, lc, lc.emuArgs, grid, block, 0);
   llKernel<T><<<grid, block, 0, lc.stream>>>(*lc.comm, a);
   return cudaGetLastError();
 }

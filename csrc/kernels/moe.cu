@@ -404,50 +404,40 @@ __global__ void __launch_bounds__(kMoeThreads) moeDispatchKernel(const flagcxDev
   dispatchBody(c, a);
 }
 __global__ void __launch_bounds__(kMoeThreads)
-    moeDispatchKernelEmu(const flagcxDevComm *cs, const MoeArgs *as) {
-  dispatchBody(cs[blockIdx.y], as[blockIdx.y]);
+    moeDispatchKernelEmu(const __grid_constant__ EmuLaunch<MoeArgs> e) {
+  dispatchBody(e.comm[blockIdx.y], e.args[blockIdx.y]);
 }
 __global__ void __launch_bounds__(kMoeThreads) moeCombineKernel(const flagcxDevComm c, const MoeArgs a) {
   combineReduceBody(c, a);
 }
 __global__ void __launch_bounds__(kMoeThreads)
-    moeCombineKernelEmu(const flagcxDevComm *cs, const MoeArgs *as) {
-  combineReduceBody(cs[blockIdx.y], as[blockIdx.y]);
+    moeCombineKernelEmu(const __grid_constant__ EmuLaunch<MoeArgs> e) {
+  combineReduceBody(e.comm[blockIdx.y], e.args[blockIdx.y]);
 }
 __global__ void __launch_bounds__(FLAGCX_DEVICE_THREADS_PER_CTA) moeCombinePullKernel(const flagcxDevComm c, const MoeArgs a) {
   combinePullBody(c, a);
 }
 __global__ void __launch_bounds__(FLAGCX_DEVICE_THREADS_PER_CTA)
-    moeCombinePullKernelEmu(const flagcxDevComm *cs, const MoeArgs *as) {
-  combinePullBody(cs[blockIdx.y], as[blockIdx.y]);
+    moeCombinePullKernelEmu(const __grid_constant__ EmuLaunch<MoeArgs> e) {
+  combinePullBody(e.comm[blockIdx.y], e.args[blockIdx.y]);
 }
 
 } // namespace
 
 cudaError_t launchMoeDispatch(const LaunchCtx &lc, const MoeArgs &a) {
   dim3 grid(lc.nCtas, lc.emuRanks > 0 ? lc.emuRanks : 1), block(kMoeThreads);
-  const size_t smem = 0;
-  (void)a;
-  if (lc.emuRanks > 0) {
-    const void *blob = lc.emuBlob;
-    void *params[] = {(void *)&lc.emuComms, (void *)&blob};
-    return cudaLaunchCooperativeKernel((const void *)moeDispatchKernelEmu, grid, block, params, smem, lc.stream);
-  }
-  moeDispatchKernel<<<grid, block, smem, lc.stream>>>(*lc.comm, a);
+  if (lc.emuRanks > 0) return launchEmu(moeDispatchKernelEmu, lc, lc.emuMoe, grid, block, 0);
+  moeDispatchKernel<<<grid, block, 0, lc.stream>>>(*lc.comm, a);
   return cudaGetLastError();
 }
 
 // a.preReduce picks the kernel; the pull kind takes half as many CTAs of twice the threads.
-// In the emulated world every rank's arguments carry the same choice (lc.emuPull).
-cudaError_t launchMoeCombine(const LaunchCtx &lc, const MoeArgs &a, bool pull) {
+cudaError_t launchMoeCombine(const LaunchCtx &lc, const MoeArgs &a) {
+  const bool pull = a.preReduce == 0;
   const int ctas = pull ? (lc.nCtas + 1) / 2 : lc.nCtas;
   dim3 grid(ctas, lc.emuRanks > 0 ? lc.emuRanks : 1), block(pull ? FLAGCX_DEVICE_THREADS_PER_CTA : kMoeThreads);
-  if (lc.emuRanks > 0) {
-    const void *blob = lc.emuBlob;
-    void *params[] = {(void *)&lc.emuComms, (void *)&blob};
-    return cudaLaunchCooperativeKernel(pull ? (const void *)moeCombinePullKernelEmu : (const void *)moeCombineKernelEmu, grid, block,
-                                       params, 0, lc.stream);
-  }
+  if (lc.emuRanks > 0)
+    return launchEmu(pull ? moeCombinePullKernelEmu : moeCombineKernelEmu, lc, lc.emuMoe, grid, block, 0);
   if (pull) moeCombinePullKernel<<<grid, block, 0, lc.stream>>>(*lc.comm, a);
   else moeCombineKernel<<<grid, block, 0, lc.stream>>>(*lc.comm, a);
   return cudaGetLastError();

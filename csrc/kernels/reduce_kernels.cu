@@ -511,8 +511,8 @@ __global__ void __launch_bounds__(FLAGCX_DEVICE_THREADS_PER_CTA)
 // Emulated world: one cooperative launch, blockIdx.y plays the rank.
 template <typename T, int OP, int NR>
 __global__ void __launch_bounds__(FLAGCX_DEVICE_THREADS_PER_CTA)
-    reduceKernelEmu(const flagcxDevComm *cs, const CollArgs *as) {
-  reduceBody<T, OP, NR>(cs[blockIdx.y], stageArgs(as[blockIdx.y]));
+    reduceKernelEmu(const __grid_constant__ EmuLaunch<CollArgs> e) {
+  reduceBody<T, OP, NR>(e.comm[blockIdx.y], stageArgs(e.args[blockIdx.y]));
 }
 
 // ---------------------------------------------------------------------------
@@ -522,7 +522,6 @@ template <typename T, int OP, int NR>
 cudaError_t launchReduceT(const LaunchCtx &lc, const CollArgs &a) {
   dim3 grid(lc.nCtas, lc.emuRanks > 0 ? lc.emuRanks : 1), block(lc.nThreads);
   if (lc.emuRanks > 0) {
-    void *params[] = {(void *)&lc.emuComms, (void *)&lc.emuArgs};
     size_t emuSmem = 0;
     if (NR > 0 && lc.emuBulk) {
       emuSmem = kBulkRingBytes;
@@ -534,8 +533,7 @@ cudaError_t launchReduceT(const LaunchCtx &lc, const CollArgs &a) {
         emuConfigured = true;
       }
     }
-    return cudaLaunchCooperativeKernel((const void *)reduceKernelEmu<T, OP, NR>, grid, block, params, emuSmem,
-                                       lc.stream);
+    return launchEmu(reduceKernelEmu<T, OP, NR>, lc, lc.emuArgs, grid, block, emuSmem);
   }
   size_t smem = 0;
   if (NR > 0 && a.bulkStage) {
