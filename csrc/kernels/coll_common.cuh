@@ -159,10 +159,7 @@ __device__ __forceinline__ bool ctaWaitFlag(const flagcxDevComm &c, const unsign
 }
 __device__ __forceinline__ void ctaRaiseFlag(unsigned long long *flag, unsigned long long v) {
   __syncthreads();
-  if (threadIdx.x == 0) {
-    fcxdev::fenceSys();
-    fcxdev::stReleaseSys(flag, v);
-  }
+  if (threadIdx.x == 0) fcxdev::stReleaseSys(flag, v);
 }
 
 __device__ void ctaCopyShare(char *dst, const char *src, size_t bytes, int b, int g) {
