@@ -155,6 +155,7 @@ flagcxResult_t allocLocalDeviceState(flagcxComm *c) {
   FCX_CUDACHECK(cudaMalloc(&c->localSync, localBytes));
   FCX_CUDACHECK(cudaMemset(c->localSync, 0, localBytes));
   c->putArrival = (unsigned int *)((char *)c->localSync + syncWords * sizeof(uint64_t));
+  c->tickets = c->putArrival + 32; // in a line of its own
   FCX_CUDACHECK(cudaHostAlloc((void **)&c->rmaCounter, sizeof(uint64_t), cudaHostAllocMapped));
   *c->rmaCounter = 0;
   FCX_CUDACHECK(cudaHostAlloc((void **)&c->status, sizeof(flagcxDevStatus), cudaHostAllocMapped));

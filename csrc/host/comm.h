@@ -134,6 +134,7 @@ struct flagcxComm {
   size_t bounceBytes[2] = {0, 0};
   int winSeq = 0;                  // window registrations so far (same on every rank)
   unsigned int *putArrival = nullptr; // device word used by put kernels
+  unsigned int *tickets = nullptr;    // two words that the kernels draw work from (inside localSync)
   volatile uint64_t *rmaCounter = nullptr; // pinned: one-sided operations completed
   uint64_t rmaIssued = 0;
   fcx::Window *oneSideSignalWin = nullptr;

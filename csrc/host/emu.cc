@@ -220,6 +220,7 @@ flagcxResult_t emuSubmitMoe(flagcxComm *c, EmuMoeOp op, const MoeArgs &args, int
   w->posted = 0;
   std::fill(w->has.begin(), w->has.end(), 0);
   LaunchCtx lc = emuLaunchCtx(w, stream);
+  lc.nCtas = w->nCtas; // the launcher knows how many of its kernel's CTAs run at once
   lc.emuMoe = w->moe.data();
   const cudaError_t e = op == kEmuMoeDispatch ? launchMoeDispatch(lc, w->moe[0]) : launchMoeCombine(lc, w->moe[0]);
   if (e != cudaSuccess) {

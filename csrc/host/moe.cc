@@ -23,6 +23,7 @@ struct flagcxMoe {
   // local
   int *pos = nullptr, *route = nullptr, *expertOffsets = nullptr, *lead = nullptr;
   int lastTokens = 0;
+  int preReduce = 0; // decided by the dispatch, for the combine that follows it
   const int *lastIdx = nullptr;
 };
 
@@ -56,6 +57,20 @@ void symFree(flagcxComm *c, void *ptr, Window *win, bool isVmm) {
   }
 }
 
+// Pre-reducing on the expert rank pays when a token has, on average, at least two experts
+// per rank it goes to (one row crosses NVLink instead of two or more; 523 -> 370 us on two
+// B200s with 64 experts, top-8); with eight ranks, 256 experts and top-8 a token reaches
+// 5.25 ranks, the saving is a third, and the extra local pass and barrier cost more (885
+// against 692 us).  Expected ranks per token for uniform routing: n (1 - (1 - 1/n)^k).
+int preReduceFor(const flagcxMoe *m) {
+  const double n = m->comm->nranks, k = m->topk;
+  double miss = 1.0;
+  for (int i = 0; i < m->topk; ++i) miss *= 1.0 - 1.0 / n;
+  const double ranksPerToken = n * (1.0 - miss);
+  const int64_t dflt = k / ranksPerToken >= 2.0 ? 1 : 0;
+  return readParam("MOE_COMBINE_REDUCE", dflt) != 0 ? 1 : 0;
+}
+
 void fillArgs(flagcxMoe *m, MoeArgs &a, int nTokens) {
   flagcxComm *c = m->comm;
   memset(&a, 0, sizeof a);
@@ -71,19 +86,8 @@ void fillArgs(flagcxMoe *m, MoeArgs &a, int nTokens) {
   a.grpRecordsPerSender = m->grpRecordsPerSender;
   a.maxT = m->maxTokens;
   a.dedup = readParam("MOE_DEDUP", 1) != 0 ? 1 : 0;
-  // Pre-reducing on the expert rank pays when a token has, on average, at least two experts
-  // per rank it goes to (one row crosses NVLink instead of two or more; 523 -> 370 us on two
-  // B200s with 64 experts, top-8); with eight ranks, 256 experts and top-8 a token reaches
-  // 5.25 ranks, the saving is a third, and the extra local pass and barrier cost more (885
-  // against 692 us).  Expected ranks per token for uniform routing: n (1 - (1 - 1/n)^k).
-  {
-    const double n = c->nranks, k = m->topk;
-    double miss = 1.0;
-    for (int i = 0; i < m->topk; ++i) miss *= 1.0 - 1.0 / n;
-    const double ranksPerToken = n * (1.0 - miss);
-    const int64_t dflt = k / ranksPerToken >= 2.0 ? 1 : 0;
-    a.preReduce = readParam("MOE_COMBINE_REDUCE", dflt) != 0 ? 1 : 0;
-  }
+  a.preReduce = m->preReduce;
+  a.tickets = c->tickets;
   a.lead = m->lead;
   a.pos = m->pos;
   a.route = m->route;
@@ -178,6 +182,7 @@ flagcxResult_t flagcxMoeDispatch(flagcxMoe_t m, const void *x, const int *topkId
   flagcxComm *c = m->comm;
   if (c->asyncError.load() != flagcxSuccess) return (flagcxResult_t)c->asyncError.load();
   cudaStream_t s = stream ? stream->base : nullptr;
+  m->preReduce = preReduceFor(m);
   MoeArgs a;
   fillArgs(m, a, nTokens);
   a.x = (const __nv_bfloat16 *)x;

@@ -2,6 +2,8 @@
 #pragma once
 #include <cuda_runtime.h>
 
+#include <atomic>
+
 #include "coll_args.h"
 
 namespace fcx {
@@ -43,6 +45,27 @@ cudaError_t launchEmu(void (*kernel)(EmuLaunch<Args>), const LaunchCtx &lc, cons
   }
   void *params[] = {&e};
   return cudaLaunchCooperativeKernel((const void *)kernel, grid, block, params, sharedBytes, lc.stream);
+}
+
+// How many CTAs per rank of a kernel may be part of such a launch (all must run at once): at least 1
+// where one fits at all.  The answer is the device's and is kept per kernel.
+template <auto Kernel>
+cudaError_t emuCtasPerRank(int threads, int ranks, int *ctas) {
+  static std::atomic<int> perDevice[64];
+  int dev = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e != cudaSuccess) return e;
+  int all = dev < 64 ? perDevice[dev].load(std::memory_order_relaxed) : 0;
+  if (!all) {
+    int sms = 0, perSm = 0;
+    e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSm, (const void *)Kernel, threads, 0);
+    if (e != cudaSuccess) return e;
+    all = sms * perSm;
+    if (dev < 64) perDevice[dev].store(all, std::memory_order_relaxed);
+  }
+  *ctas = all / ranks > 1 ? all / ranks : 1;
+  return cudaSuccess;
 }
 
 cudaError_t launchMoeDispatch(const LaunchCtx &lc, const MoeArgs &a);

@@ -19,6 +19,8 @@
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 
+#include <algorithm>
+
 #include "launch.h"
 #include "moe_args.h"
 #include "prims.cuh"
@@ -30,32 +32,34 @@ namespace {
 // registers for them; the host launches twice as many CTAs as it would of the 512-thread kind.
 constexpr int kMoeThreads = 256;
 
-// One warp copies one row (H bf16) to every non-null destination.  The row is read once, eight
-// 16-byte loads in flight per lane, and each piece goes to all destinations: a token's row was
-// read again for every rank it went to (and every local copy re-read the leader row), with four
-// loads in flight, which with 8 warps per SM is 16 KiB of the 35 that latency asks for.  Eight
-// emulated ranks, 512 tokens x 7168, top 8 of 256: dispatch 225 -> 209 us; with two vectors of
-// every row in flight in the pulling combine 189 -> 163.
-__device__ __forceinline__ void warpCopyRow(char *const (&dst)[FLAGCX_MOE_MAX_TOPK], const char *src, int vecs, int lane,
-                                            bool srcIsPeerWritten) {
-  constexpr int U = 8;
-  const uint4 *s = (const uint4 *)src;
-  for (int v0 = lane; v0 < vecs; v0 += 32 * U) {
-    uint4 r[U];
+// A row of vecs 16-byte vectors is copied in pieces of at most 32 x kMoePiece vectors, one warp
+// each, so that the warps of a CTA share its rows evenly however few they are.
+constexpr int kMoePiece = 8;
+struct RowPieces {
+  int count, vecs; // pieces per row, vectors per piece
+  __device__ __forceinline__ explicit RowPieces(int rowVecs) {
+    count = (rowVecs + 32 * kMoePiece - 1) / (32 * kMoePiece);
+    vecs = ((rowVecs + count - 1) / count + 31) & ~31;
+  }
+};
+
+// One warp copies the vectors [first, end) of a row to the first n of the rows dst.  The piece is
+// read once, all of a lane's loads in flight, and then goes to every destination.
+__device__ __forceinline__ void warpCopyPiece(char *const *dst, int n, const char *src, int first, int end, int lane,
+                                              bool srcIsPeerWritten) {
+  uint4 r[kMoePiece];
 #pragma unroll
-    for (int u = 0; u < U; ++u) {
-      const int v = v0 + 32 * u;
-      if (v < vecs) r[u] = srcIsPeerWritten ? ldSys16(s + v) : s[v];
+  for (int u = 0; u < kMoePiece; ++u) {
+    const int v = first + lane + 32 * u;
+    if (v < end) r[u] = srcIsPeerWritten ? ldSys16((const uint4 *)src + v) : ((const uint4 *)src)[v];
+  }
+  for (int k = 0; k < n; ++k) {
+    uint4 *d = (uint4 *)dst[k];
+#pragma unroll
+    for (int u = 0; u < kMoePiece; ++u) {
+      const int v = first + lane + 32 * u;
+      if (v < end) st16(d + v, r[u]);
     }
-#pragma unroll
-    for (int k = 0; k < FLAGCX_MOE_MAX_TOPK; ++k)
-      if (dst[k]) {
-#pragma unroll
-        for (int u = 0; u < U; ++u) {
-          const int v = v0 + 32 * u;
-          if (v < vecs) st16((uint4 *)dst[k] + v, r[u]);
-        }
-      }
   }
 }
 
@@ -127,163 +131,235 @@ __device__ __forceinline__ void weightedRowSum(const char *rows[FLAGCX_MOE_MAX_T
   }
 }
 
+// Start of CTA b's range of T tokens: at most ceil(T / g) of them, every CTA within one of that.
+__device__ __forceinline__ int firstToken(int T, int b, int g) { return (int)((long)T * b / g); }
+
 // The whole dispatch is this one kernel: histogram of the routing, exchange of the
 // counts, the copies, and the local fan-out of rows that several experts of one rank want.
+// Bound: memory (eight emulated ranks, 512 tokens x 7168, top 8 of 256: 640 MB, 97 us of the 126
+// at the rate of a copy), then two barriers and about 6 us of counting and routing.  One warp per
+// row, one load of the routing table at a time, and one CTA of 8 warps per SM took 173 us; the
+// routes of four tokens at once, pieces of rows and two to three CTAs per SM brought it here.
+struct DispatchShared {
+  int base[FLAGCX_MOE_MAX_EXPERTS];
+  union {
+    struct { int tot[FLAGCX_MOE_MAX_EXPERTS], before[FLAGCX_MOE_MAX_EXPERTS], mine[FLAGCX_MOE_MAX_EXPERTS]; };
+    struct { // rows that a token goes to, or the row that a group has and then those it is copied to
+      char *row[kMoeThreads][FLAGCX_MOE_MAX_TOPK];
+      int nRows[kMoeThreads];
+    };
+  };
+  int grpN[FLAGCX_MAX_RANKS], nRec;
+};
+
 __device__ void dispatchBody(const flagcxDevComm &c, const MoeArgs &a) {
-  __shared__ int tot[FLAGCX_MOE_MAX_EXPERTS], base[FLAGCX_MOE_MAX_EXPERTS], before[FLAGCX_MOE_MAX_EXPERTS],
-      mineCnt[FLAGCX_MOE_MAX_EXPERTS];
-  __shared__ int grpN[FLAGCX_MAX_RANKS];
+  __shared__ DispatchShared s;
   const int b = blockIdx.x, g = gridDim.x, rank = c.rank, n = c.nRanks;
   const int t = threadIdx.x, nt = blockDim.x;
   // this CTA's tokens: a contiguous range, so that "how many earlier pairs chose expert e"
   // splits into the pairs of earlier CTAs' ranges and the pairs of this range
-  const int tpc = (a.T + g - 1) / g;
-  const int tlo = b * tpc < a.T ? b * tpc : a.T, thi = tlo + tpc < a.T ? tlo + tpc : a.T;
+  const int tlo = firstToken(a.T, b, g), thi = firstToken(a.T, b + 1, g);
   const int lo = tlo * a.K, hi = thi * a.K, items = a.T * a.K;
   // 0. every CTA counts the whole routing table (a few dozen shared-memory atomics per
   // thread): no separate counting kernel, no global atomics, no memset
-  for (int e = t; e < a.E; e += nt) tot[e] = before[e] = mineCnt[e] = 0;
-  if (t < FLAGCX_MAX_RANKS) grpN[t] = 0;
+  for (int e = t; e < a.E; e += nt) s.tot[e] = s.before[e] = s.mine[e] = 0;
+  if (t < FLAGCX_MAX_RANKS) s.grpN[t] = 0;
   __syncthreads();
-  for (int i = t; i < items; i += nt) {
-    const int e = a.topkIdx[i];
-    const bool valid = e >= 0 && e < a.E;
-    if (i < lo) { if (valid) atomicAdd(&before[e], 1); }
-    else if (i < hi) {
-      if (valid) a.pos[i] = atomicAdd(&mineCnt[e], 1); // index within this CTA's range, completed below
-      else {
-        a.pos[i] = -1;
-        fcxdev::reportError(c.status, FLAGCX_DEV_BOUNDS, FLAGCX_DEV_AT_KERNEL, 0xffffffffu, (unsigned long long)i);
-      }
-    } else if (valid) atomicAdd(&tot[e], 1);
+  constexpr int kAhead = 8; // entries of the table that a thread has on their way
+  for (int i0 = t; i0 < items; i0 += kAhead * nt) {
+    int es[kAhead];
+#pragma unroll
+    for (int u = 0; u < kAhead; ++u) es[u] = i0 + u * nt < items ? a.topkIdx[i0 + u * nt] : 0;
+#pragma unroll
+    for (int u = 0; u < kAhead; ++u) {
+      const int i = i0 + u * nt, e = es[u];
+      if (i >= items) break;
+      const bool valid = e >= 0 && e < a.E;
+      if (i < lo) { if (valid) atomicAdd(&s.before[e], 1); }
+      else if (i < hi) {
+        if (valid) a.pos[i] = atomicAdd(&s.mine[e], 1); // index within this CTA's range, completed below
+        else {
+          a.pos[i] = -1;
+          fcxdev::reportError(c.status, FLAGCX_DEV_BOUNDS, FLAGCX_DEV_AT_KERNEL, 0xffffffffu, (unsigned long long)i);
+        }
+      } else if (valid) atomicAdd(&s.tot[e], 1);
+    }
   }
-  __syncthreads();
-  for (int e = t; e < a.E; e += nt) tot[e] += before[e] + mineCnt[e];
   __syncthreads();
   // 1. publish my per-expert counts in every rank's table (row `rank`), mine included;
   // every CTA writes the same values and reads them back from its own peers' CTA
-  for (int p = 0; p < n; ++p) {
-    int *dst = a.countsAll[p] + (size_t)rank * a.E;
-    for (int e = t; e < a.E; e += nt) dst[e] = tot[e];
+  for (int e = t; e < a.E; e += nt) {
+    const int cnt = s.tot[e] + s.before[e] + s.mine[e];
+#pragma unroll
+    for (int p = 0; p < FLAGCX_MAX_RANKS; ++p)
+      if (p < n) a.countsAll[p][(size_t)rank * a.E + e] = cnt;
   }
   if (!ctaBarrier(c, b)) return;
   // 2. where my rows start inside each destination's expert-grouped buffer
   const int *tab = a.countsAll[rank];
   for (int e = t; e < a.E; e += nt) {
-    int s = 0;
+    int cnt[FLAGCX_MAX_RANKS], all = 0, lower = 0;
     // rows written by peers: system-scope loads, never a stale cached line
-    for (int q = 0; q < n; ++q) s += ldSysElem(tab + (size_t)q * a.E + e);
-    tot[e] = s;
+#pragma unroll
+    for (int q = 0; q < FLAGCX_MAX_RANKS; ++q) cnt[q] = q < n ? ldSysElem(tab + (size_t)q * a.E + e) : 0;
+#pragma unroll
+    for (int q = 0; q < FLAGCX_MAX_RANKS; ++q) {
+      all += cnt[q];
+      if (q < rank) lower += cnt[q];
+    }
+    s.tot[e] = all;
+    s.base[e] = lower + s.before[e]; // pairs of lower ranks and of earlier CTAs' ranges come first
   }
   __syncthreads();
   for (int e = t; e < a.E; e += nt) {
-    int d = e / a.EPR, s = 0;
-    for (int e2 = d * a.EPR; e2 < e; ++e2) s += tot[e2];
-    for (int q = 0; q < rank; ++q) s += ldSysElem(tab + (size_t)q * a.E + e);
-    base[e] = s + before[e]; // pairs of earlier CTAs' ranges come first
+    int sum = 0;
+    for (int e2 = e / a.EPR * a.EPR; e2 < e; ++e2) sum += s.tot[e2];
+    s.base[e] += sum;
   }
-  __syncthreads();
   if (b == 0) {
     // this rank's own expert boundaries, for whoever runs the experts
     for (int le = t; le <= a.EPR; le += nt) {
-      int s = 0;
-      for (int e2 = 0; e2 < le; ++e2) s += tot[rank * a.EPR + e2];
-      a.expertOffsets[le] = s;
+      int sum = 0;
+      for (int e2 = 0; e2 < le; ++e2) sum += s.tot[rank * a.EPR + e2];
+      a.expertOffsets[le] = sum;
     }
     if (t == 0) {
       long total = 0;
-      for (int le = 0; le < a.EPR; ++le) total += tot[rank * a.EPR + le];
+      for (int le = 0; le < a.EPR; ++le) total += s.tot[rank * a.EPR + le];
       if ((size_t)total > a.capacity)
         fcxdev::reportError(c.status, FLAGCX_DEV_BOUNDS, FLAGCX_DEV_AT_KERNEL, (unsigned)rank, (unsigned long long)total);
     }
   }
-  // 3. one warp per token.  The first expert of each destination rank gets the row over
-  // NVLink, straight into its final place; the destination is left a group record (all rows
-  // of that token there, leader first) from which it makes the other copies locally.
-  const int warpsPerCta = nt >> 5, warp = t >> 5, lane = t & 31;
+  // 3. eight lanes per token work out where its rows go.  The first expert of each destination
+  // rank gets the row over NVLink, straight into its final place; the destination is left a group
+  // record (all rows of that token there, leader first) from which it makes the other copies
+  // locally.  Then one warp per piece of a row moves the data.
+  const int warps = nt >> 5, warp = t >> 5, lane = t & 31;
   const int vecs = a.H / 8; // 16-byte vectors per row
   const size_t rowBytes = (size_t)a.H * 2;
   const int capPer = ((a.maxT + g - 1) / g) * a.K;
-  for (int tok = tlo + warp; tok < thi; tok += warpsPerCta) {
-    int d = -1, row = 0;
-    bool valid = false;
-    if (lane < a.K) {
-      const int i = tok * a.K + lane, e = a.topkIdx[i], rel = a.pos[i];
-      valid = rel >= 0;
-      if (valid) {
-        d = e / a.EPR;
-        row = base[e] + rel;
-        a.pos[i] = row; // any value >= 0 tells combine that the pair is real
-        a.route[2 * i] = d;
-        a.route[2 * i + 1] = row;
-        valid = (size_t)row < a.capacity; // rows past the capacity are reported by the receiver and dropped
+  const RowPieces pieces(vecs);
+  static_assert(FLAGCX_MOE_MAX_TOPK == 8, "a quarter of a warp per token");
+  for (int tok0 = tlo; tok0 < thi; tok0 += kMoeThreads) {
+    const int nTok = thi - tok0 < kMoeThreads ? thi - tok0 : kMoeThreads;
+    __syncthreads(); // the tables of counts, or the last batch's rows, have been read
+    for (int j0 = warp * 4; j0 < nTok; j0 += warps * 4) { // the whole warp stays together
+      const int j = j0 + (lane >> 3), k = lane & 7, tok = tok0 + j;
+      int d = 0, row = 0;
+      bool valid = false;
+      if (j < nTok && k < a.K) {
+        const int i = tok * a.K + k, e = a.topkIdx[i], rel = a.pos[i];
+        valid = rel >= 0;
+        if (valid) {
+          d = e / a.EPR;
+          row = s.base[e] + rel;
+          a.pos[i] = row; // any value >= 0 tells combine that the pair is real
+          a.route[2 * i] = d;
+          a.route[2 * i + 1] = row;
+          valid = (size_t)row < a.capacity; // rows past the capacity are reported by the receiver and dropped
+        }
+      }
+      // pairs of one token that go to one rank form a group; others (no pair, bad pair) are alone
+      const int alone = FLAGCX_MAX_RANKS * 4 + lane;
+      const unsigned members = __match_any_sync(0xffffffffu, valid && a.dedup ? (lane >> 3) * FLAGCX_MAX_RANKS + d : alone);
+      const int leader = __ffs(members) - 1, member = __popc(members & ((1u << lane) - 1u));
+      const bool isLeader = valid && lane == leader;
+      int idx = 0;
+      if (isLeader) idx = atomicAdd(&s.grpN[d], 1);
+      idx = __shfl_sync(0xffffffffu, idx, leader);
+      // the token's groups, packed: entry j = pair index of the j-th leader, -1 after the last
+      const unsigned leaders = (__ballot_sync(0xffffffffu, isLeader) >> (lane & 24)) & 0xffu;
+      const int at = __popc(leaders & ((1u << k) - 1u)), nLead = __popc(leaders);
+      if (j < nTok) {
+        if (isLeader) {
+          a.lead[tok * a.K + at] = k;
+          s.row[j][at] = a.recv[d] + (size_t)row * rowBytes;
+        }
+        if (k >= nLead && k < a.K) a.lead[tok * a.K + k] = -1;
+        if (k == 0) s.nRows[j] = nLead;
+      }
+      if (valid && idx < capPer) {
+        int *rec = a.grpList[d] + ((size_t)rank * a.grpRecordsPerSender + (size_t)b * capPer + idx) * FLAGCX_MOE_MAX_TOPK;
+        rec[member] = row;
+        if (isLeader)
+          for (int m = __popc(members); m < FLAGCX_MOE_MAX_TOPK; ++m) rec[m] = -1;
       }
     }
-    int firstLane = lane;
-    for (int j = a.K - 1; j >= 0; --j) { // the smallest earlier lane with the same destination wins
-      const int dj = __shfl_sync(0xffffffffu, valid ? d : -1, j);
-      if (a.dedup && valid && j < lane && dj == d) firstLane = j;
+    __syncthreads();
+    for (int i = warp; i < nTok * pieces.count; i += warps) {
+      const int j = i / pieces.count, first = (i - j * pieces.count) * pieces.vecs;
+      const int end = first + pieces.vecs < vecs ? first + pieces.vecs : vecs;
+      warpCopyPiece(s.row[j], s.nRows[j], (const char *)(a.x + (size_t)(tok0 + j) * a.H), first, end, lane, false);
     }
-    // lanes of one group find each other; the others (no pair, bad pair) are alone
-    const unsigned members = __match_any_sync(0xffffffffu, valid ? firstLane : 32 + lane);
-    const int member = __popc(members & ((1u << lane) - 1u)), groupSize = __popc(members);
-    const bool isFirst = valid && member == 0;
-    int idx = 0;
-    if (isFirst) idx = atomicAdd(&grpN[d], 1);
-    idx = __shfl_sync(0xffffffffu, idx, firstLane);
-    // the token's groups, packed: entry j = pair index of the j-th leader, -1 after the last
-    const unsigned leaders = __ballot_sync(0xffffffffu, isFirst);
-    if (lane < a.K) a.lead[tok * a.K + lane] = -1;
-    __syncwarp();
-    if (isFirst) a.lead[tok * a.K + __popc(leaders & ((1u << lane) - 1u))] = lane;
-    if (valid && idx < capPer) {
-      int *rec = a.grpList[d] + ((size_t)rank * a.grpRecordsPerSender + (size_t)b * capPer + idx) * FLAGCX_MOE_MAX_TOPK;
-      rec[member] = row;
-      if (isFirst)
-        for (int j = groupSize; j < FLAGCX_MOE_MAX_TOPK; ++j) rec[j] = -1;
-    }
-    char *dst[FLAGCX_MOE_MAX_TOPK];
-#pragma unroll
-    for (int k = 0; k < FLAGCX_MOE_MAX_TOPK; ++k) { // lanes from K on hold no pair
-      const int dk = __shfl_sync(0xffffffffu, d, k), rowk = __shfl_sync(0xffffffffu, row, k);
-      const bool fk = __shfl_sync(0xffffffffu, isFirst ? 1 : 0, k) != 0;
-      dst[k] = fk ? a.recv[dk] + (size_t)rowk * rowBytes : nullptr;
-    }
-    warpCopyRow(dst, (const char *)(a.x + (size_t)tok * a.H), vecs, lane, false);
   }
   __syncthreads();
-  if (t < n) a.grpCount[t][(size_t)rank * FLAGCX_COLL_BARRIER_SLOTS + b] = grpN[t] < capPer ? grpN[t] : capPer;
+  if (t < n) a.grpCount[t][(size_t)rank * FLAGCX_COLL_BARRIER_SLOTS + b] = s.grpN[t] < capPer ? s.grpN[t] : capPer;
   if (!ctaBarrier(c, b)) return;
-  // 4. the copies the senders' CTA b left to this rank: row to row inside my own buffer
-  for (int q = 0; q < n; ++q) {
-    const int cnt = ldSysElem(a.grpCount[rank] + (size_t)q * FLAGCX_COLL_BARRIER_SLOTS + b);
-    const int *recs = a.grpList[rank] + ((size_t)q * a.grpRecordsPerSender + (size_t)b * capPer) * FLAGCX_MOE_MAX_TOPK;
-    for (int r = warp; r < cnt; r += warpsPerCta) {
-      int rows[FLAGCX_MOE_MAX_TOPK];
-      loadGroup(recs + (size_t)r * FLAGCX_MOE_MAX_TOPK, rows);
-      if ((size_t)rows[0] >= a.capacity) continue;
-      char *dst[FLAGCX_MOE_MAX_TOPK];
-      dst[0] = nullptr;
+  // 4. the copies the senders' CTA b left to this rank: row to row inside my own buffer.  A thread
+  // looks at one record; those with more than one row are collected, and their pieces shared out.
+  int start[FLAGCX_MAX_RANKS + 1]; // records of senders 0 .. q-1
+  start[0] = 0;
 #pragma unroll
-      for (int j = 1; j < FLAGCX_MOE_MAX_TOPK; ++j)
-        dst[j] = rows[j] >= 0 && (size_t)rows[j] < a.capacity ? a.recv[rank] + (size_t)rows[j] * rowBytes : nullptr;
-      if (rows[1] >= 0) warpCopyRow(dst, a.recv[rank] + (size_t)rows[0] * rowBytes, vecs, lane, true); // packed: none after -1
+  for (int q = 0; q < FLAGCX_MAX_RANKS; ++q)
+    start[q + 1] = q < n ? ldSysElem(a.grpCount[rank] + (size_t)q * FLAGCX_COLL_BARRIER_SLOTS + b) : 0;
+#pragma unroll
+  for (int q = 0; q < FLAGCX_MAX_RANKS; ++q) start[q + 1] += start[q];
+  for (int r0 = 0; r0 < start[FLAGCX_MAX_RANKS]; r0 += nt) {
+    if (t == 0) s.nRec = 0;
+    __syncthreads();
+    const int r = r0 + t;
+    if (r < start[FLAGCX_MAX_RANKS]) {
+      int q = 0, before = 0;
+#pragma unroll
+      for (int p = 1; p < FLAGCX_MAX_RANKS; ++p)
+        if (r >= start[p]) { q = p; before = start[p]; }
+      const int *rec = a.grpList[rank] +
+                       ((size_t)q * a.grpRecordsPerSender + (size_t)b * capPer + (r - before)) * FLAGCX_MOE_MAX_TOPK;
+      int rows[FLAGCX_MOE_MAX_TOPK];
+      loadGroup(rec, rows);
+      if (rows[1] >= 0 && (size_t)rows[0] < a.capacity) { // packed: no row after -1
+        const int at = atomicAdd(&s.nRec, 1);
+        int m = 0;
+#pragma unroll
+        for (int k = 0; k < FLAGCX_MOE_MAX_TOPK; ++k)
+          if (rows[k] >= 0 && (size_t)rows[k] < a.capacity) s.row[at][m++] = a.recv[rank] + (size_t)rows[k] * rowBytes;
+        s.nRows[at] = m;
+      }
     }
+    __syncthreads();
+    const int nRec = s.nRec;
+    for (int i = warp; i < nRec * pieces.count; i += warps) {
+      const int j = i / pieces.count, first = (i - j * pieces.count) * pieces.vecs;
+      const int end = first + pieces.vecs < vecs ? first + pieces.vecs : vecs;
+      warpCopyPiece(s.row[j] + 1, s.nRows[j] - 1, s.row[j][0], first, end, lane, true);
+    }
+    __syncthreads();
   }
 }
 
 // Pull-everything combine: the token's owner reads each (token, expert) row and weights it.
 // Independent of the dispatch's CTA layout (it needs only the route), so it runs as CTAs of
 // 512 threads: measured faster that way (402 against 527 us on two B200s for the same
-// number of warps in 256-thread CTAs).
+// number of warps in 256-thread CTAs).  A warp draws a part of a token at a time, so that few tokens
+// occupy all warps and many end together.  Eight emulated ranks, 512 tokens x 7168: 135 -> 99 us with
+// twice the CTAs (107), the parts drawn by ticket, and a cheaper barrier; 530 MB, 81 us for a copy.
 __device__ void combinePullBody(const flagcxDevComm &c, const MoeArgs &a) {
   const int b = blockIdx.x, g = gridDim.x;
   const int t = threadIdx.x, nt = blockDim.x;
-  if (!ctaBarrier(c, b)) return; // every rank's expert outputs are complete
-  const int warpsPerCta = nt >> 5, warp = t >> 5, lane = t & 31;
+  const int warpsPerCta = nt >> 5, lane = t & 31;
   const int vecs = a.H / 8;
   const size_t rowBytes = (size_t)a.H * 2;
-  for (int tok = b * warpsPerCta + warp; tok < a.T; tok += g * warpsPerCta) {
+  constexpr int U = 2; // vectors of every row in flight per lane
+  // four parts or more per warp, of whole rounds of the loop below
+  const int rounds = (vecs + 32 * U - 1) / (32 * U), wanted = a.T > 0 ? (4 * g * warpsPerCta + a.T - 1) / a.T : 1;
+  const int perPart = (rounds + wanted - 1) / wanted, parts = (rounds + perPart - 1) / perPart;
+  const Tickets tickets{a.tickets};
+  const bool met = ctaBarrier(c, b); // every rank's expert outputs are complete
+  int item = met ? (int)tickets.take() : a.T * parts;
+  while (item < a.T * parts) {
+    const int next = (int)tickets.take(); // on its way while this one is worked on
+    const int tok = item / parts, first = (item - tok * parts) * perPart * 32 * U;
+    const int end = first + perPart * 32 * U < vecs ? first + perPart * 32 * U : vecs;
     const char *rows[FLAGCX_MOE_MAX_TOPK];
     float w[FLAGCX_MOE_MAX_TOPK];
 #pragma unroll
@@ -300,13 +376,12 @@ __device__ void combinePullBody(const flagcxDevComm &c, const MoeArgs &a) {
       }
     }
     uint4 *dst = (uint4 *)(a.out + (size_t)tok * a.H);
-    constexpr int U = 2; // vectors of every row in flight per lane
-    for (int v0 = lane; v0 < vecs; v0 += 32 * U) {
+    for (int v0 = first + lane; v0 < end; v0 += 32 * U) {
       uint4 r[U][FLAGCX_MOE_MAX_TOPK];
 #pragma unroll
       for (int u = 0; u < U; ++u) {
         const int v = v0 + 32 * u;
-        if (v < vecs) {
+        if (v < end) {
 #pragma unroll
           for (int k = 0; k < FLAGCX_MOE_MAX_TOPK; ++k)
             if (rows[k]) r[u][k] = ldSys16(rows[k] + (size_t)v * 16);
@@ -315,7 +390,7 @@ __device__ void combinePullBody(const flagcxDevComm &c, const MoeArgs &a) {
 #pragma unroll
       for (int u = 0; u < U; ++u) {
         const int v = v0 + 32 * u;
-        if (v < vecs) {
+        if (v < end) {
           float acc[8] = {0, 0, 0, 0, 0, 0, 0, 0};
 #pragma unroll
           for (int k = 0; k < FLAGCX_MOE_MAX_TOPK; ++k)
@@ -332,8 +407,10 @@ __device__ void combinePullBody(const flagcxDevComm &c, const MoeArgs &a) {
         }
       }
     }
+    item = next;
   }
-  ctaBarrier(c, b); // peers may overwrite their expert outputs only after everyone has read them
+  tickets.leave();
+  if (met) ctaBarrier(c, b); // peers may overwrite their expert outputs only after everyone has read them
 }
 
 // Pre-reducing combine.  Everything is organised per CTA index, like the dispatch: the
@@ -345,8 +422,7 @@ __device__ void combineReduceBody(const flagcxDevComm &c, const MoeArgs &a) {
   const int warpsPerCta = nt >> 5, warp = t >> 5, lane = t & 31;
   const int vecs = a.H / 8;
   const size_t rowBytes = (size_t)a.H * 2;
-  const int tpc = (a.T + g - 1) / g; // the dispatch's token ranges
-  const int tlo = b * tpc < a.T ? b * tpc : a.T, thi = tlo + tpc < a.T ? tlo + tpc : a.T;
+  const int tlo = firstToken(a.T, b, g), thi = firstToken(a.T, b + 1, g); // the dispatch's token ranges
   const int capPer = ((a.maxT + g - 1) / g) * a.K;
   // 0. the gate weight of each of my pairs goes next to the row it weights
   for (int i = tlo * a.K + t; i < thi * a.K; i += nt) {
@@ -400,21 +476,24 @@ __device__ void combineReduceBody(const flagcxDevComm &c, const MoeArgs &a) {
 }
 
 
-__global__ void __launch_bounds__(kMoeThreads) moeDispatchKernel(const flagcxDevComm c, const MoeArgs a) {
+__global__ void __launch_bounds__(kMoeThreads)
+    moeDispatchKernel(const __grid_constant__ flagcxDevComm c, const __grid_constant__ MoeArgs a) {
   dispatchBody(c, a);
 }
 __global__ void __launch_bounds__(kMoeThreads)
     moeDispatchKernelEmu(const __grid_constant__ EmuLaunch<MoeArgs> e) {
   dispatchBody(e.comm[blockIdx.y], e.args[blockIdx.y]);
 }
-__global__ void __launch_bounds__(kMoeThreads) moeCombineKernel(const flagcxDevComm c, const MoeArgs a) {
+__global__ void __launch_bounds__(kMoeThreads)
+    moeCombineKernel(const __grid_constant__ flagcxDevComm c, const __grid_constant__ MoeArgs a) {
   combineReduceBody(c, a);
 }
 __global__ void __launch_bounds__(kMoeThreads)
     moeCombineKernelEmu(const __grid_constant__ EmuLaunch<MoeArgs> e) {
   combineReduceBody(e.comm[blockIdx.y], e.args[blockIdx.y]);
 }
-__global__ void __launch_bounds__(FLAGCX_DEVICE_THREADS_PER_CTA) moeCombinePullKernel(const flagcxDevComm c, const MoeArgs a) {
+__global__ void __launch_bounds__(FLAGCX_DEVICE_THREADS_PER_CTA)
+    moeCombinePullKernel(const __grid_constant__ flagcxDevComm c, const __grid_constant__ MoeArgs a) {
   combinePullBody(c, a);
 }
 __global__ void __launch_bounds__(FLAGCX_DEVICE_THREADS_PER_CTA)
@@ -424,22 +503,40 @@ __global__ void __launch_bounds__(FLAGCX_DEVICE_THREADS_PER_CTA)
 
 } // namespace
 
+// The emulated world has fewer CTAs per rank to offer than a GPU of its own.  The pre-reducing
+// combine must run as many as the dispatch that left it its records: what both kernels have room for.
+static cudaError_t emuMoeCtas(const LaunchCtx &lc, bool preReduce, int *ctas) {
+  int forDispatch = 0, forCombine = lc.nCtas;
+  cudaError_t e = emuCtasPerRank<moeDispatchKernelEmu>(kMoeThreads, lc.emuRanks, &forDispatch);
+  if (e == cudaSuccess && preReduce) e = emuCtasPerRank<moeCombineKernelEmu>(kMoeThreads, lc.emuRanks, &forCombine);
+  *ctas = std::min(lc.nCtas, std::min(forDispatch, forCombine));
+  return e;
+}
+
 cudaError_t launchMoeDispatch(const LaunchCtx &lc, const MoeArgs &a) {
-  dim3 grid(lc.nCtas, lc.emuRanks > 0 ? lc.emuRanks : 1), block(kMoeThreads);
-  if (lc.emuRanks > 0) return launchEmu(moeDispatchKernelEmu, lc, lc.emuMoe, grid, block, 0);
-  moeDispatchKernel<<<grid, block, 0, lc.stream>>>(*lc.comm, a);
+  if (lc.emuRanks > 0) {
+    int ctas = 0;
+    const cudaError_t e = emuMoeCtas(lc, a.preReduce != 0, &ctas);
+    return e != cudaSuccess ? e : launchEmu(moeDispatchKernelEmu, lc, lc.emuMoe, dim3(ctas, lc.emuRanks), dim3(kMoeThreads), 0);
+  }
+  moeDispatchKernel<<<lc.nCtas, kMoeThreads, 0, lc.stream>>>(*lc.comm, a);
   return cudaGetLastError();
 }
 
 // a.preReduce picks the kernel; the pull kind takes half as many CTAs of twice the threads.
 cudaError_t launchMoeCombine(const LaunchCtx &lc, const MoeArgs &a) {
   const bool pull = a.preReduce == 0;
-  const int ctas = pull ? (lc.nCtas + 1) / 2 : lc.nCtas;
-  dim3 grid(ctas, lc.emuRanks > 0 ? lc.emuRanks : 1), block(pull ? FLAGCX_DEVICE_THREADS_PER_CTA : kMoeThreads);
-  if (lc.emuRanks > 0)
-    return launchEmu(pull ? moeCombinePullKernelEmu : moeCombineKernelEmu, lc, lc.emuMoe, grid, block, 0);
-  if (pull) moeCombinePullKernel<<<grid, block, 0, lc.stream>>>(*lc.comm, a);
-  else moeCombineKernel<<<grid, block, 0, lc.stream>>>(*lc.comm, a);
+  const int pullCtas = (lc.nCtas + 1) / 2, pullThreads = FLAGCX_DEVICE_THREADS_PER_CTA;
+  if (lc.emuRanks > 0) {
+    int ctas = 0;
+    cudaError_t e = pull ? emuCtasPerRank<moeCombinePullKernelEmu>(pullThreads, lc.emuRanks, &ctas) : emuMoeCtas(lc, true, &ctas);
+    if (e != cudaSuccess) return e;
+    if (pull)
+      return launchEmu(moeCombinePullKernelEmu, lc, lc.emuMoe, dim3(std::min(ctas, pullCtas), lc.emuRanks), dim3(pullThreads), 0);
+    return launchEmu(moeCombineKernelEmu, lc, lc.emuMoe, dim3(ctas, lc.emuRanks), dim3(kMoeThreads), 0);
+  }
+  if (pull) moeCombinePullKernel<<<pullCtas, pullThreads, 0, lc.stream>>>(*lc.comm, a);
+  else moeCombineKernel<<<lc.nCtas, kMoeThreads, 0, lc.stream>>>(*lc.comm, a);
   return cudaGetLastError();
 }
 

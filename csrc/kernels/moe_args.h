@@ -37,6 +37,7 @@ struct MoeArgs {
   int *lead;               // local [T*K]: per token, the pair indices of its group leaders packed to the front, then -1
   float *wRow[FLAGCX_MAX_RANKS];     // wRow[p]: rank p's gate weight per received row (pushed by the combine)
   char *partial[FLAGCX_MAX_RANKS];   // partial[p]: rank p's pre-reduced rows, indexed by the group's leader row
+  unsigned *tickets;                 // local: two words for Tickets, zero between launches
   int T, H, K, E, EPR;
   size_t capacity;         // rows in recv / expertOut
 };

@@ -90,3 +90,42 @@ def test_capacity_overflow_is_reported_not_written():
         assert comms[0].async_error() == capi.flagcxInvalidArgument
     finally:
         capi.Comm.emu_world_destroy(comms)
+
+
+# more tokens than a CTA's table holds (256), more groups than it looks at in one turn, rows that
+# end inside a piece (257 vectors: pieces of 160 and 97) and inside a round of the combine
+@pytest.mark.parametrize("T,H,ctas", [(1, 8, 3), (256, 64, 1), (257, 64, 1), (600, 264, 2), (31, 2056, 1)])
+@pytest.mark.parametrize("reduce", [1, 0])
+def test_few_ctas_and_ragged_rows(T, H, ctas, reduce, monkeypatch):
+    monkeypatch.setenv("FLAGCX_MOE_CTAS", str(ctas))
+    monkeypatch.setenv("FLAGCX_MOE_COMBINE_REDUCE", str(reduce))
+    n, E, K = 2, 8, 5
+    comms = capi.Comm.emu_world(n, 0)
+    try:
+        moes = [MoeDispatcher(comms[r], T, H, K, E, T * K * n) for r in range(n)]
+        g = torch.Generator().manual_seed(T)
+        for t in (T, max(1, T // 3), T):  # a second batch of another size, and a third
+            xs = [torch.randn(t, H, generator=g).to(torch.bfloat16).cuda() for _ in range(n)]
+            routed = [route(torch.randn(t, E, generator=g).cuda(), K) for _ in range(n)]
+            for r in range(n):
+                moes[r].dispatch(xs[r], routed[r][0])
+            for m in moes:
+                offs = m.expert_offsets.cpu().tolist()
+                for le in range(E // n):
+                    scale = moes.index(m) * (E // n) + le + 1
+                    m.expert_out[offs[le]:offs[le + 1]] = (m.recv_rows[offs[le]:offs[le + 1]].float() * scale).to(torch.bfloat16)
+            outs = [torch.full((t, H), float("nan"), dtype=torch.bfloat16, device="cuda") for _ in range(n)]
+            for r in range(n):
+                moes[r].combine(routed[r][1], outs[r])
+            torch.cuda.synchronize()
+            assert all(c.async_error() == 0 for c in comms)
+            for r in range(n):
+                idx, w = routed[r]
+                ref = xs[r].float() * (w * (idx.float() + 1)).sum(1, keepdim=True)
+                # all summands have one sign, so the three roundings to 8 significant bits (the expert's,
+                # the pre-reduced row's, the result's) change the result by 2^-8 of its value each
+                assert ((outs[r].float() - ref).abs() <= 3.02 * 2.0 ** -8 * ref.abs() + 1e-6).all()
+        for m in moes:
+            m.close()
+    finally:
+        capi.Comm.emu_world_destroy(comms)
