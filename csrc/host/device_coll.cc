@@ -179,6 +179,7 @@ void initArgs(flagcxComm *c, CollArgs &a, int kind, flagcxDataType_t dt) {
   a.elemSize = (int)getFlagcxDataTypeSize(dt);
   a.scale = 1.0f;
   a.flags = kFlagBeginBarrier | kFlagEndBarrier;
+  a.tickets = c->tickets;
   for (int p = 0; p < c->nranks; ++p) {
     a.meta[p] = (unsigned long long *)((char *)c->internalWin->peer[p] + c->layout.metaOff);
     a.ptrPad[p] = (unsigned long long *)((char *)c->internalWin->peer[p] + c->layout.ptrPadOff);

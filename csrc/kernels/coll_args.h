@@ -96,6 +96,7 @@ struct CollArgs {
   unsigned long long *ringNext, *ringMine;
   unsigned long long ringBase;
   size_t ringSlotElems;
+  unsigned *tickets;   // local: two words for Tickets (prims.cuh), zero between launches
   size_t llSlotBytes;
   uint32_t llEpoch;    // value of the flags of this operation (never 0)
   uint32_t llPad;

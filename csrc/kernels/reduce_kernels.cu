@@ -24,6 +24,15 @@ namespace {
 // ---------------------------------------------------------------------------
 // reduce family
 // ---------------------------------------------------------------------------
+// Bound: memory, by the SM that gets least of it.  Large ranges are drawn by ticket instead of
+// cut into equal shares: eight emulated ranks x 32 MiB bf16 119 -> 97 us (5.5 TB/s with both
+// barriers; the main loop alone 105 -> 90), fp32 217 -> 180.  From kDrawItems items of 16 loads per
+// warp on; with less (1 Mi elements: 4 packs a thread) the barriers are most of the time and both
+// ways take the same.
+constexpr int kDrawItems = 2;
+// Loads in flight per thread: 16 where few CTAs run (32 CTAs: 209 against 250 us with 8), 8 where
+// they fill the GPU (144 CTAs: 97 against 105 us with 16, fp32 180 against 212).
+constexpr unsigned kDrawHalfCtas = 128;
 template <typename T, int OP, int NR>
 struct Reducer {
   using Acc = typename Elem<T>::Acc;
@@ -124,11 +133,53 @@ struct Reducer {
     }
   }
 
+  // Whole packs [0, packs) of a range that starts at element sb of the inputs, drawn by the warps
+  // in items of 32 x U packs; every pack's U x NR loads are under way before the first is used.
+  template <int U>
+  static __device__ __forceinline__ void drawPacks(const CollArgs &a, size_t sb, size_t packs, char *const *dst, int nDst,
+                                                   size_t dstBase) {
+    const Tickets tickets{a.tickets};
+    const int lane = threadIdx.x & 31;
+    const size_t items = (packs + 32 * U - 1) / (32 * U);
+    for (size_t item = tickets.take(); item < items;) {
+      const size_t next = tickets.take(); // on its way while this one is worked on
+      const size_t first = item * (32 * U) + lane;
+      uint4 v[U][NR];
+#pragma unroll
+      for (int u = 0; u < U; ++u)
+        if (first + u * 32 < packs) {
+#pragma unroll
+          for (int p = 0; p < NR; ++p) v[u][p] = ldSys16(a.in[p] + sb * sizeof(T) + ((first + u * 32) << 4));
+        }
+#pragma unroll
+      for (int u = 0; u < U; ++u)
+        if (first + u * 32 < packs) {
+          Acc acc[N];
+          addUp(a, v[u], acc);
+          storePack(a, dst, nDst, dstBase + (first + u * 32) * N, acc);
+        }
+      item = next;
+    }
+    tickets.leave();
+  }
+
+  static __device__ __forceinline__ void addUp(const CollArgs &a, const uint4 (&v)[NR > 0 ? NR : 1], Acc (&acc)[N]) {
+    const T *e0 = (const T *)&v[0];
+#pragma unroll
+    for (int i = 0; i < N; ++i) acc[i] = toAcc<T>(e0[i]);
+#pragma unroll
+    for (int p = 1; p < NR; ++p) {
+      const T *ep = (const T *)&v[p];
+#pragma unroll
+      for (int i = 0; i < N; ++i) acc[i] = combine<OP, Acc>(acc[i], toAcc<T>(ep[i]), a.redOp);
+    }
+  }
+
   // Reduces elements [sb, se) of the inputs (indices into in[p]) and stores them at
   // element index (i - sb + dstBase) of each destination.  The CTA takes its share
-  // of the range in 16-byte units.
+  // of the range in 16-byte units, or (mayDraw) draws them where that pays.
   static __device__ void slice(const CollArgs &a, int nRanks, size_t sb, size_t se, char *const *dst, int nDst,
-                               size_t dstBase, int b, int g) {
+                               size_t dstBase, int b, int g, bool mayDraw = false) {
     if (se <= sb) return;
     const size_t elems = se - sb;
     const size_t outSize = a.outMode == kOutFloat ? 4 : (a.outMode == kOutBf16 ? 2 : sizeof(T));
@@ -139,7 +190,19 @@ struct Reducer {
     size_t ub, ue;
     ctaShare((elems * sizeof(T) + 15) >> 4, b, g, &ub, &ue);
     size_t eb = ub * N, ee = ue * N < elems ? ue * N : elems; // this CTA's elements, relative to sb
-    if (vec) {
+    bool drawn = false;
+    if constexpr (NR > 0) {
+      constexpr int U = 16 / NR; // peer loads take microseconds: 16 of them in flight per thread
+      const size_t packs = elems / N;
+      drawn = vec && mayDraw && packs >= (size_t)kDrawItems * 32 * U * (blockDim.x >> 5) * g;
+      if (drawn) {
+        if (gridDim.x * gridDim.y >= kDrawHalfCtas) drawPacks<U / 2>(a, sb, packs, dst, nDst, dstBase);
+        else drawPacks<U>(a, sb, packs, dst, nDst, dstBase);
+        eb = packs * N; // what is left is less than a pack: the last CTA's
+        ee = b == g - 1 ? elems : eb;
+      }
+    }
+    if (vec && !drawn) {
       const size_t fullEnd = ee / N * N; // whole packs only
       const size_t stride = (size_t)blockDim.x * N;
       size_t e = eb + (size_t)threadIdx.x * N;
@@ -155,15 +218,7 @@ struct Reducer {
 #pragma unroll
           for (int u = 0; u < U; ++u) {
             Acc acc[N];
-            const T *e0 = (const T *)&v[u][0];
-#pragma unroll
-            for (int i = 0; i < N; ++i) acc[i] = toAcc<T>(e0[i]);
-#pragma unroll
-            for (int p = 1; p < NR; ++p) {
-              const T *ep = (const T *)&v[u][p];
-#pragma unroll
-              for (int i = 0; i < N; ++i) acc[i] = combine<OP, Acc>(acc[i], toAcc<T>(ep[i]), a.redOp);
-            }
+            addUp(a, v[u], acc);
             storePack(a, dst, nDst, dstBase + e + u * stride, acc);
           }
         }
@@ -399,6 +454,7 @@ __device__ void reduceBody(const flagcxDevComm &c, CollArgs &a) {
     if (!ctaBarrier(c, b)) return;
   learnPointers(c, a, b);
   const bool bulk = NR > 0 && a.bulkStage && learntPointersAligned(c, a);
+  const bool direct = !a.userIn && !a.userOut; // else CTA b must take what CTA b has staged, and only that
   {
     const size_t outEs = a.outMode == kOutFloat ? 4 : (a.outMode == kOutBf16 ? 2 : sizeof(T));
     const size_t inEnd = a.kind == kReduceScatter ? a.inStride * (size_t)(n - 1) + a.count * sizeof(T)
@@ -418,7 +474,7 @@ __device__ void reduceBody(const flagcxDevComm &c, CollArgs &a) {
   char *local[1] = {a.out[rank]};
   switch (a.kind) {
     case kAllReduceOneShot:
-      R::slice(a, n, 0, a.count, local, 1, 0, b, g);
+      R::slice(a, n, 0, a.count, local, 1, 0, b, g, direct);
       break;
     case kAllReduceTwoShot: {
       size_t s = sliceElems(a.count, n, sizeof(T));
@@ -427,7 +483,7 @@ __device__ void reduceBody(const flagcxDevComm &c, CollArgs &a) {
       if (bulk) {
         if (!R::sliceBulk(c, a, sb, se, a.out, n, sb, b, g)) return;
       } else {
-        R::slice(a, n, sb, se, a.out, n, sb, b, g);
+        R::slice(a, n, sb, se, a.out, n, sb, b, g, direct);
       }
       break;
     }
@@ -436,12 +492,12 @@ __device__ void reduceBody(const flagcxDevComm &c, CollArgs &a) {
       if (bulk) {
         if (!R::sliceBulk(c, a, sb, sb + a.count, local, 1, 0, b, g)) return;
       } else {
-        R::slice(a, n, sb, sb + a.count, local, 1, 0, b, g);
+        R::slice(a, n, sb, sb + a.count, local, 1, 0, b, g, direct);
       }
       break;
     }
     case kReduceToRoot:
-      if (rank == a.root) R::slice(a, n, 0, a.count, local, 1, 0, b, g);
+      if (rank == a.root) R::slice(a, n, 0, a.count, local, 1, 0, b, g, direct);
       break;
     case kReduceScatterRing:
       if (!ringReduceScatter<T, OP>(c, a, a.count, a.count * (size_t)n, (T *)a.out[rank], b, g)) return;

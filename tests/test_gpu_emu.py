@@ -137,6 +137,40 @@ def test_allreduce_in_place_and_large(n):
         check_close(xs[r], ref, capi.BFLOAT16, n, f"in-place rank {r}")
 
 
+# Warps draw packs by ticket from 2 items of 32 x (16 / ranks) packs per warp and rank slice on: just
+# below, at and beyond that line, with a remainder of less than a pack; on few CTAs (16 loads per
+# thread) and on 128 (8 loads).  Twice each: the tickets are back at zero for the second launch.
+@pytest.mark.parametrize("n,nctas", [(2, 1), (4, 2), (8, 1), (8, 16), (2, 64)])
+@pytest.mark.parametrize("dt", [capi.FLOAT, capi.BFLOAT16, capi.HALF])
+@pytest.mark.parametrize("extra", [-1, 0, 1])
+def test_reductions_by_ticket(n, nctas, dt, extra):
+    comms = world(n)
+    per = 16 // capi.DT_SIZE[dt]
+    line = 2 * 32 * (16 // n) * 16 * nctas
+    block = (line + extra) * per
+    count = block * n - (3 if extra == 1 else 0)  # the last rank's slice ends inside a pack
+    xs = make_inputs(n, count, dt)
+    ref = reference(xs, capi.SUM)
+    for _ in range(2):
+        outs = [torch.full_like(x, float("nan")) for x in xs]
+        for r in range(n):
+            comms[r].all_reduce_fused(xs[r], outs[r], count, dt, capi.SUM, algo=capi.ALGO_TWOSHOT, nctas=nctas)
+        torch.cuda.synchronize()
+        assert_no_device_error(comms)
+        check_close(outs[0], ref, dt, n, "two-shot")
+        for r in range(1, n):
+            assert torch.equal(outs[r], outs[0])
+    block = min(block, count // n)
+    scattered = [torch.full((block,), float("nan"), dtype=torch.float32, device="cuda") for _ in range(n)]
+    wide = capi.FLOAT if dt != capi.FLOAT else capi.NUM_TYPES
+    for r in range(n):
+        comms[r].reduce_scatter_fused(xs[r], scattered[r], block, dt, capi.SUM, scale=0.5, out_dtype=wide, nctas=nctas)
+    torch.cuda.synchronize()
+    assert_no_device_error(comms)
+    for r in range(n):
+        check_close(scattered[r], ref[r * block:(r + 1) * block] * 0.5, capi.FLOAT, n, f"reduce-scatter rank {r}")
+
+
 @pytest.mark.parametrize("n", [2, 4])
 @pytest.mark.parametrize("algo", [capi.ALGO_ONESHOT, capi.ALGO_TWOSHOT])
 def test_allreduce_fused_scale_cast_residual(n, algo):
