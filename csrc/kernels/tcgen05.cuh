@@ -139,6 +139,15 @@ __device__ __forceinline__ uint32_t clusterCtaRank() {
 __device__ __forceinline__ void clusterSync() {
   asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
+// The same where nothing is to be published: prior accesses need only have been issued.
+__device__ __forceinline__ void clusterSyncRelaxed() {
+  asm volatile("barrier.cluster.arrive.relaxed.aligned;\n\tbarrier.cluster.wait.aligned;" ::: "memory");
+}
+// A kernel launched with programmatic serialization may start before the one in front of it has
+// ended: nothing it reads or writes in global memory may come before the wait, which returns when
+// all of that kernel's work is done and visible.  The second lets the next such kernel start.
+__device__ __forceinline__ void waitForEarlierGrid() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void letNextGridStart() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 // shared::cluster address of the same shared variable in CTA `rank` of the cluster
 __device__ __forceinline__ uint32_t mapToCta(uint32_t localSmemAddr, uint32_t rank) {
   uint32_t r;

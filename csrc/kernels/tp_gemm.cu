@@ -188,6 +188,10 @@ __global__ void __launch_bounds__(kThreads, 1)
   __syncthreads();
   if (PAIR) clusterSync(); // the partner's barriers exist before anything is signalled on them
   fenceAfterSync();
+  if (a.mode == kPlain) { // the fused modes are launched without programmatic serialization
+    waitForEarlierGrid();
+    letNextGridStart();
+  }
   const uint32_t tmemBase = s.tmemBase;
   volatile int *abortFlag = &s.abortFlag;
 
@@ -501,23 +505,21 @@ cudaError_t launchTpGemm(cudaStream_t stream, const CUtensorMap &tmA, const CUte
     if (e != cudaSuccess) return e;
     configured[pair] = true;
   }
-  if (!pair) {
-    tpGemmKernel<false><<<nCtas, kThreads, tpGemmSmemBytes(false), stream>>>(tmA, tmB, sm, c, a);
-    return cudaGetLastError();
-  }
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(nCtas & ~1);
+  cfg.gridDim = dim3(pair ? nCtas & ~1 : nCtas);
   cfg.blockDim = dim3(kThreads);
-  cfg.dynamicSmemBytes = tpGemmSmemBytes(true);
+  cfg.dynamicSmemBytes = tpGemmSmemBytes(pair);
   cfg.stream = stream;
-  cudaLaunchAttribute attr[1];
+  cudaLaunchAttribute attr[2];
   attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = 2;
+  attr[0].val.clusterDim.x = pair ? 2 : 1;
   attr[0].val.clusterDim.y = 1;
   attr[0].val.clusterDim.z = 1;
+  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
-  cfg.numAttrs = 1;
-  return cudaLaunchKernelEx(&cfg, tpGemmKernel<true>, tmA, tmB, sm, c, a);
+  cfg.numAttrs = a.mode == kPlain ? 2 : 1;
+  return cudaLaunchKernelEx(&cfg, pair ? tpGemmKernel<true> : tpGemmKernel<false>, tmA, tmB, sm, c, a);
 }
 
 } // namespace fcx

@@ -66,6 +66,39 @@ def test_gemm_whose_last_wave_is_nearly_empty(M, N, K):
     assert bool(((out.double() - ref).abs() <= bound).all())
 
 
+# A product starts while the one in front of it ends.  Each reads what the last wrote, into buffers
+# that are used again every third time: by the split kernel, the persistent one (CTA pairs and single
+# CTAs), and both (full waves and a split last one); plainly and captured.
+@pytest.mark.parametrize("M,N", [(128, 1024), (256, 2048), (640, 8192), (2048, 3328), (384, 8192)])
+def test_products_that_follow_one_another(M, N):
+    from flagcx_b200.parallel.tp import gemm_bf16
+    g = torch.Generator(device="cuda").manual_seed(M)
+    x = torch.randn(M, N, generator=g, device="cuda").to(torch.bfloat16)
+    w = (torch.randn(N, N, generator=g, device="cuda") * N ** -0.5).to(torch.bfloat16)
+
+    def chain(wait):
+        bufs = [torch.full((M, N), float("nan"), dtype=torch.bfloat16, device="cuda") for _ in range(3)]
+        src = x
+        for i in range(7):
+            gemm_bf16(src, w, bufs[i % 3])
+            if wait:
+                torch.cuda.synchronize()
+            src = bufs[i % 3]
+        return src
+
+    want = chain(True)
+    assert bool(torch.isfinite(want).all())
+    for _ in range(3):
+        assert torch.equal(chain(False), want)
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        got = chain(False)
+    for _ in range(3):
+        got.zero_()
+        graph.replay()
+        assert torch.equal(got, want)
+
+
 @pytest.mark.skipif(torch.cuda.device_count() < 2, reason="needs at least 2 GPUs")
 def test_fused_tensor_parallel_kernels_on_real_peers():
     n = 8 if torch.cuda.device_count() >= 8 else 4 if torch.cuda.device_count() >= 4 else 2
