@@ -103,6 +103,11 @@ __device__ __forceinline__ void mbarExpect(uint64_t *bar, uint32_t bytes) {
   asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(sharedAddr(bar)), "r"(bytes) : "memory");
 }
 
+// The weight gradient's sum over CTAs is launched with programmatic serialization: it may be set up
+// while the backward runs (letNextGridStart), and reads nothing before that is done and visible.
+__device__ __forceinline__ void letNextGridStart() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void waitForEarlierGrid() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
 struct Pack8 {
   uint4 raw;
   __device__ float get(int i) const { return __bfloat162float(((const bf16 *)&raw)[i]); }
@@ -110,79 +115,63 @@ struct Pack8 {
 };
 
 // ---------------------------------------------------------------------------
-// RMSNorm: y = x * rstd * w,  rstd = rsqrt(mean(x^2) + eps).  One CTA per row,
-// H a multiple of 8; a thread owns packs t, t+blockDim, ...
+// RMSNorm: y = x * rstd * w,  rstd = rsqrt(mean(x^2) + eps), H a multiple of 8.  A group of GT
+// threads takes a row and holds it in registers (PPT packs of 8 per thread); a CTA has four warps
+// or one group.  The row and the weights are on their way before the sum of squares is taken; the
+// hardware deals the CTAs out.  Bound: HBM for many rows, the chain load -> sum -> store for few.
+// Four packs per thread where they hold the row (eight of 256 threads beyond 8192 elements), us
+// against one warp per row up to 4096 elements and 512 threads beyond: 128 x 4096 8.3 -> 3.4, 1021 x
+// 4096 10.1 -> 6.1, 4096 x 4096 16.9 -> 14.4, 3000 x 2560 12.2 -> 9.1, 512 x 8192 6.2 -> 6.1, 1000 x
+// 16384 16.4 -> 14.5; at 512 threads with one pack each 1021 x 4096 takes 8.0, at 256 with two 6.3.
 // ---------------------------------------------------------------------------
-template <int MAXP>
-__global__ void rmsnormFwd(const bf16 *__restrict__ x, const bf16 *__restrict__ w, bf16 *__restrict__ y,
-                           float *__restrict__ rstdOut, int H, float eps) {
-  __shared__ float red[32];
-  const size_t row = blockIdx.x;
-  const uint4 *xr = (const uint4 *)(x + row * H);
-  const int nPacks = H / 8;
-  Pack8 px[MAXP];
-  float ss = 0.f;
-#pragma unroll
-  for (int k = 0; k < MAXP; ++k) {
-    int p = threadIdx.x + k * blockDim.x;
-    if (p < nPacks) {
-      px[k].raw = xr[p];
-#pragma unroll
-      for (int i = 0; i < 8; ++i) { float v = px[k].get(i); ss += v * v; }
-    }
-  }
-  ss = blockSum(ss, red);
-  const float rstd = rsqrtf(ss / H + eps);
-  if (threadIdx.x == 0) rstdOut[row] = rstd;
-  uint4 *yr = (uint4 *)(y + row * H);
-#pragma unroll
-  for (int k = 0; k < MAXP; ++k) {
-    int p = threadIdx.x + k * blockDim.x;
-    if (p < nPacks) {
-      Pack8 pw, po;
-      pw.raw = ((const uint4 *)w)[p];
-#pragma unroll
-      for (int i = 0; i < 8; ++i) po.set(i, px[k].get(i) * rstd * pw.get(i));
-      yr[p] = po.raw;
-    }
-  }
-}
+template <int GT>
+constexpr int kNormFwdThreads = GT < 128 ? 128 : GT;
 
-// The same for H <= 4096 with one WARP per row: a lane keeps its share of the row in
-// registers (PPL packs of 8), the sum of squares needs shuffles only, and a CTA of eight
-// warps has eight rows in flight with no block-wide barrier.
-template <int PPL>
-__global__ void __launch_bounds__(256)
-rmsnormFwdWarp(const bf16 *__restrict__ x, const bf16 *__restrict__ w, bf16 *__restrict__ y, float *__restrict__ rstdOut,
-               long rows, int H, float eps) {
-  const int lane = threadIdx.x & 31;
-  const long row = (long)blockIdx.x * 8 + (threadIdx.x >> 5);
-  if (row >= rows) return;
-  const int nPacks = H / 8;
+template <int GT, int PPT>
+__global__ void __launch_bounds__(kNormFwdThreads<GT>)
+rmsnormFwd(const bf16 *__restrict__ x, const bf16 *__restrict__ w, bf16 *__restrict__ y, float *__restrict__ rstdOut, long rows,
+           int H, float eps) {
+  constexpr int T = kNormFwdThreads<GT>, G = T / GT;
+  __shared__ float red[T / 32];
+  const int group = threadIdx.x / GT, t = threadIdx.x % GT, nPacks = H / 8;
+  const long row = (long)blockIdx.x * G + group;
+  const bool live = row < rows;
   const uint4 *xr = (const uint4 *)(x + row * H);
-  Pack8 px[PPL];
+  Pack8 px[PPT], pw[PPT];
+#pragma unroll
+  for (int k = 0; k < PPT; ++k) {
+    const int p = t + k * GT;
+    px[k].raw = live && p < nPacks ? xr[p] : make_uint4(0, 0, 0, 0);
+  }
+#pragma unroll
+  for (int k = 0; k < PPT; ++k) {
+    const int p = t + k * GT;
+    if (p < nPacks) pw[k].raw = ((const uint4 *)w)[p];
+  }
   float ss = 0.f;
 #pragma unroll
-  for (int k = 0; k < PPL; ++k) {
-    const int p = lane + k * 32;
-    if (p < nPacks) {
-      px[k].raw = xr[p];
+  for (int k = 0; k < PPT; ++k)
 #pragma unroll
-      for (int i = 0; i < 8; ++i) { float v = px[k].get(i); ss += v * v; }
-    }
-  }
+    for (int i = 0; i < 8; ++i) { const float v = px[k].get(i); ss += v * v; }
   ss = warpSum(ss);
+  if constexpr (GT > 32) {
+    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = ss;
+    __syncthreads();
+    ss = 0.f;
+#pragma unroll
+    for (int i = 0; i < GT / 32; ++i) ss += red[group * (GT / 32) + i];
+  }
+  if (!live) return;
   const float rstd = rsqrtf(ss / H + eps);
-  if (lane == 0) rstdOut[row] = rstd;
+  if (t == 0) rstdOut[row] = rstd;
   uint4 *yr = (uint4 *)(y + row * H);
 #pragma unroll
-  for (int k = 0; k < PPL; ++k) {
-    const int p = lane + k * 32;
+  for (int k = 0; k < PPT; ++k) {
+    const int p = t + k * GT;
     if (p < nPacks) {
-      Pack8 pw, po;
-      pw.raw = ((const uint4 *)w)[p];
+      Pack8 po;
 #pragma unroll
-      for (int i = 0; i < 8; ++i) po.set(i, px[k].get(i) * rstd * pw.get(i));
+      for (int i = 0; i < 8; ++i) po.set(i, px[k].get(i) * rstd * pw[k].get(i));
       yr[p] = po.raw;
     }
   }
@@ -204,6 +193,7 @@ rmsnormBwdFewRows(const bf16 *__restrict__ g, const bf16 *__restrict__ x, const 
   extern __shared__ __align__(128) unsigned char slots[];
   __shared__ float red[32];
   __shared__ __align__(8) uint64_t full[kNormFewRows];
+  letNextGridStart();
   const int nPacks = H / 8;
   const uint32_t rowBytes = (uint32_t)H * 2u;
   // a slot holds the g row, the x row and, when a gradient of the same shape is to be added
@@ -332,6 +322,7 @@ rmsnormBwdRing(const bf16 *__restrict__ g, const bf16 *__restrict__ x, const bf1
   constexpr int G = kNormThreads / GT;
   __shared__ float red[2][kNormThreads / 32];
   __shared__ __align__(8) uint64_t full[G * kNormMaxStages];
+  letNextGridStart();
   const int group = threadIdx.x / GT, t = threadIdx.x % GT;
   const int nPacks = H / 8;
   const uint32_t rowBytes = (uint32_t)H * 2u;
@@ -455,6 +446,7 @@ rmsnormBwdRing(const bf16 *__restrict__ g, const bf16 *__restrict__ x, const bf1
 __global__ void columnSumToBf16(const float *__restrict__ partial, bf16 *__restrict__ dw, int R, int H) {
   __shared__ float tile[32][33];
   const int c = blockIdx.x * 32 + threadIdx.x;
+  waitForEarlierGrid();
   float acc = 0.f;
   if (c < H)
     for (int r = threadIdx.y; r < R; r += 32) acc += partial[(size_t)r * H + c];
@@ -1021,25 +1013,16 @@ cudaError_t launchCeRows(bf16 *logits, const long *targets, float *loss, long ro
 // ---------------------------------------------------------------------------
 namespace fcxops {
 
-cudaError_t rmsnormForward(const void *x, const void *w, void *y, float *rstd, long rows, int H, float eps, int sms,
+cudaError_t rmsnormForward(const void *x, const void *w, void *y, float *rstd, long rows, int H, float eps,
                            cudaStream_t stream) {
-  const int threads = 512, packs = H / 8;
-  const int maxp = (packs + threads - 1) / threads;
-  auto launch = [&](auto tag) {
-    rmsnormFwd<decltype(tag)::value><<<(unsigned)rows, threads, 0, stream>>>((const bf16 *)x, (const bf16 *)w, (bf16 *)y,
-                                                                             rstd, H, eps);
+  auto launch = [&](auto gt, auto ppt) {
+    constexpr int GT = decltype(gt)::value, PPT = decltype(ppt)::value, G = kNormFwdThreads<GT> / GT;
+    rmsnormFwd<GT, PPT><<<(unsigned)((rows + G - 1) / G), kNormFwdThreads<GT>, 0, stream>>>(
+        (const bf16 *)x, (const bf16 *)w, (bf16 *)y, rstd, rows, H, eps);
+    return cudaGetLastError();
   };
-  auto launchWarp = [&](auto tag) { // one warp per row, eight rows per CTA
-    rmsnormFwdWarp<decltype(tag)::value><<<(unsigned)((rows + 7) / 8), 256, 0, stream>>>((const bf16 *)x, (const bf16 *)w,
-                                                                                       (bf16 *)y, rstd, rows, H, eps);
-  };
-  if (packs <= 32 * 4) launchWarp(std::integral_constant<int, 4>());
-  else if (packs <= 32 * 8) launchWarp(std::integral_constant<int, 8>());
-  else if (packs <= 32 * 16) launchWarp(std::integral_constant<int, 16>());
-  else if (maxp <= 1) launch(std::integral_constant<int, 1>());
-  else if (maxp <= 2) launch(std::integral_constant<int, 2>());
-  else launch(std::integral_constant<int, 4>());
-  return cudaGetLastError();
+  if (H / 8 > 256 * 4) return launch(std::integral_constant<int, 256>(), std::integral_constant<int, 8>());
+  return withNormShape(H / 8, launch);
 }
 
 int rmsnormPartials(long rows, int H, int sms) {
@@ -1082,8 +1065,16 @@ cudaError_t rmsnormBackward(const void *g, const void *x, const void *w, const f
       return cudaGetLastError();
     }));
   }
-  columnSumToBf16<<<(H + 31) / 32, dim3(32, 32), 0, stream>>>(partial, (bf16 *)dw, ctas, H);
-  return cudaGetLastError();
+  cudaLaunchConfig_t cfg = {};
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.gridDim = dim3((unsigned)((H + 31) / 32));
+  cfg.blockDim = dim3(32, 32);
+  cfg.stream = stream;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, columnSumToBf16, (const float *)partial, (bf16 *)dw, ctas, H);
 }
 
 cudaError_t rope(void *x, const int *positions, int tokens, int heads, int D, float logTheta, float sign, cudaStream_t stream) {

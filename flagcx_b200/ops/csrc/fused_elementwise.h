@@ -8,7 +8,7 @@
 
 namespace fcxops {
 
-cudaError_t rmsnormForward(const void *x, const void *w, void *y, float *rstd, long rows, int H, float eps, int sms,
+cudaError_t rmsnormForward(const void *x, const void *w, void *y, float *rstd, long rows, int H, float eps,
                            cudaStream_t stream);
 // partial: scratch of rmsnormPartials(rows, H, sms) x H floats; add may be null
 int rmsnormPartials(long rows, int H, int sms);

@@ -44,7 +44,7 @@ std::vector<at::Tensor> rmsnorm_fwd(const at::Tensor &x, const at::Tensor &w, do
   auto rstd = at::empty({rows}, x.options().dtype(at::kFloat));
   if (rows > 0)
     checkLaunch(fcxops::rmsnormForward(data(x), data(w), data(y), rstd.data_ptr<float>(), rows, H, (float)eps,
-                                          smCount(), at::cuda::getCurrentCUDAStream()));
+                                          at::cuda::getCurrentCUDAStream()));
   return {y, rstd};
 }
 

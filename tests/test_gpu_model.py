@@ -66,6 +66,26 @@ def test_rmsnorm_backward_at_the_edges_of_its_row_groups(rows, H, skip):
     assert bool(((dw.double() - rdw).abs() <= rdw.abs() * 2 ** -8 + terms * 2 ** -16).all())
 
 
+# one row per warp up to 256 threads per row, the ends of each (a pack less, a pack more), CTAs whose
+# last rows do not exist, and eight packs per thread
+@pytest.mark.parametrize("H", [8, 256, 264, 1024, 1032, 2048, 2056, 4096, 4104, 8192, 8200, 16384])
+@pytest.mark.parametrize("rows", [1, 3, 4, 301])
+def test_norm_forward_at_the_edges_of_its_groups(H, rows):
+    ops = _ops()
+    g = torch.Generator(device="cuda").manual_seed(H + rows)
+    x = torch.randn(rows, H, generator=g, device="cuda").to(torch.bfloat16)
+    w = (1 + 0.1 * torch.randn(H, generator=g, device="cuda")).to(torch.bfloat16)
+    y, rstd = ops.ext().rmsnorm_fwd(x, w, 1e-5)
+    want = torch.rsqrt(x.double().square().mean(-1) + 1e-5)
+    # fp32 sums of H squares, then rsqrtf: a few units in the last place of H additions at most
+    assert bool(((rstd.double() - want).abs() <= want * (H + 8) * 2 ** -24).all())
+    ref = x.double() * want[:, None] * w.double()
+    assert bool(((y.double() - ref).abs() <= ref.abs() * (2 ** -8 + (H + 16) * 2 ** -24)).all())  # and one rounding to bf16
+    x[0, H // 2] = float("inf")  # the row's sum: 0 for what is finite, NaN for the infinity
+    y2, _ = ops.ext().rmsnorm_fwd(x, w, 1e-5)
+    assert bool(y2[0, H // 2].isnan()) and int(y2[0].isnan().sum()) == 1 and torch.equal(y2[1:], y[1:])
+
+
 def test_norm_backward_from_two_threads_with_different_sizes():
     """The backward of an autograd graph runs without the GIL, so its launches interleave with
     another thread's; 8 and 256 columns share a kernel and ask for 3 and 144 KiB of shared memory."""
