@@ -38,14 +38,18 @@ class MoeDispatcher:
         """x: [T, hidden] bf16; topk_idx: [T, topk] int32 (global expert ids)."""
         assert x.dtype == torch.bfloat16 and x.is_contiguous() and topk_idx.dtype == torch.int32 and topk_idx.is_contiguous()
         self._idx = topk_idx  # the combine reads it again
-        capi.check(capi.lib().flagcxMoeDispatch(self.h, capi._ptr(x), capi._ptr(topk_idx), x.shape[0],
-                                                capi._stream_arg(stream)), "flagcxMoeDispatch", self.comm.h)
+        code = capi._call("flagcxMoeDispatch")(self.h, capi._addr(x), capi._addr(topk_idx), x.shape[0],
+                                               None if stream is None else capi._stream_arg(stream))
+        if code:
+            capi.check(code, "flagcxMoeDispatch", self.comm.h)
 
     def combine(self, topk_weights: torch.Tensor, out: torch.Tensor, stream=None) -> None:
         """topk_weights: [T, topk] fp32; out: [T, hidden] bf16."""
         assert topk_weights.dtype == torch.float32 and topk_weights.is_contiguous() and out.is_contiguous()
-        capi.check(capi.lib().flagcxMoeCombine(self.h, capi._ptr(topk_weights), capi._ptr(out), out.shape[0],
-                                               capi._stream_arg(stream)), "flagcxMoeCombine", self.comm.h)
+        code = capi._call("flagcxMoeCombine")(self.h, capi._addr(topk_weights), capi._addr(out), out.shape[0],
+                                              None if stream is None else capi._stream_arg(stream))
+        if code:
+            capi.check(code, "flagcxMoeCombine", self.comm.h)
 
     def close(self) -> None:
         if self.h:

@@ -27,10 +27,14 @@ def gemm_bf16(a: torch.Tensor, b: torch.Tensor, out: torch.Tensor | None = None,
     assert b.shape[1] == K
     if out is None:
         out = torch.empty(M, N, dtype=torch.bfloat16, device=a.device)
-    if stream is None:
-        stream = torch.cuda.current_stream(a.device)
-    capi.check(capi.lib().flagcxGemmBf16(capi._ptr(a), capi._ptr(b), capi._ptr(out), M, N, K,
-                                         capi._stream_arg(stream)), "flagcxGemmBf16")
+    if stream is None and a.is_cuda:  # the current stream without a torch.cuda.Stream around it (2 us)
+        on = capi.CudaStream(torch._C._cuda_getCurrentRawStream(a.get_device()))
+        arg = C.byref(on)
+    else:
+        arg = capi._stream_arg(torch.cuda.current_stream(a.device) if stream is None else stream)
+    code = capi._call("flagcxGemmBf16")(capi._addr(a), capi._addr(b), capi._addr(out), M, N, K, arg)
+    if code:
+        capi.check(code, "flagcxGemmBf16")
     return out
 
 
