@@ -625,7 +625,7 @@ __global__ void crossEntropyFwdBwd(bf16 *__restrict__ logits, const long *__rest
 }
 
 // ---------------------------------------------------------------------------
-// The same operation, persistent, for vocabularies up to 8 x 16 x 2048 = 262144.  A cluster
+// The same operation, persistent, for vocabularies up to 262144.  A cluster
 // of C CTAs walks over rows; each CTA's 1/C of a row comes into a shared-memory slot by bulk
 // copy, moves on into registers (PPT packs of 8 per thread), and the copy of the next row
 // into the slot starts at once: while a row is being reduced, scaled and stored, the next one
@@ -634,13 +634,48 @@ __global__ void crossEntropyFwdBwd(bf16 *__restrict__ logits, const long *__rest
 // (maximum, sum), one cluster barrier, and every warp combines all pairs of the cluster.  A
 // warp whose logits are all -inf (a masked stretch) contributes nothing.
 //
+// DEAL: rows are not cut into equal shares; the grid has a cluster for every row, and a cluster that
+// runs takes over rows whose clusters have not started (cluster launch control) until none is left.
+// The answer for the row after next is asked for while a row is worked on and reaches the other
+// CTAs with the pairs.
+//
 // Bound: HBM (one read and one write of the logits).  The kernel below it in this file, which
 // loads, reduces and stores one row per CTA with nothing overlapped, took 458 us for
-// 4096 x 128256; this one takes 355 (5.9 TB/s, 0.90 of a copy).
+// 4096 x 128256; this one takes 331 (6.3 TB/s, 0.97 of a copy).  The CTAs of a cluster wait for one
+// another at every row, so a row goes to as few as can hold it: with up to 21 packs per thread (128
+// registers, two CTAs per SM) 3 instead of 4 here, 349 -> 331; 2048 x 151936 in 4 instead of 8 261 ->
+// 214; with 5, 6 and 7 CTAs 376, 400 and 445.  Dealt against equal shares: 4096 x 32000 93.4 -> 85.2,
+// 8192 x 8192 46.6 -> 45.5, 16384 x 1024 45.2 -> 47.0: from four packs per thread on.
 // ---------------------------------------------------------------------------
 constexpr int kCeRowThreads = 256, kCeRowWarps = kCeRowThreads / 32;
-constexpr int kCeRowMaxPacks = 16 * kCeRowThreads; // packs of a row that one CTA can hold
+constexpr int kCeRowPacks = 21 * kCeRowThreads;         // packs of a row that one CTA can hold
+constexpr int kCeRowMaxPacks = 8 * 16 * kCeRowThreads;  // longer rows go to crossEntropyCluster
 constexpr uint32_t kCeBulkPiece = 32768;
+
+// Cluster launch control: asks for a cluster of this grid that has not started yet; the answer (16
+// bytes) arrives at `answer` and is counted on the mbarrier.
+__device__ __forceinline__ void askForCluster(uint4 *answer, uint64_t *bar) {
+  mbarExpect(bar, 16);
+  asm volatile("clusterlaunchcontrol.try_cancel.async.shared::cta.mbarrier::complete_tx::bytes.b128 [%0], [%1];" ::"r"(
+                   sharedAddr(answer)),
+               "r"(sharedAddr(bar))
+               : "memory");
+}
+// blockIdx.x of the first CTA of the cluster that the answer hands over, -1: none is left.
+__device__ __forceinline__ int clusterHandedOver(const uint4 *answer) {
+  uint32_t ok, x;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t.reg .b128 h;\n\t"
+      "ld.shared.b128 h, [%2];\n\t"
+      "clusterlaunchcontrol.query_cancel.is_canceled.pred.b128 p, h;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t"
+      "mov.u32 %1, 0;\n\t"
+      "@p clusterlaunchcontrol.query_cancel.get_first_ctaid::x.b32.b128 %1, h;\n\t}"
+      : "=r"(ok), "=r"(x)
+      : "r"(sharedAddr(answer))
+      : "memory");
+  return ok ? (int)x : -1;
+}
 
 __device__ __forceinline__ void clusterSyncAll() {
   asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
@@ -659,17 +694,24 @@ __device__ __forceinline__ uint32_t maxBf16x2(uint32_t a, uint32_t b) {
   return r;
 }
 
-template <int PPT>
+template <int PPT, bool DEAL>
 __global__ void __launch_bounds__(kCeRowThreads, PPT > 10 ? 2 : PPT > 8 ? 3 : PPT == 8 ? 4 : PPT == 4 ? 5 : 8)
 crossEntropyRows(bf16 *__restrict__ logits, const long *__restrict__ targets, float *__restrict__ loss, long rows, int V,
                  float gradScale, int packsPerCta) {
   extern __shared__ __align__(128) unsigned char ceSlot[];
   __shared__ float2 stat[2][kCeRowWarps]; // (maximum, sum) of every warp, two rows deep
-  __shared__ __align__(8) uint64_t bar;
+  __shared__ __align__(8) uint64_t bar, dealBar;
+  __shared__ __align__(16) uint4 answer[2];
+  __shared__ int dealt[2], dealOver; // of the cluster's first CTA: the row after next (-1: none); no more requests
   cg::cluster_group cluster = cg::this_cluster();
   const int C = (int)cluster.num_blocks(), cr = (int)cluster.block_rank();
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const long step = gridDim.x / C;
+  const bool dealer = DEAL && cr == 0 && tid == 0;
+  auto takeAnswer = [&](uint32_t nth) { // dealer: what came of the nth request
+    const int first = mbarWaitBounded(&dealBar, nth & 1u) ? clusterHandedOver(&answer[nth & 1u]) : -1;
+    return first < 0 ? -1 : first / C;
+  };
   const int p0 = cr * packsPerCta, n = max(0, min(packsPerCta, V / 8 - p0));
   const uint32_t bytes = (uint32_t)n * 16u;
   const uint4 *slot = (const uint4 *)ceSlot;
@@ -680,18 +722,33 @@ crossEntropyRows(bf16 *__restrict__ logits, const long *__restrict__ targets, fl
     for (uint32_t off = 0; off < bytes; off += kCeBulkPiece)
       bulkLoad(ceSlot + off, part(row) + off, min(kCeBulkPiece, bytes - off), &bar);
   };
-  long row = blockIdx.x / C;
+  long row = blockIdx.x / C, next = row + step;
   if (tid == 0) {
     mbarInit(&bar);
+    if (DEAL) mbarInit(&dealBar);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     if (row < rows && n > 0) issue(row);
   }
-  __syncthreads();
+  if constexpr (DEAL) {
+    if (dealer) {
+      dealOver = 0;
+      askForCluster(&answer[0], &dealBar);
+      dealt[1] = takeAnswer(0);
+    }
+    if (C > 1) clusterSyncAll(); else __syncthreads();
+    next = *cluster.map_shared_rank(&dealt[1], 0);
+  } else {
+    __syncthreads();
+  }
   constexpr float kLog2e = 1.4426950408889634f;
   // A copy that never arrived makes the loss and the gradient of its row NaN, and those of the rows
   // after it, which are not fetched; it is given as long again to land before the CTA may leave.
   bool ok = true;
-  for (int it = 0; row < rows; row += step, ++it) {
+  for (int it = 0; DEAL || row < rows; ++it) {
+    if (dealer && next >= 0 && !dealOver) {
+      asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); // the last answer has been read
+      askForCluster(&answer[(it + 1) & 1], &dealBar);
+    }
     if (n > 0 && ok && !(ok = mbarWaitBounded(&bar, (uint32_t)it & 1u)) && tid == 0) mbarWaitBounded(&bar, (uint32_t)it & 1u);
     const long tLocal = targets[row] - (long)p0 * 8; // index of the target inside this CTA's part, if it is here
     const bool own = tLocal >= 0 && tLocal < (long)n * 8;
@@ -704,7 +761,7 @@ crossEntropyRows(bf16 *__restrict__ logits, const long *__restrict__ targets, fl
       v[k][0] = q.x; v[k][1] = q.y; v[k][2] = q.z; v[k][3] = q.w;
     }
     __syncthreads(); // the slot has been read
-    if (tid == 0 && row + step < rows && n > 0 && ok) issue(row + step);
+    if (tid == 0 && (DEAL ? next >= 0 : next < rows) && n > 0 && ok) issue(next);
     uint32_t m2 = 0xff80ff80u;
 #pragma unroll
     for (int k = 0; k < PPT; ++k)
@@ -724,10 +781,12 @@ crossEntropyRows(bf16 *__restrict__ logits, const long *__restrict__ targets, fl
       }
     sum = warpSum(ok ? sum : NAN);
     if (lane == 0) stat[it & 1][warp] = make_float2(wmax, sum);
+    if (dealer) dealt[it & 1] = next >= 0 && !dealOver ? takeAnswer(it + 1) : -1;
     __syncwarp();
     // One barrier per row: the pairs of the row before last are overwritten only now, when
     // every CTA has passed the last row's barrier and so has read them.
     if (C > 1) clusterSyncAll(); else __syncthreads();
+    const long after = DEAL ? *cluster.map_shared_rank(&dealt[it & 1], 0) : next + step;
     float M = -INFINITY, S = 0.f;
     float2 st[2];
 #pragma unroll
@@ -742,6 +801,9 @@ crossEntropyRows(bf16 *__restrict__ logits, const long *__restrict__ targets, fl
     for (int j = 0; j < 2; ++j)
       if (st[j].y != 0.f) S += st[j].y * __expf(st[j].x - M);
     S = warpSum(S);
+    // A cluster that has lost a copy takes no further row (nor one that has met a NaN, which its
+    // sums do not tell apart): rows that nobody takes over start clusters of their own.
+    if (dealer && S != S) dealOver = 1;
     if (own && tid == 0) loss[row] = M + __logf(S) - tgtLogit;
     const float f = __expf(wmax - M) / S * gradScale;
     uint4 *out = (uint4 *)part(row);
@@ -760,6 +822,9 @@ crossEntropyRows(bf16 *__restrict__ logits, const long *__restrict__ targets, fl
     // the one element that is softmax - 1, redone in fp32 by the thread that stored its pack
     if (own && tid == (int)((tLocal >> 3) % kCeRowThreads))
       ((bf16 *)out)[tLocal] = __float2bfloat16_rn(exp2f(fmaf(tgtLogit, kLog2e, -ref)) * f - gradScale);
+    if (DEAL && next < 0) break;
+    row = next;
+    next = after;
   }
   __syncwarp();
   if (C > 1) clusterSyncAll(); // no CTA leaves while another may still read its pairs
@@ -974,10 +1039,10 @@ cudaError_t withNormShape(int packs, F &&f) {
   return ppt(std::integral_constant<int, 512>());
 }
 
-template <int PPT>
+template <int PPT, bool DEAL>
 cudaError_t launchCeRows(bf16 *logits, const long *targets, float *loss, long rows, int V, float gradScale, int C, int per,
                          int sms, cudaStream_t stream) {
-  auto kern = crossEntropyRows<PPT>;
+  auto kern = crossEntropyRows<PPT, DEAL>;
   const int smem = per * 16;
   cudaLaunchConfig_t cfg = {};
   cudaLaunchAttribute attr[1];
@@ -991,10 +1056,10 @@ cudaError_t launchCeRows(bf16 *logits, const long *targets, float *loss, long ro
   cfg.attrs = attr;
   cfg.numAttrs = 1;
   constexpr int kMost = PPT * kCeRowThreads * 16;
-  if constexpr (kMost > (47 << 10)) RETURN_IF(allowShared<crossEntropyRows<PPT>>(kMost)); // beyond what a kernel gets without asking
-  // As many clusters as run at once: rows are dealt out evenly, so a second wave would be waste.
+  if constexpr (kMost > (47 << 10)) RETURN_IF((allowShared<crossEntropyRows<PPT, DEAL>>(kMost))); // beyond what a kernel gets without asking
+  // Equal shares: as many clusters as run at once, a second wave would be waste.
   long clusters = rows;
-  if (rows * C > sms) {
+  if (!DEAL && rows * C > sms) {
     static fcxops::ClusterCount count;
     int dev = 0, active = 0;
     RETURN_IF(cudaGetDevice(&dev));
@@ -1103,35 +1168,50 @@ cudaError_t swigluBackward(const void *g, const void *ab, void *dab, size_t T, i
 
 cudaError_t crossEntropy(void *logits, const long *targets, float *loss, long rows, int V, float gradScale, int sms,
                          cudaStream_t stream) {
-  // Smallest cluster whose per-CTA part of a row fits the registers of crossEntropyRows; more
+  // Many rows: the fewest CTAs whose part of a row fits the registers of crossEntropyRows, rows dealt
+  // out.  From eight rounds of the CTAs that run at once on: with 8 it gains 2 % (1230 x 48440), with 14
+  // 5 to 9 (1410 x 86736, 4096 x 32000), with 3 to 5 the first requests cost more (700 x 65536 42.0 ->
+  // 43.2, 2228 x 5520 14.4 -> 16.4).  Fewer rows: equal shares, at most 64 KiB of a row per CTA, and more
   // CTAs per row while that leaves SMs idle and a CTA still has two packs per thread.  Longer
   // rows: up to 200 KiB of shared memory per CTA; failing that, the kernel that streams the
   // row three times.
   const int packs = V / 8;
   int cluster = 0, per = 0;
-  static const size_t partKb = std::getenv("FLAGCX_OPS_CE_PART_KB") ? (size_t)atoi(std::getenv("FLAGCX_OPS_CE_PART_KB")) : 64;
+  static const size_t partKb = std::getenv("FLAGCX_OPS_CE_PART_KB") ? (size_t)atoi(std::getenv("FLAGCX_OPS_CE_PART_KB")) : kCeRowPacks * 16 >> 10;
   static const bool forceStreaming = std::getenv("FLAGCX_OPS_CE_STREAMING") && atoi(std::getenv("FLAGCX_OPS_CE_STREAMING")) != 0;
   if (!forceStreaming) {
-    for (int c : {1, 2, 4, 8}) {
-      per = (packs + c - 1) / c;
-      if (per <= kCeRowMaxPacks && ((size_t)per * 16 <= partKb << 10 || c == 8)) { cluster = c; break; }
-    }
-    if (cluster) {
-      while (cluster < 8 && rows * cluster < 2 * sms && packs >= 4 * kCeRowThreads * cluster) cluster *= 2;
-      per = (packs + cluster - 1) / cluster;
-      auto go = [&](auto tag) {
-        return launchCeRows<decltype(tag)::value>((bf16 *)logits, targets, loss, rows, V, gradScale, cluster, per, sms, stream);
+    if (packs <= kCeRowMaxPacks) {
+      auto fits = [&](int c, int most, size_t kb) {
+        per = (packs + c - 1) / c;
+        return per <= most && ((size_t)per * 16 <= kb << 10 || c == 8);
       };
+      cluster = 1;
+      while (!fits(cluster, kCeRowPacks, partKb)) ++cluster; // 8 do
+      const int perSm = per <= 4 * kCeRowThreads ? 5 : per <= 8 * kCeRowThreads ? 4 : per <= 10 * kCeRowThreads ? 3 : 2;
+      const bool deal = per > 2 * kCeRowThreads && rows * cluster >= 8L * perSm * sms && rows * cluster <= 0x7fffffffL;
+      if (!deal) {
+        cluster = 1;
+        while (!fits(cluster, 16 * kCeRowThreads, std::min<size_t>(partKb, 64))) cluster *= 2;
+        while (cluster < 8 && rows * cluster < 2 * sms && packs >= 4 * kCeRowThreads * cluster) cluster *= 2;
+        per = (packs + cluster - 1) / cluster;
+      }
       // Packs per thread decide the registers (4 each), and they how many CTAs share an SM: 10 let
-      // three, 16 two, 13 waste less of them than 16.  Without these two 1024 x 65544 took 79.9 us
-      // instead of 61.2, 1024 x 151936 170.9 instead of 134.7, 4096 x 100352 327.5 instead of 295.5.
+      // three, 21 two, 13, 16 and 18 leave fewer threads without a pack.  Without 10 and 13 1024 x 65544
+      // took 79.9 us instead of 61.2, 4096 x 100352 327.5 instead of 295.5.
+      auto go = [&](auto tag) {
+        constexpr int PPT = decltype(tag)::value;
+        auto launch = deal ? launchCeRows<PPT, (PPT > 2)> : launchCeRows<PPT, (PPT > 16)>;
+        return launch((bf16 *)logits, targets, loss, rows, V, gradScale, cluster, per, sms, stream);
+      };
       if (per <= kCeRowThreads) return go(std::integral_constant<int, 1>());
       if (per <= 2 * kCeRowThreads) return go(std::integral_constant<int, 2>());
       if (per <= 4 * kCeRowThreads) return go(std::integral_constant<int, 4>());
       if (per <= 8 * kCeRowThreads) return go(std::integral_constant<int, 8>());
       if (per <= 10 * kCeRowThreads) return go(std::integral_constant<int, 10>());
       if (per <= 13 * kCeRowThreads) return go(std::integral_constant<int, 13>());
-      return go(std::integral_constant<int, 16>());
+      if (per <= 16 * kCeRowThreads) return go(std::integral_constant<int, 16>());
+      if (per <= 18 * kCeRowThreads) return go(std::integral_constant<int, 18>());
+      return go(std::integral_constant<int, 21>());
     }
     per = (packs + 7) / 8;
     if (per * 16 <= kCePartBytes) cluster = 8;

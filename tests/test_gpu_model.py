@@ -310,6 +310,35 @@ def test_cross_entropy_at_the_edges_of_its_row_split(T, V):
     assert bool(((logits.double() - d).abs() <= d.abs() * 2 ** -7 + 2 ** -15 / T * (d < 0)).all())
 
 
+# Rows dealt out: the edges of what one CTA holds (256 threads x 4, 8, 10, 13, 16, 18, 21 packs of 8) with
+# as few rows as are dealt, and one, two, three, five and seven CTAs per row.  Two rows hold a NaN: they
+# are lost, and their clusters take over no others, which are done all the same.
+@pytest.mark.parametrize("T,V", [(5925, 4104), (5920, 8192), (4737, 8200), (4736, 16384), (3555, 16392), (3552, 20480), (2370, 20488),
+                                 (2368, 26624), (2368, 26632), (2369, 32768), (2368, 32776), (2368, 36864), (2368, 36872),
+                                 (2371, 43008), (1184, 43016), (790, 86024), (475, 172040), (340, 262144)])
+def test_cross_entropy_of_rows_dealt_out(T, V):
+    ops = _ops()
+    g = torch.Generator(device="cuda").manual_seed(V)
+    logits = (torch.randn(T, V, generator=g, device="cuda") * 3).to(torch.bfloat16)
+    tgt = torch.randint(0, V // 2, (T,), generator=g, device="cuda")
+    tgt[0] = V - 1
+    logits[1::2, V // 2:] = float("-inf")
+    bad = [3, T // 2]
+    logits[bad, 1] = float("nan")
+    lp = logits.double().log_softmax(-1)
+    at = torch.arange(T, device="cuda")
+    want = -lp[at, tgt]
+    d = lp.exp_()
+    d[at, tgt] -= 1
+    loss = ops.ext().cross_entropy_fwd_bwd_(logits, tgt, 1.0)
+    good = torch.ones(T, dtype=torch.bool, device="cuda")
+    good[bad] = False
+    assert bool(loss[~good].isnan().all()) and bool(logits[~good].isnan().any(1).all())
+    assert bool(((loss.double() - want).abs()[good] <= 1e-5 * want[good].abs() + 1e-5).all())
+    # bounds of the test above, for a scale of 1
+    assert bool(((logits.double() - d).abs() <= d.abs() * 2 ** -7 + 2 ** -15 * (d < 0))[good].all())
+
+
 def test_adamw_matches_torch():
     ops = _ops()
     torch.manual_seed(5)

@@ -79,3 +79,18 @@ def test_cross_entropy_without_one_row(lib, rows, V):
     assert torch.equal(loss[~lost], whole[1][~lost]) and torch.equal(d[~lost], whole[0][~lost])
     again = _cross_entropy(lib, logits, targets, -1)
     assert all(torch.equal(a, b) for a, b in zip(again, whole))
+
+
+# rows dealt out to the clusters: the one that lost a copy had the next two rows already, and takes no more
+@pytest.mark.parametrize("rows,V", [(8000, 8192), (2400, 43008), (1000, 128256), (400, 262144)])
+def test_cross_entropy_of_rows_dealt_out_without_one(lib, rows, V):
+    g = torch.Generator(device="cuda").manual_seed(V)
+    logits = torch.randn(rows, V, generator=g, device="cuda").to(torch.bfloat16)
+    targets = torch.randint(0, V, (rows,), generator=g, device="cuda")
+    whole = _cross_entropy(lib, logits, targets, -1)
+    held = rows // 2 + 1
+    d, loss = _cross_entropy(lib, logits, targets, held)
+    lost = loss.isnan()
+    assert bool(lost[held]) and not bool(lost[:held].any()) and int(lost.sum()) <= 3
+    assert bool(d[lost].isnan().all())
+    assert torch.equal(loss[~lost], whole[1][~lost]) and torch.equal(d[~lost], whole[0][~lost])
