@@ -31,6 +31,11 @@ namespace {
 // CTAs of 8 warps: the combine keeps eight 16-byte loads per lane in flight and wants the
 // registers for them; the host launches twice as many CTAs as it would of the 512-thread kind.
 constexpr int kMoeThreads = 256;
+// In the emulated world, where all ranks' CTAs share the SMs, the dispatch runs as one CTA of twice
+// the threads per SM: CTAs of one SM wait for each other's system-wide releases in a barrier (8
+// tokens of 7168 a rank 22.5 -> 18.8 us against two CTAs per SM, 400 of 2048 22.7 -> 18.2, 512 of 7168
+// the same).
+constexpr int kMoeEmuThreads = 512;
 
 // A row of vecs 16-byte vectors is copied in pieces of at most 32 x kMoePiece vectors, one warp
 // each, so that the warps of a CTA share its rows evenly however few they are.
@@ -139,14 +144,16 @@ __device__ __forceinline__ int firstToken(int T, int b, int g) { return (int)((l
 // Bound: memory (eight emulated ranks, 512 tokens x 7168, top 8 of 256: 640 MB, 97 us of the 126
 // at the rate of a copy), then two barriers and about 6 us of counting and routing.  One warp per
 // row, one load of the routing table at a time, and one CTA of 8 warps per SM took 173 us; the
-// routes of four tokens at once, pieces of rows and two to three CTAs per SM brought it here.
+// routes of four tokens at once, pieces of rows and 16 warps per SM brought it here.
+constexpr int kMoeTable = 256; // tokens, or group records, that a CTA looks at before it moves their rows
+static_assert(kMoeThreads >= kMoeTable, "a thread looks at one record");
 struct DispatchShared {
   int base[FLAGCX_MOE_MAX_EXPERTS];
   union {
     struct { int tot[FLAGCX_MOE_MAX_EXPERTS], before[FLAGCX_MOE_MAX_EXPERTS], mine[FLAGCX_MOE_MAX_EXPERTS]; };
     struct { // rows that a token goes to, or the row that a group has and then those it is copied to
-      char *row[kMoeThreads][FLAGCX_MOE_MAX_TOPK];
-      int nRows[kMoeThreads];
+      char *row[kMoeTable][FLAGCX_MOE_MAX_TOPK];
+      int nRows[kMoeTable];
     };
   };
   int grpN[FLAGCX_MAX_RANKS], nRec;
@@ -240,8 +247,8 @@ __device__ void dispatchBody(const flagcxDevComm &c, const MoeArgs &a) {
   const int capPer = ((a.maxT + g - 1) / g) * a.K;
   const RowPieces pieces(vecs);
   static_assert(FLAGCX_MOE_MAX_TOPK == 8, "a quarter of a warp per token");
-  for (int tok0 = tlo; tok0 < thi; tok0 += kMoeThreads) {
-    const int nTok = thi - tok0 < kMoeThreads ? thi - tok0 : kMoeThreads;
+  for (int tok0 = tlo; tok0 < thi; tok0 += kMoeTable) {
+    const int nTok = thi - tok0 < kMoeTable ? thi - tok0 : kMoeTable;
     __syncthreads(); // the tables of counts, or the last batch's rows, have been read
     for (int j0 = warp * 4; j0 < nTok; j0 += warps * 4) { // the whole warp stays together
       const int j = j0 + (lane >> 3), k = lane & 7, tok = tok0 + j;
@@ -304,11 +311,11 @@ __device__ void dispatchBody(const flagcxDevComm &c, const MoeArgs &a) {
     start[q + 1] = q < n ? ldSysElem(a.grpCount[rank] + (size_t)q * FLAGCX_COLL_BARRIER_SLOTS + b) : 0;
 #pragma unroll
   for (int q = 0; q < FLAGCX_MAX_RANKS; ++q) start[q + 1] += start[q];
-  for (int r0 = 0; r0 < start[FLAGCX_MAX_RANKS]; r0 += nt) {
+  for (int r0 = 0; r0 < start[FLAGCX_MAX_RANKS]; r0 += kMoeTable) {
     if (t == 0) s.nRec = 0;
     __syncthreads();
     const int r = r0 + t;
-    if (r < start[FLAGCX_MAX_RANKS]) {
+    if (t < kMoeTable && r < start[FLAGCX_MAX_RANKS]) {
       int q = 0, before = 0;
 #pragma unroll
       for (int p = 1; p < FLAGCX_MAX_RANKS; ++p)
@@ -480,7 +487,7 @@ __global__ void __launch_bounds__(kMoeThreads)
     moeDispatchKernel(const __grid_constant__ flagcxDevComm c, const __grid_constant__ MoeArgs a) {
   dispatchBody(c, a);
 }
-__global__ void __launch_bounds__(kMoeThreads)
+__global__ void __launch_bounds__(kMoeEmuThreads)
     moeDispatchKernelEmu(const __grid_constant__ EmuLaunch<MoeArgs> e) {
   dispatchBody(e.comm[blockIdx.y], e.args[blockIdx.y]);
 }
@@ -507,7 +514,7 @@ __global__ void __launch_bounds__(FLAGCX_DEVICE_THREADS_PER_CTA)
 // combine must run as many as the dispatch that left it its records: what both kernels have room for.
 static cudaError_t emuMoeCtas(const LaunchCtx &lc, bool preReduce, int *ctas) {
   int forDispatch = 0, forCombine = lc.nCtas;
-  cudaError_t e = emuCtasPerRank<moeDispatchKernelEmu>(kMoeThreads, lc.emuRanks, &forDispatch);
+  cudaError_t e = emuCtasPerRank<moeDispatchKernelEmu>(kMoeEmuThreads, lc.emuRanks, &forDispatch);
   if (e == cudaSuccess && preReduce) e = emuCtasPerRank<moeCombineKernelEmu>(kMoeThreads, lc.emuRanks, &forCombine);
   *ctas = std::min(lc.nCtas, std::min(forDispatch, forCombine));
   return e;
@@ -517,7 +524,7 @@ cudaError_t launchMoeDispatch(const LaunchCtx &lc, const MoeArgs &a) {
   if (lc.emuRanks > 0) {
     int ctas = 0;
     const cudaError_t e = emuMoeCtas(lc, a.preReduce != 0, &ctas);
-    return e != cudaSuccess ? e : launchEmu(moeDispatchKernelEmu, lc, lc.emuMoe, dim3(ctas, lc.emuRanks), dim3(kMoeThreads), 0);
+    return e != cudaSuccess ? e : launchEmu(moeDispatchKernelEmu, lc, lc.emuMoe, dim3(ctas, lc.emuRanks), dim3(kMoeEmuThreads), 0);
   }
   moeDispatchKernel<<<lc.nCtas, kMoeThreads, 0, lc.stream>>>(*lc.comm, a);
   return cudaGetLastError();
