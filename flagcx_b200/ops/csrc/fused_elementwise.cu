@@ -285,10 +285,12 @@ rmsnormBwdFewRows(const bf16 *__restrict__ g, const bf16 *__restrict__ x, const 
 // copies that complete on one mbarrier per slot, and reduces its rows by itself: shuffles, and for
 // GT > 32 one named barrier of the group.  So a CTA has 512 / GT rows in work and as many or more
 // on their way, and nothing waits for the whole block.  Bound: the chain wait -> dot product ->
-// sum -> store of each row, and 128 registers (four packs per thread spill 16 bytes).  Device time
+// sum -> store of each row, and 128 registers (with four packs per thread and the weights widened
+// ahead of the loop 16 bytes too few: 8192 x 8192 96.0 us instead of 86.0, which is 6.2 TB/s, 4096 x 4096
+// 30.9 instead of 28.8).  Device time
 // with the sum over CTAs and a skip gradient, against one row per CTA at every size: 8192 x 1024
 // 37.1 -> 18.8 us, 8192 x 256 34.2 -> 8.7, 4096 x 2560 27.9 -> 20.4, 2048 x 5120 28.7 -> 19.0,
-// 4096 x 4096 31.4 -> 29.1, 2048 x 16384 58.1 -> 51.0.
+// 2048 x 16384 58.1 -> 51.0.
 constexpr int kNormThreads = 512, kNormMaxStages = 6, kNormPacks = 4, kNormRingBytes = 200 << 10;
 
 // Sum over a group of GT threads; every thread gets it.  red holds one float per warp of the
@@ -364,6 +366,10 @@ rmsnormBwdRing(const bf16 *__restrict__ g, const bf16 *__restrict__ x, const bf1
     ok = __all_sync(0xffffffffu, mbarWaitBounded(&bars[s], phase));
     if (!ok) break;
     const uint4 *gs = (const uint4 *)(slots + (size_t)s * slotBytes), *xs = gs + nPacks, *as = xs + nPacks;
+    if constexpr (PPT == 4) // the weights stay packed: widened ahead of the loop they take 16 registers more than there are
+#pragma unroll
+      for (int k = 0; k < PPT; ++k)
+        asm volatile("" : "+r"(pw[k].raw.x), "+r"(pw[k].raw.y), "+r"(pw[k].raw.z), "+r"(pw[k].raw.w));
     Pack8 pg[PPT], px[PPT], pa[PPT];
     float dot = 0.f;
 #pragma unroll
