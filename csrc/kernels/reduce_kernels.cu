@@ -140,20 +140,21 @@ struct Reducer {
                                                    size_t dstBase) {
     const Tickets tickets{a.tickets};
     const int lane = threadIdx.x & 31;
-    const size_t items = (packs + 32 * U - 1) / (32 * U);
-    for (size_t item = tickets.take(); item < items;) {
-      const size_t next = tickets.take(); // on its way while this one is worked on
-      const size_t first = item * (32 * U) + lane;
+    const unsigned items = (unsigned)((packs + 32 * U - 1) / (32 * U)); // 2^32 of them would be 4 TB of input
+    for (unsigned item = tickets.take(); item < items;) {
+      const unsigned next = tickets.take(); // on its way while this one is worked on
+      const size_t first = (size_t)item * (32 * U) + lane, off = sb * sizeof(T) + (first << 4);
+      const int left = first + 32 * U <= packs ? 32 * U : first < packs ? (int)(packs - first) : 0;
       uint4 v[U][NR];
 #pragma unroll
       for (int u = 0; u < U; ++u)
-        if (first + u * 32 < packs) {
+        if (u * 32 < left) {
 #pragma unroll
-          for (int p = 0; p < NR; ++p) v[u][p] = ldSys16(a.in[p] + sb * sizeof(T) + ((first + u * 32) << 4));
+          for (int p = 0; p < NR; ++p) v[u][p] = ldSys16(a.in[p] + off + u * 512);
         }
 #pragma unroll
       for (int u = 0; u < U; ++u)
-        if (first + u * 32 < packs) {
+        if (u * 32 < left) {
           Acc acc[N];
           addUp(a, v[u], acc);
           storePack(a, dst, nDst, dstBase + (first + u * 32) * N, acc);

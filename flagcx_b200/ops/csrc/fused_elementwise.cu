@@ -1088,8 +1088,9 @@ cudaError_t rmsnormForward(const void *x, const void *w, void *y, float *rstd, l
                            cudaStream_t stream) {
   auto launch = [&](auto gt, auto ppt) {
     constexpr int GT = decltype(gt)::value, PPT = decltype(ppt)::value, G = kNormFwdThreads<GT> / GT;
-    rmsnormFwd<GT, PPT><<<(unsigned)((rows + G - 1) / G), kNormFwdThreads<GT>, 0, stream>>>(
-        (const bf16 *)x, (const bf16 *)w, (bf16 *)y, rstd, rows, H, eps);
+    if constexpr (GT <= 256) // rows beyond 8192 elements take the line after the lambda
+      rmsnormFwd<GT, PPT><<<(unsigned)((rows + G - 1) / G), kNormFwdThreads<GT>, 0, stream>>>(
+          (const bf16 *)x, (const bf16 *)w, (bf16 *)y, rstd, rows, H, eps);
     return cudaGetLastError();
   };
   if (H / 8 > 256 * 4) return launch(std::integral_constant<int, 256>(), std::integral_constant<int, 8>());
