@@ -10,6 +10,7 @@ compiles it.  Nothing falls back silently: a missing library raises.
 from __future__ import annotations
 
 import ctypes as C
+import operator
 import os
 from typing import Optional, Sequence
 
@@ -288,7 +289,7 @@ class Comm:
 
     # -- collectives (buffers: numpy arrays, torch tensors or raw addresses) ---------
     def all_reduce(self, send, recv, count, dtype, op=SUM, stream=None):
-        code = _call("flagcxAllReduce")(_addr(send), _addr(recv), count, dtype, op, self.h,
+        code = _call("flagcxAllReduce")(_addr(send), _addr(recv), operator.index(count), dtype, op, self.h,
                                         None if stream is None else _stream_arg(stream))
         if code:
             check(code, "flagcxAllReduce", self.h)
