@@ -98,7 +98,7 @@ flagcxResult_t flagcxGemmBf16(const void *A, const void *B, void *D, int M, int 
   FCXCHECK(checkShape(M, N, K));
   CUtensorMap ta, tb;
   FCXCHECK(cu::tensorMap2dBf16(&ta, A, M, K, 128, 64));
-  const bool pair = usePair(M);
+  bool pair = usePair(M);
   const int forced = (int)readParam("GEMM_SPLIT", 0);
   SplitGemmPlan plan = splitPlan(M, N, K, pair, forced, forced > 1 ? (int)readParam("GEMM_SPLIT_N", 256) : 256);
   if (plan.tileN) {
@@ -107,6 +107,12 @@ flagcxResult_t flagcxGemmBf16(const void *A, const void *B, void *D, int M, int 
     if (e != cudaSuccess) { FCX_WARN("GEMM launch failed: %s", cudaGetErrorString(e)); return flagcxUnhandledDeviceError; }
     return flagcxSuccess;
   }
+  const int sms = smCount();
+  if (!pair) { // an odd number of 128-row blocks
+    const int64_t want = readParam("GEMM_PAIR", 1);
+    pair = want > 1 || (want == 1 && pairForOddRows(M, N, K, sms, groupRows(true), groupRows(false), forced == 1));
+  }
+  const int padded = pair ? (M + 255) / 256 * 256 : M; // rows in whole tiles
   FCXCHECK(cu::tensorMap2dBf16(&tb, B, N, K, pair ? 128 : 256, 64));
   flagcxDevComm c;
   memset(&c, 0, sizeof c);
@@ -115,15 +121,14 @@ flagcxResult_t flagcxGemmBf16(const void *A, const void *B, void *D, int M, int 
   TpGemmArgs a;
   memset(&a, 0, sizeof a);
   a.D = (__nv_bfloat16 *)D;
-  a.M = M; a.N = N; a.K = K;
+  a.M = padded; a.N = N; a.K = K;
+  a.rows = M;
   a.mode = kPlain;
-  a.rowsPerRank = M;
+  a.rowsPerRank = padded;
   a.groupRows = groupRows(pair);
-  int tiles = (M / 128) * (N / 256);
-  if (pair) tiles = 2 * ((M / 256) * (N / 256));
-  const int sms = smCount();
+  const int tiles = (padded / 128) * (N / 256);
   SplitGemmTail tail;
-  if (forced != 1) tail = tailPlan(M, N, K, pair, pair ? sms / 2 : sms, groupRows(pair), &plan);
+  if (forced != 1) tail = tailPlan(padded, N, K, pair, pair ? sms / 2 : sms, groupRows(pair), &plan);
   a.tiles = tail.first;
   cudaError_t e = launchTpGemm(stream ? stream->base : nullptr, ta, tb, nullptr, c, a, std::min(tiles, sms), pair);
   if (e == cudaSuccess && tail.count) {

@@ -108,9 +108,10 @@ __global__ void __launch_bounds__(kThreads, 1)
     // part q of one of the persistent kernel's tiles (its order: tileCoords in tp_gemm.cu)
     const int down = tail.tileRows / BM, per = down * (256 / BN), t = tail.first + tile / per, q = tile % per;
     const int wide = N / 256, g = t / (tail.groupRows * wide), wg = t - g * tail.groupRows * wide;
-    const int gsize = min(tail.groupRows, tilesM / down - g * tail.groupRows);
+    const int gsize = min(tail.groupRows, (tilesM + down - 1) / down - g * tail.groupRows);
     tm = (g * tail.groupRows + wg % gsize) * down + q % down;
     tn = wg / gsize * (256 / BN) + q / down;
+    if (tm >= tilesM) return; // the whole cluster: half a tile that lies beyond the output
   }
   const int kb0 = (int)((long)kBlocks * part / S), kb1 = (int)((long)kBlocks * (part + 1) / S);
 

@@ -291,6 +291,8 @@ __global__ void __launch_bounds__(kThreads, 1)
       fenceAfterSync();
       // rows q*32 .. q*32+31 of the tile belong to this warp; all of them have one owner
       const size_t growBase = (size_t)tm * TM + ctaRank * BM + q * 32;
+      // the second half of a pair's last tile may lie beyond the output (its rows of A came as zeros)
+      const bool live = a.mode != kPlain || growBase < (size_t)a.rows;
       bf16 *dbase;
       int owner = rank;
       const bf16 *others = nullptr; // reduce-scatter, own rows: slice 0 of the partial sums of these rows
@@ -325,7 +327,7 @@ __global__ void __launch_bounds__(kThreads, 1)
       dbase += (size_t)tn * BN;
       const size_t sliceElems = (size_t)a.rowsPerRank * a.N;
 #pragma unroll 1
-      for (int cb = 0; cb < BN / kEpiCols; ++cb) {
+      for (int cb = 0; live && cb < BN / kEpiCols; ++cb) {
         // TMA stores alternate between the warp's two staging buffers; a buffer is
         // rewritten only after the engine has read its previous contents out
         uint4 *buf = (tmaOut && (cb & 1)) ? s.extra + (warp - 2) * (32 * kEpiCols * 2 / 16) : stg;

@@ -22,6 +22,7 @@ struct TpGemmArgs {
   int rowsPerRank;  // M / nRanks
   int piecesPerChunk; // all-gather mode: a 128-row chunk travels in this many 4 KiB pieces per peer
   int tiles;          // plain mode: only the first so many tiles of the order (0: all)
+  int rows;           // plain mode: rows that exist; M (and rowsPerRank) count whole tiles
   int groupRows;      // tile order: this many row blocks are walked together, column by column
   unsigned long long epoch; // call counter of this handle, starts at 1
   // all-gather -> GEMM

@@ -66,6 +66,29 @@ def test_gemm_whose_last_wave_is_nearly_empty(M, N, K):
     assert bool(((out.double() - ref).abs() <= bound).all())
 
 
+# CTA pairs whose last row of tiles is half empty: alone, in the order's last group, over several
+# waves, and with the last wave (the half tile is in it) on the split kernel.  Rows of A behind its
+# end would make a sum infinite, rows of the output behind its end must stay as they are.
+@pytest.mark.parametrize("M,N,K,split", [(128, 256, 64, 1), (640, 512, 320, 1), (2176, 768, 192, 1), (3712, 4352, 256, 1),
+                                         (2176, 2816, 8192, 0), (4736, 1024, 4096, 0)])
+def test_cta_pairs_with_an_odd_number_of_row_blocks(M, N, K, split, monkeypatch):
+    from flagcx_b200.parallel.tp import gemm_bf16
+    monkeypatch.setenv("FLAGCX_GEMM_PAIR", "2")
+    monkeypatch.setenv("FLAGCX_GEMM_SPLIT", str(split))
+    g = torch.Generator(device="cuda").manual_seed(M + N + K)
+    wide = torch.full((M + 128, K), float("inf"), dtype=torch.bfloat16, device="cuda")
+    wide[:M] = torch.randn(M, K, generator=g, device="cuda")
+    b = torch.randn(N, K, generator=g, device="cuda").to(torch.bfloat16)
+    out = torch.full((M + 128, N), 7.0, dtype=torch.bfloat16, device="cuda")
+    a = wide[:M]
+    gemm_bf16(a, b, out[:M])
+    ref = a.double() @ b.double().T
+    # the bound of the tests above
+    bound = ref.abs() * 2 ** -8 + (a.double().abs() @ b.double().abs().T) * K * 2 ** -24
+    assert bool(((out[:M].double() - ref).abs() <= bound).all())
+    assert bool((out[M:] == 7).all())
+
+
 # A product starts while the one in front of it ends.  Each reads what the last wrote, into buffers
 # that are used again every third time: by the split kernel, the persistent one (CTA pairs and single
 # CTAs), and both (full waves and a split last one); plainly and captured.
