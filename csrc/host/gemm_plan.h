@@ -94,23 +94,26 @@ inline SplitGemmTail tailPlan(int M, int N, int K, bool pair, int units, int gro
   return t;
 }
 
-// CTA pairs for an odd number of 128-row blocks: the pairs' last row of tiles is half empty, but a
-// wave of pairs is quicker than one of single CTAs (which load every tile of B once for 128 rows,
-// not 256) and costs more at its end, where two CTAs wait for each other: 0.4 us and 0.2 a wave.
-// Set by 90 shapes (4736 x 5632 x 7360 290 -> 263 us; with few K steps 4224 x 4352 x 256 15.8 against
-// 18.1, which stays) and tried on 120 others of 640 to 6272 rows and 75 tiles or more: 4.5 % less time
-// on average (5504 x 4608 x 1856 79.9 -> 69.7), none slower, 5.1 % if the better side were always known.
-inline bool pairForOddRows(int M, int N, int K, int sms, int groupPair, int groupSingle, bool noTail) {
+// Whether the persistent kernel takes CTA pairs.  A K step of pairs is quicker (single CTAs load every
+// tile of B once for 128 rows, not 256); the end of a wave of pairs costs more, where two CTAs wait for
+// each other; and with an odd number of 128-row blocks the pairs' last row of tiles is half empty.  So
+// single CTAs are the quicker side up to seven K steps (to twelve in a single wave), and about where
+// pairs need a wave more.
+// Set by 550 shapes of 256 to 6272 rows and 75 tiles or more, tried on 240 others against pairs for
+// even numbers of blocks and single CTAs for odd ones: 1.8 % less time over the even ones (5888 x 4608
+// x 256 24.6 -> 21.0 us, 5888 x 5888 x 384 33.9 -> 30.2), 4.3 % over the odd (1152 x 4608 x 2304
+// 32.8 -> 28.6, 5504 x 4608 x 1856 79.9 -> 69.7), none slower by more than the 0.3 us that two
+// runs of one route differ by; 2.0 and 4.6 % if the better side were always known.
+inline bool pairsQuicker(int M, int N, int K, int sms, int groupPair, int groupSingle, bool noTail) {
   const int kb = K / 64;
   auto us = [&](bool pair) {
     const int rows = pair ? (M + 255) / 256 * 256 : M, units = pair ? sms / 2 : sms;
-    const int tiles = rows / (pair ? 256 : 128) * (N / 256);
-    const double wave = pair ? kb * 0.33 + 0.2 : kb * 0.363, fixed = pair ? 0.4 : 0;
-    int waves = (tiles + units - 1) / units;
+    const int tiles = rows / (pair ? 256 : 128) * (N / 256), waves = (tiles + units - 1) / units;
+    const double wave = pair ? kb * 0.30 + 0.45 : kb * 0.363;
     SplitGemmPlan plan;
     if (noTail || !tailPlan(rows, N, K, pair, units, pair ? groupPair : groupSingle, &plan).count)
-      return fixed + waves * wave;
-    return fixed + (waves - 1) * wave + 10.5 + (kb + plan.parts - 1) / plan.parts * 0.3625;
+      return waves * wave + (pair && waves == 1 ? 0.5 : 0);
+    return (waves - 1) * wave + 10.5 + (kb + plan.parts - 1) / plan.parts * 0.3625;
   };
   return us(true) < us(false);
 }

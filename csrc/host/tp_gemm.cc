@@ -98,7 +98,7 @@ flagcxResult_t flagcxGemmBf16(const void *A, const void *B, void *D, int M, int 
   FCXCHECK(checkShape(M, N, K));
   CUtensorMap ta, tb;
   FCXCHECK(cu::tensorMap2dBf16(&ta, A, M, K, 128, 64));
-  bool pair = usePair(M);
+  bool pair = usePair(M); // what the estimates of splitPlan compare with
   const int forced = (int)readParam("GEMM_SPLIT", 0);
   SplitGemmPlan plan = splitPlan(M, N, K, pair, forced, forced > 1 ? (int)readParam("GEMM_SPLIT_N", 256) : 256);
   if (plan.tileN) {
@@ -108,10 +108,8 @@ flagcxResult_t flagcxGemmBf16(const void *A, const void *B, void *D, int M, int 
     return flagcxSuccess;
   }
   const int sms = smCount();
-  if (!pair) { // an odd number of 128-row blocks
-    const int64_t want = readParam("GEMM_PAIR", 1);
-    pair = want > 1 || (want == 1 && pairForOddRows(M, N, K, sms, groupRows(true), groupRows(false), forced == 1));
-  }
+  const int64_t want = readParam("GEMM_PAIR", 1);
+  pair = want > 1 || (want == 1 && pairsQuicker(M, N, K, sms, groupRows(true), groupRows(false), forced == 1));
   const int padded = pair ? (M + 255) / 256 * 256 : M; // rows in whole tiles
   FCXCHECK(cu::tensorMap2dBf16(&tb, B, N, K, pair ? 128 : 256, 64));
   flagcxDevComm c;

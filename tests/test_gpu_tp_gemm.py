@@ -68,12 +68,15 @@ def test_gemm_whose_last_wave_is_nearly_empty(M, N, K):
 
 # CTA pairs whose last row of tiles is half empty: alone, in the order's last group, over several
 # waves, and with the last wave (the half tile is in it) on the split kernel.  Rows of A behind its
-# end would make a sum infinite, rows of the output behind its end must stay as they are.
-@pytest.mark.parametrize("M,N,K,split", [(128, 256, 64, 1), (640, 512, 320, 1), (2176, 768, 192, 1), (3712, 4352, 256, 1),
-                                         (2176, 2816, 8192, 0), (4736, 1024, 4096, 0)])
-def test_cta_pairs_with_an_odd_number_of_row_blocks(M, N, K, split, monkeypatch):
+# end would make a sum infinite, rows of the output behind its end must stay as they are.  And what
+# the size picks (pair 1): both sides for even and odd numbers of blocks.
+@pytest.mark.parametrize("M,N,K,split,pair", [(128, 256, 64, 1, 2), (640, 512, 320, 1, 2), (2176, 768, 192, 1, 2),
+                                              (3712, 4352, 256, 1, 2), (2176, 2816, 8192, 0, 2), (4736, 1024, 4096, 0, 2),
+                                              (2304, 3072, 256, 0, 1), (2304, 3072, 1024, 0, 1),
+                                              (2176, 3072, 256, 0, 1), (2176, 3072, 1024, 0, 1)])
+def test_cta_pairs_with_an_odd_number_of_row_blocks(M, N, K, split, pair, monkeypatch):
     from flagcx_b200.parallel.tp import gemm_bf16
-    monkeypatch.setenv("FLAGCX_GEMM_PAIR", "2")
+    monkeypatch.setenv("FLAGCX_GEMM_PAIR", str(pair))
     monkeypatch.setenv("FLAGCX_GEMM_SPLIT", str(split))
     g = torch.Generator(device="cuda").manual_seed(M + N + K)
     wide = torch.full((M + 128, K), float("inf"), dtype=torch.bfloat16, device="cuda")
