@@ -102,8 +102,9 @@ inline SplitGemmTail tailPlan(int M, int N, int K, bool pair, int units, int gro
 // Set by 550 shapes of 256 to 6272 rows and 75 tiles or more, tried on 240 others against pairs for
 // even numbers of blocks and single CTAs for odd ones: 1.8 % less time over the even ones (5888 x 4608
 // x 256 24.6 -> 21.0 us, 5888 x 5888 x 384 33.9 -> 30.2), 4.3 % over the odd (1152 x 4608 x 2304
-// 32.8 -> 28.6, 5504 x 4608 x 1856 79.9 -> 69.7), none slower by more than the 0.3 us that two
-// runs of one route differ by; 2.0 and 4.6 % if the better side were always known.
+// 32.8 -> 28.6, 640 x 4608 x 7104 45.9 -> 40.6), none slower by more than the 0.3 us that two
+// runs of one route differ by; 2.0 and 4.6 % if the better side were always known.  5504 x 4352 x 896
+// stays with single CTAs, 37.4 against 35.8.
 inline bool pairsQuicker(int M, int N, int K, int sms, int groupPair, int groupSingle, bool noTail) {
   const int kb = K / 64;
   auto us = [&](bool pair) {
