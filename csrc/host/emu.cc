@@ -16,18 +16,19 @@
 
 namespace fcx {
 
+constexpr int kMoeKinds = 100; // beyond the families of device_coll.cc
+
 struct EmuWorld {
   int n = 0, dev = 0;
   std::vector<flagcxComm *> comms;
   std::vector<void *> internalBase;
   // pending submissions of the current collective
   int posted = 0;
-  int family = -1, nCtas = 0;
+  int kind = -1, nCtas = 0; // what the ranks have posted: a kernel family, or kMoeKinds + EmuMoeOp
   std::vector<char> has;
   std::vector<CollArgs> coll;
   std::vector<P2pArgs> p2p;
   std::vector<MoeArgs> moe;
-  EmuMoeOp moeOp = kEmuMoeDispatch;
   std::vector<flagcxDevComm> devs; // what the launch in preparation hands to its kernel
   int maxGrid = 0;
 };
@@ -148,28 +149,39 @@ static LaunchCtx emuLaunchCtx(EmuWorld *w, cudaStream_t stream) {
   return lc;
 }
 
-flagcxResult_t emuSubmit(flagcxComm *c, int family, const CollArgs *coll, const P2pArgs *p2p, int nCtas,
-                         cudaStream_t stream) {
-  EmuWorld *w = c->emu;
-  const int n = w->n, r = c->rank;
+// Counts rank r's post in; *all tells whether it was the last one.  A launch takes the argument
+// blocks of one kind from every rank, so a rank that posts another kind is refused.
+static flagcxResult_t emuPost(EmuWorld *w, int r, int kind, int nCtas, bool *all) {
   if (w->has[r]) {
-    FCX_WARN("emulated rank %d posted a second collective before the others posted their first", r);
+    FCX_WARN("emulated rank %d posted a second operation before the others posted their first", r);
     return flagcxInvalidUsage;
   }
-  if (w->posted == 0) { w->family = family; w->nCtas = nCtas; }
-  if (family != w->family) {
+  if (w->posted == 0) { w->kind = kind; w->nCtas = nCtas; }
+  if (kind != w->kind) {
     FCX_WARN("emulated ranks posted different kinds of operations");
     return flagcxInvalidUsage;
   }
   w->nCtas = std::min(w->nCtas, nCtas);
+  w->has[r] = 1;
+  *all = ++w->posted == w->n;
+  if (*all) {
+    w->posted = 0;
+    std::fill(w->has.begin(), w->has.end(), 0);
+  }
+  return flagcxSuccess;
+}
+
+flagcxResult_t emuSubmit(flagcxComm *c, int family, const CollArgs *coll, const P2pArgs *p2p, int nCtas,
+                         cudaStream_t stream) {
+  EmuWorld *w = c->emu;
+  const int n = w->n, r = c->rank;
+  bool all = false;
+  FCXCHECK(emuPost(w, r, family, nCtas, &all));
   if (coll) w->coll[r] = *coll;
   if (p2p) w->p2p[r] = *p2p;
-  w->has[r] = 1;
-  if (++w->posted < n) return flagcxSuccess;
+  if (!all) return flagcxSuccess;
 
   // everybody is here: complete the peer tables and launch once
-  w->posted = 0;
-  std::fill(w->has.begin(), w->has.end(), 0);
   LaunchCtx lc = emuLaunchCtx(w, stream);
   cudaError_t e;
   if (family == 3) {
@@ -203,22 +215,10 @@ flagcxResult_t emuSubmit(flagcxComm *c, int family, const CollArgs *coll, const 
 // The same for the expert-parallel kernels.
 flagcxResult_t emuSubmitMoe(flagcxComm *c, EmuMoeOp op, const MoeArgs &args, int nCtas, cudaStream_t stream) {
   EmuWorld *w = c->emu;
-  const int n = w->n, r = c->rank;
-  if (w->has[r]) {
-    FCX_WARN("emulated rank %d posted a second operation before the others posted their first", r);
-    return flagcxInvalidUsage;
-  }
-  if (w->posted == 0) { w->moeOp = op; w->nCtas = nCtas; }
-  if (op != w->moeOp) {
-    FCX_WARN("emulated ranks posted different kinds of operations");
-    return flagcxInvalidUsage;
-  }
-  w->nCtas = std::min(w->nCtas, nCtas);
-  w->moe[r] = args;
-  w->has[r] = 1;
-  if (++w->posted < n) return flagcxSuccess;
-  w->posted = 0;
-  std::fill(w->has.begin(), w->has.end(), 0);
+  bool all = false;
+  FCXCHECK(emuPost(w, c->rank, kMoeKinds + op, nCtas, &all));
+  w->moe[c->rank] = args;
+  if (!all) return flagcxSuccess;
   LaunchCtx lc = emuLaunchCtx(w, stream);
   lc.nCtas = w->nCtas; // the launcher knows how many of its kernel's CTAs run at once
   lc.emuMoe = w->moe.data();

@@ -129,3 +129,40 @@ def test_few_ctas_and_ragged_rows(T, H, ctas, reduce, monkeypatch):
             m.close()
     finally:
         capi.Comm.emu_world_destroy(comms)
+
+
+# Four ranks of which two post: nothing is launched before the others have.  Both orders, in a new
+# world and in one whose last operation was of the second kind.
+@pytest.mark.parametrize("used", [False, True])
+@pytest.mark.parametrize("first", ["dispatch", "all_reduce"])
+def test_ranks_that_post_different_operations_are_refused(first, used):
+    n, T, H, E, K = 4, 8, 64, 8, 2
+    comms = capi.Comm.emu_world(n, 0)
+    try:
+        moes = [MoeDispatcher(comms[r], T, H, K, E, T * K * n) for r in range(n)]
+        g = torch.Generator().manual_seed(1)
+        xs = [torch.randn(T, H, generator=g).to(torch.bfloat16).cuda() for _ in range(n)]
+        routed = [route(torch.randn(T, E, generator=g).cuda(), K) for _ in range(n)]
+        outs = [torch.empty_like(x) for x in xs]
+        post = {"dispatch": lambda r: moes[r].dispatch(xs[r], routed[r][0]),
+                "all_reduce": lambda r: comms[r].all_reduce(xs[r], outs[r], T * H, capi.BFLOAT16)}
+        second = "all_reduce" if first == "dispatch" else "dispatch"
+        if used:
+            for r in range(n):
+                post[second](r)
+        post[first](0)
+        with pytest.raises(RuntimeError):
+            post[second](1)
+        for r in range(1, n):  # the others still complete what rank 0 has posted
+            post[first](r)
+        torch.cuda.synchronize()
+        assert all(c.async_error() == 0 for c in comms)
+        if first == "all_reduce":
+            ref = sum(x.double() for x in xs)
+            assert float((outs[2].double() - ref).abs().max()) < 0.05
+        else:  # every row that was dispatched has arrived
+            assert sum(int(m.expert_offsets[-1]) for m in moes) == n * T * K
+        for m in moes:
+            m.close()
+    finally:
+        capi.Comm.emu_world_destroy(comms)
