@@ -161,7 +161,12 @@ struct Reducer {
         }
       item = next;
     }
-    tickets.leave();
+  }
+  // Whether a range of so many elements is drawn (where every pointer is aligned).  Known before the
+  // first barrier and the same for all CTAs of a rank: then each of them ends with Tickets::leave().
+  static __device__ __forceinline__ bool draws(size_t elems, int g) {
+    if constexpr (NR > 0) return elems / N >= (size_t)kDrawItems * 32 * (16 / NR) * (blockDim.x >> 5) * g;
+    else return false;
   }
 
   static __device__ __forceinline__ void addUp(const CollArgs &a, const uint4 (&v)[NR > 0 ? NR : 1], Acc (&acc)[N]) {
@@ -178,9 +183,9 @@ struct Reducer {
 
   // Reduces elements [sb, se) of the inputs (indices into in[p]) and stores them at
   // element index (i - sb + dstBase) of each destination.  The CTA takes its share
-  // of the range in 16-byte units, or (mayDraw) draws them where that pays.
+  // of the range in 16-byte units, or (draw) draws them.
   static __device__ void slice(const CollArgs &a, int nRanks, size_t sb, size_t se, char *const *dst, int nDst,
-                               size_t dstBase, int b, int g, bool mayDraw = false) {
+                               size_t dstBase, int b, int g, bool draw = false) {
     if (se <= sb) return;
     const size_t elems = se - sb;
     const size_t outSize = a.outMode == kOutFloat ? 4 : (a.outMode == kOutBf16 ? 2 : sizeof(T));
@@ -195,7 +200,7 @@ struct Reducer {
     if constexpr (NR > 0) {
       constexpr int U = 16 / NR; // peer loads take microseconds: 16 of them in flight per thread
       const size_t packs = elems / N;
-      drawn = vec && mayDraw && packs >= (size_t)kDrawItems * 32 * U * (blockDim.x >> 5) * g;
+      drawn = vec && draw;
       if (drawn) {
         if (gridDim.x * gridDim.y >= kDrawHalfCtas) drawPacks<U / 2>(a, sb, packs, dst, nDst, dstBase);
         else drawPacks<U>(a, sb, packs, dst, nDst, dstBase);
@@ -444,18 +449,16 @@ __device__ bool ringReduceScatter(const flagcxDevComm &c, const CollArgs &a, siz
   return true;
 }
 
+// From the first barrier to the last store of this CTA; *done: nothing was given up on the way.
 template <typename T, int OP, int NR>
-__device__ void reduceBody(const flagcxDevComm &c, CollArgs &a) {
+__device__ __forceinline__ void reduceRanges(const flagcxDevComm &c, CollArgs &a, bool draw, bool *done) {
   const int b = blockIdx.x, g = gridDim.x, rank = c.rank, n = c.nRanks;
   using R = Reducer<T, OP, NR>;
 
-  copyIn(a, rank, b, g);
-  publishPointers(c, a, b);
   if (a.flags & kFlagBeginBarrier)
     if (!ctaBarrier(c, b)) return;
   learnPointers(c, a, b);
   const bool bulk = NR > 0 && a.bulkStage && learntPointersAligned(c, a);
-  const bool direct = !a.userIn && !a.userOut; // else CTA b must take what CTA b has staged, and only that
   {
     const size_t outEs = a.outMode == kOutFloat ? 4 : (a.outMode == kOutBf16 ? 2 : sizeof(T));
     const size_t inEnd = a.kind == kReduceScatter ? a.inStride * (size_t)(n - 1) + a.count * sizeof(T)
@@ -475,7 +478,7 @@ __device__ void reduceBody(const flagcxDevComm &c, CollArgs &a) {
   char *local[1] = {a.out[rank]};
   switch (a.kind) {
     case kAllReduceOneShot:
-      R::slice(a, n, 0, a.count, local, 1, 0, b, g, direct);
+      R::slice(a, n, 0, a.count, local, 1, 0, b, g, draw);
       break;
     case kAllReduceTwoShot: {
       size_t s = sliceElems(a.count, n, sizeof(T));
@@ -484,7 +487,7 @@ __device__ void reduceBody(const flagcxDevComm &c, CollArgs &a) {
       if (bulk) {
         if (!R::sliceBulk(c, a, sb, se, a.out, n, sb, b, g)) return;
       } else {
-        R::slice(a, n, sb, se, a.out, n, sb, b, g, direct);
+        R::slice(a, n, sb, se, a.out, n, sb, b, g, draw);
       }
       break;
     }
@@ -493,12 +496,12 @@ __device__ void reduceBody(const flagcxDevComm &c, CollArgs &a) {
       if (bulk) {
         if (!R::sliceBulk(c, a, sb, sb + a.count, local, 1, 0, b, g)) return;
       } else {
-        R::slice(a, n, sb, sb + a.count, local, 1, 0, b, g, direct);
+        R::slice(a, n, sb, sb + a.count, local, 1, 0, b, g, draw);
       }
       break;
     }
     case kReduceToRoot:
-      if (rank == a.root) R::slice(a, n, 0, a.count, local, 1, 0, b, g, direct);
+      if (rank == a.root) R::slice(a, n, 0, a.count, local, 1, 0, b, g, draw);
       break;
     case kReduceScatterRing:
       if (!ringReduceScatter<T, OP>(c, a, a.count, a.count * (size_t)n, (T *)a.out[rank], b, g)) return;
@@ -553,7 +556,29 @@ __device__ void reduceBody(const flagcxDevComm &c, CollArgs &a) {
     }
     default: break;
   }
+  *done = true;
+}
 
+template <typename T, int OP, int NR>
+__device__ void reduceBody(const flagcxDevComm &c, CollArgs &a) {
+  const int b = blockIdx.x, g = gridDim.x, rank = c.rank;
+  copyIn(a, rank, b, g);
+  publishPointers(c, a, b);
+  // With staging CTA b must take what CTA b has staged, and only that.
+  size_t drawn = 0; // elements that this rank's CTAs may draw
+  if (!a.userIn && !a.userOut) {
+    if (a.kind == kAllReduceTwoShot) {
+      const size_t s = sliceElems(a.count, c.nRanks, sizeof(T)), sb = s * rank;
+      drawn = sb < a.count ? (s < a.count - sb ? s : a.count - sb) : 0;
+    } else if (a.kind == kAllReduceOneShot || a.kind == kReduceScatter || (a.kind == kReduceToRoot && rank == a.root)) {
+      drawn = a.count;
+    }
+  }
+  const bool draw = Reducer<T, OP, NR>::draws(drawn, g);
+  bool done = false;
+  reduceRanges<T, OP, NR>(c, a, draw, &done);
+  if (draw) Tickets{a.tickets}.leave(); // also where a wait has run out: the next launch starts at zero
+  if (!done) return;
   if (a.flags & kFlagEndBarrier)
     if (!ctaBarrier(c, b)) return;
   copyOut(a, rank, b, g);

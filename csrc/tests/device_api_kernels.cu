@@ -248,6 +248,12 @@ __global__ void kCWrappers(TestArgs a) {
   if (threadIdx.x == 0) resultOf(a, c.rank)[0] = good;
 }
 
+// 11. moves rank 0's count of barriers in slot nWords by `iterations`, which puts it out of step
+// with its peers, or back.
+__global__ void kShiftEpoch(TestArgs a) {
+  if (blockIdx.y == 0 && threadIdx.x == 0) a.comms[0].barrierEpoch[a.nWords] += (long long)a.iterations;
+}
+
 } // namespace
 
 extern "C" int fcxDevTestSizes(int *devCommBytes, int *devMemBytes) {
@@ -286,6 +292,7 @@ extern "C" int fcxDevTestLaunch(int which, const void *dComms, const void *dMems
     case 8: fn = (const void *)kReset; break;
     case 9: fn = (const void *)kWaitTimesOut; break;
     case 10: fn = (const void *)kCWrappers; break;
+    case 11: fn = (const void *)kShiftEpoch; break;
     default: return (int)cudaErrorInvalidValue;
   }
   return (int)cudaLaunchCooperativeKernel(fn, dim3(1, nRanks), dim3(256), params, 0, (cudaStream_t)stream);

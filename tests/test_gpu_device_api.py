@@ -166,6 +166,46 @@ def test_unsatisfied_wait_returns_false_and_reports():
         w.close()
 
 
+# Two of rank 0's four CTAs wait in vain before they reduce anything, the others draw their work.
+# A launch that is already queued behind that one starts with all of it.
+@pytest.mark.parametrize("kind", ["one-shot", "two-shot", "reduce-scatter"])
+def test_launch_queued_behind_one_whose_barrier_ran_out(kind):
+    w = World(2, timeout_ms=100)
+    try:
+        n, ctas, count = w.n, 4, 1 << 19
+        g = torch.Generator().manual_seed(3)
+        xs = [torch.randn(count, generator=g).cuda() for _ in range(n)]
+        outs = [[torch.full((count,), float("nan"), device="cuda") for _ in range(n)] for _ in range(2)]
+
+        def shift(by):
+            for slot in (1, 2):
+                assert w.lib.fcxDevTestLaunch(11, w.d_comms.data_ptr(), w.d_mems.data_ptr(), w.results.data_ptr(), n, slot, by,
+                                              None) == 0
+
+        def launch(out):
+            for r in range(n):
+                if kind == "reduce-scatter":
+                    w.comms[r].reduce_scatter_fused(xs[r], out[r], count // n, capi.FLOAT, capi.SUM, nctas=ctas)
+                else:
+                    w.comms[r].all_reduce_fused(xs[r], out[r], count, capi.FLOAT, capi.SUM, nctas=ctas,
+                                                algo=capi.ALGO_ONESHOT if kind == "one-shot" else capi.ALGO_TWOSHOT)
+
+        # rank 0 is two barriers ahead: its first wait runs out, while its peer's two barriers pass; then
+        # one barrier ahead of its peer's two, which is in step again
+        shift(2)
+        launch(outs[0])
+        shift(-1)
+        launch(outs[1])
+        torch.cuda.synchronize()
+        assert w.comms[0].async_error() == capi.flagcxRemoteError
+        ref = xs[0] + xs[1]
+        for r in range(n):
+            want = ref[r * count // n:(r + 1) * count // n] if kind == "reduce-scatter" else ref
+            assert torch.equal(outs[1][r][:want.numel()], want), r
+    finally:
+        w.close()
+
+
 def test_one_sided_host_api_put_get_signal_counter():
     """flagcxOneSideRegister / Put / Get / BatchPut / ReadCounter / WaitCounter / PutSignal /
     Signal / WaitSignal between two emulated ranks."""
