@@ -71,6 +71,11 @@ inline size_t sliceElems(size_t count, int nRanks, size_t elemSize) {
   return (s + perPack - 1) / perPack * perPack;
 }
 
+// Loads in flight per thread of a reduction whose packs are drawn by ticket: 16, since loads from a
+// peer take microseconds, but 8 (true) in an emulated world whose CTAs (`ctas` per rank) fill the one GPU
+// that holds all inputs: 144 CTAs 97 against 105 us with 16, fp32 180 against 212; 32 CTAs 250 against 209.
+__host__ __device__ inline bool drawHalfLoads(unsigned ctas, unsigned emuRanks) { return emuRanks > 1 && ctas * emuRanks >= 128; }
+
 struct CollArgs {
   const char *in[FLAGCX_MAX_RANKS]; // in[p]: rank p's input as mapped here
   char *out[FLAGCX_MAX_RANKS];      // out[p]: rank p's output as mapped here

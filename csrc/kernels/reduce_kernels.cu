@@ -30,9 +30,6 @@ namespace {
 // warp on; with less (1 Mi elements: 4 packs a thread) the barriers are most of the time and both
 // ways take the same.
 constexpr int kDrawItems = 2;
-// Loads in flight per thread: 16 where few CTAs run (32 CTAs: 209 against 250 us with 8), 8 where
-// they fill the GPU (144 CTAs: 97 against 105 us with 16, fp32 180 against 212).
-constexpr unsigned kDrawHalfCtas = 128;
 template <typename T, int OP, int NR>
 struct Reducer {
   using Acc = typename Elem<T>::Acc;
@@ -202,7 +199,7 @@ struct Reducer {
       const size_t packs = elems / N;
       drawn = vec && draw;
       if (drawn) {
-        if (gridDim.x * gridDim.y >= kDrawHalfCtas) drawPacks<U / 2>(a, sb, packs, dst, nDst, dstBase);
+        if (drawHalfLoads(gridDim.x, gridDim.y)) drawPacks<U / 2>(a, sb, packs, dst, nDst, dstBase);
         else drawPacks<U>(a, sb, packs, dst, nDst, dstBase);
         eb = packs * N; // what is left is less than a pack: the last CTA's
         ee = b == g - 1 ? elems : eb;

@@ -18,6 +18,7 @@
 #include "../host/reg_cache.h"
 #include "../host/shm.h"
 #include "../host/tuner.h"
+#include "../kernels/coll_args.h"
 #include "flagcx_net.h"
 #include "flagcx_p2p.h"
 
@@ -483,8 +484,14 @@ static void testGemmPlan() {
       }
 }
 
+static void testDrawHalfLoads() {
+  EXPECT(!drawHalfLoads(1, 1) && !drawHalfLoads(128, 1)); // one rank per GPU: never
+  EXPECT(drawHalfLoads(18, 8) && drawHalfLoads(64, 2) && !drawHalfLoads(4, 8) && !drawHalfLoads(15, 8));
+}
+
 int main() {
   testGemmPlan();
+  testDrawHalfLoads();
   testRegCache();
   testShmRing();
   testParams();
