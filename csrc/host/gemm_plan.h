@@ -32,6 +32,10 @@ inline double splitUs(const SplitGemmKind &k, int parts, long tiles, int kb, dou
 // tiles the persistent kernel keeps what it had when a split cost 2 us more: two parts or more, and
 // 1.7 us to be gained (given away: 1664 x 768 x 1024 9.6 against 10.6, 128 x 9728 x 1280 11.3 against
 // 13.3).
+// pair: that the number of 128-row blocks is even.  The persistent kernel may yet take pairs for an odd
+// one (pairsQuicker); its estimate here stays that of single CTAs, with which the split was right on
+// all of 30 shapes where the estimate for pairs would have left it (3 to 22 % quicker: 1152 x 2048 x 2816
+// 16.1 against 19.7, 128 x 13312 x 11328 58.4 against 65.6).
 // Clusters stay within what is co-resident: a second wave costs more than the split gains (28
 // clusters of 5: 37 us against 27).
 // forced: 1 = never split, 2 to 8 = split over so many CTAs with tiles of forcedTileN.
@@ -97,23 +101,27 @@ inline SplitGemmTail tailPlan(int M, int N, int K, bool pair, int units, int gro
 // Whether the persistent kernel takes CTA pairs.  A K step of pairs is quicker (single CTAs load every
 // tile of B once for 128 rows, not 256); the end of a wave of pairs costs more, where two CTAs wait for
 // each other; and with an odd number of 128-row blocks the pairs' last row of tiles is half empty.  So
-// single CTAs are the quicker side up to seven K steps (to twelve in a single wave), and about where
-// pairs need a wave more.
-// Set by 550 shapes of 256 to 6272 rows and 75 tiles or more, tried on 240 others against pairs for
+// single CTAs are the quicker side up to seven K steps, and about where pairs need a wave more.  In a
+// single wave they are up to eleven, where 75 tiles or more occupy half of the SMs with either kind
+// (2560 x 1792 x 576 9.3 against 9.7 us, 512 x 9472 x 896 12.6 against 12.1), and up to eight with
+// fewer tiles (384 x 4096 x 512 8.3 against 8.4, 256 x 3584 x 832 10.0 against 9.5; a lone block of 128
+// rows gains from the second CTA that fetches half of B: 128 x 14848 x 7296 56.0 against 47.3).
+// Several waves were set by 550 shapes of 256 to 6272 rows and tried on 240 others against pairs for
 // even numbers of blocks and single CTAs for odd ones: 1.8 % less time over the even ones (5888 x 4608
 // x 256 24.6 -> 21.0 us, 5888 x 5888 x 384 33.9 -> 30.2), 4.3 % over the odd (1152 x 4608 x 2304
 // 32.8 -> 28.6, 640 x 4608 x 7104 45.9 -> 40.6), none slower by more than the 0.3 us that two
 // runs of one route differ by; 2.0 and 4.6 % if the better side were always known.  5504 x 4352 x 896
-// stays with single CTAs, 37.4 against 35.8.
+// stays with single CTAs, 37.4 against 35.8.  A single wave by 244 shapes: at worst 0.2 us are given
+// away, for odd and even numbers of blocks alike.
 inline bool pairsQuicker(int M, int N, int K, int sms, int groupPair, int groupSingle, bool noTail) {
   const int kb = K / 64;
   auto us = [&](bool pair) {
     const int rows = pair ? (M + 255) / 256 * 256 : M, units = pair ? sms / 2 : sms;
     const int tiles = rows / (pair ? 256 : 128) * (N / 256), waves = (tiles + units - 1) / units;
-    const double wave = pair ? kb * 0.30 + 0.45 : kb * 0.363;
+    const double wave = pair ? kb * 0.30 + 0.45 : kb * 0.363, only = M / 128 * (N / 256) > sms / 2 ? 0.27 : 0.085;
     SplitGemmPlan plan;
     if (noTail || !tailPlan(rows, N, K, pair, units, pair ? groupPair : groupSingle, &plan).count)
-      return waves * wave + (pair && waves == 1 ? 0.5 : 0);
+      return waves * wave + (pair && waves == 1 ? only : 0);
     return (waves - 1) * wave + 10.5 + (kb + plan.parts - 1) / plan.parts * 0.3625;
   };
   return us(true) < us(false);

@@ -98,7 +98,7 @@ flagcxResult_t flagcxGemmBf16(const void *A, const void *B, void *D, int M, int 
   FCXCHECK(checkShape(M, N, K));
   CUtensorMap ta, tb;
   FCXCHECK(cu::tensorMap2dBf16(&ta, A, M, K, 128, 64));
-  bool pair = usePair(M); // what the estimates of splitPlan compare with
+  bool pair = usePair(M); // for splitPlan's estimates; what the persistent kernel takes is decided below
   const int forced = (int)readParam("GEMM_SPLIT", 0);
   SplitGemmPlan plan = splitPlan(M, N, K, pair, forced, forced > 1 ? (int)readParam("GEMM_SPLIT_N", 256) : 256);
   if (plan.tileN) {

@@ -476,6 +476,11 @@ static void testGemmPlan() {
   EXPECT(pairs(2560, 2560, 576) && pairs(8192, 3584, 8192));  // 13.1 against 13.6, 380 against 413 in a loop
   EXPECT(pairs(1152, 4608, 2304) && pairs(640, 4608, 7104));  // 28.7 against 32.8, 41.1 against 45.9
   EXPECT(!pairs(2688, 3584, 640) && !pairs(896, 5376, 2944)); // a wave more: 17.3 against 14.9, 33.5 against 23.4
+  // ... in a single wave, of few tiles and of more
+  EXPECT(pairs(256, 3584, 832) && pairs(768, 2048, 960) && pairs(128, 4608, 960)); // 9.5 against 10.0, 10.1 against 10.5, 10.1 against 10.9
+  EXPECT(!pairs(512, 3328, 256) && !pairs(384, 4096, 512));   // 7.1 against 6.8, 8.4 against 8.3
+  EXPECT(pairs(512, 9472, 896) && pairs(768, 5376, 960));     // 12.1 against 12.6, 11.6 against 11.8
+  EXPECT(!pairs(2560, 1792, 576) && !pairs(3584, 1280, 704)); // 9.7 against 9.3, 10.3 against 10.2
   for (int M = 128; M <= 8192; M += 128) // a plan never asks for more parts than K has steps or than run at once
     for (int N = 256; N <= 8192; N += 768)
       for (int K = 64; K <= 8192; K += 192) {
