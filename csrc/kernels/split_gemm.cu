@@ -16,9 +16,10 @@
 // Bound, 128 x 3584 x 8192 (112 CTAs, 4 parts): 10 us in which the weights come out of HBM at 5.9
 // TB/s, and 3.6 us behind them: accumulators to shared memory 0.6, cluster barrier 0.7, the sum 2.3,
 // which is 48 KB into every SM at the 14 bytes a clock that distributed shared memory gives (loads,
-// stores and bulk copies alike).  The sum's loads are all under way at once, a part that failed
-// says so in its values (NaN) instead of a flag of its own, the last barrier publishes nothing,
-// and the kernel is launched while the one in front of it ends: 20.5 -> 17.5 us back to back.
+// stores and bulk copies alike).  The sum's loads are all under way at once, the marks of
+// parts that failed come with them (0.1 us with 8 parts: 128 x 256 x 8192 9.09 -> 9.24), the last
+// barrier publishes nothing, and the kernel is launched while the one in front of it ends: 20.5 -> 17.5
+// us back to back.
 #include <cuda_bf16.h>
 
 #include <atomic>
@@ -33,7 +34,15 @@ using bf16 = __nv_bfloat16;
 using namespace tc;
 
 constexpr int BM = 128, BK = 64, kThreads = 256;
-constexpr unsigned long long kWaitLimitNs = 4000000000ull; // 4 s
+
+// How long a wait may take, the K step whose operands are not fetched, and what is done about them
+// once the CTA has given up (a test of the waits that run out sets all three).
+#ifndef FLAGCX_GEMM_WAIT_NS
+#define FLAGCX_GEMM_WAIT_NS 4000000000ull
+#define FLAGCX_GEMM_HELD_BACK(tile, kb) false
+#define FLAGCX_GEMM_GIVEN_UP(load)
+#endif
+constexpr unsigned long long kWaitLimitNs = FLAGCX_GEMM_WAIT_NS;
 
 template <int BN>
 struct __align__(1024) Smem {
@@ -43,6 +52,7 @@ struct __align__(1024) Smem {
   uint64_t full[STAGES], empty[STAGES], done;
   uint32_t tmemBase;
   int abortFlag;
+  int lost; // this part has no sum.  Outside the ring, where copies may land late
 };
 
 __device__ __forceinline__ float4 ldCluster16(uint32_t addr) {
@@ -51,6 +61,12 @@ __device__ __forceinline__ float4 ldCluster16(uint32_t addr) {
                : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w)
                : "r"(addr)
                : "memory");
+  return v;
+}
+
+__device__ __forceinline__ int ldClusterInt(uint32_t addr) {
+  int v;
+  asm volatile("ld.shared::cluster.s32 %0, [%1];" : "=r"(v) : "r"(addr) : "memory");
   return v;
 }
 
@@ -121,6 +137,7 @@ __global__ void __launch_bounds__(kThreads, 1)
     for (int i = 0; i < STAGES; ++i) { mbarInit(&s.full[i], 1); mbarInit(&s.empty[i], 1); }
     mbarInit(&s.done, 1);
     s.abortFlag = 0;
+    s.lost = 0;
     mbarInitFence();
   }
   if (warp == 1) { tmemAlloc(&s.tmemBase, BN); tmemRelinquish(); }
@@ -132,22 +149,21 @@ __global__ void __launch_bounds__(kThreads, 1)
   const uint32_t tmemBase = s.tmemBase;
   volatile int *abortFlag = &s.abortFlag;
 
+  int issued = 0; // K steps whose operands thread 0 has asked for
+  auto load = [&](int kb, int stage) {
+    mbarExpectTx(&s.full[stage], kStageBytes);
+    tmaLoad2d(s.a[stage], &tmA, kb * BK, tm * BM, &s.full[stage]);
+    tmaLoad2d(s.b[stage], &tmB, kb * BK, tn * BN, &s.full[stage]);
+  };
   if (warp == 0) {
     if (lane == 0) { // TMA producer
-      int stage = 0, issued = 0;
+      int stage = 0;
       uint32_t phase = 0;
       for (int kb = kb0; kb < kb1; ++kb) {
         if (!mbarWait(&s.empty[stage], phase ^ 1, abortFlag, kWaitLimitNs)) break;
-        mbarExpectTx(&s.full[stage], kStageBytes);
-        tmaLoad2d(s.a[stage], &tmA, kb * BK, tm * BM, &s.full[stage]);
-        tmaLoad2d(s.b[stage], &tmB, kb * BK, tn * BN, &s.full[stage]);
+        if (!FLAGCX_GEMM_HELD_BACK(tile, kb)) load(kb, stage);
         ++issued;
         if (++stage == STAGES) { stage = 0; phase ^= 1; }
-      }
-      if (*abortFlag) { // given up: copies that are still under way land before the CTA goes on
-        int never = 0;
-        for (int j = issued > STAGES ? issued - STAGES : 0; j < issued; ++j)
-          mbarWait(&s.full[j % STAGES], (uint32_t)(j / STAGES) & 1u, &never, kWaitLimitNs);
       }
     }
     __syncwarp();
@@ -189,13 +205,19 @@ __global__ void __launch_bounds__(kThreads, 1)
             make_float4(__uint_as_float(r[4 * i]), __uint_as_float(r[4 * i + 1]), __uint_as_float(r[4 * i + 2]),
                         __uint_as_float(r[4 * i + 3]));
     }
-  } else { // with this part NaN the whole tile is, in every CTA of the cluster
-    for (int i = threadIdx.x; i < BM * kChunks; i += kThreads) tileBuf[i] = make_float4(NAN, NAN, NAN, NAN);
+  } else if (threadIdx.x == 0) {
+    s.lost = 1;
+    // given up: copies that are still under way land before the CTA goes on
+    int never = 0;
+    for (int j = issued > STAGES ? issued - STAGES : 0; j < issued; ++j)
+      mbarWait(&s.full[j % STAGES], (uint32_t)(j / STAGES) & 1u, &never, kWaitLimitNs);
+    FLAGCX_GEMM_GIVEN_UP(load);
   }
   fenceBeforeSync();
   __syncwarp();
   clusterSync();
   const uint32_t base = smemAddr(tileBuf);
+  const int lost = lane < S ? ldClusterInt(mapToCta(smemAddr(&s.lost), lane)) : 0; // on its way during the sum
   const int r0 = BM * part / S, r1 = BM * (part + 1) / S;
   bf16 *out = D + (size_t)tm * BM * N + tn * BN;
   switch (S) {
@@ -204,6 +226,11 @@ __global__ void __launch_bounds__(kThreads, 1)
     case 4: addParts<BN, 4>(base, S, r0, r1, out, N); break;
     case 8: addParts<BN, 8>(base, S, r0, r1, out, N); break;
     default: addParts<BN, 0>(base, S, r0, r1, out, N);
+  }
+  if (__any_sync(0xffffffffu, lost)) { // the tile becomes NaN, in every CTA of the cluster: each thread's sums again
+    __align__(8) const __nv_bfloat162 o[2] = {__floats2bfloat162_rn(NAN, NAN), __floats2bfloat162_rn(NAN, NAN)};
+    for (int i = threadIdx.x; i < (r1 - r0) * kChunks; i += kThreads)
+      *reinterpret_cast<uint2 *>(out + (size_t)(r0 + i / kChunks) * N + i % kChunks * 4) = *reinterpret_cast<const uint2 *>(o);
   }
   // no CTA leaves while another may still read its part: the stores above have taken what they read
   __syncwarp();

@@ -49,6 +49,14 @@ def build_opwait(verbose: bool = False) -> str:
                                ["-O3", "--use_fast_math"], verbose)
 
 
+def build_gemmwait(verbose: bool = False) -> str:
+    """The GEMM with K split over a cluster, with a short wait limit (csrc/tests/gemm_wait_limits.cu),
+    loaded by tests/test_gpu_op_wait_limits.py."""
+    kernels = os.path.join(ROOT, "csrc", "kernels")
+    deps = [os.path.join(kernels, f) for f in ("split_gemm.cu", "split_gemm.h", "tcgen05.cuh")]
+    return _build_test_kernels("gemm_wait_limits.cu", "libflagcx_gemmwait.so", deps, ["-O3"], verbose)
+
+
 def build_bounds(jobs: int | None = None, verbose: bool = False) -> str:
     """The kernels once more with -DFLAGCX_BOUNDS_CHECK (csrc/build/bounds/libflagcx.so): every
     kernel verifies the extent of its accesses first; tests/test_gpu_bounds_build.py runs
@@ -66,6 +74,7 @@ def build(verbose: bool = False) -> None:
     build_bounds(verbose=verbose)
     build_devtest(verbose=verbose)
     build_opwait(verbose=verbose)
+    build_gemmwait(verbose=verbose)
     try:
         from flagcx_b200.torch_backend import build as tb
     except ImportError:

@@ -1,5 +1,6 @@
-"""What the model kernels make of a copy that never comes: the wait for it runs out (20 ms in this
-build of them), the kernel ends, what depends on it is NaN and everything else is right."""
+"""What the model kernels and the GEMM that splits K make of a copy that never comes, or too late: the
+wait for it runs out (20 ms in this build of them), the kernel ends, what depends on it is NaN and
+everything else is right."""
 import ctypes
 
 import pytest
@@ -94,3 +95,46 @@ def test_cross_entropy_of_rows_dealt_out_without_one(lib, rows, V):
     assert bool(lost[held]) and not bool(lost[:held].any()) and int(lost.sum()) <= 3
     assert bool(d[lost].isnan().all())
     assert torch.equal(loss[~lost], whole[1][~lost]) and torch.equal(d[~lost], whole[0][~lost])
+
+
+@pytest.fixture(scope="module")
+def gemm():
+    from flagcx_b200.build import build_gemmwait
+    torch.cuda.init()
+    so = ctypes.CDLL(build_gemmwait())
+    so.split_gemm.argtypes = [ctypes.c_void_p] * 3 + [ctypes.c_int] * 5
+    yield so
+    so.hold_back_step(-1, -1)
+
+
+# A step of the first, a middle and the last part, which arrives when its CTA has given up: the whole
+# ring is asked for by then (parts of 2 steps, fewer than there are stages) or the producer still waits
+# for a stage (parts of 21).
+@pytest.mark.parametrize("K,parts", [(1024, 8), (512, 3), (1344, 1), (5376, 4)])
+@pytest.mark.parametrize("tile_n", [256, 128, 64])
+def test_split_gemm_of_operands_that_come_too_late(gemm, K, parts, tile_n):
+    M, N, steps = 256, 512, K // 64
+    g = torch.Generator(device="cuda").manual_seed(K)
+    a = torch.randn(M, K, generator=g, device="cuda").to(torch.bfloat16)
+    b = torch.randn(N, K, generator=g, device="cuda").to(torch.bfloat16)
+
+    def run(tile, kb):
+        assert gemm.hold_back_step(tile, kb) == 0
+        out = torch.full((M, N), 7.0, dtype=torch.bfloat16, device="cuda")
+        assert gemm.split_gemm(a.data_ptr(), b.data_ptr(), out.data_ptr(), M, N, K, parts, tile_n) == 0
+        return out
+
+    whole = run(-1, -1)
+    ref = a.double() @ b.double().T
+    # one rounding to bf16 and fp32 sums of K products
+    bound = ref.abs() * 2 ** -8 + (a.double().abs() @ b.double().abs().T) * K * 2 ** -24
+    assert bool(((whole.double() - ref).abs() <= bound).all())
+    tile = 3 if N // tile_n > 1 else 1
+    down, across = tile % (M // 128), tile // (M // 128)  # neighbours share their rows of B
+    lost = torch.zeros(M, N, dtype=torch.bool, device="cuda")
+    lost[down * 128:(down + 1) * 128, across * tile_n:(across + 1) * tile_n] = True
+    for kb in (0, steps // 2, steps - 1):
+        out = run(tile, kb)
+        assert torch.equal(out.isnan(), lost), kb
+        assert torch.equal(out[~lost], whole[~lost]), kb
+    assert torch.equal(run(-1, -1), whole)
