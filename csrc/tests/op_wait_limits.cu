@@ -1,14 +1,22 @@
 // op_wait_limits.cu -- the model kernels with a wait limit of 20 ms and a row whose copy is never
-// started, so that the waits for it run out; tests/test_gpu_op_wait_limits.py checks what the
-// kernels make of that.
+// started, so that the waits for it run out, or with answers to requests for a row that count as
+// not seen in time; tests/test_gpu_op_wait_limits.py checks what the kernels make of that.
 #define FLAGCX_OPS_WAIT_NS 20000000ull
 #define FLAGCX_OPS_HELD_BACK(row) ((long)(row) == heldBackRow)
+#define FLAGCX_OPS_UNSEEN(request) (blockIdx.x == unseen[0] && (request) == unseen[1] ? unseen[2] : 0)
 static __device__ long heldBackRow = -1;
+static __device__ unsigned unseen[3] = {0, 0, 0};
 #include "../../flagcx_b200/ops/csrc/fused_elementwise.cu"
 
 extern "C" {
 
 int hold_back(long row) { return cudaMemcpyToSymbol(heldBackRow, &row, sizeof row); }
+
+// Of the requests of the cluster that starts with CTA `block`, `waits` waits for the nth do not see its answer.
+int leave_unseen(unsigned block, unsigned nth, unsigned waits) {
+  const unsigned u[3] = {block, nth, waits};
+  return cudaMemcpyToSymbol(unseen, u, sizeof u);
+}
 
 int norm_partials(long rows, int H, int sms) { return fcxops::rmsnormPartials(rows, H, sms); }
 

@@ -59,11 +59,13 @@ __device__ __forceinline__ float blockMax(float v, float *red) {
 
 __device__ __forceinline__ uint32_t sharedAddr(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }
 
-// How long a copy may take before a kernel gives up on it, and the row that is never fetched
-// (a test of the waits that run out sets both; there is none otherwise).
+// How long a copy may take before a kernel gives up on it, the row that is never fetched, and how
+// many of the two waits for the answer to a request are taken as having run out (a test of the waits
+// that run out sets all three; there are none otherwise).
 #ifndef FLAGCX_OPS_WAIT_NS
 #define FLAGCX_OPS_WAIT_NS 1000000000ull
 #define FLAGCX_OPS_HELD_BACK(row) false
+#define FLAGCX_OPS_UNSEEN(request) 0
 #endif
 
 // Waits for a phase of an mbarrier for at most about one second.
@@ -708,15 +710,24 @@ crossEntropyRows(bf16 *__restrict__ logits, const long *__restrict__ targets, fl
   __shared__ float2 stat[2][kCeRowWarps]; // (maximum, sum) of every warp, two rows deep
   __shared__ __align__(8) uint64_t bar, dealBar;
   __shared__ __align__(16) uint4 answer[2];
-  __shared__ int dealt[2], dealOver; // of the cluster's first CTA: the row after next (-1: none); no more requests
+  // of the cluster's first CTA: the row after next (-1: none); 0, or no more requests (bit 1: an answer was not seen)
+  __shared__ int dealt[2], dealOver;
   cg::cluster_group cluster = cg::this_cluster();
   const int C = (int)cluster.num_blocks(), cr = (int)cluster.block_rank();
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const long step = gridDim.x / C;
   const bool dealer = DEAL && cr == 0 && tid == 0;
-  auto takeAnswer = [&](uint32_t nth) { // dealer: what came of the nth request
-    const int first = mbarWaitBounded(&dealBar, nth & 1u) ? clusterHandedOver(&answer[nth & 1u]) : -1;
-    return first < 0 ? -1 : first / C;
+  // Dealer: what came of the nth request.  The row that it hands over is nobody else's, so the answer
+  // is given as long again to be seen; if it is not, a row may be done by nobody, and which one is not
+  // known: the rows that this cluster has become NaN.
+  auto takeAnswer = [&](uint32_t nth) {
+    for (int wait = 0; wait < 2; ++wait)
+      if (mbarWaitBounded(&dealBar, nth & 1u) && wait >= FLAGCX_OPS_UNSEEN(nth)) {
+        const int first = clusterHandedOver(&answer[nth & 1u]);
+        return first < 0 ? -1 : first / C;
+      }
+    dealOver = 2;
+    return -1;
   };
   const int p0 = cr * packsPerCta, n = max(0, min(packsPerCta, V / 8 - p0));
   const uint32_t bytes = (uint32_t)n * 16u;
@@ -787,7 +798,10 @@ crossEntropyRows(bf16 *__restrict__ logits, const long *__restrict__ targets, fl
       }
     sum = warpSum(ok ? sum : NAN);
     if (lane == 0) stat[it & 1][warp] = make_float2(wmax, sum);
-    if (dealer) dealt[it & 1] = next >= 0 && !dealOver ? takeAnswer(it + 1) : -1;
+    if (dealer) {
+      dealt[it & 1] = next >= 0 && !dealOver ? takeAnswer(it + 1) : -1;
+      if (dealOver & 2) stat[it & 1][0].y = NAN;
+    }
     __syncwarp();
     // One barrier per row: the pairs of the row before last are overwritten only now, when
     // every CTA has passed the last row's barrier and so has read them.
@@ -809,7 +823,7 @@ crossEntropyRows(bf16 *__restrict__ logits, const long *__restrict__ targets, fl
     S = warpSum(S);
     // A cluster that has lost a copy takes no further row (nor one that has met a NaN, which its
     // sums do not tell apart): rows that nobody takes over start clusters of their own.
-    if (dealer && S != S) dealOver = 1;
+    if (dealer && S != S) dealOver |= 1;
     if (own && tid == 0) loss[row] = M + __logf(S) - tgtLogit;
     const float f = __expf(wmax - M) / S * gradScale;
     uint4 *out = (uint4 *)part(row);

@@ -20,6 +20,7 @@ def lib():
     so.cross_entropy.argtypes = [ctypes.c_void_p] * 3 + [ctypes.c_long, ctypes.c_int, ctypes.c_float, ctypes.c_int]
     yield so
     so.hold_back(-1)
+    so.leave_unseen(0, 0, 0)
 
 
 def _norm_backward(lib, t, rows, H, skip, held):
@@ -95,6 +96,31 @@ def test_cross_entropy_of_rows_dealt_out_without_one(lib, rows, V):
     assert bool(lost[held]) and not bool(lost[:held].any()) and int(lost.sum()) <= 3
     assert bool(d[lost].isnan().all())
     assert torch.equal(loss[~lost], whole[1][~lost]) and torch.equal(d[~lost], whole[0][~lost])
+
+
+# The answer to a cluster's first request, or a later one, is not seen in time.  Seen while the cluster
+# waits once more, the row that it hands over is done like any other; not seen at all, that row is left
+# as it was, and the cluster's own rows tell.
+@pytest.mark.parametrize("rows,V,ctas", [(8000, 8192, 1), (1000, 128256, 3)])
+@pytest.mark.parametrize("nth", [0, 1, 2])
+def test_cross_entropy_of_rows_dealt_out_without_an_answer(lib, rows, V, ctas, nth):
+    g = torch.Generator(device="cuda").manual_seed(V)
+    logits = torch.randn(rows, V, generator=g, device="cuda").to(torch.bfloat16)
+    targets = torch.randint(0, V, (rows,), generator=g, device="cuda")
+    whole = _cross_entropy(lib, logits, targets, -1)
+    try:
+        assert lib.leave_unseen(5 * ctas, nth, 1) == 0
+        late = _cross_entropy(lib, logits, targets, -1)
+        assert all(torch.equal(a, b) for a, b in zip(late, whole))
+        assert lib.leave_unseen(5 * ctas, nth, 2) == 0
+        d, loss = _cross_entropy(lib, logits, targets, -1)
+    finally:
+        lib.leave_unseen(0, 0, 0)
+    lost, undone = loss.isnan(), loss == 7.0
+    assert 1 <= int(lost.sum()) <= 2 and bool(d[lost].isnan().all())
+    assert int(undone.sum()) == 1 and torch.equal(d[undone], logits[undone])
+    rest = ~(lost | undone)
+    assert torch.equal(loss[rest], whole[1][rest]) and torch.equal(d[rest], whole[0][rest])
 
 
 @pytest.fixture(scope="module")
