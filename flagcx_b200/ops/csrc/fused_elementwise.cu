@@ -752,6 +752,7 @@ crossEntropyRows(bf16 *__restrict__ logits, const long *__restrict__ targets, fl
       askForCluster(&answer[0], &dealBar);
       dealt[1] = takeAnswer(0);
     }
+    __syncwarp(); // the cluster barrier wants whole warps, and the dealer's lane has been away
     if (C > 1) clusterSyncAll(); else __syncthreads();
     next = *cluster.map_shared_rank(&dealt[1], 0);
   } else {
