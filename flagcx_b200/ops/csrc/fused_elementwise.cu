@@ -650,9 +650,10 @@ __global__ void crossEntropyFwdBwd(bf16 *__restrict__ logits, const long *__rest
 // Bound: HBM (one read and one write of the logits).  The kernel below it in this file, which
 // loads, reduces and stores one row per CTA with nothing overlapped, took 458 us for
 // 4096 x 128256; this one takes 331 (6.3 TB/s, 0.97 of a copy).  The CTAs of a cluster wait for one
-// another at every row, so a row goes to as few as can hold it: with up to 21 packs per thread (128
-// registers, two CTAs per SM) 3 instead of 4 here, 349 -> 331; 2048 x 151936 in 4 instead of 8 261 ->
-// 214; with 5, 6 and 7 CTAs 376, 400 and 445.  Dealt against equal shares: 4096 x 32000 93.4 -> 85.2,
+// another at every row, so a row goes to as few as can hold it: with up to 21 packs per thread (two
+// CTAs per SM, and all of their 128 registers: 12 bytes spilled made it 449) 3 instead of 4 here,
+// 349 -> 331; 2048 x 151936 in 4 instead of 8 261 -> 214; with 5, 6 and 7 CTAs 376, 400 and 445.  Dealt
+// against equal shares: 4096 x 32000 93.4 -> 85.2,
 // 8192 x 8192 46.6 -> 45.5, 16384 x 1024 45.2 -> 47.0: from four packs per thread on.
 // ---------------------------------------------------------------------------
 constexpr int kCeRowThreads = 256, kCeRowWarps = kCeRowThreads / 32;
@@ -752,8 +753,12 @@ crossEntropyRows(bf16 *__restrict__ logits, const long *__restrict__ targets, fl
       askForCluster(&answer[0], &dealBar);
       dealt[1] = takeAnswer(0);
     }
-    __syncwarp(); // the cluster barrier wants whole warps, and the dealer's lane has been away
-    if (C > 1) clusterSyncAll(); else __syncthreads();
+    if (C > 1) {
+      __syncwarp(); // the cluster barrier wants whole warps, and the dealer's lane has been away
+      clusterSyncAll();
+    } else {
+      __syncthreads();
+    }
     next = *cluster.map_shared_rank(&dealt[1], 0);
   } else {
     __syncthreads();
