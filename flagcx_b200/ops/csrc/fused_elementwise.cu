@@ -450,14 +450,15 @@ rmsnormBwdRing(const bf16 *__restrict__ g, const bf16 *__restrict__ x, const bf1
 }
 
 // dw[c] = sum over the CTAs' partials, in a fixed order, rounded to bf16 once.
-// Block (32, 32): 32 neighbouring columns, 32 lanes over the rows.
-__global__ void columnSumToBf16(const float *__restrict__ partial, bf16 *__restrict__ dw, int R, int H) {
+// Block (32, 32): 32 neighbouring columns, 32 lanes over the rows.  The partials may still be in
+// writing when this kernel starts, so they are read through L2, never as read-only data.
+__global__ void columnSumToBf16(const float *partial, bf16 *__restrict__ dw, int R, int H) {
   __shared__ float tile[32][33];
   const int c = blockIdx.x * 32 + threadIdx.x;
   waitForEarlierGrid();
   float acc = 0.f;
   if (c < H)
-    for (int r = threadIdx.y; r < R; r += 32) acc += partial[(size_t)r * H + c];
+    for (int r = threadIdx.y; r < R; r += 32) acc += __ldcg(partial + (size_t)r * H + c);
   tile[threadIdx.y][threadIdx.x] = acc;
   __syncthreads();
   if (threadIdx.y == 0 && c < H) {
