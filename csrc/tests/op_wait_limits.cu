@@ -18,6 +18,11 @@ int leave_unseen(unsigned block, unsigned nth, unsigned waits) {
   return cudaMemcpyToSymbol(unseen, u, sizeof u);
 }
 
+int norm_forward(const void *x, const void *w, void *y, float *rstd, long rows, int H) {
+  const cudaError_t e = fcxops::rmsnormForward(x, w, y, rstd, rows, H, 1e-5f, nullptr);
+  return e != cudaSuccess ? e : cudaDeviceSynchronize();
+}
+
 int norm_partials(long rows, int H, int sms) { return fcxops::rmsnormPartials(rows, H, sms); }
 
 int norm_backward(const void *g, const void *x, const void *w, const float *rstd, const void *add, void *dx, void *dw,

@@ -1045,9 +1045,9 @@ cudaError_t allowShared(int bytes) {
 }
 
 // Calls f(GT, PPT) for rows of `packs` packs of 8: the smallest group whose threads hold a row
-// with at most four packs each (512 threads and four packs: 16384 elements), so three or four in
-// every group but the smallest.
-template <typename F>
+// with at most four packs each, so three or four in every group but the smallest.  MOST is the largest
+// group there is to be (512 threads and four packs: 16384 elements); a row that it cannot hold is refused.
+template <int MOST, typename F>
 cudaError_t withNormShape(int packs, F &&f) {
   auto ppt = [&](auto gt) -> cudaError_t {
     constexpr int GT = decltype(gt)::value;
@@ -1063,7 +1063,9 @@ cudaError_t withNormShape(int packs, F &&f) {
   if (packs <= 64 * kNormPacks) return ppt(std::integral_constant<int, 64>());
   if (packs <= 128 * kNormPacks) return ppt(std::integral_constant<int, 128>());
   if (packs <= 256 * kNormPacks) return ppt(std::integral_constant<int, 256>());
-  return ppt(std::integral_constant<int, 512>());
+  if constexpr (MOST == 512)
+    if (packs <= 512 * kNormPacks) return ppt(std::integral_constant<int, 512>());
+  return cudaErrorInvalidValue;
 }
 
 template <int PPT, bool DEAL>
@@ -1109,19 +1111,19 @@ cudaError_t rmsnormForward(const void *x, const void *w, void *y, float *rstd, l
                            cudaStream_t stream) {
   auto launch = [&](auto gt, auto ppt) {
     constexpr int GT = decltype(gt)::value, PPT = decltype(ppt)::value, G = kNormFwdThreads<GT> / GT;
-    if constexpr (GT <= 256) // rows beyond 8192 elements take the line after the lambda
-      rmsnormFwd<GT, PPT><<<(unsigned)((rows + G - 1) / G), kNormFwdThreads<GT>, 0, stream>>>(
-          (const bf16 *)x, (const bf16 *)w, (bf16 *)y, rstd, rows, H, eps);
+    rmsnormFwd<GT, PPT><<<(unsigned)((rows + G - 1) / G), kNormFwdThreads<GT>, 0, stream>>>(
+        (const bf16 *)x, (const bf16 *)w, (bf16 *)y, rstd, rows, H, eps);
     return cudaGetLastError();
   };
-  if (H / 8 > 256 * 4) return launch(std::integral_constant<int, 256>(), std::integral_constant<int, 8>());
-  return withNormShape(H / 8, launch);
+  const int packs = H / 8;
+  if (packs > 256 * kNormPacks && packs <= 256 * 8) return launch(std::integral_constant<int, 256>(), std::integral_constant<int, 8>());
+  return withNormShape<256>(packs, launch);
 }
 
 int rmsnormPartials(long rows, int H, int sms) {
   if (rmsnormRowPerCta(rows, H, sms)) return (int)std::max<long>(1, std::min<long>(rows, sms * 2));
   int ctas = 0;
-  withNormShape(H / 8, [&](auto gt, auto) {
+  withNormShape<512>(H / 8, [&](auto gt, auto) {
     constexpr int G = kNormThreads / decltype(gt)::value;
     ctas = (int)std::max<long>(1, std::min<long>((rows + G - 1) / G, sms));
     return cudaSuccess;
@@ -1145,7 +1147,7 @@ cudaError_t rmsnormBackward(const void *g, const void *x, const void *w, const f
     if (H / 8 <= kNormBwdThreads) RETURN_IF(launch(std::integral_constant<int, 1>()));
     else RETURN_IF(launch(std::integral_constant<int, 2>()));
   } else {
-    RETURN_IF(withNormShape(H / 8, [&](auto gt, auto ppt) {
+    RETURN_IF(withNormShape<512>(H / 8, [&](auto gt, auto ppt) {
       constexpr int GT = decltype(gt)::value, PPT = decltype(ppt)::value, G = kNormThreads / GT;
       // slots of all groups, two for each at least: one CTA per SM
       const size_t slots = (size_t)H * (add ? 6 : 4) * G;

@@ -15,12 +15,24 @@ def lib():
     torch.cuda.init()
     so = ctypes.CDLL(build_opwait())
     so.hold_back.argtypes = [ctypes.c_long]
+    so.norm_forward.argtypes = [ctypes.c_void_p] * 4 + [ctypes.c_long, ctypes.c_int]
     so.norm_partials.argtypes = [ctypes.c_long, ctypes.c_int, ctypes.c_int]
     so.norm_backward.argtypes = [ctypes.c_void_p] * 8 + [ctypes.c_long, ctypes.c_int, ctypes.c_int]
     so.cross_entropy.argtypes = [ctypes.c_void_p] * 3 + [ctypes.c_long, ctypes.c_int, ctypes.c_float, ctypes.c_int]
     yield so
     so.hold_back(-1)
     so.leave_unseen(0, 0, 0)
+
+
+# the longest rows of every group of threads, and rows that no kernel holds
+@pytest.mark.parametrize("H,held", [(1024, 1), (2048, 1), (4096, 1), (8192, 1), (8200, 1), (16384, 1), (16392, 0), (32768, 0)])
+def test_norm_forward_takes_rows_that_a_kernel_holds_and_no_others(lib, H, held):
+    g = torch.Generator(device="cuda").manual_seed(H)
+    x = torch.randn(5, H, generator=g, device="cuda").to(torch.bfloat16)
+    w, y, rstd = torch.ones_like(x[0]), torch.full_like(x, 7.0), torch.full((5,), 7.0, device="cuda")
+    assert (lib.norm_forward(*[t.data_ptr() for t in (x, w, y, rstd)], 5, H) == 0) == bool(held)
+    ref = x.double() * torch.rsqrt(x.double().square().mean(-1, keepdim=True) + 1e-5) if held else torch.full_like(x, 7.0).double()
+    assert bool(((y.double() - ref).abs() <= ref.abs() * 2 ** -8).all())  # one rounding to bf16, and fp32 in front of it
 
 
 def _norm_backward(lib, t, rows, H, skip, held):
