@@ -22,6 +22,7 @@ struct flagcxMoe {
   size_t grpCountOff = 0, wRowOff = 0; // byte offsets of the count table and the per-row weights inside `grp`
   // local
   int *pos = nullptr, *route = nullptr, *expertOffsets = nullptr, *lead = nullptr;
+  unsigned *tickets = nullptr; // not the communicator's: layers of a lone rank may run at the same time
   int lastTokens = 0;
   int preReduce = 0; // decided by the dispatch, for the combine that follows it
   const int *lastIdx = nullptr;
@@ -87,7 +88,7 @@ void fillArgs(flagcxMoe *m, MoeArgs &a, int nTokens) {
   a.maxT = m->maxTokens;
   a.dedup = readParam("MOE_DEDUP", 1) != 0 ? 1 : 0;
   a.preReduce = m->preReduce;
-  a.tickets = c->tickets;
+  a.tickets = m->tickets;
   a.lead = m->lead;
   a.pos = m->pos;
   a.route = m->route;
@@ -145,6 +146,8 @@ flagcxResult_t flagcxMoeCreate(flagcxComm_t comm, int maxTokens, int hidden, int
   FCX_CUDACHECK(cudaMalloc((void **)&m->route, sizeof(int) * items * 2));
   FCX_CUDACHECK(cudaMalloc((void **)&m->expertOffsets, sizeof(int) * (m->epr + 1)));
   FCX_CUDACHECK(cudaMalloc((void **)&m->lead, sizeof(int) * items));
+  FCX_CUDACHECK(cudaMalloc((void **)&m->tickets, 2 * sizeof(unsigned)));
+  FCX_CUDACHECK(cudaMemset(m->tickets, 0, 2 * sizeof(unsigned)));
   FCX_CUDACHECK(cudaMemset(m->table, 0, sizeof(int) * (size_t)comm->nranks * nExperts));
   FCX_CUDACHECK(cudaDeviceSynchronize());
   *out = m;
@@ -165,6 +168,7 @@ flagcxResult_t flagcxMoeDestroy(flagcxMoe_t m) {
   cudaFree(m->route);
   cudaFree(m->expertOffsets);
   cudaFree(m->lead);
+  cudaFree(m->tickets);
   delete m;
   return flagcxSuccess;
 }

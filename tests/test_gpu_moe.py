@@ -166,3 +166,37 @@ def test_ranks_that_post_different_operations_are_refused(first, used):
             m.close()
     finally:
         capi.Comm.emu_world_destroy(comms)
+
+
+# A lone rank has no barriers that would keep its layers apart: two of them on two streams, each with
+# its own tokens and weights, over and over.
+def test_two_layers_of_one_rank_at_the_same_time(monkeypatch):
+    monkeypatch.setenv("FLAGCX_MOE_COMBINE_REDUCE", "0")
+    comm = capi.Comm.init_rank(1, capi.get_unique_id(), 0)
+    try:
+        T, H, E, K = 700, 2048, 16, 4
+        streams = [torch.cuda.Stream() for _ in range(2)]
+        g = torch.Generator().manual_seed(5)
+        layers = []
+        for _ in streams:
+            m = MoeDispatcher(comm, T, H, K, E, T * K)
+            x = torch.randn(T, H, generator=g).to(torch.bfloat16).cuda()
+            idx, w = route(torch.randn(T, E, generator=g).cuda(), K)
+            layers.append((m, x, idx, w, torch.empty(20, T, H, dtype=torch.bfloat16, device="cuda")))
+        for (m, x, idx, w, outs), s in zip(layers, streams):
+            m.dispatch(x, idx)
+            m.expert_out.copy_(m.recv_rows)
+        torch.cuda.synchronize()
+        for i in range(20):
+            for (m, x, idx, w, outs), s in zip(layers, streams):
+                m.combine(w, outs[i], stream=s)
+        torch.cuda.synchronize()
+        assert comm.async_error() == 0, comm.last_error()
+        for m, x, idx, w, outs in layers:
+            ref = x.float() * w.sum(1, keepdim=True)
+            # fp32 sums of K products, rounded to bf16 once
+            assert bool(((outs.float() - ref).abs() <= ref.abs() * 2 ** -8 + x.float().abs() * K * 2 ** -23).all())
+            assert bool((outs == outs[0]).all())
+            m.close()
+    finally:
+        comm.destroy()
