@@ -30,8 +30,9 @@ inline double splitUs(const SplitGemmKind &k, int parts, long tiles, int kb, dou
 // 128 x 256 x 256 to 2048 x 6144 x 8192, every kind and size that the shape allows: the smallest
 // estimate takes 1.002 of the quickest on average, 1.08 at worst (256 x 2816 x 3072).  Beyond 32
 // tiles the persistent kernel keeps what it had when a split cost 2 us more: two parts or more, and
-// 1.7 us to be gained (given away: 1664 x 768 x 1024 9.6 against 10.6, 128 x 9728 x 1280 11.3 against
-// 13.3).
+// 1.7 us to be gained (given away: 3456 x 512 x 1472 12.0 against 12.6, 2432 x 512 x 1152 10.5 against
+// 10.9, 1664 x 768 x 1024 10.1 against 10.3; with the pairs that this takes now the persistent kernel has
+// caught up at 128 x 9728 x 1280, 12.8 against 12.7).
 // pair: that the number of 128-row blocks is even.  The persistent kernel may yet take pairs for an odd
 // one (pairsQuicker); its estimate here stays that of single CTAs, with which the split was right on
 // all of 30 shapes where the estimate for pairs would have left it (3 to 22 % quicker: 1152 x 2048 x 2816
@@ -70,14 +71,15 @@ inline SplitGemmPlan splitPlan(int M, int N, int K, bool pair, int forced = 0, i
 
 // The tiles of the persistent kernel's last wave, where handing them to the split kernel (parts
 // CTAs per tile) is quicker than a wave of whole tiles in which most SMs are idle: 8192 x 3584
-// x 8192 is 6 waves of 74 CTA pairs and 4 tiles, 336 -> 322 us.  A wave costs 0.363 us per K step, of
+// x 8192 is 6 waves of 74 CTA pairs and 4 tiles, 327 -> 314 us in short runs (under the power limit of a
+// long one 370 to 380, and the difference within what the clock moves).  A wave costs 0.363 us per K step, of
 // pairs 0.33 (several waves: the clock is lower than in splitPlan's single one); the split kernel
 // the larger of its K steps and its operands out of L2, and 14.5 us for the exchange and the second
-// launch.  Measured on 90 shapes, none lost (6400 x 768 x 8896 142 -> 92, 1792 x 3072 x 7424 74 -> 62).
-// Since the second launch starts while the first kernel ends it costs less; with 10.5 us 768 x 8448 x 6336
-// would gain (88 -> 76), 6400 x 4096 x 7040 and 5504 x 3584 x 2880 nothing.  The gain falls with the
-// number of full waves (on average 17 % after one, 11 after two, 3 after six, 1 after eight); beyond
-// nine it is within the noise.
+// launch.  Measured on 90 shapes, none lost (6400 x 768 x 8896 90 -> 68, 1792 x 3072 x 7424 75 -> 63).
+// Since the second launch starts while the first kernel ends it costs less: with 10.5 us 1024 x 4864 x
+// 3072 would take 32.7 instead of 35.2 us, 768 x 8448 x 6336 65.3 instead of 67.5, 6400 x 4096 x 7040 246
+// instead of 249, 5504 x 3584 x 2880 the same.  The gain falls with the number of full waves (on average
+// 17 % after one, 11 after two, 3 after six, 1 after eight); beyond nine it is within the noise.
 inline SplitGemmTail tailPlan(int M, int N, int K, bool pair, int units, int groupRows, SplitGemmPlan *plan) {
   SplitGemmTail t;
   const int kb = K / 64, tiles = (M / (pair ? 256 : 128)) * (N / 256), rest = tiles % units;

@@ -112,7 +112,8 @@ __device__ __forceinline__ void ctaShare(size_t n, int b, int g, size_t *begin, 
 // 8 x 32 MiB on one GPU: 105 us with shares, 89 with tickets).  Where what a CTA touches is not
 // tied to what the same CTA of a peer has staged, warps draw numbered items of their rank's work
 // instead.  words[0] is the next number, words[1] counts CTAs that are through; the last of them
-// sets both back to zero for the rank's next launch (launches of a rank follow one another).
+// sets both back to zero for the next launch with these words (such launches follow one another: a
+// rank's collectives, or the combines of one expert-parallel layer).
 struct Tickets {
   unsigned *words;
   __device__ __forceinline__ unsigned take() const { // the whole warp gets one number

@@ -9,11 +9,13 @@ pytestmark = pytest.mark.gpu
 
 @pytest.mark.parametrize("M,N,K", [(128, 256, 64), (128, 256, 256), (256, 512, 128), (1024, 3584, 1024),
                                    (2048, 1024, 8192)])
-@pytest.mark.parametrize("pair", [1, 0])
+@pytest.mark.parametrize("pair", [2, 1, 0])
 def test_tcgen05_gemm_matches_fp32_reference(M, N, K, pair, monkeypatch):
-    """pair=1: CTA pairs (cta_group::2, 256-row tiles) where M allows; pair=0: single CTAs."""
+    """pair=2: the persistent kernel with CTA pairs (cta_group::2, 256-row tiles); 0: with single CTAs;
+    1: whatever the size picks, the split kernel among it."""
     from flagcx_b200.parallel.tp import gemm_bf16
     monkeypatch.setenv("FLAGCX_GEMM_PAIR", str(pair))
+    monkeypatch.setenv("FLAGCX_GEMM_SPLIT", "0" if pair == 1 else "1")
     g = torch.Generator(device="cuda").manual_seed(M + N + K)
     a = (torch.randn(M, K, generator=g, device="cuda") * 0.5).to(torch.bfloat16)
     b = (torch.randn(N, K, generator=g, device="cuda") * 0.5).to(torch.bfloat16)
@@ -52,9 +54,11 @@ def test_gemm_with_k_split_over_a_cluster(M, N, K, parts, tile_n, monkeypatch):
 
 # full waves by the persistent kernel, the rest of the tiles by the split one: CTA pairs, single
 # CTAs, and row blocks that do not fill the tile order's last group
-@pytest.mark.parametrize("M,N,K", [(2048, 2816, 8192), (1408, 3584, 4096), (2816, 1792, 4096)])
-def test_gemm_whose_last_wave_is_nearly_empty(M, N, K):
+@pytest.mark.parametrize("M,N,K,pair", [(2048, 2816, 8192, 1), (1408, 3584, 4096, 1), (2816, 1792, 4096, 1),
+                                        (1408, 3584, 4096, 0), (2816, 1792, 4096, 0)])
+def test_gemm_whose_last_wave_is_nearly_empty(M, N, K, pair, monkeypatch):
     from flagcx_b200.parallel.tp import gemm_bf16
+    monkeypatch.setenv("FLAGCX_GEMM_PAIR", str(pair))
     g = torch.Generator(device="cuda").manual_seed(M + N + K)
     a = torch.randn(M, K, generator=g, device="cuda").to(torch.bfloat16)
     b = torch.randn(N, K, generator=g, device="cuda").to(torch.bfloat16)
