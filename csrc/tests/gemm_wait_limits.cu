@@ -10,6 +10,7 @@
     mbarWait(&s.full[j % STAGES], (uint32_t)(j / STAGES) & 1u, &never, kWaitLimitNs);                       \
   }
 static __device__ int heldBack[2] = {-1, -1};
+#define fcx fcx_gemmwait // in a process that has the library, whose functions would be taken for these
 #include "../kernels/split_gemm.cu"
 
 namespace {
